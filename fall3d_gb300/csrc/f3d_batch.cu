@@ -49,6 +49,7 @@ struct Scen {
   int log_cap = 0, nlog = 0;
   int bstep = 0, iiter0 = 0;
   float *c_a = nullptr, *c_b = nullptr;  // the context's buffers when it joined
+  CMaps m_a{}, m_b{};                    // and their tensor maps
   int state = 0;                         // 0 free, 1 running, 2 done, 3 failed
   int status = 0;
   std::string error;
@@ -58,7 +59,6 @@ struct Scen {
 
 struct f3d_batch {
   cudaStream_t stream = nullptr;
-  BatchFork fork;  // second stream of the odd-nx part of the step kernel
   int cap = 0;
   std::vector<Scen> slot;
   std::vector<int> active;  // running slots in batch order
@@ -69,8 +69,8 @@ struct f3d_batch {
   // pinned staging of the tables
   BatchAux* h_aux = nullptr;
   FusedArgs* h_args = nullptr;
-  F2Maps* h_maps = nullptr;  // the scenarios' tensor maps (shape 3), batch order
-  F2Maps* d_maps = nullptr;
+  BatchMaps* h_maps = nullptr;  // the scenarios' tensor maps, batch order
+  BatchMaps* d_maps = nullptr;
   int *h_item_off = nullptr, *h_bstep = nullptr, *h_iiter0 = nullptr;
   // graph of one step
   cudaGraphExec_t exec = nullptr;
@@ -78,7 +78,6 @@ struct f3d_batch {
   bool tables_dirty = true, graph_dirty = true;
   int use_graph = 1;
   int shape = 0, grid = 0, max_nz = 0, max_nc = 0, max_nsou = 0;
-  int split = 0, total = 0;  // items of the even-nx scenarios come first (shape 3)
   int graph_kernels = 0;     // kernels in one replay of the graph
   long long batch_steps = 0;
   double cell_class_steps = 0.0;
@@ -89,12 +88,7 @@ namespace {
 int table_rebuild(f3d_batch* b) {
   const int n = (int)b->active.size();
   BK(cudaStreamSynchronize(b->stream));  // the previous step no longer reads the tables
-  // batch order: scenarios with an even nx first (the shape-3 kernel runs
-  // them and the others in two launches)
-  std::stable_partition(b->active.begin(), b->active.end(),
-                        [&](int id) { return (b->slot[id].x->g.nx & 1) == 0; });
   int off = 0;
-  b->split = -1;
   b->max_nz = 0;
   b->max_nc = 0;
   const int nsou_blocks = (b->max_nsou + 127) / 128;
@@ -102,11 +96,13 @@ int table_rebuild(f3d_batch* b) {
   for (int q = 0; q < n; ++q) {
     Scen& s = b->slot[b->active[q]];
     f3d_ctx* x = s.x;
-    FusedArgs a = ctx_fused_args(x);
+    FusedArgs a = ctx_fused_args(x, b->shape);
     a.c_in = s.c_a;
     a.c_out = s.c_b;
     b->h_args[q] = a;
-    b->h_maps[q] = x->maps2;
+    b->h_maps[q].met = x->maps2;
+    b->h_maps[q].a = s.m_a;
+    b->h_maps[q].b = s.m_b;
     BatchAux& u = b->h_aux[q];
     u = BatchAux{};
     u.c_a = s.c_a;
@@ -131,9 +127,8 @@ int table_rebuild(f3d_batch* b) {
     u.vz = x->vz;
     u.vset = x->vset;
     u.outmass = ctx_outmass(x);
-    if (b->split < 0 && (x->g.nx & 1)) b->split = off;
     b->h_item_off[q] = off;
-    off += fused_tiles(x->g.nx, x->g.ny, b->shape) * x->g.nc;
+    off += fused_tiles(x->g.nx, x->g.ny, b->shape) * x->g.nc * a.nchunk;
     b->h_bstep[q] = s.bstep;
     b->h_iiter0[q] = s.iiter0;
     b->max_nz = std::max(b->max_nz, x->g.nz);
@@ -142,12 +137,10 @@ int table_rebuild(f3d_batch* b) {
   }
   if ((b->max_nsou + 127) / 128 != nsou_blocks) b->graph_dirty = true;  // setsrc's grid changed
   b->h_item_off[n] = off;
-  b->total = off;
-  if (b->split < 0) b->split = off;
   if (n > 0) {
     if (upload_batch_args(b->h_args, n, b->stream)) return ctx_error(F3D_ERR_CUDA, "constant table upload failed");
     BK(cudaMemcpyAsync(b->d_aux, b->h_aux, sizeof(BatchAux) * n, cudaMemcpyHostToDevice, b->stream));
-    BK(cudaMemcpyAsync(b->d_maps, b->h_maps, sizeof(F2Maps) * n, cudaMemcpyHostToDevice, b->stream));
+    BK(cudaMemcpyAsync(b->d_maps, b->h_maps, sizeof(BatchMaps) * n, cudaMemcpyHostToDevice, b->stream));
     BK(cudaMemcpyAsync(b->d_bstep, b->h_bstep, sizeof(int) * n, cudaMemcpyHostToDevice, b->stream));
     BK(cudaMemcpyAsync(b->d_iiter0, b->h_iiter0, sizeof(int) * n, cudaMemcpyHostToDevice, b->stream));
   }
@@ -160,10 +153,10 @@ int table_rebuild(f3d_batch* b) {
 // the kernels of one batch step, in stream order
 int enqueue_step(f3d_batch* b, int commit_only_fused) {
   const int n = (int)b->active.size();
-  BK(cudaMemsetAsync(b->d_counter, 0, 2 * sizeof(int), b->stream));
+  BK(cudaMemsetAsync(b->d_counter, 0, sizeof(int), b->stream));
   if (!commit_only_fused) launch_setsrc_batch(b->d_aux, b->d_bstep, n, b->max_nc, b->max_nsou, b->stream);
-  launch_step_fused_batch(b->shape, b->grid, b->d_item_off, n, b->split, b->total, b->d_counter, b->d_bstep,
-                          b->d_iiter0, commit_only_fused ? 0 : 1, b->max_nz, b->d_maps, b->stream, &b->fork);
+  launch_step_fused_batch(b->shape, b->grid, b->d_item_off, n, b->d_counter, b->d_bstep, b->d_iiter0,
+                          commit_only_fused ? 0 : 1, b->max_nz, b->d_maps, b->stream);
   if (!commit_only_fused) {
     launch_cmass2d_batch(b->d_aux, b->d_bstep, n, b->d_red, b->stream);
     launch_batch_advance(b->d_bstep, n, b->stream);
@@ -221,19 +214,16 @@ int f3d_batch_create(int max_scenarios, f3d_batch** out) {
   const int n = max_scenarios;
   bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaStreamCreateWithFlags(&b->fork.s2, cudaStreamNonBlocking) == cudaSuccess;
-  ok = ok && cudaEventCreateWithFlags(&b->fork.a, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaEventCreateWithFlags(&b->fork.b, cudaEventDisableTiming) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_aux, sizeof(BatchAux) * n) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_item_off, sizeof(int) * (n + 1)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_bstep, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_iiter0, sizeof(int) * n) == cudaSuccess;
-  ok = ok && cudaMalloc(&b->d_counter, 2 * sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&b->d_counter, sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_red, cmass2d_batch_scratch_bytes(n)) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_aux, sizeof(BatchAux) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_args, sizeof(FusedArgs) * n) == cudaSuccess;
-  ok = ok && cudaMallocHost(&b->h_maps, sizeof(F2Maps) * n) == cudaSuccess;
-  ok = ok && cudaMalloc(&b->d_maps, sizeof(F2Maps) * n) == cudaSuccess;
+  ok = ok && cudaMallocHost(&b->h_maps, sizeof(BatchMaps) * n) == cudaSuccess;
+  ok = ok && cudaMalloc(&b->d_maps, sizeof(BatchMaps) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_item_off, sizeof(int) * (n + 1)) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_bstep, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_iiter0, sizeof(int) * n) == cudaSuccess;
@@ -263,11 +253,7 @@ int f3d_batch_destroy(f3d_batch* b) {
   cudaFreeHost(b->h_item_off);
   cudaFreeHost(b->h_bstep);
   cudaFreeHost(b->h_iiter0);
-  if (b->fork.s2) cudaStreamSynchronize(b->fork.s2);
   if (b->ev) cudaEventDestroy(b->ev);
-  if (b->fork.a) cudaEventDestroy(b->fork.a);
-  if (b->fork.b) cudaEventDestroy(b->fork.b);
-  if (b->fork.s2) cudaStreamDestroy(b->fork.s2);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return F3D_OK;
@@ -310,6 +296,8 @@ int f3d_batch_add(f3d_batch* b, f3d_ctx* x, const f3d_met_series* met, const f3d
   s.iiter0 = 0;
   s.c_a = x->c32;
   s.c_b = x->c32b;
+  s.m_a = x->cmap;
+  s.m_b = x->cmapb;
   s.state = 1;
   b->active.push_back(id);
   b->tables_dirty = b->graph_dirty = true;
@@ -371,6 +359,7 @@ int f3d_batch_step(f3d_batch* b, int* n_running) {
     ++s.bstep;
     ++s.steps;
     std::swap(x->c32, x->c32b);
+    std::swap(x->cmap, x->cmapb);
     if (x->iiter == 1 || std::fmod(x->time, 600.0) <= x->dt) {  // endstep.f90:51
       if (s.log && s.nlog < s.log_cap) {
         if (!synced) {

@@ -312,16 +312,26 @@ void launch_setdivu(Dims d, double dX1, double dX2, const double* dz, const doub
 }
 
 // reamet.f90:146 (PRATE mm/s -> mm/h when wet deposition is on) and
-// reamet.f90:153 (vz(:,:,1) = 0).
-__global__ void k_reamet_fix(Dims d, int wetdep, double* vz, double* prate) {
+// reamet.f90:153 (vz(:,:,1) = 0); with wet deposition also the highest level
+// it reaches at any column, max over zi of the levels with zlayer <= zi
+// (wetdep.f90:37), for the step kernel's column pieces.
+__global__ void k_reamet_fix(Dims d, int wetdep, double* vz, double* prate, const double* zi, const double* zlayer,
+                             int* nwet) {
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= d.plane()) return;
   vz[p] = 0.0;
-  if (wetdep) prate[p] = prate[p] * 3600.0;
+  if (!wetdep) return;
+  prate[p] = prate[p] * 3600.0;
+  const double z = zi[p];
+  int top = 0;
+  for (int k = 1; k <= d.nz; ++k)
+    if (zlayer[k - 1] <= z) top = k;
+  if (top > 0) atomicMax(nwet, top);
 }
 
-void launch_reamet_fix(Dims d, int wetdep, double* vz, double* prate, cudaStream_t s) {
-  k_reamet_fix<<<(unsigned)((d.plane() + 255) / 256), 256, 0, s>>>(d, wetdep, vz, prate);
+void launch_reamet_fix(Dims d, int wetdep, double* vz, double* prate, const double* zi, const double* zlayer,
+                       int* nwet, cudaStream_t s) {
+  k_reamet_fix<<<(unsigned)((d.plane() + 255) / 256), 256, 0, s>>>(d, wetdep, vz, prate, zi, zlayer, nwet);
   count_launch();
 }
 

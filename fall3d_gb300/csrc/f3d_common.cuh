@@ -121,18 +121,23 @@ __device__ __forceinline__ double minmod_div(double a, double b, double dx, doub
   return __longlong_as_double(__double_as_longlong(q) | (ba & (long long)0x8000000000000000ULL));
 }
 
-// Grid geometry of one scenario (interior nx, ny, nz; halo arrays are
-// (nx+2)(ny+2)(nz+2), x fastest).
+// Grid geometry of one scenario (interior nx, ny, nz; halo arrays are rows of
+// px values, (ny+2)(nz+2) rows, x fastest).  The row pitch px is nx+2, or for
+// the precision form's state nx+2 rounded up to a multiple of 4 values, so
+// that tensor copies (16-byte row strides) can stage it; the padding stays 0.
 struct Dims {
-  int nx, ny, nz;
+  int nx, ny, nz, px;
+  Dims() = default;
+  F3D_HD Dims(int nx_, int ny_, int nz_) : nx(nx_), ny(ny_), nz(nz_), px(nx_ + 2) {}
+  F3D_HD Dims(int nx_, int ny_, int nz_, int px_) : nx(nx_), ny(ny_), nz(nz_), px(px_) {}
   F3D_HD long long C(int i, int j, int k) const {
-    return (long long)i + (long long)(nx + 2) * ((long long)j + (long long)(ny + 2) * k);
+    return (long long)i + (long long)px * ((long long)j + (long long)(ny + 2) * k);
   }
   F3D_HD long long M(int i, int j, int k) const {
     return (long long)(i - 1) + (long long)nx * ((long long)(j - 1) + (long long)ny * (k - 1));
   }
   F3D_HD long long P(int i, int j) const { return (long long)(i - 1) + (long long)nx * (j - 1); }
-  F3D_HD long long halo() const { return (long long)(nx + 2) * (ny + 2) * (nz + 2); }
+  F3D_HD long long halo() const { return (long long)px * (ny + 2) * (nz + 2); }
   F3D_HD long long cells() const { return (long long)nx * ny * nz; }
   F3D_HD long long plane() const { return (long long)nx * ny; }
 };

@@ -6,7 +6,8 @@
 //   met      vx vy vz tempe vptemp rho rkhor rkh1 rkver divu: nx*ny*nz each
 //   vset     nc * nx*ny*nz, vdep nc * nx*ny          binary64
 //   2-D      ustar zi rl znt prate ldu                binary64
-//   FP32 form: binary32 copies of vx vy vz rho rkhor rkh1 rkver vset vdep dz
+//   FP32 form: binary32 copies of vx vy vz rho rkhor rkh1 rkver vset vdep dz,
+//            and the step kernel's fields (StepFields)
 //   scratch  reduction partials, setvset chain buffers, small results.
 // Everything of one step is enqueued on the context's stream without a host
 // synchronisation; the host keeps only the scalars of the time loop.
@@ -49,6 +50,9 @@ int* small_step_status(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 26
 double* small_pref_cd(f3d_ctx* x) { return x->small + 32; }
 unsigned long long* small_pref_dtcn(f3d_ctx* x) { return reinterpret_cast<unsigned long long*>(x->small + 33); }
 int* small_pref_status(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 34); }
+// the highest wet level of an update and of the look-ahead one
+int* small_nwet(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 17); }
+int* small_pref_nwet(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 35); }
 // the non-finite counts of f3d_count_nonfinite: in c, in cdry + cwet
 unsigned long long* small_nonfinite(f3d_ctx* x) { return reinterpret_cast<unsigned long long*>(x->small + 40); }
 
@@ -72,7 +76,7 @@ int dalloc(f3d_ctx* x, T** p, size_t n) {
 int met_set_alloc(f3d_ctx* x, f3d_met_set* m) {
   const Dims d = x->d;
   const size_t s3 = (size_t)d.cells(), pl = (size_t)d.plane(), nc = (size_t)x->g.nc;
-  const size_t hsz = (size_t)f3d::halo_pitch(d.nx) * (d.ny + 2) * (d.nz + 2);
+  const size_t hsz = (size_t)d.halo(), hpl = (size_t)d.px * (d.ny + 2);
   int rc = 0;
 #define A(p, n) \
   if (!rc) rc = dalloc(x, &m->p, (n))
@@ -109,18 +113,19 @@ int met_set_alloc(f3d_ctx* x, f3d_met_set* m) {
     A(rkver32, s3);
     A(vset32, s3 * nc);
     A(vdep32, pl * nc);
-    A(lrho32, s3);
-    A(pkx32, s3);
-    A(pky32, s3);
-    A(pkz32, s3);
-    A(vk32, s3 * nc);
-    A(vxh, hsz);
-    A(vyh, hsz);
-    A(lrhoh, hsz);
-    A(pkxh, hsz);
-    A(pkyh, hsz);
-    A(pkzh, hsz);
-    A(vkh, hsz * nc);
+    A(sf.ux, hsz);
+    A(sf.kx, hsz);
+    A(sf.uy, hsz);
+    A(sf.ky, hsz);
+    A(sf.l, hsz);
+    A(sf.fx, hsz);
+    A(sf.fy, hsz);
+    A(sf.fz, hsz);
+    A(sf.vk, hsz * nc);
+    A(sf.ex, 2 * (size_t)(d.nz + 2) * (d.ny + 2));
+    A(sf.ey, 2 * (size_t)(d.nz + 2) * d.px);
+    A(sf.ez, hpl);
+    A(sf.tab, (size_t)d.nz + 2);
   }
 #undef A
   return rc;
@@ -132,7 +137,9 @@ void met_set_swap(f3d_ctx* x, f3d_met_set* m) {
   F3D_MET_SET_D(F3D_X)
   F3D_MET_SET_F(F3D_X)
 #undef F3D_X
+  std::swap(x->sf, m->sf);
   std::swap(x->maps2, m->maps2);
+  std::swap(x->nwet, m->nwet);
 }
 
 }  // namespace
@@ -150,11 +157,7 @@ void refresh_fp32_class(f3d_ctx* x, int ic) {
   const size_t s3 = (size_t)d.cells();
   cudaStream_t s = x->stream;
   launch_d2f(x->vset32 + ic * s3, x->vset + ic * s3, (long long)s3, s);
-  launch_vk32((long long)s3, 1, x->vz32, x->vset32 + ic * s3, x->vk32 + ic * s3, s);
-  const float* vs = x->vk32 + ic * s3;
-  const int hp = halo_pitch(d.nx);
-  float* vd = x->vkh + (size_t)ic * (size_t)hp * (d.ny + 2) * (d.nz + 2);
-  launch_to_halo(d, hp, 1, &vs, &vd, s);
+  launch_step_vk(d, 1, x->vz, x->vset + ic * s3, x->sf.vk + (size_t)ic * d.halo(), s);
 }
 }  // namespace f3d
 
@@ -188,9 +191,11 @@ long long footprint_bytes(const f3d_grid* g) {
   b += 4LL * s3 * nc;                          // vsettl iteration counts
   b += 8LL * 3 * pl * (nc + 1);                // cdry cwet cload
   if (g->precision == F3D_PREC_FP32) {
-    b += 2 * 4LL * halo * nc;
-    b += 4LL * (11 * s3 + s3 * nc + pl * nc + nz + 1) + 8LL * pl + nc;
-    b += 4LL * (6 + nc) * f3d::halo_pitch(g->nx) * (ny + 2) * (nz + 2);  // padded halo-layout met fields
+    const long long hp = f3d::halo_pitch(g->nx), phalo = hp * (ny + 2) * (nz + 2);  // padded rows
+    b += 2 * 4LL * phalo * nc;
+    b += 4LL * (7 * s3 + s3 * nc + pl * nc + nz + 1) + 8LL * pl + nc;
+    b += 4LL * (8 + nc) * phalo;  // the step kernel's fields
+    b += 4LL * (2 * (nz + 2) * (ny + 2 + hp) + hp * (ny + 2)) + (long long)sizeof(f3d::ZTab) * (nz + 2);
   } else {
     b += 8LL * halo * nc;
     b += 8LL * 4 * s3 + 8LL * pl;  // 1/rho, rkh1*rho, rkhor*rho, diffz face coefficients; lambda
@@ -374,15 +379,13 @@ void sizloop_fused(f3d_ctx* x) {
   const Dims d = x->d;
   const int nc = x->g.nc;
   cudaStream_t s = x->stream;
-  const FusedArgs a = f3d::ctx_fused_args(x);
+  const FusedArgs a = f3d::ctx_fused_args(x, x->opt_tile);
   {
     ProfScope ps(x, "step_fused");
-    if (x->opt_tile == 3)  // the 112-register build while a look-ahead update runs beside it
-      launch_step_fused2(a, x->maps2, s, x->pref_ready && cudaEventQuery(x->ev_pref) == cudaErrorNotReady);
-    else
-      launch_step_fused(a, x->opt_tile, s);
+    launch_step_fused(a, x->maps2, x->cmap, x->opt_tile, s);
   }
   std::swap(x->c32, x->c32b);
+  std::swap(x->cmap, x->cmapb);
   {
     ProfScope ps(x, "cmass2d");
     launch_cmass2d<float>(x->c32, x->vx, x->vy, x->vz, x->vset, d, 1, nc, 1, d.nz, x->g.dX1,
@@ -393,37 +396,20 @@ void sizloop_fused(f3d_ctx* x) {
 }  // namespace
 
 namespace f3d {
-FusedArgs ctx_fused_args(f3d_ctx* x) {
+FusedArgs ctx_fused_args(f3d_ctx* x, int shape) {
   const Dims d = x->d;
-  const long long hb = d.halo(), s3 = d.cells(), pl = d.plane();
   FusedArgs a{};
   a.c_in = x->c32;
   a.c_out = x->c32b;
-  a.cstride = hb;
+  a.cstride = d.halo();
   a.d = d;
   a.ncls = x->g.nc;
   a.xfirst = (x->iiter % 2 == 0) ? 1 : 0;
-  a.dt = (float)x->dt;
   a.dt64 = x->dt;
-  a.vx = x->vx32;
-  a.vy = x->vy32;
-  a.vz = x->vz32;
-  a.vk = x->vk32;
-  a.vstride = s3;
+  a.f = x->sf;
   a.vdep = x->vdep32;
-  a.dstride = pl;
   a.rkver1 = x->rkver32;
-  a.lrho = x->lrho32;
-  a.pkx = x->pkx32;
-  a.pky = x->pky32;
-  a.pkz = x->pkz32;
-  a.dz = x->dz32;
-  a.auxvx = (float)(x->dt / x->g.dX1);
-  a.auxvy = (float)(x->dt / x->g.dX2);
-  a.inv_dx = (float)(1.0 / x->g.dX1);
-  a.inv_dy = (float)(1.0 / x->g.dX2);
-  a.dtdx2 = (float)(x->dt / (x->g.dX1 * x->g.dX1));
-  a.dtdy2 = (float)(x->dt / (x->g.dX2 * x->g.dX2));
+  a.dz0 = x->h_dz0;
   a.wet_class = x->g.wetdep ? x->wet_class : nullptr;
   a.lambda2d = x->lambda2d;
   a.zi = x->zi;
@@ -433,17 +419,8 @@ FusedArgs ctx_fused_args(f3d_ctx* x) {
   a.cdry = x->cdry;
   a.vset64 = x->vset;
   a.vdep64 = x->vdep;
-  a.vxh = x->vxh;
-  a.vyh = x->vyh;
-  a.lrhoh = x->lrhoh;
-  a.pkxh = x->pkxh;
-  a.pkyh = x->pkyh;
-  a.pkzh = x->pkzh;
-  a.vkh = x->vkh;
-  a.hpitch = halo_pitch(d.nx);
-  a.hstride = (long long)a.hpitch * (d.ny + 2) * (d.nz + 2);
   a.status = small_step_status(x);
-  a.pair_aligned = (d.nx % 2 == 0) ? 1 : 0;
+  step_chunks(a, shape, x->g.wetdep ? x->nwet : 0);
   return a;
 }
 }  // namespace f3d
@@ -463,7 +440,7 @@ namespace {
 int meteo_enqueue(f3d_ctx* x, cudaStream_t s, const double* u, const double* v, const double* w,
                   const double* t, const double* tp, const double* rho, const double* ust,
                   const double* pblh, const double* rmol, const double* znt, const double* prate,
-                  const double* ldu, double* cd_state, unsigned long long* dtcn, int* status,
+                  const double* ldu, double* cd_state, unsigned long long* dtcn, int* status, int* nwet,
                   int beside_step) {
   const Dims d = x->d;
   const size_t s3 = (size_t)d.cells(), pl = (size_t)d.plane();
@@ -483,7 +460,8 @@ int meteo_enqueue(f3d_ctx* x, cudaStream_t s, const double* u, const double* v, 
   if (!rc && x->g.wetdep) rc = upload_on(x->prate, prate, pl, s);
   if (rc) return rc;
   const f3d_grid& g = x->g;
-  launch_reamet_fix(d, g.wetdep, x->vz, x->prate, s);
+  CK(cudaMemsetAsync(nwet, 0, sizeof(int), s));
+  launch_reamet_fix(d, g.wetdep, x->vz, x->prate, x->zi, x->zlayer, nwet, s);
   // meteo.f90:27 kappa3 (unscaled vx, vy)
   launch_kappa3(d, g.modkv, g.modkh, g.coord_sys, g.rkv0, g.rkh0, g.Csh, g.dX1, g.dX2, g.dx, g.dy,
                 x->dz, x->zlayer, x->Hm1, x->vx, x->vy, x->vptemp, x->ustar, x->zi, x->rl, x->rkver,
@@ -518,20 +496,8 @@ int meteo_enqueue(f3d_ctx* x, cudaStream_t s, const double* u, const double* v, 
     launch_d2f(x->rkver32, x->rkver, (long long)s3, s);
     launch_d2f(x->vset32, x->vset, (long long)(s3 * g.nc), s);
     launch_d2f(x->vdep32, x->vdep, (long long)(pl * g.nc), s);
-    launch_fp32_coeffs((long long)s3, x->rho, x->rkh1, x->rkhor, x->rkver, x->lrho32, x->pkx32,
-                       x->pky32, x->pkz32, s);
-    launch_vk32((long long)s3, g.nc, x->vz32, x->vset32, x->vk32, s);
-    {  // halo-layout copies for the two-columns-per-lane kernel
-      const float* src[6] = {x->vx32, x->vy32, x->lrho32, x->pkx32, x->pky32, x->pkz32};
-      float* dst[6] = {x->vxh, x->vyh, x->lrhoh, x->pkxh, x->pkyh, x->pkzh};
-      const int hp = halo_pitch(d.nx);
-      launch_to_halo(d, hp, 6, src, dst, s);
-      for (int c = 0; c < g.nc; ++c) {
-        const float* vs = x->vk32 + (size_t)c * s3;
-        float* vd = x->vkh + (size_t)c * (size_t)hp * (d.ny + 2) * (d.nz + 2);
-        launch_to_halo(d, hp, 1, &vs, &vd, s);
-      }
-    }
+    launch_step_fields(d, g.nc, g.safety_factor, g.dX1, g.dX2, x->dz, dtcn, x->vx, x->vy, x->vz, x->rho, x->rkh1,
+                       x->rkhor, x->rkver, x->vset, x->sf, s);
   }
   CK(cudaGetLastError());
   return F3D_OK;
@@ -540,7 +506,8 @@ int meteo_enqueue(f3d_ctx* x, cudaStream_t s, const double* u, const double* v, 
 // What follows an update on the host: finddt.f90:58-66 from the CFL
 // maximum, the wet-scavenging rate of the new dt (wetdep.f90:31), the
 // aggregation flags (Fall3d.f90:94-96).
-int meteo_finish(f3d_ctx* x, unsigned long long dtcn_bits, int status) {
+int meteo_finish(f3d_ctx* x, unsigned long long dtcn_bits, int status, int nwet) {
+  x->nwet = nwet;
   if (status) return f3d::ctx_error(F3D_ERR_NOCONV, "No convergence in vsettl routine");
   double dtcn;
   memcpy(&dtcn, &dtcn_bits, sizeof dtcn);
@@ -567,7 +534,7 @@ int prefetch_setup(f3d_ctx* x) {
   if (int rc = met_set_alloc(x, &m)) return rc;
   if (x->prec == F3D_PREC_FP32 && x->fused_ok) {  // tensor maps of the second set's fields
     met_set_swap(x, &m);
-    const int r2 = f3d::make_fused2_maps(f3d::ctx_fused_args(x), &x->maps2);
+    const int r2 = f3d::make_step_maps(f3d::ctx_fused_args(x, 3), &x->maps2);
     met_set_swap(x, &m);
     if (r2) return f3d::ctx_error(F3D_ERR_CUDA, "cuTensorMapEncodeTiled failed for the second met set");
   }
@@ -580,7 +547,7 @@ int prefetch_setup(f3d_ctx* x) {
   CK(cudaEventCreateWithFlags(&x->ev_pref, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&x->ev_free, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&x->ev_staged, cudaEventDisableTiming));
-  CK(cudaMallocHost((void**)&x->pref_host, 2 * sizeof(unsigned long long)));
+  CK(cudaMallocHost((void**)&x->pref_host, 3 * sizeof(unsigned long long)));
   CK(cudaStreamSynchronize(x->stream));  // the zero fills of the new buffers
   x->pref_alloc = 1;
   return F3D_OK;
@@ -624,11 +591,12 @@ int prefetch_start(f3d_ctx* x, const f3d_met_series* met, int itime) {
   met_set_swap(x, &x->shadow);
   const int rc = meteo_enqueue(x, s, f3[0], f3[1], f3[2], f3[3], f3[4], f3[5], f2[0], f2[1], f2[2], f2[3],
                                src2[4] ? f2[4] : nullptr, nullptr, small_pref_cd(x), small_pref_dtcn(x),
-                               small_pref_status(x), 1);
+                               small_pref_status(x), small_pref_nwet(x), 1);
   met_set_swap(x, &x->shadow);
   if (rc) return rc;
   CK(cudaMemcpyAsync(x->pref_host, small_pref_dtcn(x), sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(x->pref_host + 1, small_pref_status(x), sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(x->pref_host + 2, small_pref_nwet(x), sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(x->ev_pref, s));
   x->pref_ready = 1;
   x->pref_itime = itime;
@@ -641,14 +609,15 @@ int prefetch_start(f3d_ctx* x, const f3d_met_series* met, int itime) {
 int prefetch_commit(f3d_ctx* x) {
   CK(cudaEventSynchronize(x->ev_pref));
   const unsigned long long bits = x->pref_host[0];
-  int status = 0;
+  int status = 0, nwet = 0;
   memcpy(&status, x->pref_host + 1, sizeof status);
+  memcpy(&nwet, x->pref_host + 2, sizeof nwet);
   CK(cudaStreamWaitEvent(x->stream, x->ev_pref, 0));
   met_set_swap(x, &x->shadow);
   x->pref_ready = 0;
   CK(cudaMemcpyAsync(small_cd_prev(x), small_cd(x), sizeof(double), cudaMemcpyDeviceToDevice, x->stream));
   CK(cudaMemcpyAsync(small_cd(x), small_pref_cd(x), sizeof(double), cudaMemcpyDeviceToDevice, x->stream));
-  return meteo_finish(x, bits, status);
+  return meteo_finish(x, bits, status, nwet);
 }
 
 }  // namespace
@@ -705,8 +674,9 @@ int f3d_ctx_create(const f3d_grid* g, f3d_ctx** out) {
   x->g = *g;
   x->g.dz = x->g.zlayer = x->g.Hm1 = x->g.topg = nullptr;
   x->g.diam = x->g.rhop = x->g.psi = x->g.sphe = nullptr;
-  x->d = Dims{g->nx, g->ny, g->nz};
   x->prec = g->precision;
+  x->d = x->prec == F3D_PREC_FP32 ? Dims{g->nx, g->ny, g->nz, f3d::halo_pitch(g->nx)} : Dims{g->nx, g->ny, g->nz};
+  x->h_dz0 = (float)g->dz[0];
   x->h_diam.assign(g->diam, g->diam + g->nc);
   x->h_rhop.assign(g->rhop, g->rhop + g->nc);
   x->h_zlayer.assign(g->zlayer, g->zlayer + g->nz);
@@ -714,8 +684,7 @@ int f3d_ctx_create(const f3d_grid* g, f3d_ctx** out) {
   for (int k = 1; k < g->nz; ++k)
     if (!(g->zlayer[k] >= g->zlayer[k - 1])) x->fused_ok = 0;
   if (x->d.halo() >= (1LL << 31) || x->d.cells() >= (1LL << 31)) x->fused_ok = 0;
-  if ((long long)f3d::halo_pitch(g->nx) * (g->ny + 2) * (g->nz + 2) >= (1LL << 31)) x->fused_ok = 0;
-  if (g->nz > f3d::fused2_max_nz()) x->fused_ok = 0;  // the shape-3 kernel's per-level table
+  if (g->nz > f3d::fused2_max_nz()) x->fused_ok = 0;  // the step kernel's per-level table
   // the highest priority: a look-ahead meteo update on the context's second
   // stream (lowest priority) runs in what the steps leave free
   int prio_least = 0, prio_greatest = 0;
@@ -804,8 +773,10 @@ int f3d_ctx_create(const f3d_grid* g, f3d_ctx** out) {
       rc = f3d::ctx_error(F3D_ERR_CUDA, "upload failed");
     launch_d2f(x->dz32, x->dz, (long long)nz + 1, x->stream);
     if (cudaStreamSynchronize(x->stream) != cudaSuccess) rc = f3d::ctx_error(F3D_ERR_CUDA, "sync failed");
-    // the tensor maps of the shape-3 step kernel: the fields stay at these addresses
-    if (!rc && x->fused_ok && f3d::make_fused2_maps(f3d::ctx_fused_args(x), &x->maps2) != 0)
+    // the tensor maps of the step kernel: the fields and state buffers stay at these addresses
+    if (!rc && x->fused_ok &&
+        (f3d::make_step_maps(f3d::ctx_fused_args(x, 3), &x->maps2) != 0 ||
+         f3d::make_c_maps(x->d, g->nc, x->c32, &x->cmap) != 0 || f3d::make_c_maps(x->d, g->nc, x->c32b, &x->cmapb) != 0))
       rc = f3d::ctx_error(F3D_ERR_CUDA, "cuTensorMapEncodeTiled failed for the step kernel's met fields");
   }
   if (rc) {
@@ -828,16 +799,17 @@ int f3d_meteo(f3d_ctx* x, const double* u, const double* v, const double* w, con
   // the chain state this update starts from (a checkpoint replays the update)
   CK(cudaMemcpyAsync(small_cd_prev(x), small_cd(x), sizeof(double), cudaMemcpyDeviceToDevice, s));
   if (int rc = meteo_enqueue(x, s, u, v, w, t, tp, rho, ust, pblh, rmol, znt, prate, ldu, small_cd(x),
-                             small_dtcn(x), small_status(x), 0))
+                             small_dtcn(x), small_status(x), small_nwet(x), 0))
     return rc;
   struct {
     unsigned long long dtcn;
-    int status;
+    int status, nwet;
   } h{};
   CK(cudaMemcpyAsync(&h.dtcn, small_dtcn(x), sizeof h.dtcn, cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(&h.status, small_status(x), sizeof h.status, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&h.nwet, small_nwet(x), sizeof h.nwet, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  return meteo_finish(x, h.dtcn, h.status);
+  return meteo_finish(x, h.dtcn, h.status, h.nwet);
 }
 
 int f3d_source(f3d_ctx* x, int nsou, const int* isrc, const int* jsrc, const int* ksrc,
@@ -1020,17 +992,19 @@ int f3d_set_time(f3d_ctx* x, double time, int iiter) {
 int f3d_download(f3d_ctx* x, double* c, double* cdry, double* cwet, double* vset, double* vdep) {
   if (!x) return f3d::ctx_error(F3D_ERR_ARG, "NULL context");
   const Dims d = x->d;
-  const size_t hb = (size_t)d.halo() * x->g.nc, pl = (size_t)d.plane(), nc = (size_t)x->g.nc;
+  // the caller's c has rows of nx+2 values; the precision form's own are padded (Dims::px)
+  const size_t rows = (size_t)(d.ny + 2) * (d.nz + 2) * x->g.nc, hb = (size_t)(d.nx + 2) * rows;
+  const size_t pl = (size_t)d.plane(), nc = (size_t)x->g.nc;
   cudaStream_t s = x->stream;
   auto kind = [](const void* p) { return is_dev(p) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost; };
   if (c) {
     if (x->prec == F3D_PREC_FP32) {
       if (is_dev(c)) {
-        launch_f2d(c, x->c32, (long long)hb, s);
+        launch_f2d_rows(c, d.nx + 2, x->c32, d.px, d.nx + 2, (long long)rows, s);
       } else {
         double* tmp = nullptr;
         CK(cudaMallocAsync((void**)&tmp, hb * sizeof(double), s));
-        launch_f2d(tmp, x->c32, (long long)hb, s);
+        launch_f2d_rows(tmp, d.nx + 2, x->c32, d.px, d.nx + 2, (long long)rows, s);
         CK(cudaMemcpyAsync(c, tmp, hb * sizeof(double), cudaMemcpyDeviceToHost, s));
         CK(cudaFreeAsync(tmp, s));
       }
@@ -1050,7 +1024,8 @@ int f3d_upload_state(f3d_ctx* x, const double* c, const double* cdry, const doub
                      double erumass, double outmass, double cd) {
   if (!x) return f3d::ctx_error(F3D_ERR_ARG, "NULL context");
   const Dims d = x->d;
-  const size_t hb = (size_t)d.halo() * x->g.nc, pl = (size_t)d.plane(), nc = (size_t)x->g.nc;
+  const size_t rows = (size_t)(d.ny + 2) * (d.nz + 2) * x->g.nc, hb = (size_t)(d.nx + 2) * rows;
+  const size_t pl = (size_t)d.plane(), nc = (size_t)x->g.nc;
   cudaStream_t s = x->stream;
   int rc = 0;
   if (c) {
@@ -1058,7 +1033,7 @@ int f3d_upload_state(f3d_ctx* x, const double* c, const double* cdry, const doub
       double* tmp = nullptr;
       CK(cudaMallocAsync((void**)&tmp, hb * sizeof(double), s));
       rc = upload(x, tmp, c, hb);
-      launch_d2f(x->c32, tmp, (long long)hb, s);
+      launch_d2f_rows(x->c32, d.px, tmp, d.nx + 2, d.nx + 2, (long long)rows, s);
       CK(cudaFreeAsync(tmp, s));
     } else {
       rc = upload(x, x->c64, c, hb);
@@ -1095,8 +1070,10 @@ const long long kCkptAggr = 0x5247474146334446LL;  // the optional aggregation s
 int f3d_ctx_save(f3d_ctx* x, const char* path) {
   if (!x || !path) return f3d::ctx_error(F3D_ERR_ARG, "NULL argument");
   const Dims d = x->d;
-  const size_t hb = (size_t)d.halo() * x->g.nc, pl2 = (size_t)d.plane() * (x->g.nc + 1);
+  const size_t rows = (size_t)(d.ny + 2) * (d.nz + 2) * x->g.nc, hb = (size_t)(d.nx + 2) * rows;
+  const size_t pl2 = (size_t)d.plane() * (x->g.nc + 1);
   const size_t esz = x->prec == F3D_PREC_FP32 ? sizeof(float) : sizeof(double);
+  const size_t wid = (size_t)(d.nx + 2) * esz;  // the file's rows hold nx+2 values
   CkptHeader h{};
   memcpy(h.magic, kCkptMagic, 8);
   h.version = 1;
@@ -1120,8 +1097,8 @@ int f3d_ctx_save(f3d_ctx* x, const char* path) {
   }
   CK(cudaMemcpyAsync(&h.outmass, small_outmass(x), sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(&h.cd_prev, small_cd_prev(x), sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(c.data(), x->prec == F3D_PREC_FP32 ? (const void*)x->c32 : (const void*)x->c64, hb * esz,
-                     cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpy2DAsync(c.data(), wid, x->prec == F3D_PREC_FP32 ? (const void*)x->c32 : (const void*)x->c64,
+                       (size_t)d.px * esz, wid, rows, cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(cdry.data(), x->cdry, pl2 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(cwet.data(), x->cwet, pl2 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -1154,8 +1131,10 @@ int f3d_ctx_restore(f3d_ctx* x, const char* path) {
     fclose(f);
     return f3d::ctx_error(F3D_ERR_ARG, "checkpoint of a different grid, class count or precision");
   }
-  const size_t hb = (size_t)d.halo() * x->g.nc, pl2 = (size_t)d.plane() * (x->g.nc + 1);
+  const size_t rows = (size_t)(d.ny + 2) * (d.nz + 2) * x->g.nc, hb = (size_t)(d.nx + 2) * rows;
+  const size_t pl2 = (size_t)d.plane() * (x->g.nc + 1);
   const size_t esz = x->prec == F3D_PREC_FP32 ? sizeof(float) : sizeof(double);
+  const size_t wid = (size_t)(d.nx + 2) * esz;
   std::vector<unsigned char> c(hb * esz);
   std::vector<double> cdry(pl2), cwet(pl2);
   ok = fread(c.data(), 1, c.size(), f) == c.size() && fread(cdry.data(), sizeof(double), pl2, f) == pl2 &&
@@ -1171,8 +1150,8 @@ int f3d_ctx_restore(f3d_ctx* x, const char* path) {
     return f3d::ctx_error(F3D_ERR_ARG, "aggregation is on in only one of the checkpoint and the context");
   f3d::ctx_prefetch_drop(x);
   cudaStream_t s = x->stream;
-  CK(cudaMemcpyAsync(x->prec == F3D_PREC_FP32 ? (void*)x->c32 : (void*)x->c64, c.data(), hb * esz,
-                     cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpy2DAsync(x->prec == F3D_PREC_FP32 ? (void*)x->c32 : (void*)x->c64, (size_t)d.px * esz, c.data(), wid,
+                       wid, rows, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(x->cdry, cdry.data(), pl2 * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(x->cwet, cwet.data(), pl2 * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(small_outmass(x), &h.outmass, sizeof(double), cudaMemcpyHostToDevice, s));

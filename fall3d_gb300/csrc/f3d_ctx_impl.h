@@ -11,7 +11,7 @@
 
 // The fields a meteo update writes and the steps read (f3d_meteo): the
 // binary64 met and coefficients, the plain form's diffusion factors, the
-// binary32 copies and the halo-layout copies of the precision form.  A
+// binary32 copies and the step kernel's fields of the precision form.  A
 // look-ahead update (F3D_OPT_PREFETCH) fills a second set of them for the
 // next DBS snapshot and the two sets are exchanged at the update.
 #define F3D_MET_SET_D(X) \
@@ -21,16 +21,16 @@
   X(double, lrho64) X(double, pkx64) X(double, pky64) X(double, rksz64)
 #define F3D_MET_SET_F(X) \
   X(float, vx32) X(float, vy32) X(float, vz32) X(float, rho32) X(float, rkhor32) X(float, rkh132) \
-  X(float, rkver32) X(float, vset32) X(float, vdep32) X(float, lrho32) X(float, pkx32) X(float, pky32) \
-  X(float, pkz32) X(float, vk32) X(float, vxh) X(float, vyh) X(float, lrhoh) X(float, pkxh) \
-  X(float, pkyh) X(float, pkzh) X(float, vkh)
+  X(float, rkver32) X(float, vset32) X(float, vdep32)
 
 struct f3d_met_set {
 #define F3D_X(T, n) T* n = nullptr;
   F3D_MET_SET_D(F3D_X)
   F3D_MET_SET_F(F3D_X)
 #undef F3D_X
+  f3d::StepFields sf{};  // the fused step kernel's fields and their tensor maps
   f3d::F2Maps maps2{};
+  int nwet = 0;  // the highest level with zlayer <= zi (wetdep.f90:37)
 };
 
 struct f3d_ctx {
@@ -45,6 +45,7 @@ struct f3d_ctx {
   std::vector<double> h_diam, h_rhop;  // host copies (output class selections)
   std::vector<double> h_zlayer;        // host copy (gravity current levels)
   double hm11 = 1.0;                   // Hm1(1,1)
+  float h_dz0 = 0.0f;                  // dz(0)
   // gravity current (f3d_set_gravity_current)
   f3d_gravity_current gc{};
   int gc_on = 0;
@@ -73,19 +74,17 @@ struct f3d_ctx {
   float *vx32 = nullptr, *vy32 = nullptr, *vz32 = nullptr, *rho32 = nullptr, *rkhor32 = nullptr,
         *rkh132 = nullptr, *rkver32 = nullptr, *vset32 = nullptr, *vdep32 = nullptr,
         *dz32 = nullptr;
-  // fused FP32 step: second concentration buffer, 1/rho, K*rho products,
-  // per-column wet rate, per-class wet-deposition switch
+  // fused FP32 step: second concentration buffer (and the two buffers' tensor
+  // maps), per-column wet rate, per-class wet-deposition switch
   float* c32b = nullptr;
-  float *lrho32 = nullptr, *pkx32 = nullptr, *pky32 = nullptr, *pkz32 = nullptr;
+  f3d::CMaps cmap{}, cmapb{};
   // plain form: 1/rho, rkh1*rho, rkhor*rho and the diffz face coefficients
   // of the current meteo update (the class-independent factors of the
   // diffusion sweeps)
   double *lrho64 = nullptr, *pkx64 = nullptr, *pky64 = nullptr, *rksz64 = nullptr;
-  float* vk32 = nullptr;  // vz + vset per class
-  // the fused met fields in the halo layout of c (two-columns-per-lane kernel)
-  float *vxh = nullptr, *vyh = nullptr, *lrhoh = nullptr, *pkxh = nullptr, *pkyh = nullptr,
-        *pkzh = nullptr, *vkh = nullptr;
-  f3d::F2Maps maps2{};  // tensor maps of those fields (shape-3 step kernel)
+  f3d::StepFields sf{};  // the fused step kernel's fields (halo layout of c) and their tensor maps
+  f3d::F2Maps maps2{};
+  int nwet = 0;  // the highest level with zlayer <= zi at any column (wetdep.f90:37)
   double* lambda2d = nullptr;
   unsigned char* wet_class = nullptr;
   int opt_fused = 1, opt_tile = 3;
@@ -142,8 +141,9 @@ int ctx_run_prepare(f3d_ctx* x, const f3d_met_series* met, const f3d_src_series*
 void ctx_advance(f3d_ctx* x);
 // the mass-budget log of endstep.f90:51 when due
 int ctx_log(f3d_ctx* x, f3d_log_record* log, int log_cap, int* nlog);
-// arguments of the fused precision-form step for the context's state
-FusedArgs ctx_fused_args(f3d_ctx* x);
+// arguments of the fused precision-form step for the context's state, with
+// the column pieces of a launch of its own for tile shape `shape`
+FusedArgs ctx_fused_args(f3d_ctx* x, int shape);
 int ctx_check_step_status(f3d_ctx* x);
 inline double* ctx_outmass(f3d_ctx* x) { return x->small; }
 // gravity current (f3d_gravity.cu): addradialwind on the scaled winds of
@@ -157,8 +157,8 @@ int agg_setsrc(f3d_ctx* x);
 int agg_restore_vset(f3d_ctx* x, int times);
 // a zero-filled device allocation owned by the context
 int ctx_alloc(f3d_ctx* x, void** p, size_t bytes);
-// the binary32 copies of class ic's settling velocity (vset32, vk32 and
-// its halo-layout copy) after vset changed on the device
+// the binary32 copies of class ic's settling velocity (vset32 and the step
+// kernel's vz+vset) after vset changed on the device
 void refresh_fp32_class(f3d_ctx* x, int ic);
 // waits for a look-ahead meteo update in flight and drops it (its chain
 // state is not committed)

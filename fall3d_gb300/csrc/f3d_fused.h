@@ -7,26 +7,55 @@
 
 namespace f3d {
 
+// Per-level factors of the step (binary32, rounded once from binary64), with
+// dzz = 2/(dz(k)+dz(k-1)) of advctzc.f90:34 and diffz.f90:25.
+struct ZTab {
+  float a, b;     // lim_coef_z: dt/4*dz(k-1)*dzz, dt^2/8*dzz
+  float rdz;      // 1/dz(k): the slope between k and k+1
+  float dtdzz;    // dt*dzz
+  float dtrdz;    // dt/dz(k)
+  float pad[3];
+};
+
+// Fields of the step kernel, filled at every meteo update.  3-D fields have
+// the halo layout of the precision form's c: rows of d.px values (nx+2
+// rounded up to a multiple of 4, so that tensor copies can stage them),
+// planes 0..nz+1; ghost rows and columns hold what makes the interior
+// formulas give the reference's boundary faces.
+struct StepFields {
+  float* ux;  // Courant velocity vx*dt/dX1, ghost columns = the adjacent cell's
+  float* kx;  // limiter coefficient of work(i,2), advctx.f90:40-43: 0.5*C*(1-C), C = 0.5*|ux(i)+ux(i-1)|
+  float* uy;  // vy*dt/dX2, ghost rows = the adjacent cell's
+  float* ky;
+  float* l;   // 1/rho, ghosts = the adjacent cell's
+  float* fx;  // face (i,i+1): 0.5*dt/dX1^2*(P(i)+P(i+1)), P = rkh1*rho; faces 0 and nx: dt/dX1^2*P(1), P(nx)
+  float* fy;  // face (j,j+1) likewise, P = rkhor*rho
+  float* fz;  // face (k,k+1): 0.5*(P(k)+P(k+1))/dz(k), P = rkver*rho; plane 0: P(1)/dz(0),
+              // plane nz: P(nz)/dz(nz), plane nz+1: P(nz-1)/dz(nz-1)
+  float* vk;  // vz+vset, class blocks
+  // the faces of the first and last cells on their inner side, which the
+  // reference does not average (diffx.f90:22-33, 44-55): dt/dX1^2*P(2) and
+  // P(nx-1) at [side][k][j] (nz+2 planes of ny+2), dt/dX2^2*P(2), P(ny-1) at
+  // [side][k][i] (nz+2 planes of px), P(2)/dz(1) of diffz at [j][i] (px)
+  float *ex, *ey, *ez;
+  ZTab* tab;  // levels 0..nz+1
+};
+
 struct FusedArgs {
-  const float* c_in;  // class blocks of (nx+2)(ny+2)(nz+2), after setsrc
+  const float* c_in;  // class blocks of d.halo() values, after setsrc
   float* c_out;       // same layout; receives the step's result incl. ghosts
   long long cstride;
   Dims d;
   int ncls;
   int xfirst;  // iiter even: x before y (sizloop.f90:42-48)
-  float dt;
+  // the column is cut into nchunk pieces marched by different blocks: levels
+  // 1..kfirst, then pieces of klen levels
+  int nchunk, kfirst, klen;
   double dt64;
-  // binary32 coefficients (scaled fields of meteo.f90:108-112)
-  const float *vx, *vy, *vz;
-  const float* vk;  // vz + vset, class blocks of nx*ny*nz
-  long long vstride;
+  StepFields f;
   const float* vdep;  // class blocks of nx*ny
-  long long dstride;
   const float* rkver1;  // rkver(:,:,1) (setbcc bottom)
-  const float* lrho;    // 1/rho
-  const float *pkx, *pky, *pkz;  // rkh1*rho, rkhor*rho, rkver*rho
-  const float* dz;      // dz(0:nz)
-  float auxvx, auxvy, inv_dx, inv_dy, dtdx2, dtdy2;
+  float dz0;
   // binary64 deposits
   const unsigned char* wet_class;  // per class: wet deposition applies (or NULL)
   const double* lambda2d;          // min(dt*a*prate^b,1) per column
@@ -35,43 +64,49 @@ struct FusedArgs {
   const double* dz64;
   double* cwet;  // (nx,ny,0:nc)
   double* cdry;
-  const double* vset64;  // class blocks, vstride apart
+  const double* vset64;  // class blocks of nx*ny*nz
   const double* vdep64;  // class blocks of nx*ny
-  // the same binary32 fields in the halo layout of c, ghost entries zero, but
-  // with the row pitch hpitch = nx+2 rounded up to a multiple of 4 (padding
-  // zero), so that a tensor copy can stage them: used by the
-  // two-columns-per-lane kernel (tile shape 3)
-  const float *vxh, *vyh, *lrhoh, *pkxh, *pkyh, *pkzh;
-  const float* vkh;  // class blocks of hstride values
-  int hpitch;
-  long long hstride;  // hpitch * (ny+2) * (nz+2)
-  int pair_aligned;  // nx even: every even column starts an 8-byte pair
-  int* status;       // device status word: F3D_STEP_STAGING_TIMEOUT is or-ed into it
+  int* status;           // device status word: F3D_STEP_STAGING_TIMEOUT is or-ed into it
 };
 
 // a staging wait of the step kernel gave up (a tensor copy did not arrive)
 #define F3D_STEP_STAGING_TIMEOUT 0x100
 
-// Tensor maps of the met fields for the shape-3 step kernel's tensor copies:
-// boxes of 68 x 32 x 1 values (x, rows, planes) of the padded halo layout.
+// Tensor maps of a context's met fields and of a state buffer for the step
+// kernel's tensor copies: boxes of 68 values (x) by the tile region's rows by
+// one plane.  [0]: 32-row boxes, [1]: 16-row boxes.
 struct F2Maps {
-  enum { VK = 0, VX, VY, L, PZ, PX, PY, N };
-  CUtensorMap m[N];
+  enum { VK = 0, UX, KX, UY, KY, L, FZ, FX, FY, N };
+  CUtensorMap m[2][N];
+};
+struct CMaps {
+  CUtensorMap m[2];
 };
 // 0 on success
-int make_fused2_maps(const FusedArgs& a, F2Maps* out);
-// the largest nz the shape-3 kernel's shared memory holds
+int make_step_maps(const FusedArgs& a, F2Maps* out);
+int make_c_maps(Dims d, int ncls, const float* c, CMaps* out);
+// the largest nz whose per-level table the step kernel's shared memory holds
 int fused2_max_nz();
 inline int halo_pitch(int nx) { return (nx + 2 + 3) & ~3; }
 
-// tile region (x by y) / threads: 0 = 32x32 / 256 (default), 1 = 32x64 / 512,
-// 2 = 32x32 / 512, 3 = 64x32 / 512 with two columns per lane.
-void launch_step_fused(const FusedArgs& a, int shape, cudaStream_t s);
-// beside != 0: the 112-register build, which leaves room for a look-ahead
-// meteo update's settling chain on the same SMs (same results)
-void launch_step_fused2(const FusedArgs& a, const F2Maps& maps, cudaStream_t s, int beside = 0);
-// met fields (nx,ny,nz) -> halo layout of row pitch hp (ghost entries untouched)
-void launch_to_halo(Dims d, int hp, int nfield, const float* const* src, float* const* dst, cudaStream_t s);
+// How a context's column is cut (nchunk, kfirst, klen) so that the tiles of
+// all classes fill the device: nwet = highest level any wet deposition
+// reaches (0: none), which the first piece must hold.
+void step_chunks(FusedArgs& a, int shape, int nwet);
+
+// Tile shapes (F3D_OPT_TILE), region x by y / threads: 0, 1 and 2 = 64x16 /
+// 512 (a row per warp, two blocks per SM), 3 = 64x32 / 512 (two rows per
+// warp, the default); two columns per lane.  Results do not depend on the
+// shape.
+void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s);
+// The step kernel's fields from the scaled binary64 fields of a meteo update
+// whose finddt maximum is at *dtcn (dt = safety/max(dtcn,1e-13)).
+void launch_step_fields(Dims d, int nc, double safety, double dX1, double dX2, const double* dz,
+                        const unsigned long long* dtcn, const double* vx, const double* vy, const double* vz,
+                        const double* rho, const double* rkh1, const double* rkhor, const double* rkver,
+                        const double* vset, const StepFields& f, cudaStream_t s);
+// vz+vset of one class block
+void launch_step_vk(Dims d, int nc, const double* vz, const double* vset, float* vk, cudaStream_t s);
 // tiles of one class of an nx x ny grid for a tile shape
 int fused_tiles(int nx, int ny, int shape);
 
@@ -79,31 +114,15 @@ int fused_tiles(int nx, int ny, int shape);
 // memory (c_in / c_out are the scenario's two buffers), then one persistent
 // launch over the work items of all of them.
 #define F3D_BATCH_MAX 128
-int upload_batch_args(const FusedArgs* h, int n, cudaStream_t s);
-int upload_batch_args2(const FusedArgs* h, int n, cudaStream_t s);  // the shape-3 kernel's table
-int fused2_batch_grid(int max_nz);
-// items [0, split) belong to scenarios with an even nx (two counters)
-// maps: the scenarios' tensor maps (device array in batch order)
-// fork: when both parts exist, the odd-nx part runs on fork->s2 as a
-// parallel branch (fork->a recorded on s, fork->b on s2, s waits for it), so
-// that its blocks fill the SMs the even-nx part's last blocks leave free
-struct BatchFork {
-  cudaStream_t s2 = nullptr;
-  cudaEvent_t a = nullptr, b = nullptr;
+struct BatchMaps {  // a scenario's tensor maps (device array in batch order)
+  F2Maps met;
+  CMaps a, b;
 };
-void launch_step_fused2_batch(int grid, const int* item_off, int nscen, int split, int total, int* counter,
-                              const int* bstep, const int* iiter0, int commit, int max_nz, const F2Maps* maps,
-                              cudaStream_t s, const BatchFork* fork = nullptr);
+int upload_batch_args(const FusedArgs* h, int n, cudaStream_t s);
 // sets the kernel's shared-memory limit and returns its persistent grid (-1 on error)
 int fused_batch_grid(int shape, int max_nz);
-// counter: two ints; split / total: see launch_step_fused2_batch (shape 3)
-void launch_step_fused_batch(int shape, int grid, const int* item_off, int nscen, int split, int total,
-                             int* counter, const int* bstep, const int* iiter0, int commit, int max_nz,
-                             const F2Maps* maps, cudaStream_t s, const BatchFork* fork = nullptr);
-void launch_vk32(long long n, int nc, const float* vz, const float* vset, float* vk, cudaStream_t s);
+void launch_step_fused_batch(int shape, int grid, const int* item_off, int nscen, int* counter, const int* bstep,
+                             const int* iiter0, int commit, int max_nz, const BatchMaps* maps, cudaStream_t s);
 void launch_wet_lambda(long long n, double dt, const double* prate, double* lam, cudaStream_t s);
-void launch_fp32_coeffs(long long n, const double* rho, const double* rkh1, const double* rkhor,
-                        const double* rkver, float* lrho, float* pkx, float* pky, float* pkz,
-                        cudaStream_t s);
 
 }  // namespace f3d

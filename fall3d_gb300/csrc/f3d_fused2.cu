@@ -1,22 +1,55 @@
-// f3d_fused2.cu -- the precision form's whole transport step in one kernel,
-// two columns per lane.
+// f3d_fused2.cu -- the precision form's whole transport step in one kernel.
 //
-// Same march as f3d_fused.cu (one CTA per tile and class, up the column;
-// iteration t: setbcc + advctzc and advctx/advcty on plane t, then diffz,
-// diffx/diffy, wetdep, accum, clip and store on plane t-1), laid out for
-// fewer instructions per cell:
+// One block owns an output tile of one class and marches up the column (or a
+// piece of it), so each concentration is read from and written to HBM once
+// per step.  The sweeps of Sources/sizloop.f90:35-71 are pipelined per
+// horizontal plane; iteration t runs
 //
-//  * a lane owns two neighbouring columns, so every field of a position pair
-//    is one 64-bit value: f32x2 arithmetic, 64-bit shared-memory accesses
-//    and 8-byte asynchronous copies; an x neighbour costs one shuffle per
-//    pair instead of one per cell;
-//  * the tile region is 64 x 32 (58 x 26 output cells, 16 warps, two rows
-//    per warp), so fewer halo cells are recomputed per output cell;
-//  * the met fields come in the halo layout of c, so one offset addresses
-//    all nine staged fields of a position and interior tiles need no bounds
-//    logic at all.
+//   A  setbcc + advctzc   plane t, per column in registers (window of the
+//                         original column c(t), c(t+1), c(t+2) and the flux
+//                         difference of the face below)
+//   B  advctx / advcty    plane t; x: warp shuffles along a row; y: the
+//                         lane's own rows and shared memory
+//   C  diffz              plane k = t-1 (needs plane t of B)
+//   D  diffx / diffy      plane k
+//   E  wetdep, accum, clip, store (plane k)
 //
-// Every cell gets the bits of the scalar formulas (f3d_fused_math.cuh).
+// A lane owns two neighbouring columns (every field of a position pair is one
+// 64-bit value), a warp HY/NW adjacent rows of the 64 x HY tile region.  The
+// x/y sweeps need +-2 cells (advection) then +-1 (diffusion), so the output
+// tile is 58 x (HY-6); halo cells are recomputed by neighbouring blocks.  The
+// ghost cells of setbcc are formed from the original column
+// (setbcc.f90:53-83) and stay unchanged through the sweeps (the reference's
+// stale ghosts).  Input and output are distinct buffers.
+//
+// Each advection sweep takes a cell's two upwind differences from one flux
+// per face, F = u*c + K*minmod (u the Courant velocity, K the limiter's
+// coefficient): c - (F(q) - F(q-1)) or c - (F(q+1) - F(q)); each diffusion
+// sweep adds the difference of its two face fluxes.  Everything that does not
+// depend on the class is part of the staged coefficients (StepFields); the
+// boundary faces of the reference come from the coefficients' ghost values.
+//
+// Staging: the ten fields iteration t+1 reads (c two planes ahead, vz+vset
+// one, the Courant velocities and limiter coefficients, 1/rho and the three
+// face coefficients) arrive by tensor copies while iteration t computes; one
+// lane of each warp issues a field's box.  A box starts at the region's first
+// column rounded down to a multiple of 4 values (16 bytes, what a tensor
+// copy needs; the region then starts 0 or 2 values into it) and is 68 wide.
+//
+// What bounds it: 400x300x50 cells and 16 classes take 0.999 ms (1.255 ms
+// before the flux form, the packed arithmetic, the coefficients formed at the
+// meteo update and the shared-memory addressing), 1.32 GB of algorithmic bytes
+// or 0.19 ms at the copy bandwidth.  A warp issues about 500 instructions per
+// plane for its 128 positions, 200 of them binary32 arithmetic, at half the
+// issue rate: with one block of 16 warps per SM (174 KB of staged fields, 128
+// registers) the dependency chains of the sweeps and the three block barriers
+// of a plane are not all covered.
+//
+// Column pieces: a march over levels k0..k1 starts at t = k0-1 from the
+// original column's planes k0-3..k0 (the advection fluxes of plane k0-1 need
+// them), so pieces are independent of one another; they let grids with few
+// tiles fill the device.  Every value is formed by the same operations
+// whatever the tile shape or the pieces, so results do not depend on them.
 #include <algorithm>
 #include <type_traits>
 
@@ -28,58 +61,52 @@ namespace {
 
 using namespace fz;
 
-constexpr int HX = 64, HY = 32, NW = 16, NT = 32 * NW, RPW = HY / NW, TX = HX - 6, TY = HY - 6,
-              NP = HX * HY;
-// The staged fields are boxes of RS x HY values: a tensor copy's first column
-// must lie on a 16-byte boundary, so a box starts at the region's first
-// column rounded down to a multiple of 4 (gx0 is even: the region then
-// starts 0 or 2 values into the box) and is 4 values wider than the region.
-constexpr int RS = HX + 4, FS = RS * HY;
+constexpr int HX = 64, TX = HX - 6, RS = HX + 4;
 constexpr int GUARD = 512;  // bytes before the staging area (reads one row above a field)
+
+template <int HY_, int NW_>
+struct Shape {
+  static constexpr int HYR = HY_, NWARP = NW_, NT = 32 * NW_, RPW = HY_ / NW_, TY = HY_ - 6, FS = RS * HY_,
+                       NP = HX * HY_, MAP = HY_ == 32 ? 0 : 1;
+  static_assert(HY_ % NW_ == 0 && NW_ >= NF, "rows must divide among warps; a warp issues one field's copies");
+};
+constexpr int HY = 32, NW = 16;  // the default shape
+using Tall = Shape<HY, NW>;
+using Flat = Shape<16, 16>;
 
 // value of the column to the left / right of each of the lane's two columns
 __device__ __forceinline__ float2 left2(float2 v) { return make_float2(shup(v.y), v.x); }
 __device__ __forceinline__ float2 right2(float2 v) { return make_float2(v.y, shdn(v.x)); }
-__device__ __forceinline__ float2 sel2(bool cx, bool cy, float2 a, float2 b) {
-  return make_float2(cx ? a.x : b.x, cy ? a.y : b.y);
-}
 __device__ __forceinline__ float cmp(const float2& v, int c) { return c ? v.y : v.x; }
 __device__ __forceinline__ float& cmp(float2& v, int c) { return c ? v.y : v.x; }
 
-__device__ __forceinline__ void cp_async8(unsigned dst, const float* src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0));
-}
-__device__ __forceinline__ void cp_async4s(unsigned dst, const float* src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 4 : 0));
-}
-
 __device__ __forceinline__ float2 lds2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void sts2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+__device__ __forceinline__ float2 ldg2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
 
-size_t fused2_smem(int nz) {
-  return 128 + GUARD + sizeof(float) * ((size_t)2 * NF * FS + 4 * (size_t)NP + HX) +
-         (2 * sizeof(double) + sizeof(int)) * TX * TY + sizeof(ZT32) * (size_t)(nz + 1) + 32;
+template <class S>
+size_t step_smem(int nz) {
+  return GUARD + sizeof(float) * ((size_t)(2 * NF + NA) * S::FS + 3 * (size_t)S::NP + HX) +
+         sizeof(ZTab) * (size_t)(nz + 2) + 64;
 }
 
 // ------------------------------------------------ tensor copies (TMA)
-// Elected thread 0 stages the eight met fields of a plane with
-// cp.async.bulk.tensor into the buffer of that plane; completion is counted
-// in bytes on the buffer's mbarrier, which every thread waits on.
-__device__ __forceinline__ void mbar_init(unsigned bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+__device__ __forceinline__ void mbar_init(unsigned bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// waits for the phase of the given parity, at most ~2^20 polls; false on a timeout
+// waits for the phase of the given parity, at most 4096 polls, each of which
+// the hardware may suspend for up to a millisecond; false on a timeout
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-  for (int i = 0; i < (1 << 20); ++i) {
+  for (int i = 0; i < 4096; ++i) {
     unsigned ok;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(1000000)
         : "memory");
     if (ok) return true;
   }
@@ -93,28 +120,29 @@ __device__ __forceinline__ void tma_load3(unsigned dst, const CUtensorMap* map, 
       : "memory");
 }
 
-// One tile of one class (see fused_tile in f3d_fused.cu for the arguments).
-// P8: nx is even, so every column pair starts on an 8-byte boundary and lies
-// wholly inside or wholly outside the halo array; otherwise the pairs are
-// copied and stored one value at a time.
-// The met fields come by tensor copies (maps: this scenario's tensor maps),
-// c by every thread's own cp.async copies.
-template <bool P8>
-__device__ __forceinline__ void fused2_tile(const FusedArgs& a, const F2Maps* maps, const float* c_in, float* c_out,
-                                            const int xfirst, const int commit, const int cls, const int tile,
-                                            unsigned char* smem_raw) {
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<size_t>(smem_raw) + 127) & ~(size_t)127);
-  float* stage = reinterpret_cast<float*>(base + GUARD);  // [2][NF][FS], 128-byte aligned fields
-  float* P0s = stage + 2 * NF * FS;
-  float* W1s = P0s + NP;
-  float* W2s = W1s + NP;
-  float* P1s = W2s + NP;
-  double* wacc = reinterpret_cast<double*>(P1s + NP + HX);
-  double* wlam = wacc + TX * TY;
-  int* wkz = reinterpret_cast<int*>(wlam + TX * TY);
-  ZT32* tab = reinterpret_cast<ZT32*>(wkz + TX * TY);
-  unsigned long long* mbar = reinterpret_cast<unsigned long long*>(
-      (reinterpret_cast<size_t>(tab + (a.d.nz + 1)) + 7) & ~(size_t)7);  // one per staging buffer
+// One piece of the column of one tile of one class.  maps, cmap: tensor maps
+// of the scenario's met fields and of c_in.  commit = 0 skips the deposit
+// writes (cdry, cwet) so that the autotuner can time the kernel on a live
+// state.
+template <class S, bool XFIRST>
+__device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps, const CMaps* cmap,
+                                          const float* c_in, float* c_out, const int commit, const int cls,
+                                          const int tile, const int chunk) {
+  constexpr int RPW = S::RPW, TY = S::TY, FS = S::FS, NP = S::NP, NT = S::NT, HYR = S::HYR;
+  // The block's shared memory, addressed from the array itself with no detour
+  // through an integer or a parameter: the compiler then knows the address
+  // space and emits shared-memory instructions with 32-bit addresses (with
+  // generic ones the step of 400x300x50 cells, 16 classes took 1.125 ms
+  // instead of 1.055 ms).
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  // 128-byte aligned fields: [3][NA][FS] of the fields read ahead, [2][NF-NA][FS] of the others
+  float* stage = reinterpret_cast<float*>(smem_raw + GUARD);
+  float* P0s = stage + (2 * NF + NA) * FS;                // planes the y sweeps exchange rows through:
+  float* Ws = P0s + NP;                                   // c, the advection flux, c/rho
+  float* P1s = Ws + NP;
+  ZTab* tab = reinterpret_cast<ZTab*>(P1s + NP + HX);
+  // one per staging buffer: 3 of the fields read ahead, 2 of the others
+  unsigned long long* mbar = reinterpret_cast<unsigned long long*>(tab + (a.d.nz + 2));
 
   const Dims d = a.d;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -122,369 +150,344 @@ __device__ __forceinline__ void fused2_tile(const FusedArgs& a, const F2Maps* ma
   const int i0 = 1 + (tile % tiles_x) * TX, j0 = 1 + (tile / tiles_x) * TY;
   const int gx0 = i0 - 3, gy0 = j0 - 3;
   const int oi1 = min(nx, i0 + TX - 1), oj1 = min(ny, j0 + TY - 1);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gi = gx0 + 2 * lane;  // the lane's first column; the second is gi + 1
-  const int px = nx + 2;          // halo row pitch of c
-  const int cs = px * (ny + 2);   // halo plane of c
-  const int hp = a.hpitch;        // row pitch of the met fields (padded to a multiple of 4)
-  const int hs = hp * (ny + 2);   // their plane
-  const int xs = gx0 & ~3;        // first column of the staged boxes
-  const int sft = gx0 - xs;       // the region's offset in a box row (0 or 2)
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(FULL, (int)threadIdx.x >> 5, 0);  // uniform
+  const int gi = gx0 + 2 * lane;       // the lane's first column (even); the second is gi + 1
+  const int gj0 = gy0 + RPW * warp;    // the warp's first row
+  const int px = d.px;                 // row pitch of c and of the fields (a multiple of 4)
+  const int cs = px * (ny + 2);        // their plane
+  const int xs = gx0 & ~3;             // first column of the staged boxes
+  const int sft = gx0 - xs;            // the region's offset in a box row (0 or 2)
   const int pl = nx * ny;
-  const bool edge = !(gx0 >= 1 && gx0 + HX - 1 <= nx && gy0 >= 1 && gy0 + HY - 1 <= ny);
+  const bool edge = !(gx0 >= 1 && gx0 + HX - 1 <= nx && gy0 >= 1 && gy0 + HYR - 1 <= ny);
   const bool xedge = gx0 <= 1 || gx0 + HX - 1 >= nx;  // the region holds column 1 or nx
+  // levels k0..k1 of the column, iterations ts..te
+  const int k0 = chunk == 0 ? 1 : a.kfirst + 1 + (chunk - 1) * a.klen;
+  const int k1 = chunk == 0 ? (a.nchunk > 1 ? a.kfirst : nz) : min(nz, k0 + a.klen - 1);
+  const int ts = max(1, k0 - 1), te = k1 + 1;
 
   const unsigned mbar0 = (unsigned)__cvta_generic_to_shared(mbar);
-  if (threadIdx.x == 0) {
-    mbar_init(mbar0);
-    mbar_init(mbar0 + 8);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  for (int k = threadIdx.x; k <= nz; k += NT) {
-    const float dzk = a.dz[k];
-    tab[k] = make_zt32(dzk, k > 0 ? a.dz[k - 1] : dzk, a.dt);
-  }
-  const bool wet = a.wet_class && a.wet_class[cls];
   __shared__ int s_kzmax;  // the highest wet layer of the tile: above it the wet code is skipped
-  if (threadIdx.x == 0) s_kzmax = 0;
-  __syncthreads();
-  for (int o = threadIdx.x; o < TX * TY; o += NT) {
-    const int oi = i0 + o % TX, oj = j0 + o / TX;
-    wacc[o] = 0.0;
-    wlam[o] = 0.0;
-    wkz[o] = 0;
-    if (!wet || oi > oi1 || oj > oj1) continue;
-    const int p2 = (oi - 1) + nx * (oj - 1);
-    wlam[o] = a.lambda2d[p2];
-    wacc[o] = a.cwet[(long long)(cls + 1) * pl + p2];
-    // zlayer is non-decreasing (checked on the host): the layers below the
-    // mixing height are a prefix of the column (wetdep.f90:37)
-    const double zi = a.zi[p2];
-    int kz = 0;
-    while (kz < nz && a.zlayer[kz] <= zi) ++kz;
-    wkz[o] = kz;
-    if (kz > 0) atomicMax(&s_kzmax, kz);
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < 5; ++b) mbar_init(mbar0 + 8u * b, b < 3 ? NA : NF - NA);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_kzmax = 0;
   }
+  __syncthreads();
+
+  // ------------------------------------------------ staging
+  // The staged inputs of iteration t: c and vz+vset, which the column update
+  // at its start reads, in buffer (t-ts)%3 and issued two iterations ahead;
+  // the others in buffer (t-ts)&1, one ahead.  Both are issued after the first
+  // barrier of an iteration, when every warp has left the previous iteration
+  // and this one's column update and nobody reads those buffers.  One lane of
+  // warp f issues field f's box; outside the arrays it fills zeros, planes
+  // outside 1..nz are not read and not copied.
+  const unsigned stage0 = (unsigned)__cvta_generic_to_shared(stage);
+  const bool issuer = lane == 0 && warp < NF;
+  const bool ahead = warp < NA;
+  auto prefetch = [&](const int i) {  // i = t - ts
+    if (!issuer) return;
+    const int t = ts + i;
+    if (t > te) return;
+    const int buf = ahead ? i % 3 : 3 + (i & 1);
+    const unsigned bar = mbar0 + 8u * (unsigned)buf;
+    const int slot = ahead ? buf * NA + warp : 3 * NA + (buf - 3) * (NF - NA) + warp - NA;
+    const int p = t + field_plane(warp);
+    // the warps' reads of this buffer (ordered before this point by a block
+    // barrier) come before the tensor copy overwrites it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (p >= 1 && p <= nz) {
+      mbar_expect(bar, (unsigned)(FS * sizeof(float)));
+      tma_load3(stage0 + 4u * (unsigned)(slot * FS), warp == F_C ? &cmap->m[S::MAP] : &maps->m[S::MAP][warp - 1], xs, gy0,
+                (ahead ? cls * (nz + 2) : 0) + p, bar);
+    } else {
+      mbar_expect(bar, 0u);
+    }
+  };
+  bool timed_out = false;
+  auto staged = [&](const int bar, const int phase) {
+    if (!mbar_wait(mbar0 + 8u * (unsigned)bar, (unsigned)phase)) timed_out = true;
+  };
+  prefetch(0);
+  if (ahead) prefetch(1);
+
+  for (int k = threadIdx.x; k < (nz + 2) * (int)(sizeof(ZTab) / 4); k += NT)
+    reinterpret_cast<float*>(tab)[k] = __ldg(reinterpret_cast<const float*>(a.f.tab) + k);
+  // wet deposition reaches only the first piece (step_chunks)
+  const bool wet = a.wet_class && chunk == 0 && a.wet_class[cls];
+  // zlayer is non-decreasing (checked on the host): the layers below the
+  // mixing height are a prefix of the column (wetdep.f90:37)
+  if (wet)
+    for (int o = threadIdx.x; o < TX * TY; o += NT) {
+      const int oi = i0 + o % TX, oj = j0 + o / TX;
+      if (oi > oi1 || oj > oj1) continue;
+      const double zi = a.zi[(oi - 1) + nx * (oj - 1)];
+      int kz = s_kzmax;
+      while (kz < nz && a.zlayer[kz] <= zi) ++kz;
+      if (kz > 0) atomicMax(&s_kzmax, kz);
+    }
 
   const float* __restrict__ cin = c_in + (long long)cls * a.cstride;
   float* __restrict__ cout = c_out + (long long)cls * a.cstride;
-  const float* __restrict__ vkc = a.vkh + (long long)cls * a.hstride;
-  const float dt = a.dt;
-  const float dznz = 1.0f / a.dz[nz];
-  const float auxvx = a.auxvx, auxvy = a.auxvy;
-  const float dtdx2h = 0.5f * a.dtdx2, dtdy2h = 0.5f * a.dtdy2;
+  const float* __restrict__ vkc = a.f.vk + (long long)cls * a.cstride;
 
   // ------------------------------------------------ per-position state
-  // bit 2r+c: row r (gj = gy0 + 2*warp + r), column c (gi + c); a warp owns
-  // two adjacent rows, so each row's y-neighbour on the other side is the
-  // same lane's other row
-  unsigned kin = 0, kgx = 0, kgy = 0, inr = 0;  // inr: the pair of row r lies in the halo array
-  int h0[RPW];                                  // halo offset of (gi, gj, plane 0), clamped
+  // bit 2r+c: row r (gj0 + r), column c (gi + c) is an output cell; is stored
+  // at the planes 1..nz (output cells and the tile's ghosts on the grid's faces)
+  unsigned kout = 0, kst = 0;
 #pragma unroll
   for (int r = 0; r < RPW; ++r) {
-    const int gj = gy0 + 2 * warp + r;
-    const bool yin = gj >= 1 && gj <= ny;
+    const int gj = gj0 + r;
+    const bool rows_out = gj >= j0 && gj <= oj1;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int g = gi + c;
-      const bool xin = g >= 1 && g <= nx;
+      const bool cols_out = g >= i0 && g <= oi1;
       const unsigned bit = 1u << (2 * r + c);
-      if (xin && yin) kin |= bit;
-      else if ((g == 0 || g == nx + 1) && yin) kgx |= bit;
-      else if ((gj == 0 || gj == ny + 1) && xin) kgy |= bit;
-      if (g >= 0 && g <= nx + 1 && gj >= 0 && gj <= ny + 1) inr |= bit;
+      if (rows_out && cols_out) kout |= bit;
+      if ((rows_out && ((g == 0 && i0 == 1) || (g == nx + 1 && oi1 == nx))) ||
+          (cols_out && ((gj == 0 && j0 == 1) || (gj == ny + 1 && oj1 == ny))))
+        kst |= bit;
     }
-    h0[r] = (inr >> (2 * r) & 1u) ? gi + px * gj : cs;  // clamped for pairs outside (plane 1 stays in range)
   }
-  float2 o_0[RPW], o_p1[RPW], vk0[RPW], w1k[RPW], w2km[RPW], w2k[RPW], gtop[RPW];
-  float2 ra[RPW], rb[RPW], rc[RPW], fprev[RPW], gprev[RPW], pb[RPW];
-#pragma unroll
-  for (int r = 0; r < RPW; ++r) {
-    o_0[r] = o_p1[r] = vk0[r] = w1k[r] = w2km[r] = w2k[r] = gtop[r] = make_float2(0.0f, 0.0f);
-    ra[r] = rb[r] = rc[r] = fprev[r] = gprev[r] = pb[r] = make_float2(0.0f, 0.0f);
-  }
-  const unsigned stage0 = (unsigned)__cvta_generic_to_shared(stage);
-  const unsigned sbase = stage0 + 4u * (unsigned)(2 * warp * RS + sft + 2 * lane);
-  bool timed_out = false;
-
-  // the staged inputs of iteration t into buffer t&1 (fields as in
-  // f3d_fused.cu): c by each thread for its own positions (positions outside
-  // the halo array copy nothing: zero fill), the met boxes by thread 0's
-  // tensor copies (outside the arrays: zero fill).  Group 0: the fields the
-  // advection phases read (c, vz+vset, vx, vy); group 1: those the diffusion
-  // phases read (1/rho, K*rho); 2: both.  Group 0 of iteration t+1 is issued
-  // as iteration t starts where every warp has passed the last barrier of
-  // iteration t-1 (after which nobody reads those fields of that buffer),
-  // group 1 after the first barrier of iteration t.
-  auto prefetch = [&](auto edge_c, const int t, const int group) {
-    constexpr bool EDGE = decltype(edge_c)::value;
-    const unsigned sb = sbase + 4u * (unsigned)((t & 1) * NF * FS);
-    const bool g0 = group != 1, g1 = group != 0;
-    const bool okc = g0 && t + 2 <= nz, okk = g0 && t + 1 <= nz, okv = g0 && t <= nz, okm = g1 && t <= nz,
-               okl = g1 && t >= 2 && t <= nz + 1;
-    {
-      if (threadIdx.x == 0) {
-        const unsigned bar = mbar0 + 8u * (unsigned)(t & 1);
-        const unsigned db = stage0 + 4u * (unsigned)((t & 1) * NF * FS);
-        // the warps' reads of this buffer (ordered before this point by a
-        // block barrier) come before the tensor copies overwrite it
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (g0) {  // the buffer's next phase: every met box of plane t, both groups
-          const unsigned n = (unsigned)((t + 1 <= nz) + 4 * (t <= nz) + 3 * (t >= 2 && t <= nz + 1));
-          if (n) mbar_expect(bar, n * (unsigned)(FS * sizeof(float)));
-        }
-        auto ld = [&](int field, int map, int z) { tma_load3(db + 4u * (unsigned)(field * FS), &maps->m[map], xs, gy0, z, bar); };
-        if (okk) ld(F_VK, F2Maps::VK, cls * (nz + 2) + t + 1);
-        if (okv) {
-          ld(F_VX, F2Maps::VX, t);
-          ld(F_VY, F2Maps::VY, t);
-        }
-        if (okm) {
-          ld(F_L, F2Maps::L, t);
-          ld(F_PZ, F2Maps::PZ, t);
-        }
-        if (okl) {
-          ld(F_L1, F2Maps::L, t - 1);
-          ld(F_PX, F2Maps::PX, t - 1);
-          ld(F_PY, F2Maps::PY, t - 1);
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-      const unsigned dst = sb + 4u * (unsigned)(r * RS);
-      const int ht = h0[r] + t * cs;  // this row's offset at plane t (c)
-      const bool v0 = !EDGE || (inr >> (2 * r) & 1u), v1 = !EDGE || (inr >> (2 * r + 1) & 1u);
-      auto cp = [&](int field, const float* src, int off) {
-        const unsigned dd = dst + 4u * (unsigned)(field * FS);
-        if constexpr (P8) {
-          (void)v1;
-          cp_async8(dd, src + off, v0);
-        } else {  // an odd nx: a pair may straddle the last ghost column
-          cp_async4s(dd, src + off, v0);
-          cp_async4s(dd + 4u, v1 ? src + off + 1 : src + off, v1);
-        }
-      };
-      if (okc) cp(F_C, cin, ht + 2 * cs);
-    }
-    cp_async_commit();
-  };
-  // all staged inputs of iteration t are in buffer t&1
-  auto staged = [&](const int t) {
-    cp_async_wait_all();
-    if (!mbar_wait(mbar0 + 8u * (unsigned)(t & 1), (unsigned)(((t - 1) >> 1) & 1))) timed_out = true;
-  };
-  if (edge)
-    prefetch(True_{}, 1, 2);
-  else
-    prefetch(False_{}, 1, 2);
+  kst |= kout;
+  // ghost columns of the lane's pair, ghost rows of the warp (uniform)
+  const bool gx_0 = gi == 0 || gi == nx + 1, gx_1 = gi + 1 == nx + 1;
+  auto ghost_row = [&](int r) { return gj0 + r == 0 || gj0 + r == ny + 1; };
+  const bool pair_in = gi >= 0 && gi < px;  // the pair lies in the arrays' rows
+  auto row_in = [&](int r) { return gj0 + r >= 0 && gj0 + r <= ny + 1; };
+  const int h0 = gi + px * gj0;  // offset of the first row's pair at plane 0
+  // original column c(t), c(t+1), vz+vset(t), slope(t) = (c(t+1)-c(t))/dz(t),
+  // work(t,2), the flux difference below plane t; then the advected plane
+  // t-1, 1/rho there, and the diffusive flux below it
+  float2 o0[RPW], o1[RPW], vk[RPW], sl[RPW], w2[RPW], gk[RPW], gtop[RPW];
+  float2 rb[RPW], lb[RPW], fp[RPW], gb[RPW], dqn[RPW], gy[RPW];
 
   __syncthreads();  // tables and wet state
-  // bottom ghost, first window (setbcc.f90:19-33, advctzc work(1))
+
+  // ------------------------------------------------ the first plane's window
 #pragma unroll
   for (int r = 0; r < RPW; ++r) {
-    const int gj = gy0 + 2 * warp + r;
+    const int gj = gj0 + r, h = h0 + r * px;
+    const float2 z2 = make_float2(0.0f, 0.0f);
+    const bool in = pair_in && row_in(r);
+    rb[r] = lb[r] = fp[r] = gb[r] = gtop[r] = dqn[r] = gy[r] = z2;
+    auto C = [&](int k) { return in ? *reinterpret_cast<const float2*>(cin + h + k * cs) : z2; };
+    auto V = [&](int k) { return in ? ldg2(vkc + h + k * cs) : z2; };
+    const ZTab zt = tab[ts], zm = tab[ts - 1];
+    o0[r] = C(ts);
+    o1[r] = C(ts + 1);
+    vk[r] = V(ts);
+    const float2 pk = mul2(vk[r], o0[r]);
+    sl[r] = mul2(sub2(o1[r], o0[r]), splat(zt.rdz));
+    if (ts == 1) {  // the bottom ghost (setbcc.f90:19-33); work(0,2) = work(1,2)
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      if (!(kin >> (2 * r + c) & 1u)) continue;
-      const int g = gi + c;
-      const int hb = g + px * gj, mb = (g - 1) + nx * (gj - 1);
-      const float c1 = cin[hb + cs], c2 = cin[hb + 2 * cs];
-      const float vk1 = __ldg(vkc + g + hp * gj + hs);
-      float gb;
-      if (vk1 >= 0.0f)
-        gb = 0.0f;
-      else
-        gb = c1 * (1.0f + a.dz[0] * __ldg(a.vdep + (long long)cls * a.dstride + mb) / __ldg(a.rkver1 + mb));
-      cmp(o_0[r], c) = c1;
-      cmp(o_p1[r], c) = c2;
-      cmp(vk0[r], c) = vk1;
-      float w1, w2;
-      zwork(gb, c1, c2, vk1, vk1, tab[1], w1, w2);
-      cmp(w1k[r], c) = w1;
-      cmp(w2k[r], c) = w2;
-      cmp(w2km[r], c) = w2;
-      cmp(rc[r], c) = gb;
-      if (g >= i0 && g <= oi1 && gj >= j0 && gj <= oj1) {
-        cout[hb] = clip0(gb);  // clipped ghost (sizloop.f90:77)
-        if (g == 1 && gj == 1) cout[d.C(0, 0, 0)] = clip0(c1);  // setbcc.f90:87-91
-        if (g == nx && gj == 1) cout[d.C(nx + 1, 0, 0)] = clip0(c1);
-        if (g == 1 && gj == ny) cout[d.C(0, ny + 1, 0)] = clip0(c1);
-        if (g == nx && gj == ny) cout[d.C(nx + 1, ny + 1, 0)] = clip0(c1);
+      for (int c = 0; c < 2; ++c) {
+        const int g = gi + c;
+        if (g < 1 || g > nx || gj < 1 || gj > ny) continue;
+        const int mb = (g - 1) + nx * (gj - 1);
+        const float c1 = cmp(o0[r], c);
+        float b = 0.0f;
+        if (!(cmp(vk[r], c) >= 0.0f))
+          b = c1 * (1.0f + a.dz0 * __ldg(a.vdep + (long long)cls * pl + mb) / __ldg(a.rkver1 + mb));
+        cmp(gb[r], c) = b;
+        if (kout >> (2 * r + c) & 1u) {
+          cout[h + c] = clip0(b);  // clipped ghost (sizloop.f90:77)
+          if (g == 1 && gj == 1) cout[d.C(0, 0, 0)] = clip0(c1);  // setbcc.f90:87-91
+          if (g == nx && gj == 1) cout[d.C(nx + 1, 0, 0)] = clip0(c1);
+          if (g == 1 && gj == ny) cout[d.C(0, ny + 1, 0)] = clip0(c1);
+          if (g == nx && gj == ny) cout[d.C(nx + 1, ny + 1, 0)] = clip0(c1);
+        }
       }
+      // a NaN ghost (0/0 where the diffusivity is 0) counts as a positive
+      // slope that the other one limits, as SIGN and MIN of a NaN do
+      float2 s0 = mul2(sub2(o0[r], gb[r]), splat(zm.rdz));
+      s0 = sel2(isnan(s0.x), isnan(s0.y), splat(__int_as_float(0x7f800000)), s0);
+      w2[r] = mul2(lim_coef_z(vk[r], vk[r], zt.a, zt.b), minmod2(sl[r], s0));
+      gk[r] = mul2(splat(zt.dtdzz), sub2(pk, mul2(vk[r], gb[r])));
+    } else {  // ts >= 3: the planes below are inside the column
+      const float2 cm = C(ts - 1), cmm = C(ts - 2), vm = V(ts - 1), vmm = V(ts - 2);
+      const float2 s1 = mul2(sub2(o0[r], cm), splat(zm.rdz));
+      const float2 s2 = mul2(sub2(cm, cmm), splat(tab[ts - 2].rdz));
+      const float2 w2m = mul2(lim_coef_z(vm, vmm, zm.a, zm.b), minmod2(s1, s2));
+      w2[r] = mul2(lim_coef_z(vk[r], vm, zt.a, zt.b), minmod2(sl[r], s1));
+      gk[r] = fma2(splat(zt.dtdzz), sub2(pk, mul2(vm, cm)), sub2(w2[r], w2m));
     }
+    // the adjacent row's c of plane ts, for a y-face ghost row
+    if (edge && (gj == 0 || gj == ny + 1) && in)
+      gy[r] = *reinterpret_cast<const float2*>(cin + h + (gj == 0 ? px : -px) + ts * cs);
   }
 
   // ------------------------------------------------ one iteration of the march
+  const int kzmax = s_kzmax;
   auto plane = [&](auto edge_c, auto steady_c, const int t) {
     constexpr bool EDGE = decltype(edge_c)::value;
-    constexpr bool STEADY = decltype(steady_c)::value;  // 3 <= t <= nz-2
-    staged(t);
-    // from iteration 3 on, the previous iteration ended with the diffy
-    // barrier, after which no warp reads its advection fields
-    const bool early = STEADY || (t >= 3 && t <= nz);
-    if (early) prefetch(edge_c, t + 1, 0);
-    const float* sb = stage + (t & 1) * (NF * FS) + 2 * warp * RS + sft + 2 * lane;  // this lane's row-0 position
-    auto at = [&](int field, int r) { return sb + field * FS + r * RS; };
-    auto km = [&](int r, int c) { return (kin >> (2 * r + c) & 1u) != 0; };
+    constexpr bool STEADY = decltype(steady_c)::value;  // 3 <= t <= nz-2, plane t-1 is an output plane
+    const int k = t - 1;
+    // ghosts keep their value through the sweeps
+    auto keep = [&](float2 out, float2 in, int r) {
+      if constexpr (EDGE) {
+        if (xedge) out = sel2(gx_0, gx_1, in, out);
+        if (ghost_row(r)) out = in;
+      }
+      return out;
+    };
+    // inner faces of the grid's first and last columns and rows, plane k
+    float ex[RPW];
+    float2 ey[RPW];
+    if constexpr (EDGE) {
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) {
+        const int gj = gj0 + r;
+        ex[r] = 0.0f;
+        ey[r] = make_float2(0.0f, 0.0f);
+        if (k < k0) continue;
+        // gi is even: column 1 is a pair's second
+        if (xedge && (gi == 0 || gi == nx || gi + 1 == nx) && row_in(r))
+          ex[r] = __ldg(a.f.ex + (gi == 0 ? 0 : (nz + 2) * (ny + 2)) + k * (ny + 2) + gj);
+        if ((gj == 1 || gj == ny) && pair_in) ey[r] = ldg2(a.f.ey + (gj == 1 ? 0 : (nz + 2) * px) + k * px + gi);
+      }
+    }
+    const int i = t - ts;
+    const int ba = i % 3;
+    staged(ba, (i / 3) & 1);
+    if constexpr (EDGE) staged(3 + (i & 1), (i >> 1) & 1);
+    // the lane's row-0 pair in the buffers of this iteration
+    const float* sa0 = stage + ba * (NA * FS) + RPW * warp * RS + sft + 2 * lane;
+    const float* sb0 = stage + (3 * NA + (i & 1) * (NF - NA)) * FS + RPW * warp * RS + sft + 2 * lane;
+    auto at = [&](int field, int r) { return (field < NA ? sa0 + field * FS : sb0 + (field - NA) * FS) + r * RS; };
     float2 s2[RPW];
     if (STEADY || t <= nz) {
       float2 s1[RPW];
-      const ZT32 zn = tab[(STEADY || t + 1 <= nz) ? t + 1 : nz];
+      const ZTab zn = tab[(STEADY || t + 1 <= nz) ? t + 1 : nz];
       // ---------------- A: setbcc ghosts + advctzc for plane t
 #pragma unroll
       for (int r = 0; r < RPW; ++r) {
-        const int gj = gy0 + 2 * warp + r;
-        float2 ghost = make_float2(0.0f, 0.0f);
+        const int gj = gj0 + r;
+        float2 gxv = make_float2(0.0f, 0.0f), gyv = gxv;
         if constexpr (EDGE) {
-          // x-face ghosts from the neighbouring column's original c and vx (setbcc.f90:53-66)
-          const float2 cL = left2(o_0[r]), cR = right2(o_0[r]);
-          const float2 vxo = lds2(at(F_VX, r));
-          const float2 vL = left2(vxo), vR = right2(vxo);
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-            cmp(ghost, c) = (gi + c == 0) ? (cmp(vR, c) >= 0.0f ? 0.0f : cmp(cR, c))
-                                          : (cmp(vL, c) <= 0.0f ? 0.0f : cmp(cL, c));
-          if (gj == 0 || gj == ny + 1) {  // y-face ghosts (setbcc.f90:70-83)
-            const int ja = gj == 0 ? 1 : ny;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int g = gi + c;
-              float gv = 0.0f;
-              if (g >= 1 && g <= nx) {
-                const float cadj = cin[g + px * ja + t * cs];
-                const float v = __ldg(a.vyh + g + hp * ja + t * hs);
-                gv = (gj == 0) ? (v >= 0.0f ? 0.0f : cadj) : (v <= 0.0f ? 0.0f : cadj);
-              }
-              cmp(ghost, c) = gv;
-            }
+          if (xedge) {  // x-face ghosts from the neighbouring column's original c; their own ux is the
+                        // neighbour's (setbcc.f90:53-66)
+            const float2 u = lds2(at(F_UX, r));
+            const float cl = shup(o0[r].y);
+            gxv.x = gi == 0 ? (u.x >= 0.0f ? 0.0f : o0[r].y) : (u.x <= 0.0f ? 0.0f : cl);
+            gxv.y = u.y <= 0.0f ? 0.0f : o0[r].x;
+          }
+          if (ghost_row(r)) {  // y-face ghosts (setbcc.f90:70-83)
+            const float2 v = lds2(at(F_UY, r));
+            const bool lo = gj == 0;
+            gyv = sel2(lo ? v.x >= 0.0f : v.x <= 0.0f, lo ? v.y >= 0.0f : v.y <= 0.0f, gyv, gy[r]);
+            if (t < min(te, nz) && pair_in)  // the next plane's
+              gy[r] = *reinterpret_cast<const float2*>(cin + h0 + r * px + (lo ? px : -px) + (t + 1) * cs);
           }
         }
         {  // the column update, on every position
-          float2 w1n, w2n, o_p2 = make_float2(0.0f, 0.0f), vkp = make_float2(0.0f, 0.0f);
+          float2 c2 = make_float2(0.0f, 0.0f), vkp = make_float2(0.0f, 0.0f), gn, w2n = w2[r], sln = sl[r];
           if (STEADY || t + 1 <= nz) {
             vkp = lds2(at(F_VK, r));
             if (STEADY || t + 2 <= nz) {
-              o_p2 = lds2(at(F_C, r));
+              c2 = lds2(at(F_C, r));
             } else {  // the top ghost (setbcc.f90:37-49), vkp = vk(nz)
+              c2 = sel2(vkp.x <= 0.0f, vkp.y <= 0.0f, make_float2(0.0f, 0.0f), o1[r]);
+              gtop[r] = c2;
 #pragma unroll
               for (int c = 0; c < 2; ++c) {
-                cmp(o_p2, c) = (cmp(vkp, c) <= 0.0f) ? 0.0f : cmp(o_p1[r], c);
                 const int g = gi + c;
-                if (g >= i0 && g <= oi1 && gj >= j0 && gj <= oj1) {  // an interior position
-                  const int hb = g + px * gj;
-                  const float top = cmp(o_p1[r], c);
-                  cout[hb + (nz + 1) * cs] = clip0(cmp(o_p2, c));
+                if (kout >> (2 * r + c) & 1u) {
+                  const float top = cmp(o1[r], c);
+                  cout[h0 + r * px + c + (nz + 1) * cs] = clip0(cmp(c2, c));
                   if (g == 1 && gj == 1) cout[d.C(0, 0, nz + 1)] = clip0(top);
                   if (g == nx && gj == 1) cout[d.C(nx + 1, 0, nz + 1)] = clip0(top);
                   if (g == 1 && gj == ny) cout[d.C(0, ny + 1, nz + 1)] = clip0(top);
                   if (g == nx && gj == ny) cout[d.C(nx + 1, ny + 1, nz + 1)] = clip0(top);
                 }
               }
-              gtop[r] = o_p2;
             }
-            zwork2(o_0[r], o_p1[r], o_p2, vkp, vk0[r], zn, w1n, w2n);
-          } else {  // t == nz: work(nz+1,1) (advctzc.f90:58-64)
-            w1n = mul2(mul2(mul2(splat(dt), vk0[r]), sub2(gtop[r], o_0[r])), splat(dznz));
-            w2n = w2k[r];
+            sln = mul2(sub2(c2, o1[r]), splat(zn.rdz));
+            w2n = mul2(lim_coef_z(vkp, vk[r], zn.a, zn.b), minmod2(sln, sl[r]));
+            gn = fma2(splat(zn.dtdzz), sub2(mul2(vkp, o1[r]), mul2(vk[r], o0[r])), sub2(w2n, w2[r]));
+          } else {  // t == nz: work(nz+1,1) (advctzc.f90:58-64), work(nz+1,2) = work(nz,2)
+            gn = mul2(splat(zn.dtrdz), mul2(vk[r], sub2(gtop[r], o0[r])));
           }
-          s1[r] = line_update2(o_0[r], vk0[r], w1k[r], w1n, w2k[r], w2km[r], w2n);
-          w2km[r] = w2k[r];
-          w2k[r] = w2n;
-          w1k[r] = w1n;
-          o_0[r] = o_p1[r];
-          o_p1[r] = o_p2;
-          vk0[r] = vkp;
+          s1[r] = upwind(o0[r], vk[r], gk[r], gn);
+          w2[r] = w2n;
+          sl[r] = sln;
+          gk[r] = gn;
+          o0[r] = o1[r];
+          o1[r] = c2;
+          vk[r] = vkp;
         }
         if constexpr (EDGE) {
-          const unsigned gm = (kgx | kgy) >> (2 * r);
-          s1[r] = sel2(gm & 1u, gm & 2u, ghost, s1[r]);
+          if (xedge) s1[r] = sel2(gx_0, gx_1, gxv, s1[r]);
+          if (ghost_row(r)) s1[r] = gyv;
         }
       }
       // ---------------- B: advctx (shuffles) and advcty (shared memory)
       auto adv_x = [&](const float2* in, float2* out) {
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-          const float2 c0 = in[r];
-          const float2 v = lds2(at(F_VX, r));
-          const float2 cm = left2(c0), cp = right2(c0), vmr = left2(v);
-          float2 w1, w2;
+          const float2 c0 = in[r], u = lds2(at(F_UX, r)), cp = right2(c0);
+          const float2 dc = sub2(cp, c0);
+          const float2 wx = mul2(lds2(at(F_KX, r)), minmod2(dc, left2(dc)));
+          const float2 F = fma2(u, c0, wx);
+          float2 Fl = left2(F);
           if constexpr (EDGE) {
-            const float2 vm = sel2(gi == 1, gi + 1 == 1, v, vmr);  // v(max(1,q-1))
-            line_work2(cm, c0, cp, v, vm, auxvx, a.inv_dx, dt, w1, w2);
-#pragma unroll
-            for (int c = 0; c < 2; ++c)  // work(nx+1,1) (advctx.f90:46)
-              if (gi + c == nx + 1) cmp(w1, c) = auxvx * cmp(vmr, c) * (cmp(c0, c) - cmp(cm, c));
-          } else {
-            line_work2(cm, c0, cp, v, vmr, auxvx, a.inv_dx, dt, w1, w2);
+            if (xedge) {  // work(0,2) = work(1,2) (advctx.f90:48-50)
+              if (gi == 0) Fl.y = __fmaf_rn(u.y, c0.x, wx.y);
+            }
           }
-          const float2 w1p = right2(w1);
-          float2 w2m = left2(w2), w2p = right2(w2);
+          const float2 G = sub2(F, Fl);
+          float2 Gp = right2(G);
           if constexpr (EDGE) {
-            w2m = sel2(gi == 1, gi + 1 == 1, w2, w2m);
-            w2p = sel2(gi == nx, gi + 1 == nx, w2, w2p);
-            const float2 u = line_update2(c0, v, w1, w1p, w2, w2m, w2p);
-            out[r] = sel2(km(r, 0), km(r, 1), u, c0);
-          } else {
-            out[r] = line_update2(c0, v, w1, w1p, w2, w2m, w2p);
+            if (xedge) {  // work(n+1,1), work(n+1,2) = work(n,2) (advctx.f90:46, 52-54)
+              if (gi == nx) Gp.x = __fsub_rn(__fmaf_rn(u.x, cp.x, wx.x), F.x);
+              if (gi + 1 == nx) Gp.y = __fsub_rn(__fmaf_rn(u.y, cp.y, wx.y), F.y);
+            }
           }
+          out[r] = keep(upwind(c0, u, G, Gp), c0, r);
         }
       };
       auto adv_y = [&](const float2* in, float2* out) {
-        float* P0 = P0s + 2 * warp * HX + 2 * lane;
-        float* W1 = W1s + 2 * warp * HX + 2 * lane;
-        float* W2 = W2s + 2 * warp * HX + 2 * lane;
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) sts2(P0 + r * HX, in[r]);
+        float* P0 = P0s + RPW * warp * HX + 2 * lane;
+        float* W = Ws + RPW * warp * HX + 2 * lane;
+        sts2(P0, in[0]);
+        if (RPW > 1) sts2(P0 + (RPW - 1) * HX, in[RPW - 1]);
         __syncthreads();
-        // every thread is past iteration t-1: its staging buffer may be refilled
-        prefetch(edge_c, t + 1, early ? 1 : 2);
-        static_assert(RPW == 2, "a warp owns a pair of adjacent rows");
-        float2 w1s[RPW], w2s[RPW], vs[RPW];
-        // y-neighbours: the rows below and above this lane's pair come from
-        // the neighbouring warps, the rest from its own registers
-        vs[0] = lds2(at(F_VY, 0));
-        vs[1] = lds2(at(F_VY, 1));
-        const float2 cmv[RPW] = {lds2(P0 - HX), in[0]};
-        const float2 cpv[RPW] = {in[1], lds2(P0 + 2 * HX)};
-        const float2 vmv[RPW] = {lds2(at(F_VY, 0) - RS), vs[0]};  // vy(i, j-1)
+        prefetch(ahead ? i + 2 : i + 1);
+        const float2 cb = lds2(P0 - HX), ca = lds2(P0 + RPW * HX);
+        float2 u[RPW], wy[RPW], F[RPW];
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) u[r] = lds2(at(F_UY, r));
+        float2 dl = sub2(in[0], cb);
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-          const int gj = gy0 + 2 * warp + r;
-          const float2 c0 = in[r];
-          const float2 cm = cmv[r], cp = cpv[r];
-          const float2 v = vs[r], vmr = vmv[r];
-          if constexpr (EDGE) {  // row conditions are uniform across the warp
-            line_work2(cm, c0, cp, v, gj == 1 ? v : vmr, auxvy, a.inv_dy, dt, w1s[r], w2s[r]);
-            if (gj == ny + 1) w1s[r] = mul2(mul2(splat(auxvy), vmr), sub2(c0, cm));  // advcty.f90:45
-          } else {
-            line_work2(cm, c0, cp, v, vmr, auxvy, a.inv_dy, dt, w1s[r], w2s[r]);
-          }
+          const float2 dr = sub2(r < RPW - 1 ? in[r + 1] : ca, in[r]);
+          wy[r] = mul2(lds2(at(F_KY, r)), minmod2(dr, dl));
+          F[r] = fma2(u[r], in[r], wy[r]);
+          dl = dr;
         }
-        sts2(W1, w1s[0]);  // the row above the pair below reads it
-        sts2(W2, w2s[0]);
-        sts2(W2 + HX, w2s[1]);
+        sts2(W, F[0]);
+        if (RPW > 1) sts2(W + (RPW - 1) * HX, F[RPW - 1]);
         __syncthreads();
-        const float2 w1pv[RPW] = {w1s[1], lds2(W1 + 2 * HX)};
-        const float2 w2mv[RPW] = {lds2(W2 - HX), w2s[0]};
-        const float2 w2pv[RPW] = {w2s[1], lds2(W2 + 2 * HX)};
+        float2 G[RPW + 1];
+#pragma unroll
+        for (int r = 0; r <= RPW; ++r) {
+          const float2 Fb = r ? F[r - 1] : lds2(W - HX), Fa = r < RPW ? F[r] : lds2(W + RPW * HX);
+          G[r] = sub2(Fa, Fb);
+        }
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-          const float2 w1p = w1pv[r];
-          float2 w2m = w2mv[r], w2p = w2pv[r];
-          if constexpr (EDGE) {
-            const int gj = gy0 + 2 * warp + r;
-            if (gj == 1) w2m = w2s[r];
-            if (gj == ny) w2p = w2s[r];
-            const float2 u = line_update2(in[r], vs[r], w1s[r], w1p, w2s[r], w2m, w2p);
-            out[r] = sel2(km(r, 0), km(r, 1), u, in[r]);
-          } else {
-            out[r] = line_update2(in[r], vs[r], w1s[r], w1p, w2s[r], w2m, w2p);
+          float2 g = G[r], gp = G[r + 1];
+          if constexpr (EDGE) {  // the line's ends, as in x (uniform across the warp)
+            if (gj0 + r == 1) g = sub2(F[r], fma2(u[r], r ? in[r - 1] : cb, wy[r]));
+            if (gj0 + r == ny) gp = sub2(fma2(u[r], r < RPW - 1 ? in[r + 1] : ca, wy[r]), F[r]);
           }
+          out[r] = keep(upwind(in[r], u[r], g, gp), in[r], r);
         }
       };
+      if constexpr (!EDGE) staged(3 + (i & 1), (i >> 1) & 1);
       float2 sa[RPW];
-      if (xfirst) {  // sizloop.f90:42-48
+      if constexpr (XFIRST) {  // sizloop.f90:42-48
         adv_x(s1, sa);
         adv_y(sa, s2);
       } else {
@@ -492,351 +495,424 @@ __device__ __forceinline__ void fused2_tile(const FusedArgs& a, const F2Maps* ma
         adv_x(sa, s2);
       }
     } else {
+      if constexpr (!EDGE) staged(3 + (i & 1), (i >> 1) & 1);
 #pragma unroll
       for (int r = 0; r < RPW; ++r) s2[r] = make_float2(0.0f, 0.0f);
       __syncthreads();  // the y-sweep plane of the previous iteration is read by all warps
     }
-    if (!STEADY && t < 2) {
-#pragma unroll
-      for (int r = 0; r < RPW; ++r) {
-        if (EDGE) gprev[r] = s2[r];  // ghost value of plane t
-        ra[r] = rb[r];
-        rb[r] = rc[r];
-        rc[r] = s2[r];
-        pb[r] = lds2(at(F_PZ, r));  // rkver*rho at plane 1
-      }
-      return;
-    }
-    // ---------------- C: diffz for plane k = t-1 (diffz.f90:22-62)
-    const int k = t - 1;
+    // ---------------- C: diffz for plane k (diffz.f90:22-62)
     float2 s3[RPW], lbv[RPW];
-    const ZT32 zk = tab[k];
+    const ZTab zk = tab[k];
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-      ra[r] = rb[r];
-      rb[r] = rc[r];
-      rc[r] = (STEADY || t <= nz) ? s2[r] : gtop[r];  // c(nz+1) is the top ghost (diffz.f90:54)
-      const float2 lb = lds2(at(F_L1, r));
-      lbv[r] = lb;
-      if (STEADY || (k > 1 && k < nz)) {
-        const float2 lc = lds2(at(F_L, r)), pc = lds2(at(F_PZ, r));
-        s3[r] = diffz_mid2(pc, pb[r], rc[r], lc, rb[r], lb, fprev[r], zk);
-        pb[r] = pc;
-      } else if (k == 1) {
-        const float2 lc = lds2(at(F_L, r)), pc = lds2(at(F_PZ, r));
-        s3[r] = diffz_bottom2(pc, pb[r], rc[r], lc, rb[r], lb, ra[r], fprev[r], tab[0], tab[1]);
-        pb[r] = pc;
-      } else {  // k == nz
-        float2 la, pa;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const bool ok = (inr >> (2 * r + c) & 1u) != 0;
-          const int hh = ok ? gi + c + hp * (gy0 + 2 * warp + r) + (nz - 1) * hs : 0;
-          cmp(la, c) = __ldg(a.lrhoh + hh);
-          cmp(pa, c) = __ldg(a.pkzh + hh);
+      const float2 c0 = rb[r];
+      lbv[r] = lb[r];
+      if (STEADY || t <= nz) {
+        const float2 l = lds2(at(F_L, r)), q = mul2(s2[r], l), qb = mul2(c0, lb[r]);
+        if (STEADY || t > ts) {
+          const float2 dq = sub2(q, qb);
+          const float2 f = mul2(lds2(at(F_FZ, r)), dq);
+          if (STEADY || k > 1) {
+            s3[r] = fma2(splat(zk.dtdzz), sub2(f, fp[r]), c0);
+          } else {  // the bottom cell: its upper face not averaged, the ground face MAX(0, ...)
+            const int h = pair_in && row_in(r) ? h0 + r * px : 0;
+            const float2 up = mul2(ldg2(a.f.ez + h), dq);
+            const float2 lo = max0(mul2(ldg2(a.f.fz + h), sub2(qb, mul2(gb[r], lb[r]))));
+            s3[r] = fma2(splat(zk.dtdzz), sub2(up, lo), c0);
+          }
+          fp[r] = f;
+          if (!STEADY && t == nz) dqn[r] = dq;
         }
-        s3[r] = diffz_top2(pa, la, pb[r], rc[r], rb[r], lb, ra[r], tab[nz - 1], tab[nz]);
+        rb[r] = s2[r];
+        lb[r] = l;
+      } else {  // k == nz: the top face MIN(0, ...) with the ghost c(nz+1) (diffz.f90:50-61)
+        const int h = pair_in && row_in(r) ? h0 + r * px : 0;
+        const float2 up = min0(mul2(ldg2(a.f.fz + h + nz * cs), sub2(mul2(gtop[r], lb[r]), mul2(c0, lb[r]))));
+        const float2 lo = mul2(ldg2(a.f.fz + h + (nz + 1) * cs), dqn[r]);
+        s3[r] = fma2(splat(zk.dtrdz), sub2(up, lo), c0);
       }
-      if constexpr (EDGE) {
-        s3[r] = sel2(km(r, 0), km(r, 1), s3[r], gprev[r]);  // ghosts keep their value
-        gprev[r] = s2[r];
-      }
+      if (STEADY || k >= k0) s3[r] = keep(s3[r], c0, r);
     }
+    if (!STEADY && k < k0) return;
     // ---------------- D: diffx (shuffles) and diffy (shared memory)
     auto dif_x = [&](const float2* in, float2* out) {
 #pragma unroll
       for (int r = 0; r < RPW; ++r) {
-        const float2 l0 = lbv[r], P0 = lds2(at(F_PX, r)), c0 = in[r];
-        // the face flux (P(q)+P(q+1))*(c(q+1)/rho(q+1) - c(q)/rho(q)) is gradr at q and
-        // gradl at q+1 (diffx.f90:34-40): computed once per face, the left one by shuffle
-        const float2 q0 = mul2(c0, l0), qp = right2(q0), Pp = right2(P0);
-        const float2 fr = diff_face2(Pp, P0, qp, q0);
-        float2 u = diff_apply2(dtdx2h, fr, left2(fr), c0);
+        const float2 c0 = in[r], q = mul2(c0, lbv[r]), qp = right2(q);
+        const float2 dq = sub2(qp, q);
+        float2 fr = mul2(lds2(at(F_FX, r)), dq);
         if constexpr (EDGE) {
-          if (xedge) {  // the line's first and last cells (diffx.f90:22-33, 44-55)
-            const float2 cm = left2(c0), cp = right2(c0), qm = left2(q0), Pm = left2(P0);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int g = gi + c;
-              if (g == 1)
-                cmp(u, c) = diff_first_q(cmp(qp, c), cmp(q0, c), cmp(cm, c), cmp(l0, c), cmp(P0, c), cmp(Pp, c),
-                                         cmp(c0, c), dtdx2h);
-              else if (g == nx)
-                cmp(u, c) = diff_last_q(cmp(q0, c), cmp(qm, c), cmp(cp, c), cmp(l0, c), cmp(P0, c), cmp(Pm, c),
-                                        cmp(c0, c), dtdx2h);
-            }
+          if (xedge) {  // the line's end faces MAX(0, ...), MIN(0, ...) (diffx.f90:22-33, 44-55)
+            fr.x = gi == 0 ? fmaxf(fr.x, 0.0f) : gi == nx ? fminf(fr.x, 0.0f) : fr.x;
+            if (gi + 1 == nx) fr.y = fminf(fr.y, 0.0f);
           }
-          u = sel2(km(r, 0), km(r, 1), u, c0);  // ghosts and outside positions keep their value
         }
-        out[r] = u;
+        float2 fl = left2(fr);
+        if constexpr (EDGE) {
+          if (xedge) {  // and the inner faces of the first and last cells
+            const float dm = shup(dq.y);
+            if (gi == 0) fr.y = ex[r] * dq.y;
+            if (gi == nx) fl.x = ex[r] * dm;
+            if (gi + 1 == nx) fl.y = ex[r] * dq.x;
+          }
+        }
+        out[r] = keep(add2(c0, sub2(fr, fl)), c0, r);
       }
     };
     auto dif_y = [&](const float2* in, float2* out) {
-      float* P1 = P1s + 2 * warp * HX + 2 * lane;
-      const float2 P0v[RPW] = {lds2(at(F_PY, 0)), lds2(at(F_PY, 1))};
-      const float2 Pmv[RPW] = {lds2(at(F_PY, 0) - RS), P0v[0]};
-      const float2 Ppv[RPW] = {P0v[1], lds2(at(F_PY, 1) + RS)};
-      // neighbours read c/rho: the products c*(1/rho) of diffy.f90:34-40,
-      // each computed once by its owner; a ghost row (edge tiles) holds c
-      // itself, which is what the line's first and last cells read of it
-      const int gj0 = gy0 + 2 * warp;  // the pair's first row
+      float* P1 = P1s + RPW * warp * HX + 2 * lane;
       float2 q[RPW];
-      bool ghost[RPW];
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) q[r] = mul2(in[r], lbv[r]);
+      sts2(P1, q[0]);
+      if (RPW > 1) sts2(P1 + (RPW - 1) * HX, q[RPW - 1]);
+      __syncthreads();
+      const float2 qm = lds2(P1 - HX), qa = lds2(P1 + RPW * HX);
+      float2 dq[RPW + 1], f[RPW + 1];  // faces gj0-1/2 .. gj0+RPW-1/2
+#pragma unroll
+      for (int r = 0; r <= RPW; ++r) {
+        dq[r] = sub2(r < RPW ? q[r] : qa, r ? q[r - 1] : qm);
+        f[r] = mul2(lds2(at(F_FY, r - 1)), dq[r]);
+      }
 #pragma unroll
       for (int r = 0; r < RPW; ++r) {
-        q[r] = mul2(in[r], lbv[r]);
-        ghost[r] = EDGE && (gj0 + r == 0 || gj0 + r == ny + 1);  // uniform across the warp
-        sts2(P1 + r * HX, ghost[r] ? in[r] : q[r]);
-      }
-      __syncthreads();
-      if constexpr (!EDGE) {
-        const float2 qm[RPW] = {lds2(P1 - HX), q[0]};
-        const float2 qp[RPW] = {q[1], lds2(P1 + 2 * HX)};
-        // three faces: below the pair, between its rows (gradr of row 0 and
-        // gradl of row 1, the same operations on the same values), above it
-        const float2 fb = diff_face2(P0v[0], Pmv[0], q[0], qm[0]);
-        const float2 fm = diff_face2(Ppv[0], P0v[0], qp[0], q[0]);
-        const float2 ft = diff_face2(Ppv[1], P0v[1], qp[1], q[1]);
-        out[0] = diff_apply2(dtdy2h, fm, fb, in[0]);
-        out[1] = diff_apply2(dtdy2h, ft, fm, in[1]);
-      } else {
-        // the stored values of the rows below and above each row
-        const float2 vmv[RPW] = {lds2(P1 - HX), ghost[0] ? in[0] : q[0]};
-        const float2 vpv[RPW] = {ghost[1] ? in[1] : q[1], lds2(P1 + 2 * HX)};
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-          const int gj = gj0 + r;
-          float2 u;
-          if (gj == 1) {  // the first row (diffy.f90:22-33): the row below is the ghost, stored as c
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-              cmp(u, c) = diff_first_q(cmp(vpv[r], c), cmp(q[r], c), cmp(vmv[r], c), cmp(lbv[r], c),
-                                       cmp(P0v[r], c), cmp(Ppv[r], c), cmp(in[r], c), dtdy2h);
-          } else if (gj == ny) {  // the last row (diffy.f90:44-55): the row above is the ghost
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-              cmp(u, c) = diff_last_q(cmp(q[r], c), cmp(vmv[r], c), cmp(vpv[r], c), cmp(lbv[r], c),
-                                      cmp(P0v[r], c), cmp(Pmv[r], c), cmp(in[r], c), dtdy2h);
-          } else {  // an inner row: its two faces
-            u = diff_apply2(dtdy2h, diff_face2(Ppv[r], P0v[r], vpv[r], q[r]), diff_face2(P0v[r], Pmv[r], q[r], vmv[r]),
-                            in[r]);
+        float2 lo = f[r], up = f[r + 1];
+        if constexpr (EDGE) {  // the line's end and inner faces, as in x (uniform across the warp)
+          if (gj0 + r == 1) {
+            lo = max0(lo);
+            up = mul2(ey[r], dq[r + 1]);
           }
-          out[r] = sel2(km(r, 0), km(r, 1), u, in[r]);
+          if (gj0 + r == ny) {
+            lo = mul2(ey[r], dq[r]);
+            up = min0(up);
+          }
         }
+        out[r] = keep(add2(in[r], sub2(up, lo)), in[r], r);
       }
     };
     float2 s3a[RPW], s4[RPW];
-    if (xfirst) {  // sizloop.f90:55-61
+    if constexpr (XFIRST) {  // sizloop.f90:55-61
       dif_x(s3, s3a);
       dif_y(s3a, s4);
     } else {
       dif_y(s3, s3a);
       dif_x(s3a, s4);
     }
-    // ---------------- E: wetdep, accum, clip, store (plane k)
-    const double dzk64 = a.dz64[k];
-    if constexpr (!EDGE && STEADY) {  // interior tile, no accum: predicated stores, no divergence
-      // the pair's columns inside the output tile (columns 3 .. 3+TX-1 of the region)
-      const bool o0 = 2 * lane >= 3 && 2 * lane < 3 + TX, o1 = 2 * lane + 1 >= 3 && 2 * lane + 1 < 3 + TX;
-#pragma unroll
-      for (int r = 0; r < RPW; ++r) {
-        const int hy = 2 * warp + r;
-        if (hy < 3 || hy >= 3 + TY) continue;  // uniform across the warp
-        float2 res = s4[r];
-        if (wet && k <= s_kzmax) {  // uniform across the block
-          const int o = (2 * lane - 3) + TX * (hy - 3);
-          if (o0 && k <= wkz[o]) {  // wetdep (wetdep.f90:37-49)
-            wacc[o] = wacc[o] + dzk64 * wlam[o] * (double)res.x;
-            res.x = (float)((double)res.x * (1.0 - wlam[o]));
-          }
-          if (o1 && k <= wkz[o + 1]) {
-            wacc[o + 1] = wacc[o + 1] + dzk64 * wlam[o + 1] * (double)res.y;
-            res.y = (float)((double)res.y * (1.0 - wlam[o + 1]));
-          }
-        }
-        res = make_float2(clip0(res.x), clip0(res.y));
-        float* q = cout + gi + px * (gy0 + hy) + k * cs;
-        if (P8 && o0 && o1) {
-          *reinterpret_cast<float2*>(q) = res;
-        } else {
-          if (o0) q[0] = res.x;
-          if (o1) q[1] = res.y;
-        }
-      }
-      return;
-    }
+    // ---------------- E: wetdep, accum, clip, store (plane k); ghosts have kept their setbcc value
+    float* const q = cout + (h0 + k * cs);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-      const int hy = 2 * warp + r;
-      const int gj = gy0 + hy;
-      const int hrow = gi + px * gj + k * cs;  // halo index of the first column
       float2 res = s4[r];
-      bool st[2];
+      if (wet && k <= kzmax) {  // uniform across the block; wetdep.f90:37-49
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int g = gi + c;
-        bool out_cell;
-        st[c] = false;
-        if constexpr (EDGE) {
-          const bool rows_out = gj >= j0 && gj <= oj1;
-          const bool cols_out = g >= i0 && g <= oi1;
-          const unsigned bit = 1u << (2 * r + c);
-          if (((kgx & bit) && rows_out && ((g == 0 && i0 == 1) || (g == nx + 1 && oi1 == nx))) ||
-              ((kgy & bit) && cols_out && ((gj == 0 && j0 == 1) || (gj == ny + 1 && oj1 == ny)))) {
-            cmp(res, c) = clip0(cmp(s3[r], c));  // an outer ghost keeps its setbcc value
-            st[c] = true;
-            continue;
-          }
-          out_cell = (kin & bit) && rows_out && cols_out;
-        } else {
-          const int col = 2 * lane + c;
-          out_cell = col >= 3 && col < 3 + TX && hy >= 3 && hy < 3 + TY;
+        for (int c = 0; c < 2; ++c) {
+          const int p2 = (gi + c - 1) + nx * (gj0 + r - 1);
+          if (!(kout >> (2 * r + c) & 1u) || !(a.zlayer[k - 1] <= a.zi[p2])) continue;
+          double* cw = a.cwet + (long long)(cls + 1) * pl + p2;
+          const double lam = a.lambda2d[p2], v = (double)cmp(res, c);
+          if (commit) *cw = *cw + a.dz64[k] * lam * v;
+          cmp(res, c) = (float)(v * (1.0 - lam));
         }
-        if (!out_cell) continue;
-        float cnew = cmp(res, c);
-        if (wet && k <= s_kzmax) {
-          const int o = (g - i0) + TX * (gj - j0);
-          if (k <= wkz[o]) {  // wetdep (wetdep.f90:37-49)
-            wacc[o] = wacc[o] + dzk64 * wlam[o] * (double)cnew;
-            cnew = (float)((double)cnew * (1.0 - wlam[o]));
-          }
-        }
-        if (!STEADY && k == 1 && commit) {  // accum (accum.f90:17-25), binary64
-          const int mb = (g - 1) + nx * (gj - 1);
+      }
+      if (!STEADY && k == 1 && commit) {  // accum (accum.f90:17-25), binary64
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (!(kout >> (2 * r + c) & 1u)) continue;
+          const int mb = (gi + c - 1) + nx * (gj0 + r - 1);
           double* cd = a.cdry + (long long)(cls + 1) * pl + mb;
-          const double vsd = a.vset64[(long long)cls * a.vstride + mb] + a.vdep64[(long long)cls * pl + mb];
-          *cd = *cd - a.dt64 * (double)cnew * fmin2(0.0, vsd);
+          const double vsd = a.vset64[(long long)cls * d.cells() + mb] + a.vdep64[(long long)cls * pl + mb];
+          *cd = *cd - a.dt64 * (double)cmp(res, c) * fmin2(0.0, vsd);
         }
-        cmp(res, c) = clip0(cnew);
-        st[c] = true;
       }
-      if (P8 && st[0] && st[1])
-        *reinterpret_cast<float2*>(cout + hrow) = res;
-      else {
-        if (st[0]) cout[hrow] = res.x;
-        if (st[1]) cout[hrow + 1] = res.y;
-      }
+      res = max0(res);
+      // predicated stores (no divergence): whole pairs, and the single
+      // columns of the two lanes at the tile's sides
+      const unsigned b = kst >> (2 * r) & 3u;
+      float* const o = q + r * px;
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %0, 3;\n\t@p st.global.v2.f32 [%1], {%2, %3};\n\t}" ::"r"(b),
+                   "l"(o), "f"(res.x), "f"(res.y)
+                   : "memory");
+      asm volatile(
+          "{\n\t.reg .pred p, q, s;\n\tsetp.eq.u32 q, %0, 1;\n\tsetp.eq.u32 s, %0, 2;\n\t@q st.global.f32 [%1], %2;\n\t"
+          "@s st.global.f32 [%1+4], %3;\n\t}" ::"r"(b),
+          "l"(o), "f"(res.x), "f"(res.y)
+          : "memory");
     }
   };
 
   auto march = [&](auto edge_c) {
-    for (int t = 1; t <= 2; ++t) plane(edge_c, False_{}, t);
-    for (int t = 3; t <= nz - 2; ++t) plane(edge_c, True_{}, t);
-    for (int t = max(3, nz - 1); t <= nz + 1; ++t) plane(edge_c, False_{}, t);
+    const int t1 = max(3, k0 + 1), t2 = max(t1 - 1, min(te, nz - 2));  // steady: t1..t2
+    for (int t = ts; t < min(t1, te + 1); ++t) plane(edge_c, False_{}, t);
+    // not unrolled: a body of two planes issues 9% fewer instructions (no
+    // moves of the carried values) but misses the instruction cache more
+    // often (400x300x50, 16 classes: 1.014 ms against 0.999 ms)
+#pragma unroll 1
+    for (int t = t1; t <= t2; ++t) plane(edge_c, True_{}, t);
+    for (int t = t2 + 1; t <= te; ++t) plane(edge_c, False_{}, t);
   };
   if (edge)
     march(True_{});
   else
     march(False_{});
 
-  if (wet && commit) {
-    __syncthreads();
-    for (int o = threadIdx.x; o < TX * TY; o += NT) {
-      const int oi = i0 + o % TX, oj = j0 + o / TX;
-      if (oi > oi1 || oj > oj1) continue;
-      a.cwet[(long long)(cls + 1) * pl + (oi - 1) + nx * (oj - 1)] = wacc[o];
+  if (timed_out) {  // a tensor copy did not arrive in time: report, and let copies in flight land
+    atomicOr(a.status, F3D_STEP_STAGING_TIMEOUT);
+    for (int i = max(0, te - ts - 1); i <= te - ts; ++i) {
+      staged(i % 3, (i / 3) & 1);
+      staged(3 + (i & 1), (i >> 1) & 1);
     }
   }
-  {
-    if (timed_out) {  // a tensor copy did not arrive in time: report, and let copies in flight land
-      atomicOr(a.status, F3D_STEP_STAGING_TIMEOUT);
-      mbar_wait(mbar0 + 8u * (unsigned)(nz & 1), (unsigned)(((nz - 1) >> 1) & 1));
-      mbar_wait(mbar0 + 8u * (unsigned)((nz + 1) & 1), (unsigned)((nz >> 1) & 1));
-    }
-    __syncthreads();  // nobody waits on the barriers any more: they may be reused (next batch item)
-    if (threadIdx.x == 0) {
-      asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mbar0) : "memory");
-      asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mbar0 + 8) : "memory");
-    }
+  __syncthreads();  // nobody waits on the barriers any more: they may be reused (next batch item)
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < 5; ++b) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mbar0 + 8u * b) : "memory");
   }
 }
 
-template <bool P8>
-__global__ void __launch_bounds__(NT, 1) k_step_fused2(const FusedArgs a, const __grid_constant__ F2Maps maps) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  fused2_tile<P8>(a, &maps, a.c_in, a.c_out, a.xfirst, 1, (int)(blockIdx.x % a.ncls),
-                        (int)(blockIdx.x / a.ncls), smem_raw);
+template <class S>
+constexpr int min_blocks() {
+  return S::RPW == 1 ? 2 : 1;
 }
 
-// The same step with at most 112 registers, launched while a look-ahead
-// meteo update runs on the context's second stream: four warps of it take
-// 14336 of an SM sub-partition's 16384 registers, which leaves one
-// 64-register warp of the settling-velocity chain room beside it on each
-// sub-partition.  Same operations, same results.
-template <bool P8>
-__global__ void __maxnreg__(112) k_step_fused2_beside(const FusedArgs a, const __grid_constant__ F2Maps maps) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  fused2_tile<P8>(a, &maps, a.c_in, a.c_out, a.xfirst, 1, (int)(blockIdx.x % a.ncls),
-                        (int)(blockIdx.x / a.ncls), smem_raw);
+struct StepMaps {
+  F2Maps met;
+  CMaps c;
+};
+
+template <class S, bool XFIRST>
+__global__ void __launch_bounds__(S::NT, min_blocks<S>())
+    k_step_fused2(const FusedArgs a, const __grid_constant__ StepMaps maps) {
+  const int item = blockIdx.x / a.ncls;
+  step_tile<S, XFIRST>(a, &maps.met, &maps.c, a.c_in, a.c_out, 1, (int)(blockIdx.x % a.ncls), item / a.nchunk,
+                       item % a.nchunk);
 }
 
-// Batched form (see k_step_fused_batch in f3d_fused.cu).  The scenarios with
-// an even nx come first in the batch; their items [0, split) run in the P8
-// kernel, the rest in the other one (counter[0] and counter[1]).
-__constant__ FusedArgs c_batch2[F3D_BATCH_MAX];
+// ------------------------------------------------------------ batched form
+// The step of every scenario of a batch in one persistent launch: the work
+// items are (scenario, tile, piece, class), numbered scenario by scenario
+// (item_off[s] .. item_off[s+1]-1, class fastest); each block takes the next
+// item from a counter until none is left.  A scenario's arguments live in
+// constant memory; its buffers alternate with the number of batch steps it
+// has taken (bstep[s] even: c_in -> c_out, odd: c_out -> c_in), and the x/y
+// order follows iiter = iiter0[s] + bstep[s] + 1 (sizloop.f90:42-48).
+__constant__ FusedArgs c_batch[F3D_BATCH_MAX];
 static_assert(sizeof(FusedArgs) * F3D_BATCH_MAX <= 48 * 1024, "batch argument table exceeds constant memory");
 
-template <bool P8>
-__global__ void __launch_bounds__(NT, 1)
-    k_step_fused2_batch(const int* __restrict__ item_off, int nscen, int begin, int end, int* counter,
-                        const int* __restrict__ bstep, const int* __restrict__ iiter0, int commit,
-                        const F2Maps* __restrict__ maps) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+// a call of its own, so that the two sweep orders do not share registers
+template <class S, bool XFIRST>
+__device__ __noinline__ void step_tile_call(const FusedArgs& a, const F2Maps* maps, const CMaps* cmap,
+                                            const float* c_in, float* c_out, const int commit, const int cls,
+                                            const int tile, const int chunk) {
+  step_tile<S, XFIRST>(a, maps, cmap, c_in, c_out, commit, cls, tile, chunk);
+}
+
+template <class S>
+__global__ void __launch_bounds__(S::NT, min_blocks<S>())
+    k_step_fused2_batch(const int* __restrict__ item_off, int nscen, int* counter, const int* __restrict__ bstep,
+                        const int* __restrict__ iiter0, int commit, const BatchMaps* __restrict__ maps) {
   __shared__ int s_item;
+  __shared__ FusedArgs s_args;
+  const int total = item_off[nscen];
   for (;;) {
     __syncthreads();  // the previous item is done with shared memory
-    if (threadIdx.x == 0) s_item = begin + atomicAdd(counter, 1);
+    if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
     __syncthreads();
     const int item = s_item;
-    if (item >= end) break;
-    int lo = 0, hi = nscen;
+    if (item >= total) break;
+    int lo = 0, hi = nscen;  // item_off[lo] <= item < item_off[hi]
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
       if (item_off[mid] <= item) lo = mid;
       else hi = mid;
     }
-    const FusedArgs& a = c_batch2[lo];
-    const int local = item - item_off[lo];
+    for (int w = threadIdx.x; w < (int)(sizeof(FusedArgs) / 4); w += S::NT)
+      reinterpret_cast<int*>(&s_args)[w] = reinterpret_cast<const int*>(&c_batch[lo])[w];
+    __syncthreads();
+    const FusedArgs& a = s_args;
+    const int local = item - item_off[lo], rest = local / a.ncls;
     const int bs = bstep[lo];
     const float* cin = (bs & 1) ? a.c_out : a.c_in;
     float* cout = (bs & 1) ? const_cast<float*>(a.c_in) : a.c_out;
     const int iiter = iiter0[lo] + bs + 1;
-    fused2_tile<P8>(a, maps + lo, cin, cout, (iiter % 2 == 0) ? 1 : 0, commit, local % a.ncls,
-                          local / a.ncls, smem_raw);
+    const CMaps* cm = (bs & 1) ? &maps[lo].b : &maps[lo].a;
+    const int cls = local % a.ncls, tile = rest / a.nchunk, chunk = rest % a.nchunk;
+    if (iiter % 2 == 0)
+      step_tile_call<S, true>(a, &maps[lo].met, cm, cin, cout, commit, cls, tile, chunk);
+    else
+      step_tile_call<S, false>(a, &maps[lo].met, cm, cin, cout, commit, cls, tile, chunk);
   }
 }
 
-// met field (nx,ny,nz) -> halo layout with row pitch hp
-__global__ void k_to_halo(Dims d, int hp, const float* src, float* dst) {
-  const long long s3 = d.cells();
+// ------------------------------------------------------------ step fields
+// The class-independent fields of the step kernel from a meteo update's
+// binary64 fields, one thread per position of the halo layout (see StepFields
+// for what the ghosts hold).  dt is the update's own, formed as the host
+// does (finddt.f90:58-66).
+__global__ void k_step_fields(Dims d, double safety, double dX1, double dX2, const double* dz,
+                              const unsigned long long* dtcn, const double* vx, const double* vy, const double* rho,
+                              const double* rkh1, const double* rkhor, const double* rkver, StepFields f) {
+  const double dt = safety * (1.0 / fmax2(__longlong_as_double((long long)*dtcn), 1e-13));
+  const int nx = d.nx, ny = d.ny, nz = d.nz, px = d.px;
+  // the divisions once per thread, which takes several positions of its plane
+  const double ax = dt / dX1, ay = dt / dX2, bx = dt / (dX1 * dX1), by = dt / (dX2 * dX2);
+  const int plane = px * (ny + 2), k = blockIdx.y;
+  const double rdz = 1.0 / (k == 0 ? dz[0] : k <= nz ? dz[k] : dz[nz - 1]);
+  for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < plane; h += gridDim.x * blockDim.x) {
+    const int i = h % px, j = h / px;
+    if (h == 0 && k <= nz) {  // this level's factors
+      ZTab z{};
+      const double dk = dz[k], dm = k > 0 ? dz[k - 1] : dz[0], dzz = 2.0 / (dk + dm);
+      z.a = (float)(0.25 * dt * dm * dzz);
+      z.b = (float)(0.125 * dt * dt * dzz);
+      z.rdz = (float)(1.0 / dk);
+      z.dtdzz = (float)(dt * dzz);
+      z.dtrdz = (float)(dt / dk);
+      f.tab[k] = z;
+    }
+    if (i > nx + 1) continue;
+    const int ic = min(max(i, 1), nx), jc = min(max(j, 1), ny);
+    const long long m = d.M(ic, jc, 1), pl = d.plane();
+    const long long o = h + (long long)k * plane;
+    // rkver*rho at a level, for diffz
+    auto Z = [&](int kk) { return rkver[m + (kk - 1) * pl] * rho[m + (kk - 1) * pl]; };
+    if (k == 0 || k > nz) {
+      f.fz[o] = (float)((k == 0 ? Z(1) : Z(nz - 1)) * rdz);
+      if (k == 0) f.ez[h] = (float)(Z(2) / dz[1]);
+      continue;
+    }
+    const long long q = m + (k - 1) * pl;
+    const double r = rho[q];
+    f.ux[o] = (float)(ax * vx[q]);
+    f.uy[o] = (float)(ay * vy[q]);
+    auto K = [](double c) { return (float)(0.5 * c * (1.0 - c)); };
+    if (i >= 1 && i <= nx) f.kx[o] = K(0.5 * ax * absd(vx[q] + vx[i > 1 ? q - 1 : q]));
+    if (j >= 1 && j <= ny) f.ky[o] = K(0.5 * ay * absd(vy[q] + vy[j > 1 ? q - nx : q]));
+    f.l[o] = (float)(1.0 / r);
+    f.fz[o] = (float)((k < nz ? 0.5 * (Z(k) + Z(k + 1)) : Z(nz)) * rdz);
+    const double p = rkh1[q] * r, s = rkhor[q] * r;
+    f.fx[o] = (float)(i >= 1 && i < nx ? 0.5 * bx * (p + rkh1[q + 1] * rho[q + 1]) : bx * p);
+    f.fy[o] = (float)(j >= 1 && j < ny ? 0.5 * by * (s + rkhor[q + nx] * rho[q + nx]) : by * s);
+    if (i == 2) f.ex[(long long)k * (ny + 2) + j] = (float)(bx * p);
+    if (i == nx - 1) f.ex[(long long)(nz + 2) * (ny + 2) + (long long)k * (ny + 2) + j] = (float)(bx * p);
+    if (j == 2) f.ey[(long long)k * px + i] = (float)(by * s);
+    if (j == ny - 1) f.ey[(long long)(nz + 2) * px + (long long)k * px + i] = (float)(by * s);
+  }
+}
+
+// vz + vset per class in the halo layout (the vertical velocity of
+// advctzc.f90:23): every thread keeps vz of its cell through the classes.
+__global__ void k_step_vk(Dims d, int nc, const double* vz, const double* vset, float* vk) {
+  const long long s3 = d.cells(), hb = d.halo();
   for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < s3;
        m += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(m % d.nx) + 1;
     const long long r = m / d.nx;
     const int j = (int)(r % d.ny) + 1, k = (int)(r / d.ny) + 1;
-    dst[i + (long long)hp * (j + (long long)(d.ny + 2) * k)] = src[m];
+    const double w = vz[m];
+    float* o = vk + d.C(i, j, k);
+    for (int c = 0; c < nc; ++c) o[c * hb] = (float)(w + vset[c * s3 + m]);
   }
+}
+
+// wet-deposition rate per column for the fused kernel: lambda =
+// min(dt*a*prate^b, 1) (wetdep.f90:40), constant between meteo updates.
+__global__ void k_wet_lambda(long long n, double dt, const double* prate, double* lam) {
+  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const double aa = 8.4e-5, b = 0.79;
+  lam[p] = fmin2(dt * aa * pow(prate[p], b), 1.0);
+}
+
+int device_sms() {
+  static int nsm = 0;
+  if (!nsm) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return std::max(1, nsm);
+}
+
+// calls f with the tile shape's type
+template <class F>
+auto with_shape(int shape, F f) {
+  return shape == 3 ? f(Tall{}) : f(Flat{});
 }
 
 }  // namespace
 
-void launch_step_fused2(const FusedArgs& a, const F2Maps& maps, cudaStream_t s, int beside) {
-  const int tiles = ((a.d.nx + TX - 1) / TX) * ((a.d.ny + TY - 1) / TY);
-  const size_t sm = fused2_smem(a.d.nz);
-  auto go = [&](auto kernel) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kernel<<<tiles * a.ncls, NT, sm, s>>>(a, maps);
-  };
-  if (a.pair_aligned)
-    beside ? go(k_step_fused2_beside<true>) : go(k_step_fused2<true>);
-  else
-    beside ? go(k_step_fused2_beside<false>) : go(k_step_fused2<false>);
+void launch_wet_lambda(long long n, double dt, const double* prate, double* lam, cudaStream_t s) {
+  k_wet_lambda<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, dt, prate, lam);
+  count_launch();
+}
+
+void launch_step_fields(Dims d, int nc, double safety, double dX1, double dX2, const double* dz,
+                        const unsigned long long* dtcn, const double* vx, const double* vy, const double* vz,
+                        const double* rho, const double* rkh1, const double* rkhor, const double* rkver,
+                        const double* vset, const StepFields& f, cudaStream_t s) {
+  const long long plane = (long long)d.px * (d.ny + 2);
+  // about four blocks per SM over all planes
+  const long long nb = std::max<long long>(1, 4LL * device_sms() / (d.nz + 2));
+  k_step_fields<<<dim3((unsigned)std::min<long long>((plane + 255) / 256, nb), d.nz + 2), 256, 0, s>>>(d, safety, dX1, dX2, dz, dtcn, vx, vy,
+                                                                               rho, rkh1, rkhor, rkver, f);
+  count_launch();
+  launch_step_vk(d, nc, vz, vset, f.vk, s);
+}
+
+void launch_step_vk(Dims d, int nc, const double* vz, const double* vset, float* vk, cudaStream_t s) {
+  const int nb = (int)std::min<long long>((d.cells() + 255) / 256, 152LL * 16);
+  k_step_vk<<<nb, 256, 0, s>>>(d, nc, vz, vset, vk);
+  count_launch();
+}
+
+int fused_tiles(int nx, int ny, int shape) {
+  const int ty = with_shape(shape, [](auto s) { return decltype(s)::TY; });
+  return ((nx + TX - 1) / TX) * ((ny + ty - 1) / ty);
+}
+
+void step_chunks(FusedArgs& a, int shape, int nwet) {
+  const int nz = a.d.nz;
+  a.nchunk = 1;
+  a.kfirst = nz;
+  a.klen = nz;
+  const long long blocks = (long long)fused_tiles(a.d.nx, a.d.ny, shape) * a.ncls;
+  const long long slots = (long long)device_sms() * with_shape(shape, [](auto s) { return min_blocks<decltype(s)>(); });
+  // waves of blocks times iterations of the longest piece (plus ~3 for the start)
+  long long best = ((blocks + slots - 1) / slots) * (nz + 4);
+  for (int n = 2; n <= 16; ++n) {
+    const int len = (nz + n - 1) / n, first = std::max(len, nwet), rest = nz - first;
+    if (len < 4 || rest < 4 * (n - 1)) break;
+    const int each = (rest + n - 2) / (n - 1);
+    if (rest - each * (n - 2) < 4) continue;
+    const long long cost = ((blocks * n + slots - 1) / slots) * (std::max(first + 1, each + 2) + 3);
+    if (cost < best) {
+      best = cost;
+      a.nchunk = n;
+      a.kfirst = first;
+      a.klen = each;
+    }
+  }
+}
+
+void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s) {
+  with_shape(shape, [&](auto sh) {
+    using S = decltype(sh);
+    const size_t sm = step_smem<S>(a.d.nz);
+    StepMaps m;
+    m.met = maps;
+    m.c = c;
+    auto go = [&](auto kernel) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      kernel<<<fused_tiles(a.d.nx, a.d.ny, shape) * a.ncls * a.nchunk, S::NT, sm, s>>>(a, m);
+    };
+    a.xfirst ? go(k_step_fused2<S, true>) : go(k_step_fused2<S, false>);
+    return 0;
+  });
   count_launch();
 }
 
 int fused2_max_nz() {
-  const size_t cap = (size_t)227 * 1024, base = fused2_smem(0);
-  return cap > base ? (int)((cap - base) / sizeof(ZT32)) - 1 : 0;
+  const size_t cap = (size_t)227 * 1024, base = step_smem<Tall>(0);
+  return cap > base ? (int)((cap - base) / sizeof(ZTab)) - 1 : 0;
 }
 
 // cuTensorMapEncodeTiled, reached through the runtime's driver entry point
@@ -845,7 +921,9 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int make_fused2_maps(const FusedArgs& a, F2Maps* out) {
+// the two maps (32- and 16-row boxes) of a field: x (the padded row), y (rows
+// 0..ny+1), z (planes 0..nz+1, times the classes for class blocks)
+static int step_map(Dims d, const float* p, long long planes, CUtensorMap* m32, CUtensorMap* m16) {
   static EncodeTiledFn enc = nullptr;
   if (!enc) {
     void* fn = nullptr;
@@ -856,86 +934,62 @@ int make_fused2_maps(const FusedArgs& a, F2Maps* out) {
       return 1;
     enc = reinterpret_cast<EncodeTiledFn>(fn);
   }
-  const Dims d = a.d;
-  if (a.hpitch % 4 != 0 || a.hpitch < d.nx + 2) return 2;
-  // x (the padded row), y (rows 0..ny+1), z (planes 0..nz+1, times the classes for vz+vset)
-  auto one = [&](CUtensorMap* m, const float* p, long long planes) {
-    const cuuint64_t dim[3] = {(cuuint64_t)a.hpitch, (cuuint64_t)(d.ny + 2), (cuuint64_t)planes};
-    const cuuint64_t stride[2] = {(cuuint64_t)a.hpitch * sizeof(float),
-                                  (cuuint64_t)a.hpitch * (d.ny + 2) * sizeof(float)};
-    const cuuint32_t box[3] = {(cuuint32_t)RS, (cuuint32_t)HY, 1u};
-    const cuuint32_t es[3] = {1u, 1u, 1u};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(p), dim, stride, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
-               ? 0
-               : 3;
-  };
-  const long long np = d.nz + 2;
-  int rc = one(&out->m[F2Maps::VK], a.vkh, np * a.ncls);
-  if (!rc) rc = one(&out->m[F2Maps::VX], a.vxh, np);
-  if (!rc) rc = one(&out->m[F2Maps::VY], a.vyh, np);
-  if (!rc) rc = one(&out->m[F2Maps::L], a.lrhoh, np);
-  if (!rc) rc = one(&out->m[F2Maps::PZ], a.pkzh, np);
-  if (!rc) rc = one(&out->m[F2Maps::PX], a.pkxh, np);
-  if (!rc) rc = one(&out->m[F2Maps::PY], a.pkyh, np);
-  return rc;
+  if (d.px % 4 != 0 || d.px < d.nx + 2) return 2;
+  const cuuint64_t dim[3] = {(cuuint64_t)d.px, (cuuint64_t)(d.ny + 2), (cuuint64_t)planes};
+  const cuuint64_t stride[2] = {(cuuint64_t)d.px * sizeof(float), (cuuint64_t)d.px * (d.ny + 2) * sizeof(float)};
+  const cuuint32_t es[3] = {1u, 1u, 1u};
+  for (int q = 0; q < 2; ++q) {
+    const cuuint32_t box[3] = {(cuuint32_t)RS, q ? 16u : 32u, 1u};
+    if (enc(q ? m16 : m32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(p), dim, stride, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return 3;
+  }
+  return 0;
 }
 
-int upload_batch_args2(const FusedArgs* h, int n, cudaStream_t s) {
+int make_step_maps(const FusedArgs& a, F2Maps* out) {
+  const long long np = a.d.nz + 2;
+  const float* p[F2Maps::N] = {a.f.vk, a.f.ux, a.f.kx, a.f.uy, a.f.ky, a.f.l, a.f.fz, a.f.fx, a.f.fy};
+  for (int f = 0; f < F2Maps::N; ++f)
+    if (int rc = step_map(a.d, p[f], f == F2Maps::VK ? np * a.ncls : np, &out->m[0][f], &out->m[1][f])) return rc;
+  return 0;
+}
+
+int make_c_maps(Dims d, int ncls, const float* c, CMaps* out) {
+  return step_map(d, c, (long long)(d.nz + 2) * ncls, &out->m[0], &out->m[1]);
+}
+
+int upload_batch_args(const FusedArgs* h, int n, cudaStream_t s) {
   if (n > F3D_BATCH_MAX) return 1;
-  return cudaMemcpyToSymbolAsync(c_batch2, h, sizeof(FusedArgs) * (size_t)n, 0, cudaMemcpyHostToDevice, s) ==
+  return cudaMemcpyToSymbolAsync(c_batch, h, sizeof(FusedArgs) * (size_t)n, 0, cudaMemcpyHostToDevice, s) ==
                  cudaSuccess
              ? 0
              : 1;
 }
 
-int fused2_batch_grid(int max_nz) {
-  const size_t sm = fused2_smem(max_nz);
-  if (cudaFuncSetAttribute(k_step_fused2_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_step_fused2_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-          cudaSuccess)
-    return -1;
-  int per_sm = 0, nsm = 0, dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_fused2_batch<true>, NT, sm) != cudaSuccess)
-    return -1;
-  return per_sm < 1 ? -1 : per_sm * nsm;
+int fused_batch_grid(int shape, int max_nz) {
+  return with_shape(shape, [&](auto sh) {
+    using S = decltype(sh);
+    const size_t sm = step_smem<S>(max_nz);
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(k_step_fused2_batch<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_fused2_batch<S>, S::NT, sm) != cudaSuccess)
+      return -1;
+    return per_sm < 1 ? -1 : per_sm * device_sms();
+  });
 }
 
-void launch_step_fused2_batch(int grid, const int* item_off, int nscen, int split, int total, int* counter,
-                              const int* bstep, const int* iiter0, int commit, int max_nz, const F2Maps* maps,
-                              cudaStream_t s, const BatchFork* fork) {
-  const size_t sm = fused2_smem(max_nz);
-  const bool both = split > 0 && total > split && fork && fork->s2;
-  cudaStream_t s_odd = s;
-  if (both) {  // the two parts are independent (their own scenarios and counters)
-    cudaEventRecord(fork->a, s);
-    cudaStreamWaitEvent(fork->s2, fork->a, 0);
-    s_odd = fork->s2;
-  }
-  if (split > 0) {
-    k_step_fused2_batch<true><<<grid, NT, sm, s>>>(item_off, nscen, 0, split, counter, bstep, iiter0, commit, maps);
-    count_launch();
-  }
-  if (total > split) {
-    k_step_fused2_batch<false><<<grid, NT, sm, s_odd>>>(item_off, nscen, split, total, counter + 1, bstep, iiter0,
-                                                         commit, maps);
-    count_launch();
-  }
-  if (both) {
-    cudaEventRecord(fork->b, fork->s2);
-    cudaStreamWaitEvent(s, fork->b, 0);
-  }
-}
-
-void launch_to_halo(Dims d, int hp, int nfield, const float* const* src, float* const* dst, cudaStream_t s) {
-  const int nb = (int)std::min<long long>((d.cells() + 255) / 256, 152LL * 16);
-  for (int f = 0; f < nfield; ++f) {
-    k_to_halo<<<nb, 256, 0, s>>>(d, hp, src[f], dst[f]);
-    count_launch();
-  }
+void launch_step_fused_batch(int shape, int grid, const int* item_off, int nscen, int* counter, const int* bstep,
+                             const int* iiter0, int commit, int max_nz, const BatchMaps* maps, cudaStream_t s) {
+  with_shape(shape, [&](auto sh) {
+    using S = decltype(sh);
+    k_step_fused2_batch<S><<<grid, S::NT, step_smem<S>(max_nz), s>>>(item_off, nscen, counter, bstep, iiter0, commit,
+                                                                    maps);
+    return 0;
+  });
+  count_launch();
 }
 
 }  // namespace f3d

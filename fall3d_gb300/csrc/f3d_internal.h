@@ -167,7 +167,9 @@ void launch_meteo_scale(Dims d, int coord_sys, double dX1, double dX2, const dou
 void launch_setdivu(Dims d, double dX1, double dX2, const double* dz, const double* Hm1,
                     const double* vx, const double* vy, const double* vz, double* divu,
                     cudaStream_t s);
-void launch_reamet_fix(Dims d, int wetdep, double* vz, double* prate, cudaStream_t s);
+// reamet.f90:146, 153; *nwet = max(*nwet, layers with zlayer <= zi at any column)
+void launch_reamet_fix(Dims d, int wetdep, double* vz, double* prate, const double* zi, const double* zlayer,
+                       int* nwet, cudaStream_t s);
 
 // setvset with the cd chain.  Work buffers come from setvset_scratch_bytes.
 size_t setvset_scratch_bytes(Dims d, int np);
@@ -186,6 +188,8 @@ void launch_dmath_eval(int op, long long n, const double* x, double* y, cudaStre
 
 // Conversions for the FP32 form.
 void launch_d2f(float* dst, const double* src, long long n, cudaStream_t s);
-void launch_f2d(double* dst, const float* src, long long n, cudaStream_t s);
+// rows of w values between arrays of different row pitch
+void launch_d2f_rows(float* dst, int dpitch, const double* src, int spitch, int w, long long rows, cudaStream_t s);
+void launch_f2d_rows(double* dst, int dpitch, const float* src, int spitch, int w, long long rows, cudaStream_t s);
 
 }  // namespace f3d

@@ -171,7 +171,7 @@ __global__ void k_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_lo
   const int i = (int)(col % nx) + 1, j = (int)(col / nx) + 1;
   T* cc = c + (long long)blockIdx.y * cstride;
   const T* vs = vset + (long long)blockIdx.y * vstride;
-  const long long cb = d.C(i, j, 0), cs = (long long)(nx + 2) * (ny + 2);
+  const long long cb = d.C(i, j, 0), cs = (long long)d.px * (ny + 2);
   const long long mb = d.M(i, j, 1), ms = (long long)nx * ny;
   auto VK = [&](int k) { return vz[mb + (k - 1) * ms] + vs[mb + (k - 1) * ms]; };
   auto CO = [&](int k) { return cc[cb + k * cs]; };
@@ -336,7 +336,7 @@ __global__ void k_advcty(T* c, long long cstride, int ncls, Dims d, int iz_loc, 
   const size_t n2 = (size_t)(ny + 2) * TI;
   T* base = reinterpret_cast<T*>(smem_raw) + tx;  // [q][TI], this thread's line
   const AdvLine<T> L{base, base + n2, base + 2 * n2, base + 3 * n2, base + 4 * n2, base + 5 * n2, nullptr, nullptr};
-  const long long rowstride = nx + 2;
+  const long long rowstride = d.px;
   const long long cbase = d.C(act ? i : nx, 0, k);
   const long long vb = d.M(act ? i : nx, 1, k) - nx;  // vb + q*nx = vy(i,q,k)
   const T auxv = dt / dy, dth = dt * T(0.5), rdy = T(1) / dy;
@@ -430,7 +430,7 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
   if (col >= (long long)nx * ny) return;
   const int i = (int)(col % nx) + 1, j = (int)(col / nx) + 1;
   T* cc = c + (long long)blockIdx.y * cstride;
-  const long long cb = d.C(i, j, 0), cs = (long long)(nx + 2) * (ny + 2);
+  const long long cb = d.C(i, j, 0), cs = (long long)d.px * (ny + 2);
   const long long mb = d.M(i, j, 1), ms = (long long)nx * ny;
   auto C = [&](int k) { return cc[cb + k * cs]; };
   auto R = [&](int k) { return rho[mb + (k - 1) * ms]; };
@@ -620,7 +620,7 @@ __global__ void k_diffy(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
   T* cv = fk + n2;
   T* cl = cv + n2;
   T* ff = cl + n2;
-  const long long rowstride = nx + 2;
+  const long long rowstride = d.px;
   const long long base = d.C(act ? i : nx, 0, k);
   const DiffSrc<T> src{lrp, pkp, rho, rkh, d.M(act ? i : nx, 1, k), nx};
   if (act)
@@ -872,10 +872,25 @@ __global__ void k_d2f(float* dst, const double* src, long long n) {
        q += (long long)gridDim.x * blockDim.x)
     dst[q] = (float)src[q];
 }
-__global__ void k_f2d(double* dst, const float* src, long long n) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x)
-    dst[q] = (double)src[q];
+// the same between arrays of rows of different pitch
+template <class D, class S>
+__global__ void k_convert_rows(D* dst, int dpitch, const S* src, int spitch, int w, long long rows) {
+  const int lane = threadIdx.x & 31;
+  for (long long r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8LL)
+    for (int i = lane; i < w; i += 32) dst[r * dpitch + i] = (D)src[r * spitch + i];
+}
+template <class D, class S>
+static void convert_rows(D* dst, int dpitch, const S* src, int spitch, int w, long long rows, cudaStream_t s) {
+  if (rows <= 0) return;
+  k_convert_rows<D, S><<<(int)std::min<long long>((rows + 7) / 8, 152LL * 16), 256, 0, s>>>(dst, dpitch, src, spitch,
+                                                                                         w, rows);
+  count_launch();
+}
+void launch_d2f_rows(float* dst, int dpitch, const double* src, int spitch, int w, long long rows, cudaStream_t s) {
+  convert_rows(dst, dpitch, src, spitch, w, rows, s);
+}
+void launch_f2d_rows(double* dst, int dpitch, const float* src, int spitch, int w, long long rows, cudaStream_t s) {
+  convert_rows(dst, dpitch, src, spitch, w, rows, s);
 }
 void launch_d2f(float* dst, const double* src, long long n, cudaStream_t s) {
   if (n <= 0) return;
@@ -883,13 +898,6 @@ void launch_d2f(float* dst, const double* src, long long n, cudaStream_t s) {
   k_d2f<<<nb, 256, 0, s>>>(dst, src, n);
   count_launch();
 }
-void launch_f2d(double* dst, const float* src, long long n, cudaStream_t s) {
-  if (n <= 0) return;
-  const int nb = (int)std::min<long long>((n + 255) / 256, 152LL * 16);
-  k_f2d<<<nb, 256, 0, s>>>(dst, src, n);
-  count_launch();
-}
-
 // ---------------------------------------------------- instantiations
 #define F3D_INST(T)                                                                              \
   template void launch_setbcc<T>(T*, long long, Dims, int, int, const T*, const T*, const T*,    \

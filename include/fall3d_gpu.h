@@ -554,9 +554,9 @@ int f3d_ctx_restore(f3d_ctx* ctx, const char* path);
                             with a decreasing zlayer or >= 2^31 cells per
                             class always use the per-routine kernels.     */
 #define F3D_OPT_TILE  2  /* fused kernel tile region x by y / threads:
-                            0 = 32x32/256, 1 = 32x64/512, 2 = 32x32/512,
-                            3 = 64x32/512 with two columns per lane
-                            (default); results do not depend on it       */
+                            0, 1, 2 = 64x16/512, 3 = 64x32/512 (default),
+                            with two columns per lane; results do not
+                            depend on it                                   */
 #define F3D_OPT_GRAPH 3  /* batches: 1 = replay one CUDA graph per batch step
                             (default), 0 = launch the kernels one by one   */
 #define F3D_OPT_PREFETCH 4 /* f3d_run: 1 = compute the next DBS snapshot's
