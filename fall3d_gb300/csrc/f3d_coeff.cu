@@ -727,15 +727,16 @@ static ChainGeom chain_geom(Dims d, int np) {
 
 static constexpr int kBadCap = 8192;
 
+// The regions of launch_setvset's scratch, each on a 256-byte boundary (so
+// that what a caller puts behind them is aligned too).
+static constexpr size_t region(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+
 size_t setvset_scratch_bytes(Dims d, int np) {
   const ChainGeom g = chain_geom(d, np);
-  size_t b = sizeof(ClassConst) * (size_t)(np + 1);
-  b += 2 * sizeof(double) * (size_t)g.nseg + sizeof(int) * (size_t)g.nseg;
-  b += sizeof(int) * (kBadCap + 8) + 1024;
-  b += sizeof(int) * 256 + sizeof(unsigned long long) + 512;  // per-SM claims, segment counter
-  b += sizeof(double) * (size_t)d.cells() + 256;      // viscosity per cell
-  b += 2 * sizeof(double) * (size_t)d.cells() + 256;  // Ganser cell factors
-  return b;
+  return region(sizeof(ClassConst) * (size_t)(np + 1)) + 2 * region(sizeof(double) * (size_t)g.nseg) +
+         region(sizeof(int) * (size_t)g.nseg) + region(sizeof(int) * 8) + region(sizeof(int) * kBadCap) +
+         region(sizeof(double) * (size_t)d.cells()) + region(2 * sizeof(double) * (size_t)d.cells()) +
+         region(sizeof(int) * 256) + region(sizeof(unsigned long long));
 }
 
 void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const double* rhop,
@@ -747,7 +748,7 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
   unsigned char* p = reinterpret_cast<unsigned char*>(scratch);
   auto take = [&](size_t bytes) {
     unsigned char* r = p;
-    p += (bytes + 255) & ~size_t(255);
+    p += region(bytes);
     return r;
   };
   ClassConst* cc = reinterpret_cast<ClassConst*>(take(sizeof(ClassConst) * (size_t)(np + 1)));

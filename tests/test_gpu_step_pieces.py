@@ -73,3 +73,30 @@ def test_batch_of_pieces_equals_alone():
         f = g.fields()
         for k in ("c", "cdry", "cwet"):
             assert_same_bits(f[k], ref[k], k)
+
+
+@pytest.mark.parametrize("nx,ny,nz,nc", [(3, 3, 3, 1), (7, 5, 13, 3), (40, 30, 20, 12), (33, 31, 29, 5)])
+@pytest.mark.parametrize("modv", [1, 2, 3, 4])
+def test_setvset_segments(nx, ny, nz, nc, modv):
+    """The settling chain through the fine-grained entry point on sizes whose
+    chain has one, an odd and an even number of segments, with a short last
+    one (what the call keeps behind the segments' arrays must stay aligned),
+    against the oracle: the velocities to 1e-12, the chain's exit value too."""
+    import oracle_lib as O
+
+    r = np.random.default_rng(nx + nz)
+    T = r.uniform(215.0, 300.0, (nz, ny, nx)).astype(np.float32).astype(float)
+    rho = r.uniform(0.05, 1.25, (nz, ny, nx)).astype(np.float32).astype(float)
+    diam = np.round(2.0 ** -np.linspace(-2.0, 6.0, nc), 6) / 1e3
+    rhop, sphe = np.linspace(2500.0, 1000.0, nc), np.full(nc, 0.9)
+    psi = synth.setpsi(modv, sphe, diam)
+    v = np.zeros((nc, nz, ny, nx))
+    cd = F.setvset(nx, ny, nz, nc, nc, modv, diam, rhop, psi, sphe, T, rho, 0, 1.0, v, 1.0)
+    s = synth.make_scenario("tiny", seed=1, nx=nx, ny=ny, nz=nz, nc=nc, modv=modv)
+    s.grid.update(diam=diam, rhop=rhop, sphe=sphe, psi=psi)
+    s.met["t"][0], s.met["rho"][0] = T, rho
+    o = O.OracleCtx(s)
+    o.meteo(0)
+    ref = o.fields()["vset"]
+    assert np.max(np.abs(v / ref - 1.0)) <= 1e-12
+    assert abs(cd / o.state()["cd"] - 1.0) <= 1e-12
