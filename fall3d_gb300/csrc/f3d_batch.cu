@@ -158,7 +158,7 @@ int enqueue_step(f3d_batch* b, int commit_only_fused) {
   launch_step_fused_batch(b->shape, b->grid, b->d_item_off, n, b->d_counter, b->d_bstep, b->d_iiter0,
                           commit_only_fused ? 0 : 1, b->max_nz, b->d_maps, b->stream);
   if (!commit_only_fused) {
-    launch_cmass2d_batch(b->d_aux, b->d_bstep, n, b->d_red, b->stream);
+    launch_cmass2d_batch(b->d_aux, b->d_bstep, n, b->cap, b->d_red, b->stream);
     launch_batch_advance(b->d_bstep, n, b->stream);
   }
   return F3D_OK;
@@ -220,6 +220,7 @@ int f3d_batch_create(int max_scenarios, f3d_batch** out) {
   ok = ok && cudaMalloc(&b->d_iiter0, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_counter, sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_red, cmass2d_batch_scratch_bytes(n)) == cudaSuccess;
+  ok = ok && cudaMemsetAsync(b->d_red, 0, cmass2d_batch_scratch_bytes(n), b->stream) == cudaSuccess;  // block counters
   ok = ok && cudaMallocHost(&b->h_aux, sizeof(BatchAux) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_args, sizeof(FusedArgs) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_maps, sizeof(BatchMaps) * n) == cudaSuccess;

@@ -21,58 +21,47 @@ int reduce_blocks(long long n) {
   return (int)std::max<long long>(1, std::min<long long>((n + RB - 1) / RB, RMAXB));
 }
 
+// Sum of n DDs p[0], p[stride], ... by one warp (all lanes call it; lane 0 has
+// the sum): each lane adds its share in order, then the lanes' sums are added
+// pairwise.  A double-double addition is about 12 binary64 operations, of
+// which an SM issues two lanes per clock, so a block's reduction is left to
+// one warp per sum instead of a shuffle tree in every warp (n = 256: 13
+// additions issued instead of 47).
+__device__ __forceinline__ DD warp_sum_dd(const DD* p, int n, int stride) {
+  const int lane = threadIdx.x & 31;
+  DD v = dd_zero();
+  for (int q = lane; q < n; q += 32) v = dd_add(v, p[(long long)q * stride]);
+  for (int off = 16; off > 0; off >>= 1) v = dd_add(v, dd_shfl_down(v, off));
+  return v;
+}
+
+// The block's NS sums of its threads' v into partial[blockIdx.x * NS ...]
 template <int NS>
-__device__ void block_store_dd(DD (&v)[NS], DD* partial) {
-  __shared__ DD sh[RB / 32][NS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+__device__ void block_store_dd(const DD (&v)[NS], DD* partial) {
+  __shared__ DD sh[NS * RB];
+  const int wid = threadIdx.x >> 5;
 #pragma unroll
-  for (int s = 0; s < NS; ++s)
-    for (int off = 16; off > 0; off >>= 1) v[s] = dd_add(v[s], dd_shfl_down(v[s], off));
-  if (lane == 0)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) sh[wid][s] = v[s];
+  for (int s = 0; s < NS; ++s) sh[s * RB + threadIdx.x] = v[s];
   __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      DD a = sh[0][s];
-      for (int w = 1; w < RB / 32; ++w) a = dd_add(a, sh[w][s]);
-      partial[(long long)blockIdx.x * NS + s] = a;
-    }
+  if (wid < NS) {
+    const DD a = warp_sum_dd(sh + wid * RB, RB, 1);
+    if ((threadIdx.x & 31) == 0) partial[(long long)blockIdx.x * NS + wid] = a;
   }
 }
 
-// Sums nblk partials of NS sums; out[s] = (hi(sum_s) * f0) * f1, or with
-// accum, out[s] = out[s] + hi(sum_s) (outmass = outmass + sum(mymass),
-// cmass2d.f90:104).
+// Sums nblk partials of NS sums, a warp per sum; out[s] = (hi(sum_s) * f0) *
+// f1, or with accum, out[s] = out[s] + hi(sum_s) (outmass = outmass +
+// sum(mymass), cmass2d.f90:104).
 template <int NS>
 __global__ void k_reduce_finish(const DD* partial, int nblk, double f0, double f1, double* out,
                                 int accum) {
-  DD v[NS];
-#pragma unroll
-  for (int s = 0; s < NS; ++s) v[s] = dd_zero();
-  for (int b = threadIdx.x; b < nblk; b += RB)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) v[s] = dd_add(v[s], partial[(long long)b * NS + s]);
-  __shared__ DD sh[RB / 32][NS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int s = 0; s < NS; ++s)
-    for (int off = 16; off > 0; off >>= 1) v[s] = dd_add(v[s], dd_shfl_down(v[s], off));
-  if (lane == 0)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) sh[wid][s] = v[s];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      DD a = sh[0][s];
-      for (int w = 1; w < RB / 32; ++w) a = dd_add(a, sh[w][s]);
-      if (accum)
-        out[s] = out[s] + a.hi;
-      else
-        out[s] = a.hi * f0 * f1;
-    }
+  const int s = threadIdx.x >> 5;
+  const DD a = warp_sum_dd(partial + s, nblk, NS);
+  if ((threadIdx.x & 31) == 0) {
+    if (accum)
+      out[s] = out[s] + a.hi;
+    else
+      out[s] = a.hi * f0 * f1;
   }
 }
 }  // namespace
@@ -120,16 +109,18 @@ __device__ __forceinline__ DD ds_dd(DS a) {
   return DD{hi, a.e - (hi - a.s)};
 }
 
-// the terms of one side-face cell, classes in order: +-(w*conc)
+// the terms of one side-face cell, classes in order: +-(w*conc); eight
+// classes' loads in flight at a time
+constexpr int CB = 8;
 template <class T>
 __device__ __forceinline__ void face_terms(const T* cc, long long hb, int nc_loc, double w, int side,
                                            DS& acc) {
-  for (int q0 = 0; q0 < nc_loc; q0 += 4) {
-    T cv[4];
+  for (int q0 = 0; q0 < nc_loc; q0 += CB) {
+    T cv[CB];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) cv[u] = q0 + u < nc_loc ? cc[(q0 + u) * hb] : T(0);
+    for (int u = 0; u < CB; ++u) cv[u] = q0 + u < nc_loc ? cc[(q0 + u) * hb] : T(0);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < CB; ++u) {
       if (cv[u] == T(0)) continue;
       const double t = w * (double)cv[u];
       ds_add(acc, side ? t : -t);
@@ -137,24 +128,31 @@ __device__ __forceinline__ void face_terms(const T* cc, long long hb, int nc_loc
   }
 }
 
-// Block sum of the threads' accumulators into partial[blockIdx.x]; a warp
-// whose accumulators are all zero contributes an exact zero without the
-// binary64 shuffle reduction.
-__device__ void block_store_ds(DS a, DD* partial) {
-  __shared__ DD sh[RB / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// Block sum of the threads' accumulators by the first warp (valid in its lane
+// 0); a block whose accumulators are all zero contributes an exact zero
+// without the binary64 reduction.
+__device__ DD block_sum_ds(DS a) {
+  __shared__ DD sh[RB];
+  sh[threadIdx.x] = ds_dd(a);
   DD v = dd_zero();
-  if (__any_sync(0xffffffffu, a.s != 0.0 || a.e != 0.0)) {
-    v = ds_dd(a);
-    for (int off = 16; off > 0; off >>= 1) v = dd_add(v, dd_shfl_down(v, off));
-  }
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
+  if (__syncthreads_or(a.s != 0.0 || a.e != 0.0) && threadIdx.x < 32) v = warp_sum_dd(sh, RB, 1);
+  return v;
+}
+
+// Stores the block's sum; the last of nblk blocks to do so (counted in *done,
+// which wraps to 0 for the next launch) adds them all to *out.
+__device__ void sum_and_finish(DD v, DD* partial, int blk, int nblk, unsigned* done, double* out) {
+  __shared__ bool last;
   if (threadIdx.x == 0) {
-    DD r = sh[0];
-    for (int w = 1; w < RB / 32; ++w) r = dd_add(r, sh[w]);
-    partial[blockIdx.x] = r;
+    partial[blk] = v;
+    __threadfence();
+    last = atomicInc(done, (unsigned)nblk - 1u) == (unsigned)nblk - 1u;
   }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  const DD a = warp_sum_dd(partial, nblk, 1);
+  if (threadIdx.x == 0) *out = *out + a.hi;  // outmass = outmass + sum (cmass2d.f90:104)
 }
 
 template <class T>
@@ -178,12 +176,12 @@ __device__ __forceinline__ void cmass2d_item(int u, const Cm2Items& it, const T*
     const double w = vz[m];
     const double* vs = vset + (long long)(ic_loc - 1) * s3 + m;
     const T* cc = c0 + d.C(i, j, nz + 1);
-    for (int q0 = 0; q0 < nc_loc; q0 += 4) {
-      T cv[4];
+    for (int q0 = 0; q0 < nc_loc; q0 += CB) {
+      T cv[CB];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) cv[u] = q0 + u < nc_loc ? cc[(q0 + u) * hb] : T(0);
+      for (int u = 0; u < CB; ++u) cv[u] = q0 + u < nc_loc ? cc[(q0 + u) * hb] : T(0);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < CB; ++u) {
         if (cv[u] == T(0)) continue;  // an exact zero term (finite velocities)
         const double velo = w + vs[(q0 + u) * s3];
         ds_add(acc, da * velo * (double)cv[u]);
@@ -220,20 +218,24 @@ template <class T>
 __global__ void k_cmass2d(const T* c, const double* vx, const double* vy, const double* vz,
                           const double* vset, Dims d, int ic_loc, int nc_loc, int iz_loc,
                           int nz_loc, double dx, double dy, const double* dz, double dt,
-                          DD* partial) {
+                          DD* partial, unsigned* done, double* out) {
   const Cm2Items it = cm2_items(d, iz_loc, nz_loc);
   const int ntot = it.nT + it.nX + it.nY;
   DS acc{0.0, 0.0};
   for (int u = blockIdx.x * RB + threadIdx.x; u < ntot; u += gridDim.x * RB)
     cmass2d_item<T>(u, it, c, vx, vy, vz, vset, d, ic_loc, nc_loc, iz_loc, nz_loc, dx, dy, dz, dt,
                     acc);
-  block_store_ds(acc, partial);
+  const DD v = block_sum_ds(acc);
+  if (done)
+    sum_and_finish(v, partial, blockIdx.x, gridDim.x, done, out);
+  else if (threadIdx.x == 0)
+    partial[blockIdx.x] = v;
 }
 
 // Batched form: scenario blockIdx.y, its outflow summed over gridDim.x
 // blocks; the step's result is in the buffer the fused kernel wrote
 // (bstep even: c_b, odd: c_a).
-__global__ void k_cmass2d_batch(const BatchAux* tab, const int* bstep, DD* partial) {
+__global__ void k_cmass2d_batch(const BatchAux* tab, const int* bstep, DD* partial, unsigned* done) {
   const BatchAux& b = tab[blockIdx.y];
   const float* c = (bstep[blockIdx.y] & 1) ? b.c_a : b.c_b;
   const Dims d = b.d;
@@ -243,25 +245,8 @@ __global__ void k_cmass2d_batch(const BatchAux* tab, const int* bstep, DD* parti
   for (int u = blockIdx.x * RB + threadIdx.x; u < ntot; u += gridDim.x * RB)
     cmass2d_item<float>(u, it, c, b.vx, b.vy, b.vz, b.vset, d, 1, b.nc, 1, d.nz, b.dX1, b.dX2, b.dz,
                         b.dt, acc);
-  block_store_ds(acc, partial + (long long)blockIdx.y * gridDim.x);
-}
-
-// outmass = outmass + sum (cmass2d.f90:104), one block per scenario
-__global__ void k_cmass2d_batch_finish(const BatchAux* tab, const DD* partial, int nblk) {
-  const DD* p = partial + (long long)blockIdx.x * nblk;
-  DD v[1] = {dd_zero()};
-  for (int b = threadIdx.x; b < nblk; b += RB) v[0] = dd_add(v[0], p[b]);
-  __shared__ DD sh[RB / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int off = 16; off > 0; off >>= 1) v[0] = dd_add(v[0], dd_shfl_down(v[0], off));
-  if (lane == 0) sh[wid] = v[0];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    DD a = sh[0];
-    for (int w = 1; w < RB / 32; ++w) a = dd_add(a, sh[w]);
-    double* out = tab[blockIdx.x].outmass;
-    *out = *out + a.hi;
-  }
+  sum_and_finish(block_sum_ds(acc), partial + (long long)blockIdx.y * gridDim.x, blockIdx.x, gridDim.x,
+                 done + blockIdx.y, b.outmass);
 }
 
 size_t cmass2d_scratch_bytes(Dims d, int iz_loc, int nz_loc) {
@@ -273,14 +258,17 @@ template <class T>
 void launch_cmass2d(const T* c, const double* vx, const double* vy, const double* vz,
                     const double* vset, Dims d, int ic_loc, int nc_loc, int iz_loc, int nz_loc,
                     double dx, double dy, const double* dz, double dt, void* scratch,
-                    double* out, cudaStream_t s) {
+                    double* out, cudaStream_t s, unsigned* done) {
   const Cm2Items it = cm2_items(d, iz_loc, nz_loc);
   const int nb = reduce_blocks((long long)it.nT + it.nX + it.nY);
   DD* partial = reinterpret_cast<DD*>(scratch);
   k_cmass2d<T><<<nb, RB, 0, s>>>(c, vx, vy, vz, vset, d, ic_loc, nc_loc, iz_loc, nz_loc, dx, dy, dz,
-                                 dt, partial);
-  k_reduce_finish<1><<<1, RB, 0, s>>>(partial, nb, 1.0, 1.0, out, 1);
-  count_launch(2);
+                                 dt, partial, done, out);
+  count_launch();
+  if (!done) {
+    k_reduce_finish<1><<<1, 32, 0, s>>>(partial, nb, 1.0, 1.0, out, 1);
+    count_launch();
+  }
 }
 
 // ----------------------------------------------------------- cmass3d
@@ -329,7 +317,7 @@ void launch_cmass3d(const T* c, const double* cload, const double* cdry, const d
   const int nb = reduce_blocks(n);
   DD* partial = reinterpret_cast<DD*>(scratch);
   k_cmass3d<T><<<nb, RB, 0, s>>>(c, cload, cdry, cwet, d, nc, dz, partial);
-  k_reduce_finish<4><<<1, RB, 0, s>>>(partial, nb, dx, dy, out, 0);
+  k_reduce_finish<4><<<1, 128, 0, s>>>(partial, nb, dx, dy, out, 0);
   count_launch(2);
 }
 
@@ -435,15 +423,19 @@ void launch_finddt(Dims d, int nc, double dX1, double dX2, const double* dz, con
   count_launch();
 }
 
-size_t cmass2d_batch_scratch_bytes(int nscen) { return sizeof(DD) * (size_t)nscen * 64 + 256; }
+constexpr int CM2_BATCH_BLOCKS = 64;  // per scenario
 
-void launch_cmass2d_batch(const BatchAux* tab, const int* bstep, int nscen, void* scratch,
+size_t cmass2d_batch_scratch_bytes(int nscen) {
+  return (sizeof(DD) * CM2_BATCH_BLOCKS + sizeof(unsigned)) * (size_t)nscen + 256;
+}
+
+void launch_cmass2d_batch(const BatchAux* tab, const int* bstep, int nscen, int cap, void* scratch,
                           cudaStream_t s) {
   if (nscen <= 0) return;
   DD* partial = reinterpret_cast<DD*>(scratch);
-  k_cmass2d_batch<<<dim3(64, nscen), RB, 0, s>>>(tab, bstep, partial);
-  k_cmass2d_batch_finish<<<nscen, RB, 0, s>>>(tab, partial, 64);
-  count_launch(2);
+  unsigned* done = reinterpret_cast<unsigned*>(partial + (size_t)cap * CM2_BATCH_BLOCKS);
+  k_cmass2d_batch<<<dim3(CM2_BATCH_BLOCKS, nscen), RB, 0, s>>>(tab, bstep, partial, done);
+  count_launch();
 }
 
 // ------------------------------------------------ non-finite values
@@ -481,10 +473,10 @@ template void launch_count_nonfinite<double>(const double*, long long, unsigned 
 
 template void launch_cmass2d<double>(const double*, const double*, const double*, const double*,
                                      const double*, Dims, int, int, int, int, double, double,
-                                     const double*, double, void*, double*, cudaStream_t);
+                                     const double*, double, void*, double*, cudaStream_t, unsigned*);
 template void launch_cmass2d<float>(const float*, const double*, const double*, const double*,
                                     const double*, Dims, int, int, int, int, double, double,
-                                    const double*, double, void*, double*, cudaStream_t);
+                                    const double*, double, void*, double*, cudaStream_t, unsigned*);
 template void launch_cmass3d<double>(const double*, const double*, const double*, const double*,
                                      Dims, int, double, double, const double*, void*, double*,
                                      cudaStream_t);

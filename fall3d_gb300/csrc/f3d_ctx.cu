@@ -50,6 +50,7 @@ int* small_step_status(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 26
 double* small_pref_cd(f3d_ctx* x) { return x->small + 32; }
 unsigned long long* small_pref_dtcn(f3d_ctx* x) { return reinterpret_cast<unsigned long long*>(x->small + 33); }
 int* small_pref_status(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 34); }
+unsigned* small_done(f3d_ctx* x) { return reinterpret_cast<unsigned*>(x->small + 44); }  // cmass2d's block counter
 // the highest wet level of an update and of the look-ahead one
 int* small_nwet(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 17); }
 int* small_pref_nwet(f3d_ctx* x) { return reinterpret_cast<int*>(x->small + 35); }
@@ -368,7 +369,7 @@ void sizloop(f3d_ctx* x) {
   {
     ProfScope ps(x, "cmass2d");
     launch_cmass2d<T>(c, x->vx, x->vy, x->vz, x->vset, d, 1, nc, 1, nz, x->g.dX1, x->g.dX2, x->dz,
-                      x->dt, x->red_scratch, small_outmass(x), s);
+                      x->dt, x->red_scratch, small_outmass(x), s, small_done(x));
   }
 }
 
@@ -389,7 +390,7 @@ void sizloop_fused(f3d_ctx* x) {
   {
     ProfScope ps(x, "cmass2d");
     launch_cmass2d<float>(x->c32, x->vx, x->vy, x->vz, x->vset, d, 1, nc, 1, d.nz, x->g.dX1,
-                          x->g.dX2, x->dz, x->dt, x->red_scratch, small_outmass(x), s);
+                          x->g.dX2, x->dz, x->dt, x->red_scratch, small_outmass(x), s, small_done(x));
   }
 }
 

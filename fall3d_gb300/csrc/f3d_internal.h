@@ -114,8 +114,9 @@ struct BatchAux {
 };
 void launch_setsrc_batch(const BatchAux* tab, const int* bstep, int nscen, int max_nc, int max_nsou,
                          cudaStream_t s);
-size_t cmass2d_batch_scratch_bytes(int nscen);
-void launch_cmass2d_batch(const BatchAux* tab, const int* bstep, int nscen, void* scratch,
+// scratch for up to cap scenarios (cmass2d_batch_scratch_bytes(cap) bytes, zero before the first launch)
+size_t cmass2d_batch_scratch_bytes(int cap);
+void launch_cmass2d_batch(const BatchAux* tab, const int* bstep, int nscen, int cap, void* scratch,
                           cudaStream_t s);
 void launch_batch_advance(int* bstep, int nscen, cudaStream_t s);
 
@@ -126,12 +127,14 @@ size_t reduce_scratch_bytes(long long nterms, int nsums);
 // face cells (class independent), so size it from the grid, not the classes.
 size_t cmass2d_scratch_bytes(Dims d, int iz_loc, int nz_loc);
 // Outflow of one step: *out = *out + sum of the terms of cmass2d.f90:42-102
-// (out is the device copy of outmass).
+// (out is the device copy of outmass).  done: a device counter that is 0
+// before the launch (and after it), with which the last block adds the block
+// sums; without one a second kernel does.
 template <class T>
 void launch_cmass2d(const T* c, const double* vx, const double* vy, const double* vz,
                     const double* vset, Dims d, int ic_loc, int nc_loc, int iz_loc, int nz_loc,
                     double dx, double dy, const double* dz, double dt, void* scratch,
-                    double* out, cudaStream_t s);
+                    double* out, cudaStream_t s, unsigned* done = nullptr);
 // out[0..3] = massvol, massdep, massdry, masswet of cmass3d.f90:29-58.
 template <class T>
 void launch_cmass3d(const T* c, const double* cload, const double* cdry, const double* cwet,
