@@ -16,11 +16,11 @@
 // few tens of cells; any segment that fails the check is recomputed in order
 // from the verified exit of its predecessor.
 //
-// The drag iteration is binary64-pipe bound on GB300, so its Ganser form is
-// restated with one division, one reciprocal square root and a table-driven
-// log/exp per iteration (f3d_dmath.cuh) in place of the reference's four
-// divisions, square root and pow: the same iteration and stopping test on
-// values that differ from the reference's by a few ulp.
+// The drag iteration is binary64-pipe bound on GB300 (two lanes per SM and
+// clock), so its Ganser form is restated to issue about 26 binary64 operations
+// (GanserCell) in place of the reference's four divisions, square root and
+// pow: the same iteration and stopping test on values that differ from the
+// reference's by a few ulp.
 #include <algorithm>
 
 #include "f3d_dmath.cuh"
@@ -29,19 +29,17 @@
 namespace f3d {
 
 // ------------------------------------------------------------- kappa3
-// Sources/kappa3.f90:50-236, one thread per cell.
-__device__ void k3_similarity_grad(Dims d, int i, int j, int k, const double* dz,
-                                   const double* vx, const double* vy, const double* vptemp,
-                                   double& dvdz2, double& rich) {
-  const double gi = 9.81;
-  const double dzs = dz[k] + dz[k - 1];
-  const double gx = (vx[d.M(i, j, k + 1)] - vx[d.M(i, j, k - 1)]) / dzs;
-  const double gy = (vy[d.M(i, j, k + 1)] - vy[d.M(i, j, k - 1)]) / dzs;
-  dvdz2 = gx * gx + gy * gy;
-  dvdz2 = fmax2(dvdz2, 1e-10);
-  rich = gi * ((vptemp[d.M(i, j, k + 1)] - vptemp[d.M(i, j, k - 1)]) / (dz[k] + dz[k - 1])) /
-         (vptemp[d.M(i, j, k)] * dvdz2);
-}
+// Sources/kappa3.f90:50-236.  A thread takes K3_LEV levels of a column: what
+// depends on the column alone (the power of RAMS, the divisors) is formed once
+// and divisions by a column's or a level's divisor use its reciprocal
+// (div_rn_recip: the same quotient), since binary64 operations bound it
+// (400x300x50 cells: 2.61 ms one cell per thread, 1.51 ms so).
+constexpr int K3_LEV = 10, K3_B = 128;
+
+struct K3Level {  // of level k (kappa3.f90:64-96)
+  double zl, dzs, rdzs;  // zlayer, dz(k)+dz(k-1) and its reciprocal
+  double lc;             // 1/(1/(vkarm*zl) + 1/rlamb)
+};
 
 __global__ void k_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv0, double rkh0,
                          double Csh, double dX1, double dX2, double dx, double dy,
@@ -50,106 +48,113 @@ __global__ void k_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv
                          const double* ustar, const double* zi, const double* rl,
                          double* rkver, double* rkhor) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const long long s3 = d.cells();
-  const long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (m >= s3) return;
-  const int i = (int)(m % nx) + 1;
-  const int j = (int)((m / nx) % ny) + 1;
-  const int k = (int)(m / ((long long)nx * ny)) + 1;
-  const long long p = d.P(i, j);
   const double vkarm = 0.4, beta1 = 9.2, beta2 = 13.0, rlamb = 30.0, rkhmin = 1e2, rkvmin = 1.0;
-  const double hinf = 5.0, hsup = 5e3, alfa = 0.28, Khf = 8000.0;
-  // vertical
-  if (modkv == 0) {
-    rkver[m] = rkv0;
-  } else if (modkv == 1) {
-    if (k >= 2) {
-      double dvdz2, rich;
-      // at k = nz the reference reuses the values of the last point computed
-      // at k = nz-1, i.e. (nx, ny, nz-1) (kappa3.f90:64-71)
-      if (k < nz)
-        k3_similarity_grad(d, i, j, k, dz, vx, vy, vptemp, dvdz2, rich);
-      else
-        k3_similarity_grad(d, nx, ny, nz - 1, dz, vx, vy, vptemp, dvdz2, rich);
-      const double h = fmin2(fmax2(zi[p], hinf), hsup);
-      const double zl = zlayer[k - 1];
-      const double zeta = zl / h;
-      double kv;
-      if (zeta < 1.0) {
-        if (rl[p] >= 0.0)
-          kv = vkarm * ustar[p] * zl * (1.0 - zeta) / (1.0 + beta1 * zl * rl[p]);
-        else
-          kv = vkarm * ustar[p] * zl * (1.0 - zeta) * sqrt(1.0 - beta2 * zl * rl[p]);
-      } else {
-        const double lc = 1.0 / ((1.0 / (vkarm * zl)) + (1.0 / rlamb));
-        if (rich >= 0.0) {
-          kv = lc * lc * sqrt(dvdz2) / (1.0 + 10.0 * rich * (1.0 + 8.0 * rich));
-          kv = fmax2(kv, rkvmin);
+  const double hinf = 5.0, hsup = 5e3, alfa = 0.28, Khf = 8000.0, gi = 9.81;
+  const int k0 = blockIdx.y * K3_LEV + 1, k1 = min(nz, k0 + K3_LEV - 1);
+  __shared__ K3Level lev[K3_LEV + 1];  // levels k0-1 .. (k0-1: only for k = nz, below)
+  if (threadIdx.x <= K3_LEV) {
+    const int k = k0 - 1 + threadIdx.x;
+    if (k >= 1 && k <= nz) {
+      K3Level z;
+      z.zl = zlayer[k - 1];
+      z.dzs = dz[k] + dz[k - 1];
+      z.rdzs = 1.0 / z.dzs;
+      z.lc = 1.0 / ((1.0 / (vkarm * z.zl)) + (1.0 / rlamb));
+      lev[threadIdx.x] = z;
+    }
+  }
+  __syncthreads();
+  const long long p = blockIdx.x * (long long)K3_B + threadIdx.x, pl = d.plane();
+  if (p >= pl) return;
+  const int i = (int)(p % nx) + 1, j = (int)(p / nx) + 1;
+  // shear and Richardson number of cell (a,b) at level k < nz (kappa3.f90:64-71)
+  auto grad = [&](long long q, int k, double& dvdz2, double& rich) {
+    const K3Level& z = lev[k - k0 + 1];
+    const long long m = q + (k - 1) * pl;
+    const double gx = div_rn_recip(vx[m + pl] - vx[m - pl], z.dzs, z.rdzs);
+    const double gy = div_rn_recip(vy[m + pl] - vy[m - pl], z.dzs, z.rdzs);
+    dvdz2 = gx * gx + gy * gy;
+    dvdz2 = fmax2(dvdz2, 1e-10);
+    rich = gi * div_rn_recip(vptemp[m + pl] - vptemp[m - pl], z.dzs, z.rdzs) / (vptemp[m] * dvdz2);
+  };
+  const double us = ustar[p], rlp = rl[p];
+  const double h = fmin2(fmax2(zi[p], hinf), hsup), rh = 1.0 / h;
+  const double dXX = Hm1[p] * dX1;
+  const double ddx = i == 1 || i == nx ? dXX : 2.0 * dXX, rddx = 1.0 / ddx;
+  const double ddy = j == 1 || j == ny ? dX2 : 2.0 * dX2, rddy = 1.0 / ddy;
+  const double Kmh = modkh == 1 ? 0.075 * pow(dXX * dX2, 2.0 / 3.0) : 0.0;
+  const long long e = i == nx ? p : p + 1, w = i == 1 ? p : p - 1;
+  const long long n = j == ny ? p : p + nx, s = j == 1 ? p : p - nx;
+  for (int k = k0; k <= k1; ++k) {
+    const long long o = (k - 1) * pl, m = p + o;
+    const double zl = lev[k - k0 + 1].zl;
+    // vertical
+    if (modkv == 0) {
+      rkver[m] = rkv0;
+    } else if (modkv == 1) {
+      if (k >= 2) {
+        const double zeta = div_rn_recip(zl, h, rh);
+        double kv;
+        if (zeta < 1.0) {
+          if (rlp >= 0.0)
+            kv = vkarm * us * zl * (1.0 - zeta) / (1.0 + beta1 * zl * rlp);
+          else
+            kv = vkarm * us * zl * (1.0 - zeta) * sqrt(1.0 - beta2 * zl * rlp);
         } else {
-          kv = lc * lc * sqrt(dvdz2) * sqrt(1.0 - 18.0 * rich);
+          double dvdz2, rich;
+          // at k = nz the reference reuses the values of the last point
+          // computed at k = nz-1, i.e. (nx, ny, nz-1) (kappa3.f90:64-71)
+          if (k < nz)
+            grad(p, k, dvdz2, rich);
+          else
+            grad(pl - 1, nz - 1, dvdz2, rich);
+          const double lc = lev[k - k0 + 1].lc;
+          if (rich >= 0.0)
+            kv = lc * lc * sqrt(dvdz2) / (1.0 + 10.0 * rich * (1.0 + 8.0 * rich));
+          else
+            kv = lc * lc * sqrt(dvdz2) * sqrt(1.0 - 18.0 * rich);
           kv = fmax2(kv, rkvmin);
         }
+        rkver[m] = kv;
       }
-      rkver[m] = kv;
+    } else if (modkv == 2) {
+      const double gh = 11.6, betah = 7.8, prt = 0.95;
+      double zeta = zl * rlp;
+      double kv;
+      if (zeta < 0.0)
+        kv = vkarm * us * zl * sqrt(1.0 - gh * zeta) / prt;
+      else if (zeta > 0.0)
+        kv = vkarm * us * zl / (prt + betah * zeta);
+      else
+        kv = vkarm * us * zl / prt;
+      zeta = div_rn_recip(zl, h, rh);
+      if (zeta > 1.0) zeta = 1.0;
+      rkver[m] = kv * (1.0 - zeta);
     }
-  } else if (modkv == 2) {
-    const double gh = 11.6, betah = 7.8, prt = 0.95;
-    const double zl = zlayer[k - 1], us = ustar[p];
-    double zeta = zl * rl[p];
-    double kv;
-    if (zeta < 0.0)
-      kv = vkarm * us * zl * sqrt(1.0 - gh * zeta) / prt;
-    else if (zeta > 0.0)
-      kv = vkarm * us * zl / (prt + betah * zeta);
-    else
-      kv = vkarm * us * zl / prt;
-    const double h = fmin2(fmax2(zi[p], hinf), hsup);
-    zeta = zl / h;
-    if (zeta > 1.0) zeta = 1.0;
-    rkver[m] = kv * (1.0 - zeta);
-  }
-  // horizontal
-  if (modkh == 0) {
-    rkhor[m] = rkh0;
-  } else if (modkh == 1 || modkh == 2) {
-    const double dXX = Hm1[p] * dX1;
-    double dvxdx, dvydx, dvxdy, dvydy;
-    if (i == 1) {
-      dvxdx = (vx[d.M(2, j, k)] - vx[d.M(1, j, k)]) / dXX;
-      dvydx = (vy[d.M(2, j, k)] - vy[d.M(1, j, k)]) / dXX;
-    } else if (i == nx) {
-      dvxdx = (vx[d.M(nx, j, k)] - vx[d.M(nx - 1, j, k)]) / dXX;
-      dvydx = (vy[d.M(nx, j, k)] - vy[d.M(nx - 1, j, k)]) / dXX;
-    } else {
-      dvxdx = (vx[d.M(i + 1, j, k)] - vx[d.M(i - 1, j, k)]) / (2.0 * dXX);
-      dvydx = (vy[d.M(i + 1, j, k)] - vy[d.M(i - 1, j, k)]) / (2.0 * dXX);
+    // horizontal
+    if (modkh == 0) {
+      rkhor[m] = rkh0;
+    } else if (modkh == 1 || modkh == 2) {
+      const double dvxdx = div_rn_recip(vx[e + o] - vx[w + o], ddx, rddx);
+      const double dvydx = div_rn_recip(vy[e + o] - vy[w + o], ddx, rddx);
+      const double dvxdy = div_rn_recip(vx[n + o] - vx[s + o], ddy, rddy);
+      const double dvydy = div_rn_recip(vy[n + o] - vy[s + o], ddy, rddy);
+      double kh;
+      if (modkh == 1) {
+        const double s1 = dvxdy + dvydx;
+        kh = Csh * Csh * dXX * dX2 * sqrt(s1 * s1 + 2.0 * (dvxdx * dvxdx + dvydy * dvydy));
+        kh = 1.0 * fmax2(kh, Kmh);
+        kh = fmax2(kh, rkhmin);
+      } else {
+        const double Khn0 = (coord_sys == 0) ? 3.6e-2 : 4000.0;
+        const double s1 = dvxdx - dvydy, s2 = dvydx + dvxdy;
+        const double Kht = alfa * alfa * dXX * dX2 * sqrt(s1 * s1 + s2 * s2);
+        const double Khn = Khf * (Khn0 / Hm1[p] / dx) * (Khn0 / dy);
+        kh = (1.0 / Kht) + (1.0 / Khn);
+        kh = fmax2(1.0 / kh, rkhmin);
+      }
+      rkhor[m] = kh;
     }
-    if (j == 1) {
-      dvxdy = (vx[d.M(i, 2, k)] - vx[d.M(i, 1, k)]) / dX2;
-      dvydy = (vy[d.M(i, 2, k)] - vy[d.M(i, 1, k)]) / dX2;
-    } else if (j == ny) {
-      dvxdy = (vx[d.M(i, ny, k)] - vx[d.M(i, ny - 1, k)]) / dX2;
-      dvydy = (vy[d.M(i, ny, k)] - vy[d.M(i, ny - 1, k)]) / dX2;
-    } else {
-      dvxdy = (vx[d.M(i, j + 1, k)] - vx[d.M(i, j - 1, k)]) / (2.0 * dX2);
-      dvydy = (vy[d.M(i, j + 1, k)] - vy[d.M(i, j - 1, k)]) / (2.0 * dX2);
-    }
-    double kh;
-    if (modkh == 1) {
-      const double Kmh = 0.075 * pow(dXX * dX2, 2.0 / 3.0);
-      const double s1 = dvxdy + dvydx;
-      kh = Csh * Csh * dXX * dX2 * sqrt(s1 * s1 + 2.0 * (dvxdx * dvxdx + dvydy * dvydy));
-      kh = 1.0 * fmax2(kh, Kmh);
-      kh = fmax2(kh, rkhmin);
-    } else {
-      const double Khn0 = (coord_sys == 0) ? 3.6e-2 : 4000.0;
-      const double s1 = dvxdx - dvydy, s2 = dvydx + dvxdy;
-      const double Kht = alfa * alfa * dXX * dX2 * sqrt(s1 * s1 + s2 * s2);
-      const double Khn = Khf * (Khn0 / Hm1[p] / dx) * (Khn0 / dy);
-      kh = (1.0 / Kht) + (1.0 / Khn);
-      kh = fmax2(1.0 / kh, rkhmin);
-    }
-    rkhor[m] = kh;
   }
 }
 
@@ -158,10 +163,9 @@ void launch_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv0, dou
                    const double* zlayer, const double* Hm1, const double* vx, const double* vy,
                    const double* vptemp, const double* ustar, const double* zi, const double* rl,
                    double* rkver, double* rkhor, cudaStream_t s) {
-  const long long n = d.cells();
-  k_kappa3<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(d, modkv, modkh, coord_sys, rkv0, rkh0, Csh,
-                                                      dX1, dX2, dx, dy, dz, zlayer, Hm1, vx, vy,
-                                                      vptemp, ustar, zi, rl, rkver, rkhor);
+  k_kappa3<<<dim3((unsigned)((d.plane() + K3_B - 1) / K3_B), (d.nz + K3_LEV - 1) / K3_LEV), K3_B, 0, s>>>(
+      d, modkv, modkh, coord_sys, rkv0, rkh0, Csh, dX1, dX2, dx, dy, dz, zlayer, Hm1, vx, vy, vptemp, ustar, zi, rl,
+      rkver, rkhor);
   count_launch();
 }
 
@@ -339,11 +343,9 @@ void launch_reamet_fix(Dims d, int wetdep, double* vz, double* prate, const doub
 struct ClassConst {
   double diam, rhop, psi;
   double num;       // 4*gi*diam*rhop, the numerator of setvset.f90:104
-  double rk1, rk2;  // Ganser shape factors (setvset.f90:127-128)
-  double rk12;      // rk1 * rk2
-  double sqnum;     // sqrt(num)
-  double drk12;     // diam * rk1 * rk2
   double cd100;     // Wilson
+  // Ganser: sqrt(num); num^(1/2)*diam*rk1*rk2; 24*rk2/that; rk2*24*0.1118; rk2*0.4305; rk2
+  double ft, fg, fi, fp, fq, rk2;
   int ok;           // get_gama converged
 };
 
@@ -380,61 +382,82 @@ __global__ void k_class_consts(int np, int modv, const double* diam, const doubl
   k.rhop = rhop[ic];
   k.psi = psi[ic];
   k.num = 4.0 * gi * k.diam * k.rhop;
-  k.rk1 = k.rk2 = k.rk12 = k.sqnum = k.drk12 = k.cd100 = 0.0;
+  k.cd100 = k.ft = k.fg = k.fi = k.fp = k.fq = k.rk2 = 0.0;
   k.ok = 1;
   if (modv == 2) {
     double gama;
     if (get_gama_dev(k.diam, sphe[ic], gama) < 0) k.ok = 0;
     // gama**(-2.0/3.0): binary32 exponent (setvset.f90:120)
     const double dnd = 0.5 * (1.0 + gama) * pow(gama, (double)(-2.0f / 3.0f));
-    k.rk1 = 1.0 / (dnd / 3.0 + 2.0 / (3.0 * sqrt(k.psi)));
+    const double rk1 = 1.0 / (dnd / 3.0 + 2.0 / (3.0 * sqrt(k.psi)));
     k.rk2 = pow(10.0, 1.8148 * pow(-log10(k.psi), 0.5743));
-    k.rk12 = k.rk1 * k.rk2;
-    k.sqnum = sqrt(k.num);
-    k.drk12 = k.diam * k.rk12;
+    k.ft = sqrt(k.num);
+    // ft*diam*rk1*rk2 and 24*rk2/that rounded once (products and quotient in
+    // double-double): their errors would be the same in every cell of a class
+    double h = k.ft * k.diam, l = fma(k.ft, k.diam, -h);
+    for (const double f : {rk1, k.rk2}) {
+      const double p = h * f;
+      l = fma(h, f, -p) + l * f;
+      h = p;
+    }
+    k.fg = h + l;
+    l = l - (k.fg - h);
+    const double n = 24.0 * k.rk2, q = n / k.fg;
+    k.fi = q + (fma(-q, k.fg, n) + fma(24.0, k.rk2, -n) - q * l) / k.fg;
+    k.fp = k.rk2 * (24.0 * 0.1118);
+    k.fq = k.rk2 * 0.4305;
   } else if (modv == 3) {
     k.cd100 = 0.24 * pow(k.psi, -0.828) + 2.0 * sqrt(1.0 - k.psi);
   }
   cc[ic] = k;
 }
 
-// Sources/setvset.f90:65-181 for one call; returns iterations (0 for the
-// closed-form Dellino model) or -1 when maxit is reached.
-//
-// Ganser (setvset.f90:117-136): with R = rey*rk1*rk2 = G*v,
-// G = (rhoa/visc)*(diam*rk1*rk2), and v = T/sqrt(cd),
-// T = sqrt(4*gi*diam*rhop)*sqrt(1/(3*rhoa)),
+// A Ganser call (setvset.f90:117-136) between iterations.  With
+// R = rey*rk1*rk2 = G*v and v = T/sqrt(cd),
 //   cd = 24/(rey*rk1)*(1 + 0.1118*R^0.6567) + 0.4305*rk2/(1 + 3305/R)
-//      = rk2*((24*(R + 3305) + 0.4305*R^2)/(R*(R + 3305)) + 24*0.1118*R^(0.6567-1)).
-// The cell factors sqrt(1/(3*rhoa)) and rhoa/visc come from k_visc
-// (shared by all classes): cf.x, cf.y.
-__device__ int vsettl_dev(const ClassConst& k, int model, double rhoa, double visc, double2 cf,
-                          double& cd, double& vset, const DMathTab& tab) {
+//      = rk2*(24*0.1118*R^(0.6567-1) + 24/R + 0.4305*R/(R + 3305)),
+// and 24/R = 24/(G*T)*cd*(1/sqrt(cd)).  y = 1/sqrt(cd) is carried: it gives
+// v, R and 24/R of an iteration, the result T*y after the last one, and the
+// next call's first v.  The cell's factors come from k_visc (cf.x =
+// sqrt(1/(3*rhoa)), cf.y = cf.x*rhoa/visc, ci = 1/cf.y), the class's from
+// k_class_consts.
+struct GanserCell {
+  double T, g, i;  // v = T*y, R = g*y, rk2*24/R = i*(cd*y)
+};
+__device__ __forceinline__ bool mid_range(double x) {  // 2^-1000 <= x < 2^1000 (positive)
+  return (unsigned)(__double2hiint(x) - 0x01700000) < 0x7d000000u;
+}
+// an argument outside the fast functions' ranges
+__device__ __noinline__ double ganser_cd_slow(double rk2, double R) {
+  const double Q = R + 3305.0, N = fma(0.4305 * R, R, 24.0 * Q);
+  return rk2 * fma(24.0 * 0.1118, pow(R, kPowA), N / (R * Q));
+}
+static __device__ __noinline__ double rsqrt_slow(double x) { return rsqrt(x); }
+__device__ __forceinline__ double ganser_rsqrt(double cd) { return mid_range(cd) ? rsqrt_fast(cd) : rsqrt_slow(cd); }
+__device__ __forceinline__ void ganser_step(const ClassConst& k, const GanserCell& c, const PowTab& tab, double& cd,
+                                            double& y, double& v) {
+  v = c.T * y;
+  const double R = c.g * y;
+  if (pow_in_range(R) && mid_range(cd)) {
+    const double u = R * rcp_fast(R + 3305.0);
+    cd = fma(k.fp, pow_a(tab, R), fma(k.fq, u, c.i * (cd * y)));
+  } else {
+    cd = ganser_cd_slow(k.rk2, R);
+  }
+  y = ganser_rsqrt(cd);
+}
+// |v - vold| <= 1e-3 on the magnitude bits (the same order for non-negative
+// values; a NaN difference is above it as in binary64)
+__device__ __forceinline__ bool ganser_done(double v, double vold) {
+  return (__double_as_longlong(v - vold) & 0x7fffffffffffffffLL) <= __double_as_longlong(1e-3);
+}
+
+// Sources/setvset.f90:65-181 for one call of the other drag models; returns
+// iterations (0 for the closed-form Dellino model) or -1 when maxit is
+// reached.
+__device__ int vsettl_dev(const ClassConst& k, int model, double rhoa, double visc, double& cd, double& vset) {
   const double eps = 1e-3;
   double vold = 1e5, v = 0.0;
-  if (model == 2) {
-    const double T = k.sqnum * cf.x;
-    const double G = cf.y * k.drk12;
-    for (int it = 1; it <= 100; ++it) {
-      v = T * rsqrt(cd);
-      const double R = G * v;
-      const double L = dm_log(tab, R);
-      const double P = dm_exp(tab, fma(0.6567, L, -L));  // R^0.6567 / R
-      const double Q = R + 3305.0;
-      const double N = fma(0.4305 * R, R, 24.0 * Q);
-      cd = k.rk2 * fma(24.0 * 0.1118, P, N / (R * Q));
-      // |v - vold| <= eps on the magnitude bits (the same order for
-      // non-negative values; a NaN difference is above eps as in binary64)
-      const long long dvb = __double_as_longlong(v - vold) & 0x7fffffffffffffffLL;
-      if (it > 1 && dvb <= __double_as_longlong(eps)) {
-        vset = T * rsqrt(cd);
-        return it;
-      }
-      vold = v;
-    }
-    vset = v;
-    return -1;
-  }
   if (model == 4) {
     const double gi = 9.81, diam = k.diam;
     v = pow((diam * diam * diam * gi * (k.rhop - rhoa) * rhoa * pow(k.psi, 1.6)) / (visc * visc),
@@ -494,103 +517,175 @@ __device__ __forceinline__ void chain_cell(const ChainGeom& g, long long q, int&
 __device__ __forceinline__ double sutherland(double T) {
   const double visc0 = 1.827e-5;
   const double Tair0 = (double)291.15f;  // default-real literal (setvset.f90:23)
-  return visc0 * ((Tair0 + 120.0) / (T + 120.0)) * pow(T / Tair0, 1.5);
+  const double t = T / Tair0;
+  return visc0 * ((Tair0 + 120.0) / (T + 120.0)) * (t * sqrt(t));  // t**1.5
 }
 
 // The air viscosity of every cell, shared by all classes (setvset.f90:95-97),
-// and the Ganser iteration's cell factors sqrt(1/(3*rho)), rho/visc.
-__global__ void k_visc(long long s3, const double* tempe, const double* rho, double* visc, double2* cf) {
+// or for the Ganser iteration (model 2) its cell factors: with
+// f = sqrt(1/(3*rho)) and g = f*rho/visc, cf = (f, g) and 1/g in visc.
+__global__ void k_visc(long long s3, int modv, const double* tempe, const double* rho, double* visc, double2* cf) {
   for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < s3;
        m += (long long)gridDim.x * blockDim.x) {
     const double vs = sutherland(tempe[m]), r = rho[m];
-    visc[m] = vs;
-    cf[m] = make_double2(sqrt(1.0 / (3.0 * r)), r / vs);
+    if (modv == 2) {
+      const double f = sqrt(1.0 / (3.0 * r)), g = f * r / vs;
+      cf[m] = make_double2(f, g);
+      visc[m] = 1.0 / g;
+    } else {
+      visc[m] = vs;
+    }
   }
 }
 
-// Runs chain cells [q0, q1) from cd; writes outputs when `write`.
-__device__ void chain_run(const ChainGeom& g, long long q0, long long q1, int modv,
-                          const ClassConst* cc, const double* viscs, const double2* cf, const double* rho,
-                          double* vset, int* iters, double& cd, bool write, int& nonconv,
-                          const DMathTab& tab) {
+// What a chain run reads and writes.
+struct ChainIO {
+  const ClassConst* cc;
+  const double* visc;
+  const double2* cf;
+  const double* rho;
+  double* vset;
+  int* iters;
+};
+
+// Runs chain cells [q0, q1) from cd; writes -vset (setvset.f90:60) and the
+// iteration counts when `write`.
+__device__ void chain_run(const ChainGeom& g, long long q0, long long q1, int modv, const ChainIO& io, double& cd,
+                          bool write, int& nonconv) {
   const long long s3 = g.d.cells();
   for (long long q = q0; q < q1; ++q) {
     int ic;
     long long m;
     chain_cell(g, q, ic, m);
-    const double visc = viscs[m];
     double v;
-    const int it = vsettl_dev(cc[ic], modv, rho[m], visc, cf[m], cd, v, tab);
+    const int it = vsettl_dev(io.cc[ic], modv, io.rho[m], io.visc[m], cd, v);
     if (write) {
-      vset[(long long)ic * s3 + m] = v;
-      if (iters) iters[(long long)ic * s3 + m] = it;
-      if (it < 0 || !cc[ic].ok) nonconv = 1;
+      io.vset[(long long)ic * s3 + m] = -v;
+      if (io.iters) io.iters[(long long)ic * s3 + m] = it;
+      if (it < 0 || !io.cc[ic].ok) nonconv = 1;
     }
+  }
+}
+
+// The same for the Ganser model, cells q0 <= q < q1 written from qw on: one
+// loop over the iterations of all cells, in which a thread goes on to its
+// next cell when it is done with one, so that the lanes of a warp need not
+// wait for the one with the most iterations at every cell.  The next cell's
+// factors are loaded while the current one iterates.
+__device__ void chain_run_ganser(const ChainGeom& g, long long q0, long long qw, long long q1, const ChainIO& io,
+                                 const PowTab& tab, double& cd, double& cd_w, int& nonconv) {
+  if (q0 >= q1) return;
+  const long long s3 = g.d.cells(), pl = g.d.plane();
+  const int nz = g.d.nz;
+  int ic;
+  long long m, q = q0;
+  chain_cell(g, q, ic, m);
+  int left = nz - (int)(q % nz);  // cells of this column from q on
+  ClassConst k = io.cc[ic];
+  auto factors = [&](double2 f, double fi) { return GanserCell{k.ft * f.x, k.fg * f.y, k.fi * fi}; };
+  GanserCell c = factors(io.cf[m], io.visc[m]);
+  int icn = ic;  // the next cell, its class and factors
+  long long mn = m;
+  double2 fn;
+  double fin;
+  auto look = [&]() {
+    if (q + 1 >= q1) return;
+    if (left > 1) {
+      mn = m + pl;
+    } else {
+      chain_cell(g, q + 1, icn, mn);
+    }
+    fn = io.cf[mn];
+    fin = io.visc[mn];
+  };
+  look();
+  double y = ganser_rsqrt(cd), vold = 1e5, v;
+  int it = 0;
+  if (q == qw) cd_w = cd;
+  for (;;) {
+    ++it;
+    ganser_step(k, c, tab, cd, y, v);
+    const bool done = it > 1 && ganser_done(v, vold);
+    vold = v;
+    if (!done && it < 100) continue;
+    if (q >= qw) {
+      io.vset[(long long)ic * s3 + m] = done ? -(c.T * y) : -v;
+      if (io.iters) io.iters[(long long)ic * s3 + m] = done ? it : -1;
+      if (!done || !k.ok) nonconv = 1;
+    }
+    if (++q >= q1) break;
+    if (q == qw) cd_w = cd;
+    left = left > 1 ? left - 1 : nz;
+    m = mn;
+    if (icn != ic) {
+      ic = icn;
+      k = io.cc[ic];
+    }
+    c = factors(fn, fin);
+    it = 0;
+    vold = 1e5;
+    look();
   }
 }
 
 // Segment s of the chain: its entry cd (the chain's state for the first
 // segment, else the value a warm-up of W cells from cd = 1 reaches), its
 // cells and its exit cd.
-__device__ __forceinline__ void chain_segment(const ChainGeom& g, long long s, int modv, const ClassConst* cc,
-                                              const double* visc, const double2* cf, const double* rho,
-                                              double* vset, int* iters, const double* cd_state, double* entry,
-                                              double* exitv, int* nonconv, const DMathTab& tab) {
-  const long long q0 = s * g.S, q1 = min(g.L, q0 + g.S);
-  double cd;
+__device__ __forceinline__ void chain_segment(const ChainGeom& g, long long s, int modv, const ChainIO& io,
+                                              const double* cd_state, double* entry, double* exitv, int* nonconv,
+                                              const PowTab& tab) {
+  const long long q0 = s * g.S, q1 = min(g.L, q0 + g.S), qs = s == 0 ? 0 : max(0LL, q0 - g.W);
+  double cd = s == 0 ? *cd_state : 1.0, cd0 = cd;
   int nc_flag = 0, dummy = 0;
-  if (s == 0) {
-    cd = *cd_state;
+  if (modv == 2) {
+    chain_run_ganser(g, qs, q0, q1, io, tab, cd, cd0, nc_flag);
   } else {
-    cd = 1.0;
-    chain_run(g, max(0LL, q0 - g.W), q0, modv, cc, visc, cf, rho, vset, iters, cd, false, dummy, tab);
+    chain_run(g, qs, q0, modv, io, cd, false, dummy);
+    cd0 = cd;
+    chain_run(g, q0, q1, modv, io, cd, true, nc_flag);
   }
-  entry[s] = cd;
-  chain_run(g, q0, q1, modv, cc, visc, cf, rho, vset, iters, cd, true, nc_flag, tab);
+  entry[s] = cd0;
   exitv[s] = cd;
   nonconv[s] = nc_flag;
 }
 
 // One segment per thread; a segment's result does not depend on the thread
 // or block that computes it.
-__global__ void __launch_bounds__(64, 16)
-    k_chain_segments(ChainGeom g, int modv, const ClassConst* cc, const double* visc, const double2* cf,
-                     const double* rho, double* vset, int* iters, const double* cd_state, double* entry,
-                     double* exitv, int* nonconv) {
-  __shared__ DMathTab tab;
-  dmath_tab_init(tab);
+__global__ void __launch_bounds__(64, 8)
+    k_chain_segments(ChainGeom g, int modv, ChainIO io, const double* cd_state, double* entry, double* exitv,
+                     int* nonconv) {
+  __shared__ PowTab tab;
+  pow_tab_init(tab);
   __syncthreads();
   const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (s >= g.nseg) return;
-  chain_segment(g, s, modv, cc, visc, cf, rho, vset, iters, cd_state, entry, exitv, nonconv, tab);
+  chain_segment(g, s, modv, io, cd_state, entry, exitv, nonconv, tab);
 }
 
 // The same segments computed beside the step kernel (a look-ahead meteo
-// update on a second stream): blocks of four warps, one per SM sub-partition,
-// at most 64 registers and 2.5 KB of shared memory, which is what a resident
-// step-kernel block (four 112-register warps per sub-partition, 222 KB)
-// leaves free.  Only the first block that starts on an SM works (claim[smid]);
-// later ones on the same SM return at once, so that an SM idle at launch
-// time does not fill up with chain blocks and shut the steps out.  The
-// working blocks take segments from a counter until none is left.
-__global__ void __launch_bounds__(128, 8)
-    k_chain_beside(ChainGeom g, int modv, const ClassConst* cc, const double* visc, const double2* cf,
-                   const double* rho, double* vset, int* iters, const double* cd_state, double* entry,
-                   double* exitv, int* nonconv, int* claim, unsigned long long* next) {
-  __shared__ DMathTab tab;
+// update on a second stream): blocks of four warps, one per SM sub-partition.
+// Only the first block that starts on an SM works (claim[smid]); later ones on
+// the same SM return at once, so that an SM idle at launch time does not fill
+// up with chain blocks and shut the steps out.  The working blocks take
+// segments from a counter until none is left.
+__global__ void __launch_bounds__(128, 4)
+    k_chain_beside(ChainGeom g, int modv, ChainIO io, const double* cd_state, double* entry, double* exitv,
+                   int* nonconv, int* claim, unsigned long long* next) {
+  __shared__ PowTab tab;
   __shared__ int mine;
   if (threadIdx.x == 0) {
     unsigned smid;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     mine = atomicCAS(claim + (smid & 255u), 0, 1) == 0;
   }
-  dmath_tab_init(tab);
   __syncthreads();
   if (!mine) return;
+  pow_tab_init(tab);
+  __syncthreads();
   for (;;) {
     const unsigned long long s = atomicAdd(next, 1ULL);
     if (s >= (unsigned long long)g.nseg) break;
-    chain_segment(g, (long long)s, modv, cc, visc, cf, rho, vset, iters, cd_state, entry, exitv, nonconv, tab);
+    chain_segment(g, (long long)s, modv, io, cd_state, entry, exitv, nonconv, tab);
   }
 }
 
@@ -608,12 +703,10 @@ __global__ void k_chain_check(ChainGeom g, const double* entry, const double* ex
 // Sequential repair in chain order (single thread).  Segments verified above
 // stay; a recomputed segment may change its exit, so its successor is
 // re-checked until the chain agrees again.  cap overflow -> full scan.
-__global__ void k_chain_fix(ChainGeom g, int modv, const ClassConst* cc, const double* visc,
-                            const double2* cf, const double* rho, double* vset, int* iters, double* entry,
-                            double* exitv, int* nonconv, int* bad, const int* nbad, int cap,
-                            double* cd_state) {
-  __shared__ DMathTab tab;
-  dmath_tab_init(tab);
+__global__ void k_chain_fix(ChainGeom g, int modv, ChainIO io, double* entry, double* exitv, int* nonconv, int* bad,
+                            const int* nbad, int cap, double* cd_state) {
+  __shared__ PowTab tab;
+  if (*nbad > 0) pow_tab_init(tab);
   __syncthreads();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const int nb = *nbad;
@@ -639,7 +732,11 @@ __global__ void k_chain_fix(ChainGeom g, int modv, const ClassConst* cc, const d
         int nc_flag = 0;
         entry[s] = cd;
         const long long q0 = s * g.S, q1 = min(g.L, q0 + g.S);
-        chain_run(g, q0, q1, modv, cc, visc, cf, rho, vset, iters, cd, true, nc_flag, tab);
+        double cd0;
+        if (modv == 2)
+          chain_run_ganser(g, q0, q0, q1, io, tab, cd, cd0, nc_flag);
+        else
+          chain_run(g, q0, q1, modv, io, cd, true, nc_flag);
         exitv[s] = cd;
         nonconv[s] = nc_flag;
         ++s;  // the successor must be re-checked
@@ -677,51 +774,46 @@ void launch_dmath_eval(int op, long long n, const double* x, double* y, cudaStre
   count_launch();
 }
 
-// setvset.f90:48-60: the aggregate loop touches class np+1 (a gas class with
-// vset = 0 when nc > np), then vset = -vset over all classes.
+// setvset.f90:48-60 for the gas classes np+1..nc, which the chain does not
+// touch: the aggregate loop multiplies class np+1 (a gas class with vset = 0
+// when nc > np), then vset = -vset over all classes.  They keep their previous
+// value (zero of alternating sign, as the reference negates the whole array
+// at every update).
 __global__ void k_vset_finish(long long s3, int nc, int np, int aggregate, double vset_factor,
                               double* vset) {
-  const long long n = s3 * nc;
+  const long long n = s3 * (nc - np);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
        q += (long long)gridDim.x * blockDim.x) {
-    const int ic = (int)(q / s3);
-    // gas classes keep their previous value (zero of alternating sign, as the
-    // reference negates the whole array at every update)
-    double v = vset[q];
-    if (aggregate && ic == np) v = vset_factor * v;
-    vset[q] = -v;
+    double* v = vset + (long long)np * s3 + q;
+    *v = -(aggregate && q < s3 ? vset_factor * *v : *v);
   }
 }
 
-// Threads of k_chain_segments the device holds at once (blocks of 64).
-static long long chain_capacity() {
-  static long long cap = 0;
-  if (cap == 0) {
-    int dev = 0, nsm = 0, per_sm = 0;
+static int chain_sms() {
+  static int nsm = 0;
+  if (!nsm) {
+    int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chain_segments, 64, 0);
-    cap = (long long)std::max(1, nsm) * std::max(1, per_sm) * 64;
   }
-  return cap;
+  return std::max(1, nsm);
 }
 
 static ChainGeom chain_geom(Dims d, int np) {
   ChainGeom g;
   g.d = d;
   g.L = d.cells() * np;
-  // The segments are the threads of one launch: half as many as the device
-  // holds at once when the chain is long enough (measured on cfg1: the
-  // binary64 pipe stays as busy with half the threads resident, and the
-  // warm-up of W cells recomputed from the preceding segment, enough for
-  // the cd iteration to forget its guess, halves relative to the work;
-  // a quarter is slower again), else fewer, longer segments.
-  const long long cap = chain_capacity() / 2;
-  long long S = (g.L + cap - 1) / cap;
-  S = std::max<long long>(256, S);
-  g.S = S;
   g.W = 64;
-  g.nseg = (g.L + S - 1) / S;
+  // The segments are the threads of one launch.  Three warps per SM already
+  // keep the binary64 pipe busy (an iteration's 26 operations take 416 clocks
+  // of it per warp, about half of the iteration's latency), and every segment
+  // costs the W cells of its warm-up: segments of about 1024 cells, but no
+  // fewer than 3 warps per SM hold, and at most 12 warps' worth, whose
+  // different lengths (2 to 6 iterations per cell by class) even out.
+  const long long warp_row = 32LL * chain_sms();
+  const long long n = std::min(12 * warp_row, std::max(3 * warp_row, g.L / 1024));
+  g.S = std::max<long long>(64, (g.L + n - 1) / n);
+  g.nseg = (g.L + g.S - 1) / g.S;
   return g;
 }
 
@@ -743,7 +835,7 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
                     const double* psi, const double* sphe, const double* tempe,
                     const double* rho, int aggregate, double vset_factor, double* vset,
                     int* iters, double* cd_state, void* scratch, int* status, cudaStream_t s,
-                    int beside_step) {
+                    int beside_step, int have_classes) {
   const ChainGeom g = chain_geom(d, np);
   unsigned char* p = reinterpret_cast<unsigned char*>(scratch);
   auto take = [&](size_t bytes) {
@@ -764,39 +856,42 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
   cudaMemsetAsync(nbad, 0, sizeof(int), s);
   cudaMemsetAsync(status, 0, sizeof(int), s);
   if (np > 0 && g.L > 0) {
-    k_class_consts<<<(np + 31) / 32, 32, 0, s>>>(np, modv, diam, rhop, psi, sphe, cc);
-    k_visc<<<(int)std::min<long long>((d.cells() + 255) / 256, 152LL * 16), 256, 0, s>>>(d.cells(), tempe,
+    if (!have_classes) launch_class_consts(np, modv, diam, rhop, psi, sphe, scratch, s);
+    k_visc<<<(int)std::min<long long>((d.cells() + 255) / 256, 152LL * 16), 256, 0, s>>>(d.cells(), modv, tempe,
                                                                                          rho, visc, cf);
+    const ChainIO io{cc, visc, cf, rho, vset, iters};
     const int bs = 64;
     const long long nb = (g.nseg + bs - 1) / bs;
     if (beside_step) {
-      static int nsm = 0;
-      if (!nsm) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        // an SM holding this block must still take a step-kernel block
-        cudaFuncSetAttribute(k_chain_beside, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-      }
+      // an SM holding this block must still take a step-kernel block
+      static const cudaError_t carveout = cudaFuncSetAttribute(
+          k_chain_beside, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      (void)carveout;
       cudaMemsetAsync(claim, 0, sizeof(int) * 256, s);
       cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
-      k_chain_beside<<<(unsigned)(4 * std::max(1, nsm)), 128, 0, s>>>(g, modv, cc, visc, cf, rho, vset, iters,
-                                                                      cd_state, entry, exitv, nonconv, claim,
-                                                                      next);
+      k_chain_beside<<<(unsigned)(4 * chain_sms()), 128, 0, s>>>(g, modv, io, cd_state, entry, exitv, nonconv, claim,
+                                                                 next);
     } else {
-      k_chain_segments<<<(unsigned)nb, bs, 0, s>>>(g, modv, cc, visc, cf, rho, vset, iters, cd_state, entry,
-                                                   exitv, nonconv);
+      k_chain_segments<<<(unsigned)nb, bs, 0, s>>>(g, modv, io, cd_state, entry, exitv, nonconv);
     }
     k_chain_check<<<(unsigned)((g.nseg + 255) / 256), 256, 0, s>>>(g, entry, exitv, bad, nbad, kBadCap);
-    k_chain_fix<<<1, 32, 0, s>>>(g, modv, cc, visc, cf, rho, vset, iters, entry, exitv, nonconv, bad,
-                                 nbad, kBadCap, cd_state);
+    k_chain_fix<<<1, 32, 0, s>>>(g, modv, io, entry, exitv, nonconv, bad, nbad, kBadCap, cd_state);
     k_chain_status<<<(unsigned)((g.nseg + 255) / 256), 256, 0, s>>>(g, nonconv, status);
-    count_launch(6);
+    count_launch(5);
   }
-  const long long n = d.cells() * nc;
-  k_vset_finish<<<(int)std::min<long long>((n + 255) / 256, 152LL * 16), 256, 0, s>>>(
-      d.cells(), nc, np, aggregate, vset_factor, vset);
+  if (nc > np) {
+    const long long n = d.cells() * (nc - np);
+    k_vset_finish<<<(int)std::min<long long>((n + 255) / 256, 152LL * 16), 256, 0, s>>>(
+        d.cells(), nc, np, aggregate, vset_factor, vset);
+    count_launch();
+  }
+}
+
+void launch_class_consts(int np, int modv, const double* diam, const double* rhop, const double* psi,
+                         const double* sphe, void* scratch, cudaStream_t s) {
+  if (np <= 0) return;
+  k_class_consts<<<(np + 31) / 32, 32, 0, s>>>(np, modv, diam, rhop, psi, sphe,
+                                               reinterpret_cast<ClassConst*>(scratch));
   count_launch();
 }
 

@@ -77,4 +77,64 @@ __device__ __forceinline__ double dm_exp(const DMathTab& t, double a) {
   return fma(s, em1, s);
 }
 
+// ---------------------------------------------------------------- Ganser
+// The three functions of a Ganser drag iteration in as few binary64
+// operations as their accuracy (about an ulp) allows, for arguments in the
+// normal range the callers check.
+
+// x^a, a = 0.6567 - 1: with x = 2^k z, z in [1, 2), and the breakpoint c of
+// the top eight fraction bits of z, x^a = 2^(ka) c^a (1 + r)^a, r = z/c - 1,
+// |r| <= 2^-9: two table values and the binomial series to r^5 (the next term
+// is below 2^-57), 8 operations in place of the 23 of a logarithm and an
+// exponential.
+constexpr double kPowA = 0.6567 - 1.0;
+constexpr int kPowEmin = -64, kPowN = 128;  // exponents k of the table
+struct PowTab {
+  double invc[256];   // RN(1 / (1 + (j + 1/2)/256))
+  double powc[256];   // RN(invc[j]^-a)
+  double pow2[kPowN]; // RN(2^(a (kPowEmin + j)))
+};
+__device__ __forceinline__ void pow_tab_init(PowTab& t) {
+  for (int j = threadIdx.x; j < 256; j += blockDim.x) {
+    const double ic = 1.0 / (1.0 + (j + 0.5) / 256.0);
+    t.invc[j] = ic;
+    t.powc[j] = pow(ic, -kPowA);
+  }
+  for (int j = threadIdx.x; j < kPowN; j += blockDim.x) t.pow2[j] = exp2(kPowA * (kPowEmin + j));
+}
+// the biased exponent lies in the table's range
+__device__ __forceinline__ bool pow_in_range(double x) {
+  return (unsigned)((__double2hiint(x) >> 20) - (1023 + kPowEmin)) < (unsigned)kPowN;
+}
+__device__ __forceinline__ double pow_a(const PowTab& t, double x) {
+  const int hi = __double2hiint(x);
+  const int j = (hi >> 12) & 255;
+  const double z = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(x));
+  const double s = t.pow2[(hi >> 20) - (1023 + kPowEmin)] * t.powc[j];
+  const double r = fma(z, t.invc[j], -1.0);
+  constexpr double a = kPowA, c1 = a, c2 = c1 * (a - 1.0) / 2.0, c3 = c2 * (a - 2.0) / 3.0, c4 = c3 * (a - 3.0) / 4.0,
+                   c5 = c4 * (a - 4.0) / 5.0;
+  double q = fma(r, c5, c4);
+  q = fma(q, r, c3);
+  q = fma(q, r, c2);
+  q = fma(q, r, c1);
+  return fma(s * r, q, s);
+}
+
+// 1/sqrt(x) and 1/x from the hardware's approximations (relative error at
+// most 2^-20) by one step of third order each, whose own error is below
+// 2^-60; x in [2^-1000, 2^1000].
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = fma(-(x * y), y, 1.0);
+  return fma(y * h, fma(0.375, h, 0.5), y);
+}
+__device__ __forceinline__ double rcp_fast(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 }  // namespace f3d

@@ -185,7 +185,11 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
                     const double* psi, const double* sphe, const double* tempe,
                     const double* rho, int aggregate, double vset_factor, double* vset,
                     int* iters, double* cd_state, void* scratch, int* status, cudaStream_t s,
-                    int beside_step = 0);
+                    int beside_step = 0, int have_classes = 0);
+// The class constants of launch_setvset, kept at the start of its scratch: a
+// caller whose classes stay the same makes them once (have_classes).
+void launch_class_consts(int np, int modv, const double* diam, const double* rhop, const double* psi,
+                         const double* sphe, void* scratch, cudaStream_t s);
 // The drag iteration's table-driven log (op 0) and exp (op 1) on n values.
 void launch_dmath_eval(int op, long long n, const double* x, double* y, cudaStream_t s);
 
