@@ -23,16 +23,29 @@ int reduce_blocks(long long n) {
 
 // Sum of n DDs p[0], p[stride], ... by one warp (all lanes call it; lane 0 has
 // the sum): each lane adds its share in order, then the lanes' sums are added
-// pairwise.  A double-double addition is about 12 binary64 operations, of
-// which an SM issues two lanes per clock, so a block's reduction is left to
-// one warp per sum instead of a shuffle tree in every warp (n = 256: 13
-// additions issued instead of 47).
+// pairwise.  The high parts by TwoSum, its exact errors and the low parts in
+// binary64 beside it (the cascaded sum of Ogita, Rump and Oishi, below): the
+// dependent chain is one addition per term, where a double-double addition's
+// is nine.  An SM issues two lanes of binary64 per clock, so a block's
+// reduction is left to one warp per sum instead of a tree in every warp.
 __device__ __forceinline__ DD warp_sum_dd(const DD* p, int n, int stride) {
   const int lane = threadIdx.x & 31;
-  DD v = dd_zero();
-  for (int q = lane; q < n; q += 32) v = dd_add(v, p[(long long)q * stride]);
-  for (int off = 16; off > 0; off >>= 1) v = dd_add(v, dd_shfl_down(v, off));
-  return v;
+  double s = 0.0, e = 0.0;
+  auto add = [&](double hi, double lo) {
+    const double t = s + hi, bb = t - s;
+    e = e + (((s - (t - bb)) + (hi - bb)) + lo);
+    s = t;
+  };
+  for (int q = lane; q < n; q += 32) {
+    const DD v = p[(long long)q * stride];
+    add(v.hi, v.lo);
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    const double hi = __shfl_down_sync(0xffffffffu, s, off), lo = __shfl_down_sync(0xffffffffu, e, off);
+    add(hi, lo);
+  }
+  const double hi = s + e;
+  return DD{hi, e - (hi - s)};
 }
 
 // The block's NS sums of its threads' v into partial[blockIdx.x * NS ...]
