@@ -374,16 +374,17 @@ void sizloop(f3d_ctx* x) {
 }
 
 
-// The precision form's step as one fused kernel (f3d_fused.cu), then the
+// The precision form's step as one fused kernel (f3d_fused2.cu), then the
 // clipped state's boundary outflow (cmass2d) in binary64.
 void sizloop_fused(f3d_ctx* x) {
   const Dims d = x->d;
   const int nc = x->g.nc;
   cudaStream_t s = x->stream;
-  const FusedArgs a = f3d::ctx_fused_args(x, x->opt_tile);
+  const int shape = x->tile_set ? x->opt_tile : step_shape(d, nc);
+  const FusedArgs a = f3d::ctx_fused_args(x, shape);
   {
     ProfScope ps(x, "step_fused");
-    launch_step_fused(a, x->maps2, x->cmap, x->opt_tile, s);
+    launch_step_fused(a, x->maps2, x->cmap, shape, s);
   }
   std::swap(x->c32, x->c32b);
   std::swap(x->cmap, x->cmapb);
@@ -1228,6 +1229,7 @@ int f3d_set_option(f3d_ctx* x, int key, int value) {
   } else if (key == F3D_OPT_TILE) {
     if (value < 0 || value > 3) return f3d::ctx_error(F3D_ERR_ARG, "tile shape must be 0..3");
     x->opt_tile = value;
+    x->tile_set = true;
   } else if (key == F3D_OPT_PREFETCH) {
     if (!value) f3d::ctx_prefetch_drop(x);
     x->opt_prefetch = value ? 1 : 0;

@@ -88,6 +88,7 @@ struct f3d_ctx {
   double* lambda2d = nullptr;
   unsigned char* wet_class = nullptr;
   int opt_fused = 1, opt_tile = 3;
+  bool tile_set = false;  // F3D_OPT_TILE was set
   // the fused kernel applies: zlayer non-decreasing, 32-bit offsets in a class
   int fused_ok = 1;
   // sources

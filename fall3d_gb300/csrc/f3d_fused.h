@@ -96,8 +96,9 @@ void step_chunks(FusedArgs& a, int shape, int nwet);
 
 // Tile shapes (F3D_OPT_TILE), region x by y / threads: 0, 1 and 2 = 64x16 /
 // 512 (a row per warp, two blocks per SM), 3 = 64x32 / 512 (two rows per
-// warp, the default); two columns per lane.  Results do not depend on the
-// shape.
+// warp); two columns per lane.  Results do not depend on the shape.
+// step_shape: the faster one for a launch of its own, where none was set.
+int step_shape(Dims d, int ncls);
 void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s);
 // The step kernel's fields from the scaled binary64 fields of a meteo update
 // whose finddt maximum is at *dtcn (dt = safety/max(dtcn,1e-13)).

@@ -31,19 +31,24 @@
 //
 // Staging: the ten fields iteration t+1 reads (c two planes ahead, vz+vset
 // one, the Courant velocities and limiter coefficients, 1/rho and the three
-// face coefficients) arrive by tensor copies while iteration t computes; one
-// lane of each warp issues a field's box.  A box starts at the region's first
-// column rounded down to a multiple of 4 values (16 bytes, what a tensor
-// copy needs; the region then starts 0 or 2 values into it) and is 68 wide.
+// face coefficients) arrive by tensor copies, in two buffers; one lane of each
+// warp issues a field's box as soon as the last warp has read the field's
+// buffer.  A box starts at the region's first column rounded down to a
+// multiple of 4 values (16 bytes, what a tensor copy needs; the region then
+// starts 0 or 2 values into it) and is 68 wide.
 //
-// What bounds it: 400x300x50 cells and 16 classes take 0.999 ms (1.255 ms
+// What bounds it: 400x300x50 cells and 16 classes take 0.889 ms (1.255 ms
 // before the flux form, the packed arithmetic, the coefficients formed at the
 // meteo update and the shared-memory addressing), 1.32 GB of algorithmic bytes
 // or 0.19 ms at the copy bandwidth.  A warp issues about 500 instructions per
 // plane for its 128 positions, 200 of them binary32 arithmetic, at half the
 // issue rate: with one block of 16 warps per SM (174 KB of staged fields, 128
 // registers) the dependency chains of the sweeps and the three block barriers
-// of a plane are not all covered.
+// of a plane are not all covered.  The tensor copies bring 87 KB per plane and
+// SM, 6.7 TB/s over the device; when the copies of t+1 were issued after
+// iteration t's first barrier, waiting for them was the largest stall (0.999
+// ms with c and vz+vset in a third buffer, 1.03 ms without; all fields issued
+// after the iteration's last barrier 0.915 ms).
 //
 // Column pieces: a march over levels k0..k1 starts at t = k0-1 from the
 // original column's planes k0-3..k0 (the advection fluxes of plane k0-1 need
@@ -67,7 +72,7 @@ constexpr int GUARD = 512;  // bytes before the staging area (reads one row abov
 template <int HY_, int NW_>
 struct Shape {
   static constexpr int HYR = HY_, NWARP = NW_, NT = 32 * NW_, RPW = HY_ / NW_, TY = HY_ - 6, FS = RS * HY_,
-                       NP = HX * HY_, MAP = HY_ == 32 ? 0 : 1;
+                       NP = HX * HY_, MAP = HY_ == 32 ? 0 : 1, UNROLL = HY_ == 32 ? 1 : 2;
   static_assert(HY_ % NW_ == 0 && NW_ >= NF, "rows must divide among warps; a warp issues one field's copies");
 };
 constexpr int HY = 32, NW = 16;  // the default shape
@@ -86,7 +91,7 @@ __device__ __forceinline__ float2 ldg2(const float* p) { return __ldg(reinterpre
 
 template <class S>
 size_t step_smem(int nz) {
-  return GUARD + sizeof(float) * ((size_t)(2 * NF + NA) * S::FS + 3 * (size_t)S::NP + HX) +
+  return GUARD + sizeof(float) * ((size_t)2 * NF * S::FS + 3 * (size_t)S::NP + HX) +
          sizeof(ZTab) * (size_t)(nz + 2) + 64;
 }
 
@@ -135,13 +140,12 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
   // generic ones the step of 400x300x50 cells, 16 classes took 1.125 ms
   // instead of 1.055 ms).
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  // 128-byte aligned fields: [3][NA][FS] of the fields read ahead, [2][NF-NA][FS] of the others
-  float* stage = reinterpret_cast<float*>(smem_raw + GUARD);
-  float* P0s = stage + (2 * NF + NA) * FS;                // planes the y sweeps exchange rows through:
+  float* stage = reinterpret_cast<float*>(smem_raw + GUARD);  // [2][NF][FS], 128-byte aligned fields
+  float* P0s = stage + 2 * NF * FS;                       // planes the y sweeps exchange rows through:
   float* Ws = P0s + NP;                                   // c, the advection flux, c/rho
   float* P1s = Ws + NP;
   ZTab* tab = reinterpret_cast<ZTab*>(P1s + NP + HX);
-  // one per staging buffer: 3 of the fields read ahead, 2 of the others
+  // one per staging buffer
   unsigned long long* mbar = reinterpret_cast<unsigned long long*>(tab + (a.d.nz + 2));
 
   const Dims d = a.d;
@@ -168,48 +172,46 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
   const unsigned mbar0 = (unsigned)__cvta_generic_to_shared(mbar);
   __shared__ int s_kzmax;  // the highest wet layer of the tile: above it the wet code is skipped
   if (threadIdx.x == 0) {
-    for (int b = 0; b < 5; ++b) mbar_init(mbar0 + 8u * b, b < 3 ? NA : NF - NA);
+    mbar_init(mbar0, NF);
+    mbar_init(mbar0 + 8, NF);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_kzmax = 0;
   }
   __syncthreads();
 
   // ------------------------------------------------ staging
-  // The staged inputs of iteration t: c and vz+vset, which the column update
-  // at its start reads, in buffer (t-ts)%3 and issued two iterations ahead;
-  // the others in buffer (t-ts)&1, one ahead.  Both are issued after the first
-  // barrier of an iteration, when every warp has left the previous iteration
-  // and this one's column update and nobody reads those buffers.  One lane of
-  // warp f issues field f's box; outside the arrays it fills zeros, planes
+  // The staged inputs of iteration t are in buffer (t-ts)&1.  Those of t+2
+  // are issued during iteration t, a field's box after the block barrier that
+  // follows every warp's last read of the field: the advection's fields after
+  // the second barrier (early), the others, and x's when its sweep is the
+  // second, after the last.  One barrier object per buffer: with one for each
+  // of the two groups the wait is shorter but the second wait of a plane costs
+  // more (0.961 ms against 0.889 ms at 400x300x50, 16 classes).  One lane of
+  // warp f issues field f's box.  Outside the arrays it fills zeros; planes
   // outside 1..nz are not read and not copied.
   const unsigned stage0 = (unsigned)__cvta_generic_to_shared(stage);
   const bool issuer = lane == 0 && warp < NF;
-  const bool ahead = warp < NA;
-  auto prefetch = [&](const int i) {  // i = t - ts
-    if (!issuer) return;
-    const int t = ts + i;
-    if (t > te) return;
-    const int buf = ahead ? i % 3 : 3 + (i & 1);
-    const unsigned bar = mbar0 + 8u * (unsigned)buf;
-    const int slot = ahead ? buf * NA + warp : 3 * NA + (buf - 3) * (NF - NA) + warp - NA;
-    const int p = t + field_plane(warp);
+  const int f_plane = field_plane(warp);
+  const int f_z = warp <= F_VK ? cls * (nz + 2) : 0;
+  const CUtensorMap* f_map = warp == F_C ? &cmap->m[S::MAP] : &maps->m[S::MAP][issuer ? warp - 1 : 0];
+  const bool early = warp < F_L && (XFIRST || (warp != F_UX && warp != F_KX));
+  auto prefetch = [&](const int t, const bool mine) {
+    if (!issuer || !mine || t > te) return;
+    const unsigned buf = (unsigned)(t - ts) & 1u, bar = mbar0 + 8u * buf;
+    const int p = t + f_plane;
     // the warps' reads of this buffer (ordered before this point by a block
     // barrier) come before the tensor copy overwrites it
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (p >= 1 && p <= nz) {
-      mbar_expect(bar, (unsigned)(FS * sizeof(float)));
-      tma_load3(stage0 + 4u * (unsigned)(slot * FS), warp == F_C ? &cmap->m[S::MAP] : &maps->m[S::MAP][warp - 1], xs, gy0,
-                (ahead ? cls * (nz + 2) : 0) + p, bar);
-    } else {
-      mbar_expect(bar, 0u);
-    }
+    const bool ok = p >= 1 && p <= nz;
+    mbar_expect(bar, ok ? (unsigned)(FS * sizeof(float)) : 0u);
+    if (ok) tma_load3(stage0 + 4u * (buf * NF + warp) * FS, f_map, xs, gy0, f_z + p, bar);
   };
   bool timed_out = false;
-  auto staged = [&](const int bar, const int phase) {
-    if (!mbar_wait(mbar0 + 8u * (unsigned)bar, (unsigned)phase)) timed_out = true;
+  auto staged = [&](const int t) {
+    if (!mbar_wait(mbar0 + 8u * ((unsigned)(t - ts) & 1u), (unsigned)((t - ts) >> 1) & 1u)) timed_out = true;
   };
-  prefetch(0);
-  if (ahead) prefetch(1);
+  prefetch(ts, true);
+  prefetch(ts + 1, true);
 
   for (int k = threadIdx.x; k < (nz + 2) * (int)(sizeof(ZTab) / 4); k += NT)
     reinterpret_cast<float*>(tab)[k] = __ldg(reinterpret_cast<const float*>(a.f.tab) + k);
@@ -348,14 +350,9 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
         if ((gj == 1 || gj == ny) && pair_in) ey[r] = ldg2(a.f.ey + (gj == 1 ? 0 : (nz + 2) * px) + k * px + gi);
       }
     }
-    const int i = t - ts;
-    const int ba = i % 3;
-    staged(ba, (i / 3) & 1);
-    if constexpr (EDGE) staged(3 + (i & 1), (i >> 1) & 1);
-    // the lane's row-0 pair in the buffers of this iteration
-    const float* sa0 = stage + ba * (NA * FS) + RPW * warp * RS + sft + 2 * lane;
-    const float* sb0 = stage + (3 * NA + (i & 1) * (NF - NA)) * FS + RPW * warp * RS + sft + 2 * lane;
-    auto at = [&](int field, int r) { return (field < NA ? sa0 + field * FS : sb0 + (field - NA) * FS) + r * RS; };
+    staged(t);
+    const float* sb = stage + ((t - ts) & 1) * (NF * FS) + RPW * warp * RS + sft + 2 * lane;  // the row-0 pair
+    auto at = [&](int field, int r) { return sb + field * FS + r * RS; };
     float2 s2[RPW];
     if (STEADY || t <= nz) {
       float2 s1[RPW];
@@ -453,7 +450,6 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
         sts2(P0, in[0]);
         if (RPW > 1) sts2(P0 + (RPW - 1) * HX, in[RPW - 1]);
         __syncthreads();
-        prefetch(ahead ? i + 2 : i + 1);
         const float2 cb = lds2(P0 - HX), ca = lds2(P0 + RPW * HX);
         float2 u[RPW], wy[RPW], F[RPW];
 #pragma unroll
@@ -469,6 +465,7 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
         sts2(W, F[0]);
         if (RPW > 1) sts2(W + (RPW - 1) * HX, F[RPW - 1]);
         __syncthreads();
+        prefetch(t + 2, early);
         float2 G[RPW + 1];
 #pragma unroll
         for (int r = 0; r <= RPW; ++r) {
@@ -485,7 +482,6 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
           out[r] = keep(upwind(in[r], u[r], g, gp), in[r], r);
         }
       };
-      if constexpr (!EDGE) staged(3 + (i & 1), (i >> 1) & 1);
       float2 sa[RPW];
       if constexpr (XFIRST) {  // sizloop.f90:42-48
         adv_x(s1, sa);
@@ -495,7 +491,6 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
         adv_x(sa, s2);
       }
     } else {
-      if constexpr (!EDGE) staged(3 + (i & 1), (i >> 1) & 1);
 #pragma unroll
       for (int r = 0; r < RPW; ++r) s2[r] = make_float2(0.0f, 0.0f);
       __syncthreads();  // the y-sweep plane of the previous iteration is read by all warps
@@ -533,14 +528,24 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
       }
       if (STEADY || k >= k0) s3[r] = keep(s3[r], c0, r);
     }
-    if (!STEADY && k < k0) return;
-    // ---------------- D: diffx (shuffles) and diffy (shared memory)
+    if (!STEADY && k < k0) {
+      __syncthreads();
+      prefetch(t + 2, !early);
+      return;
+    }
+    // ---------------- D: diffx (shuffles) and diffy (shared memory); their
+    // coefficients are read before the barrier that frees the staging buffer
+    float2 cfx[RPW], cfy[RPW + 1];
+#pragma unroll
+    for (int r = 0; r < RPW; ++r) cfx[r] = lds2(at(F_FX, r));
+#pragma unroll
+    for (int r = 0; r <= RPW; ++r) cfy[r] = lds2(at(F_FY, r - 1));
     auto dif_x = [&](const float2* in, float2* out) {
 #pragma unroll
       for (int r = 0; r < RPW; ++r) {
         const float2 c0 = in[r], q = mul2(c0, lbv[r]), qp = right2(q);
         const float2 dq = sub2(qp, q);
-        float2 fr = mul2(lds2(at(F_FX, r)), dq);
+        float2 fr = mul2(cfx[r], dq);
         if constexpr (EDGE) {
           if (xedge) {  // the line's end faces MAX(0, ...), MIN(0, ...) (diffx.f90:22-33, 44-55)
             fr.x = gi == 0 ? fmaxf(fr.x, 0.0f) : gi == nx ? fminf(fr.x, 0.0f) : fr.x;
@@ -567,12 +572,13 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
       sts2(P1, q[0]);
       if (RPW > 1) sts2(P1 + (RPW - 1) * HX, q[RPW - 1]);
       __syncthreads();
+      prefetch(t + 2, !early);
       const float2 qm = lds2(P1 - HX), qa = lds2(P1 + RPW * HX);
       float2 dq[RPW + 1], f[RPW + 1];  // faces gj0-1/2 .. gj0+RPW-1/2
 #pragma unroll
       for (int r = 0; r <= RPW; ++r) {
         dq[r] = sub2(r < RPW ? q[r] : qa, r ? q[r - 1] : qm);
-        f[r] = mul2(lds2(at(F_FY, r - 1)), dq[r]);
+        f[r] = mul2(cfy[r], dq[r]);
       }
 #pragma unroll
       for (int r = 0; r < RPW; ++r) {
@@ -643,10 +649,11 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
   auto march = [&](auto edge_c) {
     const int t1 = max(3, k0 + 1), t2 = max(t1 - 1, min(te, nz - 2));  // steady: t1..t2
     for (int t = ts; t < min(t1, te + 1); ++t) plane(edge_c, False_{}, t);
-    // not unrolled: a body of two planes issues 9% fewer instructions (no
-    // moves of the carried values) but misses the instruction cache more
-    // often (400x300x50, 16 classes: 1.014 ms against 0.999 ms)
-#pragma unroll 1
+    // A body of two planes issues 9% fewer instructions (no moves of the
+    // carried values) but misses the instruction cache more often: with two
+    // rows per warp the second costs more (400x300x50, 16 classes: 0.912 ms
+    // against 0.889 ms), with one row the first (0.976 ms against 1.014 ms).
+#pragma unroll S::UNROLL
     for (int t = t1; t <= t2; ++t) plane(edge_c, True_{}, t);
     for (int t = t2 + 1; t <= te; ++t) plane(edge_c, False_{}, t);
   };
@@ -657,20 +664,17 @@ __device__ __forceinline__ void step_tile(const FusedArgs& a, const F2Maps* maps
 
   if (timed_out) {  // a tensor copy did not arrive in time: report, and let copies in flight land
     atomicOr(a.status, F3D_STEP_STAGING_TIMEOUT);
-    for (int i = max(0, te - ts - 1); i <= te - ts; ++i) {
-      staged(i % 3, (i / 3) & 1);
-      staged(3 + (i & 1), (i >> 1) & 1);
-    }
+    for (int t = max(ts, te - 1); t <= te; ++t) staged(t);
   }
   __syncthreads();  // nobody waits on the barriers any more: they may be reused (next batch item)
   if (threadIdx.x == 0) {
-    for (int b = 0; b < 5; ++b) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mbar0 + 8u * b) : "memory");
+    for (int b = 0; b < 2; ++b) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mbar0 + 8u * b) : "memory");
   }
 }
 
 template <class S>
 constexpr int min_blocks() {
-  return S::RPW == 1 ? 2 : 1;
+  return S::HYR == 16 ? 2 : 1;
 }
 
 struct StepMaps {
@@ -868,6 +872,15 @@ int fused_tiles(int nx, int ny, int shape) {
   const int ty = with_shape(shape, [](auto s) { return decltype(s)::TY; });
   return ((nx + TX - 1) / TX) * ((ny + ty - 1) / ty);
 }
+
+// 64x16 tiles of which every SM gets at most one take a plane in fewer
+// operations per warp than the 64x32 tiles that would leave half of the SMs
+// idle: 21.0 us against 27.2 at 12x10x8 cells and 3 classes, 24.1 against 39.9
+// at 32x28x14 and 4, 40.5 against 50.6 at 80x80x25 and 6 (96 tiles), 60.7
+// against 61.0 at 160x121x40 and 3 (117).  Beyond, their larger share of halo
+// rows costs more: 66.0 against 63.0 us at 121x101x30 and 6 classes (198 tiles),
+// 299 against 285 at 243x191x37 and 11, 976 against 889 at 400x300x50 and 16.
+int step_shape(Dims d, int ncls) { return (long long)fused_tiles(d.nx, d.ny, 0) * ncls <= device_sms() ? 0 : 3; }
 
 void step_chunks(FusedArgs& a, int shape, int nwet) {
   const int nz = a.d.nz;

@@ -71,8 +71,7 @@ __device__ __forceinline__ float2 upwind(float2 c, float2 v, float2 g, float2 gp
 // vz+vset(t+1), the Courant velocities and limiter coefficients of x and y and
 // 1/rho (t), and the diffusion's face coefficients (t-1).
 enum : int { F_C = 0, F_VK, F_UX, F_KX, F_UY, F_KY, F_L, F_FZ, F_FX, F_FY, NF };
-constexpr int NA = 2;
-// Their plane in iteration t, minus t; the first NA are staged two iterations ahead.
+// their plane in iteration t, minus t
 __host__ __device__ constexpr int field_plane(int f) { return f == F_C ? 2 : f == F_VK ? 1 : f >= F_FZ ? -1 : 0; }
 
 using False_ = std::integral_constant<bool, false>;

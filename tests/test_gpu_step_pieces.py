@@ -52,6 +52,28 @@ def test_pieces_and_edges(nx, ny, nz, nc, pblh):
         assert np.max(a["cwet"]) > 0.0
 
 
+@pytest.mark.parametrize("nx,ny,nz,nc", [(30, 20, 9, 3), (58, 10, 9, 152), (58, 10, 9, 153), (117, 41, 8, 8)])
+def test_default_shape_equals_the_set_ones(nx, ny, nz, nc):
+    """Where no tile shape was set the step picks one by the number of tiles
+    (both sides of one tile per SM): the same bits as with either."""
+    s = synth.make_scenario("small", seed=7, nx=nx, ny=ny, nz=nz, nc=nc, run_h=1.0, H=5000.0)
+    out = []
+    for tile in (None, 0, 3):
+        g = F.Context(s, F.PREC_FP32)
+        assert g.get_option(F.OPT_TILE) == 3
+        if tile is not None:
+            g.set_option(F.OPT_TILE, tile)
+        g.meteo(0)
+        g.source(0)
+        g.step(STEPS)
+        g.sync()
+        out.append((g.fields(), g.state()["outmass"]))
+    for f, om in out[1:]:
+        for k in ("c", "cdry"):
+            assert_same_bits(f[k], out[0][0][k], k)
+        assert om == out[0][1]
+
+
 def test_batch_of_pieces_equals_alone():
     """Members of different sizes in one batch: the batched launch cuts the
     columns as a launch of its own does, and the results are the same bits."""
