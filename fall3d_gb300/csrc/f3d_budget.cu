@@ -340,14 +340,29 @@ __global__ void k_getc0(double* cdry, double* cwet, double* cload, Dims d, int n
   const long long pl = d.plane();
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= pl) return;
+  // four classes' loads in flight; the sums in class order
   double sd = 0.0, sw = 0.0;
-  for (int ic = 1; ic <= np; ++ic) {
-    sd = sd + cdry[ic * pl + p];
-    sw = sw + cwet[ic * pl + p];
+  for (int i0 = 1; i0 <= nc; i0 += 4) {
+    double a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = i0 + u <= nc;
+      a[u] = in ? cdry[(i0 + u) * pl + p] : 0.0;
+      b[u] = in ? cwet[(i0 + u) * pl + p] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i0 + u > nc) break;
+      if (i0 + u <= np) {
+        sd = sd + a[u];
+        sw = sw + b[u];
+      }
+      cload[(i0 + u) * pl + p] = a[u] + b[u];
+    }
   }
   cdry[p] = sd;
   cwet[p] = sw;
-  for (int ic = 0; ic <= nc; ++ic) cload[ic * pl + p] = cdry[ic * pl + p] + cwet[ic * pl + p];
+  cload[p] = sd + sw;
 }
 
 void launch_getc0(double* cdry, double* cwet, double* cload, Dims d, int nc, int np,

@@ -20,89 +20,162 @@ namespace {
 
 constexpr int OB = 128;  // threads per block: one column (i, j) each
 
-// sum over the listed classes of c(i,j,k,ic) (0 + c1 + c2 + ...)
+// The classes of an output variable (0-based) with AOT's qeff and
+// rhop*reff of each, as a kernel parameter; more than CMAX go to device arrays.
+constexpr int CMAX = 128;
+struct OutClasses {
+  int n;
+  const int* cls_more;
+  const double *q_more, *r_more;
+  unsigned short cls[CMAX];
+  double q[CMAX], r[CMAX];
+  __device__ int at(int i) const { return cls_more ? cls_more[i] : (int)cls[i]; }
+};
+
+// A binary32 value widened with integer operations (the conversion
+// instruction goes through the binary64 pipe, which these kernels are bound
+// by); exponent 0 and 255 take the conversion.
+__device__ __forceinline__ double widen(float v) {
+  const unsigned u = __float_as_uint(v), e = (u >> 23) & 255u;
+  if (e - 1u >= 254u) return (double)v;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
+// sum over the listed classes of c(i,j,k,ic) (0 + c1 + c2 + ...).  A zero
+// leaves the sum as it is and is skipped; eight loads are in flight.
 template <class T>
-__device__ __forceinline__ double class_sum(const T* c, long long hb, long long q, const int* cls,
-                                            int ncls) {
+__device__ __forceinline__ double class_sum(const T* c, long long hb, long long q, const OutClasses& cl) {
   double s = 0.0;
-  for (int n = 0; n < ncls; ++n) s = s + (double)c[(long long)cls[n] * hb + q];
+  for (int n0 = 0; n0 < cl.n; n0 += 8) {
+    T v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = n0 + u < cl.n ? c[(long long)cl.at(n0 + u) * hb + q] : T(0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (v[u] != T(0)) s = s + widen(v[u]);
+  }
   return s;
 }
+
+// one result value, in binary64 or rounded to binary32
+__device__ __forceinline__ void put(void* out, long long p, double v, int f32) {
+  if (f32)
+    reinterpret_cast<float*>(out)[p] = (float)v;
+  else
+    reinterpret_cast<double*>(out)[p] = v;
+}
+
+// The column variables take blocks of 32 columns by 8 warps: the warps form
+// the values of 8 levels at a time, the first warp adds their terms in the
+// reference's order.  They are bound by binary64 operations (a class's
+// addition and its conversion); with the conversion in integers, zeros
+// skipped and the division by Hm1 through its reciprocal (div_rn_recip) the
+// column mass of 400x300x50 cells and 16 classes takes 323 us instead of
+// 418 us, the optical thickness 187 us instead of 400 us.
+constexpr int CW = 8;
 
 // z-cumulative concentration, g/m2 (printres_nc.f90:216-246 particles and
 // gases, :281-387 PM05/PM10/PM20): w(k) = (sum over the classes)/Hm1,
 // work2d = sum_{k<nz} dz(k)*0.5*(w(k)+w(k+1)), times 1e3.
 template <class T>
-__global__ void k_out_column(const T* c, Dims d, const int* cls, int ncls, const double* dz,
-                             const double* Hm1, double* out) {
-  const long long p = blockIdx.x * (long long)OB + threadIdx.x;
-  if (p >= d.plane()) return;
-  const int i = (int)(p % d.nx) + 1, j = (int)(p / d.nx) + 1;
+__global__ void __launch_bounds__(32 * CW) k_out_column(const T* c, Dims d, const OutClasses cl, const double* dz,
+                                                        const double* Hm1, void* out, int f32) {
+  __shared__ double w[CW][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long p = blockIdx.x * 32LL + lane, pc = min(p, d.plane() - 1);
+  const int i = (int)(pc % d.nx) + 1, j = (int)(pc / d.nx) + 1;
   const long long hb = d.halo();
-  const double h = Hm1[p];
-  double acc = 0.0;
-  double wp = class_sum<T>(c, hb, d.C(i, j, 1), cls, ncls) / h;
-  for (int k = 1; k <= d.nz - 1; ++k) {
-    const double wn = class_sum<T>(c, hb, d.C(i, j, k + 1), cls, ncls) / h;
-    acc = acc + dz[k] * 0.5 * (wp + wn);
-    wp = wn;
+  const double h = Hm1[pc], rh = 1.0 / h;
+  double acc = 0.0, wp = 0.0;
+  for (int k0 = 1; k0 <= d.nz; k0 += CW) {
+    const int k = k0 + warp;
+    if (k <= d.nz) w[warp][lane] = div_rn_recip(class_sum<T>(c, hb, d.C(i, j, k), cl), h, rh);
+    __syncthreads();
+    if (warp == 0)
+      for (int u = 0; u < CW && k0 + u <= d.nz; ++u) {
+        const double wn = w[u][lane];
+        const double two = wp + wn;
+        if (k0 + u > 1 && two != 0.0) acc = acc + dz[k0 + u - 1] * 0.5 * two;
+        wp = wn;
+      }
+    __syncthreads();
   }
-  out[p] = 1e3 * acc;
+  if (warp == 0 && p < d.plane()) put(out, p, 1e3 * acc, f32);
 }
 
 // concentration at the first layer, g/m3 (printres_nc.f90:389-493):
 // 1e3*(sum over the classes of c(i,j,1,ic))/Hm1.
 template <class T>
-__global__ void k_out_ground(const T* c, Dims d, const int* cls, int ncls, const double* Hm1,
-                             double* out) {
+__global__ void k_out_ground(const T* c, Dims d, const OutClasses cl, const double* Hm1, void* out, int f32) {
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
   if (p >= d.plane()) return;
   const int i = (int)(p % d.nx) + 1, j = (int)(p / d.nx) + 1;
-  const double s = class_sum<T>(c, d.halo(), d.C(i, j, 1), cls, ncls);
-  out[p] = 1e3 * s / Hm1[p];
+  const double s = class_sum<T>(c, d.halo(), d.C(i, j, 1), cl);
+  put(out, p, 1e3 * s / Hm1[p], f32);
 }
 
 // aerosol optical thickness (printres_nc.f90:495-540): for each aerosol
 // class in class order and each layer upwards,
 // work2d += dz(k)*0.5*(w(k)+w(k+1))*0.75*Qeff(ieff)/(rhop(ic)*reff(ieff))
-// with w = c(ic)/Hm1; qeff[n] and den[n] = rhop*reff belong to cls[n].
+// with w = c(ic)/Hm1; q[n] = qeff and r[n] = rhop*reff belong to class n.
 template <class T>
-__global__ void k_out_aot(const T* c, Dims d, const int* cls, const double* qeff, const double* den,
-                          int ncls, const double* dz, const double* Hm1, double* out) {
-  const long long p = blockIdx.x * (long long)OB + threadIdx.x;
-  if (p >= d.plane()) return;
-  const int i = (int)(p % d.nx) + 1, j = (int)(p / d.nx) + 1;
+__global__ void __launch_bounds__(32 * CW) k_out_aot(const T* c, Dims d, const OutClasses cl, const double* dz,
+                                                     const double* Hm1, void* out, int f32) {
+  __shared__ double w[CW + 1][32], term[CW][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long p = blockIdx.x * 32LL + lane, pc = min(p, d.plane() - 1);
+  const int i = (int)(pc % d.nx) + 1, j = (int)(pc / d.nx) + 1;
   const long long hb = d.halo();
-  const double h = Hm1[p];
+  const double h = Hm1[pc], rh = 1.0 / h;
+  const bool h_plain = div_in_range(h);  // 0/h is 0
   double acc = 0.0;
-  for (int n = 0; n < ncls; ++n) {
-    const T* cc = c + (long long)cls[n] * hb;
-    const double q = qeff[n], r = den[n];
-    double wp = (double)cc[d.C(i, j, 1)] / h;
-    for (int k = 1; k <= d.nz - 1; ++k) {
-      const double wn = (double)cc[d.C(i, j, k + 1)] / h;
-      acc = acc + dz[k] * 0.5 * (wp + wn) * 0.75 * q / r;
-      wp = wn;
+  for (int n = 0; n < cl.n; ++n) {
+    const T* cc = c + (long long)cl.at(n) * hb;
+    const double q = cl.q_more ? cl.q_more[n] : cl.q[n], r = cl.r_more ? cl.r_more[n] : cl.r[n], rr = 1.0 / r;
+    const bool q_plain = div_in_range(r) && fabs(q) < 1e300;  // 0*q/r is 0
+    for (int k0 = 1; k0 <= d.nz - 1; k0 += CW) {  // layers k0 .. k0+CW-1, levels to k0+CW
+      const int k = k0 + warp;
+      auto W = [&](int kk) {
+        const T v = cc[d.C(i, j, kk)];
+        return v == T(0) && h_plain ? 0.0 : div_rn_recip(widen(v), h, rh);
+      };
+      if (k <= d.nz) w[warp][lane] = W(k);
+      if (warp == 0 && k0 + CW <= d.nz) w[CW][lane] = W(k0 + CW);
+      __syncthreads();
+      if (k <= d.nz - 1) {
+        const double two = w[warp][lane] + w[warp + 1][lane];
+        term[warp][lane] = two == 0.0 && q_plain ? 0.0 : div_rn_recip(dz[k] * 0.5 * two * 0.75 * q, r, rr);
+      }
+      __syncthreads();
+      if (warp == 0)
+        for (int u = 0; u < CW && k0 + u <= d.nz - 1; ++u)
+          if (term[u][lane] != 0.0) acc = acc + term[u][lane];
     }
+    __syncthreads();
   }
-  out[p] = acc;
+  if (warp == 0 && p < d.plane()) put(out, p, acc, f32);
 }
 
 // deposit plane (printres_nc.f90:105-189): field(:,:,ic)/Hm1 of cload or cwet
-__global__ void k_out_plane(const double* f, long long n, const double* Hm1, double* out) {
+__global__ void k_out_plane(const double* f, long long n, const double* Hm1, void* out, int f32) {
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
-  if (p < n) out[p] = f[p] / Hm1[p];
+  if (p < n) put(out, p, f[p] / Hm1[p], f32);
 }
 
 // deposit thickness, cm (printres_nc.f90:191-214): 1e2*(sum over particle
-// classes of cload(ic)/rhop(ic))/Hm1.
+// classes of cload(ic)/rhop(ic))/Hm1; the reciprocals of rhop once per block.
 __global__ void k_out_thick(const double* cload, long long pl, int np, const double* rhop,
-                            const double* Hm1, double* out) {
+                            const double* Hm1, void* out, int f32) {
+  extern __shared__ double rr[];
+  for (int ic = threadIdx.x; ic < np; ic += OB) rr[ic] = 1.0 / rhop[ic];
+  __syncthreads();
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
   if (p >= pl) return;
   double s = 0.0;
-  for (int ic = 1; ic <= np; ++ic) s = s + cload[(long long)ic * pl + p] / rhop[ic - 1];
-  out[p] = 1e2 * s / Hm1[p];
+  for (int ic = 1; ic <= np; ++ic)
+    s = s + div_rn_recip(cload[(long long)ic * pl + p], rhop[ic - 1], rr[ic - 1]);
+  put(out, p, 1e2 * s / Hm1[p], f32);
 }
 
 // concentration at a flight level, g/m3 (printres_nc.f90:542-573 and
@@ -111,8 +184,8 @@ __global__ void k_out_thick(const double* cload, long long pl, int np, const dou
 // pressures bracket pnom (p(k) >= pnom > p(k+1)), 0 below the first layer
 // or when no pair of layers brackets it; times 1e3.
 template <class T>
-__global__ void k_out_fl(const T* c, Dims d, const int* cls, int ncls, const double* pres,
-                         double pnom, const double* Hm1, double* out) {
+__global__ void k_out_fl(const T* c, Dims d, const OutClasses cl, const double* pres,
+                         double pnom, const double* Hm1, void* out, int f32) {
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
   const long long pl = d.plane();
   if (p >= pl) return;
@@ -125,14 +198,14 @@ __global__ void k_out_fl(const T* c, Dims d, const int* cls, int ncls, const dou
         const double s = (pnom - pk) / (pk1 - pk);
         const double h = Hm1[p];
         const long long hb = d.halo();
-        const double wk = class_sum<T>(c, hb, d.C(i, j, k), cls, ncls) / h;
-        const double wk1 = class_sum<T>(c, hb, d.C(i, j, k + 1), cls, ncls) / h;
+        const double wk = class_sum<T>(c, hb, d.C(i, j, k), cl) / h;
+        const double wk1 = class_sum<T>(c, hb, d.C(i, j, k + 1), cl) / h;
         v = wk * (1.0 - s) + wk1 * s;
         break;
       }
     }
   }
-  out[p] = 1e3 * v;
+  put(out, p, 1e3 * v, f32);
 }
 
 // 3-D concentration, g/m3 (printres_nc.f90:575-601 all particles,
@@ -141,20 +214,28 @@ __global__ void k_out_fl(const T* c, Dims d, const int* cls, int ncls, const dou
 // Sources/ter2asl.f90:1-55 (linear in height between the terrain-following
 // levels that bracket zlayer(k) above max(0,topg); 0 below the first level
 // and above the last).
+// The model levels take a thread per column and level.
 template <class T>
-__global__ void k_out_con(const T* c, Dims d, const int* cls, int ncls, const double* Hm1,
-                          const double* zlayer, const double* topg, int asl, double* out) {
+__global__ void k_out_con(const T* c, Dims d, const OutClasses cl, const double* Hm1, void* out, int f32) {
+  const long long p = blockIdx.x * (long long)OB + threadIdx.x;
+  const long long pl = d.plane();
+  if (p >= pl) return;
+  const int i = (int)(p % d.nx) + 1, j = (int)(p / d.nx) + 1;
+  const long long hb = d.halo();
+  const double h = Hm1[p], rh = 1.0 / h;
+  for (int k = blockIdx.y + 1; k <= d.nz; k += gridDim.y)
+    put(out, (long long)(k - 1) * pl + p, 1e3 * div_rn_recip(class_sum<T>(c, hb, d.C(i, j, k), cl), h, rh), f32);
+}
+template <class T>
+__global__ void k_out_con_asl(const T* c, Dims d, const OutClasses cl, const double* Hm1, const double* zlayer,
+                              const double* topg, void* out, int f32) {
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
   const long long pl = d.plane();
   if (p >= pl) return;
   const int i = (int)(p % d.nx) + 1, j = (int)(p / d.nx) + 1;
   const long long hb = d.halo();
   const double h = Hm1[p];
-  auto val = [&](int k) { return 1e3 * (class_sum<T>(c, hb, d.C(i, j, k), cls, ncls) / h); };
-  if (!asl) {
-    for (int k = 1; k <= d.nz; ++k) out[(long long)(k - 1) * pl + p] = val(k);
-    return;
-  }
+  auto val = [&](int k) { return 1e3 * (class_sum<T>(c, hb, d.C(i, j, k), cl) / h); };
   const double zo = fmax2(0.0, topg[p]);
   for (int k = 1; k <= d.nz; ++k) {
     const double zasl = zlayer[k - 1];
@@ -168,7 +249,7 @@ __global__ void k_out_con(const T* c, Dims d, const int* cls, int ncls, const do
         }
       }
     }
-    out[(long long)(k - 1) * pl + p] = v;
+    put(out, (long long)(k - 1) * pl + p, v, f32);
   }
 }
 
@@ -176,7 +257,7 @@ __global__ void k_out_con(const T* c, Dims d, const int* cls, int ncls, const do
 // heights above sea level by ter2asl: the gravity-current winds
 // (printres_nc.f90:603-644: vx*Hm1, vy*Hm1) and Maggr (:673-690)
 __global__ void k_out_field(const double* f, int times_hm1, Dims d, const double* Hm1,
-                            const double* zlayer, const double* topg, int asl, double* out) {
+                            const double* zlayer, const double* topg, int asl, void* out, int f32) {
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
   const long long pl = d.plane();
   if (p >= pl) return;
@@ -186,7 +267,7 @@ __global__ void k_out_field(const double* f, int times_hm1, Dims d, const double
     return times_hm1 ? v * h : v;
   };
   if (!asl) {
-    for (int k = 1; k <= d.nz; ++k) out[(long long)(k - 1) * pl + p] = val(k);
+    for (int k = 1; k <= d.nz; ++k) put(out, (long long)(k - 1) * pl + p, val(k), f32);
     return;
   }
   const double zo = fmax2(0.0, topg[p]);
@@ -202,7 +283,7 @@ __global__ void k_out_field(const double* f, int times_hm1, Dims d, const double
         }
       }
     }
-    out[(long long)(k - 1) * pl + p] = v;
+    put(out, (long long)(k - 1) * pl + p, v, f32);
   }
 }
 
@@ -298,12 +379,6 @@ __global__ void k_track(const T* c, const double* cload, Dims d, int np, const i
   for (int ic = 1; ic <= np; ++ic) o[8 + 3 * nz + ic - 1] = pl4(cload + (long long)ic * pl);
 }
 
-__global__ void k_out_to_f32(const double* a, long long n, float* b) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x)
-    b[q] = (float)a[q];
-}
-
 unsigned blocks(long long n) { return (unsigned)((n + OB - 1) / OB); }
 
 // Sources/printres_nc.f90:2066-2123 (get_AOT_prop): effective radii in
@@ -344,8 +419,7 @@ double standard_pressure(double z) {
   return po2 * std::pow(To2 / T, goo * Moo / (Roo * Lo2));
 }
 
-// One device scratch block of the call: the (nx,ny[,nz]) binary64 result,
-// its binary32 copy and the class tables.
+// A device allocation of one call, given back on its stream.
 struct Scratch {
   void* p = nullptr;
   cudaStream_t s = nullptr;
@@ -354,19 +428,75 @@ struct Scratch {
   }
 };
 
-int finish(f3d_ctx* x, double* res, long long n, void* dst, int dst_type, Scratch& sc) {
-  cudaStream_t s = x->stream;
-  if (dst_type == F3D_OUT_BINARY32) {
-    float* f = reinterpret_cast<float*>(res + n);
-    k_out_to_f32<<<(unsigned)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, s>>>(res, n, f);
-    count_launch();
-    OK(cudaMemcpyAsync(dst, f, sizeof(float) * n, cudaMemcpyDefault, s));
-  } else {
-    OK(cudaMemcpyAsync(dst, res, sizeof(double) * n, cudaMemcpyDefault, s));
+// Where a call's kernel writes its n values of the wanted type: the
+// destination itself if it is aligned memory of this device, else the
+// context's plane buffer (2-D variables) or a buffer of the call (3-D), from
+// which finish() copies.
+struct Result {
+  void* p = nullptr;
+  size_t bytes = 0;
+  Scratch own;
+};
+
+int result_buffer(f3d_ctx* x, long long n, void* dst, int dst_type, Result& r) {
+  const size_t size = dst_type == F3D_OUT_BINARY32 ? sizeof(float) : sizeof(double);
+  r.bytes = size * (size_t)n;
+  cudaPointerAttributes at{};
+  int dev = -1;
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+    cudaGetLastError();
+    at.type = cudaMemoryTypeHost;
   }
+  OK(cudaGetDevice(&dev));
+  if (at.type == cudaMemoryTypeDevice && at.device == dev && reinterpret_cast<size_t>(dst) % size == 0) {
+    r.p = dst;
+  } else if (n <= x->d.plane()) {
+    if (!x->out_plane)
+      if (int rc = f3d::ctx_alloc(x, &x->out_plane, sizeof(double) * (size_t)x->d.plane())) return rc;
+    r.p = x->out_plane;
+  } else {
+    r.own.s = x->stream;
+    OK(cudaMallocAsync(&r.own.p, r.bytes, x->stream));
+    r.p = r.own.p;
+  }
+  return F3D_OK;
+}
+
+int finish(f3d_ctx* x, const Result& r, void* dst) {
+  cudaStream_t s = x->stream;
+  if (r.p != dst) OK(cudaMemcpyAsync(dst, r.p, r.bytes, cudaMemcpyDefault, s));
   OK(cudaGetLastError());
   OK(cudaStreamSynchronize(s));
-  (void)sc;
+  return F3D_OK;
+}
+
+// The kernel parameter of a class list; lists longer than it holds are copied
+// to `more` (device memory of the call).
+int class_list(f3d_ctx* x, const std::vector<int>& cls, const std::vector<double>& q, const std::vector<double>& r,
+               OutClasses& o, Scratch& more) {
+  o = OutClasses{};
+  o.n = (int)cls.size();
+  if (cls.size() <= (size_t)CMAX) {
+    for (size_t i = 0; i < cls.size(); ++i) o.cls[i] = (unsigned short)cls[i];
+    for (size_t i = 0; i < q.size(); ++i) {
+      o.q[i] = q[i];
+      o.r[i] = r[i];
+    }
+    return F3D_OK;
+  }
+  const size_t n = cls.size();
+  more.s = x->stream;
+  OK(cudaMallocAsync(&more.p, (2 * sizeof(double) + sizeof(int)) * n, x->stream));
+  double* dq = reinterpret_cast<double*>(more.p);
+  int* dc = reinterpret_cast<int*>(dq + 2 * n);
+  OK(cudaMemcpyAsync(dc, cls.data(), sizeof(int) * n, cudaMemcpyHostToDevice, x->stream));
+  if (!q.empty()) {
+    OK(cudaMemcpyAsync(dq, q.data(), sizeof(double) * n, cudaMemcpyHostToDevice, x->stream));
+    OK(cudaMemcpyAsync(dq + n, r.data(), sizeof(double) * n, cudaMemcpyHostToDevice, x->stream));
+    o.q_more = dq;
+    o.r_more = dq + n;
+  }
+  o.cls_more = dc;
   return F3D_OK;
 }
 
@@ -459,21 +589,13 @@ int f3d_output(f3d_ctx* x, int var, int index, int asl, void* dst, int dst_type)
       return f3d::ctx_error(F3D_ERR_ARG, "unknown output variable");
   }
   cudaStream_t s = x->stream;
-  Scratch sc;
-  sc.s = s;
-  const size_t tab = 3 * sizeof(double) * (cls.size() + 1);
-  OK(cudaMallocAsync(&sc.p, sizeof(double) * n + sizeof(float) * n + tab + 64, s));
-  double* res = reinterpret_cast<double*>(sc.p);
-  unsigned char* t = reinterpret_cast<unsigned char*>(sc.p) + ((sizeof(double) * n + sizeof(float) * n + 15) & ~size_t(15));
-  int* dcls = reinterpret_cast<int*>(t);
-  double* dq = reinterpret_cast<double*>(t + sizeof(double) * (cls.size() + 1));
-  double* dr = dq + cls.size() + 1;
-  if (!cls.empty()) OK(cudaMemcpyAsync(dcls, cls.data(), sizeof(int) * cls.size(), cudaMemcpyHostToDevice, s));
-  if (!q.empty()) {
-    OK(cudaMemcpyAsync(dq, q.data(), sizeof(double) * q.size(), cudaMemcpyHostToDevice, s));
-    OK(cudaMemcpyAsync(dr, r.data(), sizeof(double) * r.size(), cudaMemcpyHostToDevice, s));
-  }
-  const int ncls = (int)cls.size();
+  Scratch more;
+  OutClasses cl;
+  Result res;
+  if (int rc = class_list(x, cls, q, r, cl, more)) return rc;
+  if (int rc = result_buffer(x, n, dst, dst_type, res)) return rc;
+  const int o32 = dst_type == F3D_OUT_BINARY32;
+  const unsigned cb = (unsigned)((pl + 31) / 32);
   const bool f32 = x->prec == F3D_PREC_FP32;
   switch (var) {
     case F3D_OUT_LOAD:
@@ -481,47 +603,52 @@ int f3d_output(f3d_ctx* x, int var, int index, int asl, void* dst, int dst_type)
     case F3D_OUT_THICK:
       launch_getc0(x->cdry, x->cwet, x->cload, d, nc, np, s);
       if (var == F3D_OUT_THICK)
-        k_out_thick<<<blocks(pl), OB, 0, s>>>(x->cload, pl, np, x->rhop, x->Hm1, res);
+        k_out_thick<<<blocks(pl), OB, sizeof(double) * (np > 0 ? np : 1), s>>>(x->cload, pl, np, x->rhop, x->Hm1,
+                                                                              res.p, o32);
       else
         k_out_plane<<<blocks(pl), OB, 0, s>>>((var == F3D_OUT_LOAD ? x->cload : x->cwet) + index * pl, pl,
-                                              x->Hm1, res);
+                                              x->Hm1, res.p, o32);
       break;
     case F3D_OUT_COL_MASS:
     case F3D_OUT_PM_COL:
       if (f32)
-        k_out_column<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, dcls, ncls, x->dz, x->Hm1, res);
+        k_out_column<float><<<cb, 32 * CW, 0, s>>>(x->c32, d, cl, x->dz, x->Hm1, res.p, o32);
       else
-        k_out_column<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, dcls, ncls, x->dz, x->Hm1, res);
+        k_out_column<double><<<cb, 32 * CW, 0, s>>>(x->c64, d, cl, x->dz, x->Hm1, res.p, o32);
       break;
     case F3D_OUT_C_GRND:
     case F3D_OUT_PM_GRND:
       if (f32)
-        k_out_ground<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, dcls, ncls, x->Hm1, res);
+        k_out_ground<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, cl, x->Hm1, res.p, o32);
       else
-        k_out_ground<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, dcls, ncls, x->Hm1, res);
+        k_out_ground<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, cl, x->Hm1, res.p, o32);
       break;
     case F3D_OUT_AOT05:
       if (f32)
-        k_out_aot<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, dcls, dq, dr, ncls, x->dz, x->Hm1, res);
+        k_out_aot<float><<<cb, 32 * CW, 0, s>>>(x->c32, d, cl, x->dz, x->Hm1, res.p, o32);
       else
-        k_out_aot<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, dcls, dq, dr, ncls, x->dz, x->Hm1, res);
+        k_out_aot<double><<<cb, 32 * CW, 0, s>>>(x->c64, d, cl, x->dz, x->Hm1, res.p, o32);
       break;
     case F3D_OUT_WIND:
     case F3D_OUT_MAGGR:
       k_out_field<<<blocks(pl), OB, 0, s>>>(var == F3D_OUT_MAGGR ? x->agr_maggr : (index == 1 ? x->vx : x->vy),
-                                            var == F3D_OUT_WIND, d, x->Hm1, x->zlayer, x->topg, asl, res);
+                                            var == F3D_OUT_WIND, d, x->Hm1, x->zlayer, x->topg, asl, res.p, o32);
       break;
-    case F3D_OUT_CON:
-      if (f32)
-        k_out_con<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, dcls, ncls, x->Hm1, x->zlayer, x->topg, asl,
-                                                   res);
+    case F3D_OUT_CON: {
+      const dim3 grid(blocks(pl), (unsigned)std::min(d.nz, 65535));
+      if (f32 && asl)
+        k_out_con_asl<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, cl, x->Hm1, x->zlayer, x->topg, res.p, o32);
+      else if (asl)
+        k_out_con_asl<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, cl, x->Hm1, x->zlayer, x->topg, res.p, o32);
+      else if (f32)
+        k_out_con<float><<<grid, OB, 0, s>>>(x->c32, d, cl, x->Hm1, res.p, o32);
       else
-        k_out_con<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, dcls, ncls, x->Hm1, x->zlayer, x->topg,
-                                                    asl, res);
+        k_out_con<double><<<grid, OB, 0, s>>>(x->c64, d, cl, x->Hm1, res.p, o32);
       break;
+    }
   }
   count_launch();
-  return finish(x, res, n, dst, dst_type, sc);
+  return finish(x, res, dst);
 }
 
 int f3d_track_points(f3d_ctx* x, int npts, const double* xpts, const double* ypts, double xo, double yo,
@@ -616,23 +743,23 @@ int f3d_output_fl(f3d_ctx* x, double flight_level, const double* p, void* dst, i
   const Dims d = x->d;
   const long long pl = d.plane(), s3 = d.cells();
   const double pnom = standard_pressure(flight_level * 30.48);  // printres_nc.f90:559
-  const std::vector<int> cls = particle_classes(x);
   cudaStream_t s = x->stream;
-  Scratch sc;
+  Scratch more, sc;
+  OutClasses cl;
+  Result res;
+  if (int rc = class_list(x, particle_classes(x), {}, {}, cl, more)) return rc;
+  if (int rc = result_buffer(x, pl, dst, dst_type, res)) return rc;
   sc.s = s;
-  const size_t head = (sizeof(double) * pl + sizeof(float) * pl + 15) & ~size_t(15);
-  OK(cudaMallocAsync(&sc.p, head + sizeof(double) * s3 + sizeof(int) * (cls.size() + 1) + 64, s));
-  double* res = reinterpret_cast<double*>(sc.p);
-  double* dp = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(sc.p) + head);
-  int* dcls = reinterpret_cast<int*>(dp + s3);
+  OK(cudaMallocAsync(&sc.p, sizeof(double) * s3, s));
+  double* dp = reinterpret_cast<double*>(sc.p);
   OK(cudaMemcpyAsync(dp, p, sizeof(double) * s3, cudaMemcpyDefault, s));
-  if (!cls.empty()) OK(cudaMemcpyAsync(dcls, cls.data(), sizeof(int) * cls.size(), cudaMemcpyHostToDevice, s));
+  const int o32 = dst_type == F3D_OUT_BINARY32;
   if (x->prec == F3D_PREC_FP32)
-    k_out_fl<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, dcls, (int)cls.size(), dp, pnom, x->Hm1, res);
+    k_out_fl<float><<<blocks(pl), OB, 0, s>>>(x->c32, d, cl, dp, pnom, x->Hm1, res.p, o32);
   else
-    k_out_fl<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, dcls, (int)cls.size(), dp, pnom, x->Hm1, res);
+    k_out_fl<double><<<blocks(pl), OB, 0, s>>>(x->c64, d, cl, dp, pnom, x->Hm1, res.p, o32);
   count_launch();
-  return finish(x, res, pl, dst, dst_type, sc);
+  return finish(x, res, dst);
 }
 
 }  // extern "C"
