@@ -25,8 +25,15 @@
 // operations: the class-independent factors of a line are formed once for
 // all classes, values shared by neighbouring cells are formed once, the
 // limiter's sign and minimum logic runs on the bit patterns, and divisions
-// by a per-launch or per-meteo-update divisor use its reciprocal with
-// Markstein's correction (div_rn_recip, f3d_common.cuh).
+// by a per-launch or per-meteo-update divisor use its reciprocal with an exact
+// correction in integers (div_rn_recip, f3d_common.cuh).  What bounds them is
+// the binary64 pipe, 16 cycles per warp instruction and SM, busy 77-91% of the
+// time; per cell and class of 400x300x50 cells the sweeps issue
+//   advctzc 19.6 (28.1 before the bit patterns went through opaque moves, the
+//     upwind side was selected instead of branched to and the slope carried),
+//   advctx 11.6 (21.6), advcty 12.2 (20.6), diffz 8.9 (19.3), diffx 7.6 (9.2),
+//   diffy 6.9 (7.4),
+// and a step of 16 classes takes 13.1 ms (19.0 ms).
 #include <algorithm>
 #include <cstdio>
 
@@ -134,23 +141,24 @@ void launch_setbcc(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, cons
 template <class T>
 struct ZTab {  // per-level constants of advctzc.f90:34-36 (IEEE, as on the host)
   T dzz, dzk, dzk_1, hdzm1;  // hdzm1 = (dt*0.5)*dz(k-1), the first factors of work(k,2)
+                             // dzk_1(k) is dzk(k-1)
 };
 
 // work(k,1), work(k,2) (advctzc.f90:37-46) at a level with c0 = c(k),
 // cp = c(k+1), vk = vk(k), vk_1 = vk(k-1), given the previous level's
-// product pm = vk(k-1)*c(k-1) and difference dm = c(k)-c(k-1); returns this
-// level's p0 = vk(k)*c(k) and d0 = c(k+1)-c(k) for the next one (the
-// reference forms both twice, with the same operations).
+// product pm = vk(k-1)*c(k-1) and slope sm = (c(k)-c(k-1))*(1/dz(k-1));
+// returns this level's p0 = vk(k)*c(k) and s0 = (c(k+1)-c(k))*(1/dz(k)) for the
+// next one (the reference forms both twice, with the same operations).
 template <class T>
-__device__ __forceinline__ void adv_z_work(T c0, T cp, T vk, T vk_1, T pm, T dm, const ZTab<T>& z, T dt,
-                                           T& w1, T& w2, T& p0, T& d0) {
-  const T vk_12 = T(0.5) * (vk + vk_1);
+__device__ __forceinline__ void adv_z_work(T c0, T cp, T vk, T vk_1, T pm, T sm, const ZTab<T>& z, T dt,
+                                           T& w1, T& w2, T& p0, T& s0) {
   p0 = vk * c0;
   w1 = dt * (p0 - pm) * z.dzz;
-  d0 = cp - c0;
-  const T sigma = minmod_ref(d0 * z.dzk, dm * z.dzk_1);
-  const T Crk = absd(vk_12) * dt * z.dzk_1;
-  w2 = z.hdzm1 * (T(1) - Crk) * sigma * absd(vk_12) * z.dzz;
+  s0 = (cp - c0) * z.dzk;
+  const T sigma = minmod_ref(s0, sm);
+  const T av = absd(half_of(vk + vk_1));
+  const T Crk = av * dt * z.dzk_1;
+  w2 = z.hdzm1 * (T(1) - Crk) * sigma * av * z.dzz;
 }
 
 template <class T>
@@ -180,13 +188,13 @@ __global__ void k_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_lo
   T c_m1 = CO(kb - 1), c_0 = CO(kb), c_p1 = CO(kb + 1);
   T vk_0 = VK(kb), vk_m1 = VK(kb > 1 ? kb - 1 : 1);
   T w1_k, w2_k, w2_km, pk, dk;
-  adv_z_work(c_0, c_p1, vk_0, vk_m1, vk_m1 * c_m1, c_0 - c_m1, tab[kb], dt, w1_k, w2_k, pk, dk);
+  adv_z_work(c_0, c_p1, vk_0, vk_m1, vk_m1 * c_m1, (c_0 - c_m1) * tab[kb].dzk_1, tab[kb], dt, w1_k, w2_k, pk, dk);
   if (kb == 1) {
     w2_km = w2_k;
   } else {
     T w1_dummy, p_dummy, d_dummy;
     const T c_m2 = CO(kb - 2), vk_m2 = VK(kb - 1 > 1 ? kb - 2 : 1);
-    adv_z_work(c_m1, c_0, vk_m1, vk_m2, vk_m2 * c_m2, c_m1 - c_m2, tab[kb - 1], dt, w1_dummy, w2_km,
+    adv_z_work(c_m1, c_0, vk_m1, vk_m2, vk_m2 * c_m2, (c_m1 - c_m2) * tab[kb - 1].dzk_1, tab[kb - 1], dt, w1_dummy, w2_km,
                p_dummy, d_dummy);
   }
   for (int k = kb; k <= ke; ++k) {
@@ -199,12 +207,10 @@ __global__ void k_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_lo
       w1_n = dt * vk_0 * (c_p1 - c_0) * dznz;  // work(nz+1,1), advctzc.f90:58-64
       w2_n = w2_k;                             // kmin = nz
     }
-    T cn;
-    if (gt0(vk_0))
-      cn = c_0 - w1_k - (w2_k - w2_km);
-    else
-      cn = c_0 - w1_n - (w2_n - w2_k);
-    cc[cb + k * cs] = cn;
+    // the upwind side's operands are selected, so that a warp whose columns
+    // differ in the sign issues the three subtractions once
+    const bool up = gt0(vk_0);
+    cc[cb + k * cs] = c_0 - (up ? w1_k : w1_n) - ((up ? w2_k : w2_n) - (up ? w2_km : w2_k));
     w2_km = w2_k;
     w2_k = w2_n;
     w1_k = w1_n;
@@ -236,96 +242,97 @@ void launch_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, con
 // class: the class-independent factors of the line are formed once,
 //   a(q) = |0.5*(v(q)+v(q-1))|,  b(q) = (dt*0.5)*(1 - auxv*a(q)),
 // so that work(q,2) = dt*0.5*(1-Cri)*sigma*|v_12| is (b(q)*sigma)*a(q),
-// the reference's product left to right; then per class the line's
-// concentrations are staged with the products v(q)*c(q) and differences
-// c(q+1)-c(q) that neighbouring positions share (each formed once, as the
-// reference forms it), work(q,1), work(q,2) formed and the line updated.
+// the reference's product left to right; then per class the products
+// v(q)*c(q) and differences c(q+1)-c(q) that neighbouring positions share are
+// staged (each formed once, as the reference forms it), work(q,1), work(q,2)
+// formed and the line updated.  The kernels are bound by binary64 operations,
+// 10 per cell and class.
+// What a line's kernel stages: the x sweep (DP) the differences and products,
+// its update reads c(q) again; the y sweep (CP) c and the products, forming
+// the differences twice: reading c again costs it more than that addition
+// (400x300x20 cells, 4 classes: 0.329 ms against 0.264 ms; x 0.223 ms against
+// 0.248 ms).  A line too long for seven arrays in a block's shared memory does
+// without the products (C).
+enum AdvStage : int { ADV_DP, ADV_CP, ADV_C };
+constexpr int adv_arrays(int mode) { return mode == ADV_C ? 6 : 7; }
+
 template <class T>
 struct AdvLine {  // a line's staged arrays at stride st
-  T *v, *a, *b, *cl, *w1, *w2;
-  T *p, *dc;  // p(q) = v(q)*c(q) (1..n), dc(q) = c(q+1)-c(q) (0..n): shared by neighbours
+  T *v, *a, *b, *w1, *w2;
+  T* cd;  // dc(q) = c(q+1)-c(q) (0..n) or c(q) (0..n+1)
+  T* p;   // v(q)*c(q) (0..n, v(0) = v(1))
 };
+template <class T>
+__device__ __forceinline__ AdvLine<T> adv_line(T* base, size_t n2) {
+  return AdvLine<T>{base, base + n2, base + 2 * n2, base + 3 * n2, base + 4 * n2, base + 5 * n2, base + 6 * n2};
+}
 
-// Stages position q (0..n+1) of a class's line: c, and the products and
-// differences that work(q,1) and the limiter of neighbouring positions share.
-// c0 = c(q), c1 = c(q+1) (read only for q <= n).  SH: stage p and dc (the
-// x sweep); the y sweep's tiles of lines keep to six arrays, whose shared
-// memory lets more blocks share an SM, and form them per position.
-template <bool SH, class T>
-__device__ __forceinline__ void adv_line_stage(const AdvLine<T>& L, int q, int n, int st, T c0, T c1) {
-  L.cl[q * st] = c0;
-  if constexpr (SH) {
-    if (q >= 1 && q <= n) L.p[q * st] = L.v[q * st] * c0;
-    if (q <= n) L.dc[q * st] = c1 - c0;
-  }
+// Stages position q (0..n; without dc to n+1) of a class's line whose
+// positions are cst apart at c.
+template <int MODE, class T>
+__device__ __forceinline__ void adv_line_stage(const AdvLine<T>& L, int q, int n, int st, const T* c, long long cst) {
+  const T c0 = c[q * cst];
+  L.cd[q * st] = MODE == ADV_DP ? c[(q + 1) * cst] - c0 : c0;
+  if (MODE != ADV_C && (MODE == ADV_DP || q <= n)) L.p[q * st] = L.v[q * st] * c0;
 }
 
 template <class T>
 __device__ __forceinline__ void adv_line_coef(T vq, T vq_1, T auxv, T dth, T& a, T& b) {
-  a = absd(T(0.5) * (vq + vq_1));
+  a = absd(half_of(vq + vq_1));
   b = dth * (T(1) - auxv * a);
 }
 
 // work(q,1), work(q,2) of position q (1..n), or work(n+1,1) (advctx.f90:46)
-template <bool SH, class T>
+template <int MODE, class T>
 __device__ __forceinline__ void adv_line_work(const AdvLine<T>& L, int q, int n, int st, T dx, T rdx, T auxv) {
-  auto C = [&](int i) { return L.cl[i * st]; };
+  auto D = [&](int i) { return MODE == ADV_DP ? L.cd[i * st] : L.cd[(i + 1) * st] - L.cd[i * st]; };
+  auto P = [&](int i) { return MODE == ADV_C ? L.v[i * st] * L.cd[i * st] : L.p[i * st]; };
   if (q > n) {
-    L.w1[(n + 1) * st] = auxv * L.v[n * st] * (SH ? L.dc[n * st] : C(n + 1) - C(n));
+    L.w1[(n + 1) * st] = auxv * L.v[n * st] * D(n);
     return;
   }
-  const T vq = L.v[q * st], vq_1 = L.v[(q > 1 ? q - 1 : 1) * st];
-  if constexpr (SH) {
-    // vq_1*c(q-1) is the left neighbour's product, or v(1)*c(0) at q = 1
-    const T pl = q > 1 ? L.p[(q - 1) * st] : vq_1 * C(0);
-    L.w1[q * st] = auxv * (L.p[q * st] - pl);
-  } else {
-    L.w1[q * st] = auxv * (vq * C(q) - vq_1 * C(q - 1));
-  }
-  const T sigma = SH ? minmod_div(L.dc[q * st], L.dc[(q - 1) * st], dx, rdx)
-                     : minmod_div(C(q + 1) - C(q), C(q) - C(q - 1), dx, rdx);
+  L.w1[q * st] = auxv * (P(q) - P(q - 1));
+  const T sigma = minmod_div(D(q), D(q - 1), dx, rdx);
   L.w2[q * st] = L.b[q * st] * sigma * L.a[q * st];
 }
 
 template <class T>
-__device__ __forceinline__ T adv_line_update(const AdvLine<T>& L, int q, int n, int st) {
-  const T cq = L.cl[q * st], vq = L.v[q * st];
-  if (gt0(vq)) return cq - L.w1[q * st] - (L.w2[q * st] - L.w2[(q > 1 ? q - 1 : 1) * st]);
-  return cq - L.w1[(q + 1) * st] - (L.w2[(q < n ? q + 1 : n) * st] - L.w2[q * st]);
+__device__ __forceinline__ T adv_line_update(const AdvLine<T>& L, T cq, int q, int n, int st) {
+  // the upwind side by its index: one issue of the three subtractions
+  const int r = gt0(L.v[q * st]) ? q : q + 1;
+  return cq - L.w1[r * st] - (L.w2[(r < n ? r : n) * st] - L.w2[(r > 1 ? r - 1 : 1) * st]);
 }
 
 // One block per x line (j,k) through classes 0..ncls-1; threads stride over i.
 template <class T>
-__global__ void k_advctx(T* c, long long cstride, int ncls, Dims d, int iz_loc, const T* vx, T dx, T dt) {
+__global__ void k_advctx(T* c, long long cstride, int ncls, Dims d, int iz_loc, const T* vx, T dx, T rdx, T auxv,
+                         T dth) {
   extern __shared__ unsigned char smem_raw[];
-  const int nx = d.nx, ny = d.ny, n2 = nx + 2;
-  T* base = reinterpret_cast<T*>(smem_raw);
-  const AdvLine<T> L{base,          base + n2,     base + 2 * n2, base + 3 * n2,
-                     base + 4 * n2, base + 5 * n2, base + 6 * n2, base + 7 * n2};
+  const int nx = d.nx, ny = d.ny;
+  const AdvLine<T> L = adv_line(reinterpret_cast<T*>(smem_raw), (size_t)nx + 2);
   const int j = blockIdx.x % ny + 1, k = blockIdx.x / ny + iz_loc;
   const T* vl = vx + d.M(1, j, k) - 1;  // vl[i] = vx(i,j,k)
-  const T auxv = dt / dx, dth = dt * T(0.5), rdx = T(1) / dx;
-  for (int q = threadIdx.x + 1; q <= nx; q += blockDim.x) {
-    const T vq = vl[q];
+  for (int q = threadIdx.x; q <= nx; q += blockDim.x) {
+    const T vq = vl[q > 1 ? q : 1];
     L.v[q] = vq;
     adv_line_coef(vq, vl[q > 1 ? q - 1 : 1], auxv, dth, L.a[q], L.b[q]);
   }
   for (int ic = 0; ic < ncls; ++ic) {
     T* cc = c + (long long)ic * cstride + d.C(0, j, k);
-    __syncthreads();  // the coefficients are staged; the previous class is done with cl, w1, w2
-    for (int q = threadIdx.x; q <= nx + 1; q += blockDim.x)
-      adv_line_stage<true>(L, q, nx, 1, cc[q], q <= nx ? cc[q + 1] : T(0));
+    __syncthreads();  // the coefficients are staged; the previous class is done with p, dc, w1, w2
+    for (int q = threadIdx.x; q <= nx; q += blockDim.x) adv_line_stage<ADV_DP>(L, q, nx, 1, cc, 1);
     __syncthreads();
-    for (int q = threadIdx.x + 1; q <= nx + 1; q += blockDim.x) adv_line_work<true>(L, q, nx, 1, dx, rdx, auxv);
+    for (int q = threadIdx.x + 1; q <= nx + 1; q += blockDim.x) adv_line_work<ADV_DP>(L, q, nx, 1, dx, rdx, auxv);
     __syncthreads();
-    for (int q = threadIdx.x + 1; q <= nx; q += blockDim.x) cc[q] = adv_line_update(L, q, nx, 1);
+    for (int q = threadIdx.x + 1; q <= nx; q += blockDim.x) cc[q] = adv_line_update(L, cc[q], q, nx, 1);
   }
 }
 
 // One block per tile of TI adjacent y lines (i0..i0+TI-1) at one k, through
 // classes 0..ncls-1.
-template <class T>
-__global__ void k_advcty(T* c, long long cstride, int ncls, Dims d, int iz_loc, const T* vy, T dy, T dt) {
+template <class T, int MODE>
+__global__ void k_advcty(T* c, long long cstride, int ncls, Dims d, int iz_loc, const T* vy, T dy, T rdy, T auxv,
+                         T dth) {
   extern __shared__ unsigned char smem_raw[];
   const int nx = d.nx, ny = d.ny, TI = blockDim.x;
   const int ntile = (nx + TI - 1) / TI;
@@ -333,31 +340,28 @@ __global__ void k_advcty(T* c, long long cstride, int ncls, Dims d, int iz_loc, 
   const int tx = threadIdx.x, ty = threadIdx.y, TJ = blockDim.y;
   const int i = i0 + tx;
   const bool act = i <= nx;
-  const size_t n2 = (size_t)(ny + 2) * TI;
-  T* base = reinterpret_cast<T*>(smem_raw) + tx;  // [q][TI], this thread's line
-  const AdvLine<T> L{base, base + n2, base + 2 * n2, base + 3 * n2, base + 4 * n2, base + 5 * n2, nullptr, nullptr};
+  const AdvLine<T> L = adv_line(reinterpret_cast<T*>(smem_raw) + tx, (size_t)(ny + 2) * TI);  // [q][TI], this line
   const long long rowstride = d.px;
   const long long cbase = d.C(act ? i : nx, 0, k);
   const long long vb = d.M(act ? i : nx, 1, k) - nx;  // vb + q*nx = vy(i,q,k)
-  const T auxv = dt / dy, dth = dt * T(0.5), rdy = T(1) / dy;
   if (act)
-    for (int q = ty + 1; q <= ny; q += TJ) {
-      const T vq = vy[vb + (long long)q * nx];
+    for (int q = ty; q <= ny; q += TJ) {
+      const T vq = vy[vb + (long long)(q > 1 ? q : 1) * nx];
       L.v[q * TI] = vq;
       adv_line_coef(vq, vy[vb + (long long)(q > 1 ? q - 1 : 1) * nx], auxv, dth, L.a[q * TI], L.b[q * TI]);
     }
   for (int ic = 0; ic < ncls; ++ic) {
-    T* cc = c + (long long)ic * cstride;
+    T* cc = c + (long long)ic * cstride + cbase;
     __syncthreads();
     if (act)
-      for (int q = ty; q <= ny + 1; q += TJ)
-        adv_line_stage<false>(L, q, ny, TI, cc[cbase + q * rowstride], T(0));
+      for (int q = ty; q <= ny + 1; q += TJ) adv_line_stage<MODE>(L, q, ny, TI, cc, rowstride);
     __syncthreads();
     if (act)
-      for (int q = ty + 1; q <= ny + 1; q += TJ) adv_line_work<false>(L, q, ny, TI, dy, rdy, auxv);
+      for (int q = ty + 1; q <= ny + 1; q += TJ) adv_line_work<MODE>(L, q, ny, TI, dy, rdy, auxv);
     __syncthreads();
     if (act)
-      for (int q = ty + 1; q <= ny; q += TJ) cc[cbase + q * rowstride] = adv_line_update(L, q, ny, TI);
+      for (int q = ty + 1; q <= ny; q += TJ)
+        cc[q * rowstride] = adv_line_update(L, L.cd[q * TI], q, ny, TI);
   }
 }
 
@@ -378,22 +382,29 @@ static void set_smem(const void* fn, size_t bytes) {
 template <class T>
 void launch_advctx(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* vx, T dx,
                    T dt, int ncls, cudaStream_t s) {
-  const size_t sm = 8 * (size_t)(d.nx + 2) * sizeof(T);
+  const size_t sm = adv_arrays(ADV_DP) * (size_t)(d.nx + 2) * sizeof(T);
   set_smem((const void*)k_advctx<T>, sm);
   const int bs = d.nx >= 256 ? 256 : 128;
-  k_advctx<T><<<dim3(d.ny * nz_loc), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, vx, dx, dt);
+  k_advctx<T><<<dim3(d.ny * nz_loc), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, vx, dx, T(1) / dx, dt / dx, dt * T(0.5));
   count_launch();
 }
 
 template <class T>
 void launch_advcty(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* vy, T dy,
                    T dt, int ncls, cudaStream_t s) {
-  const int TI = pick_ti(d.ny, sizeof(T), 6);
-  const int TJ = 256 / TI;
-  const size_t sm = 6 * (size_t)(d.ny + 2) * TI * sizeof(T);
-  set_smem((const void*)k_advcty<T>, sm);
-  const int ntile = (d.nx + TI - 1) / TI;
-  k_advcty<T><<<dim3(ntile * nz_loc), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, vy, dy, dt);
+  auto go = [&](auto kernel, int arrays) {
+    const int TI = pick_ti(d.ny, sizeof(T), arrays);
+    const int TJ = 256 / TI;
+    const size_t sm = arrays * (size_t)(d.ny + 2) * TI * sizeof(T);
+    set_smem((const void*)kernel, sm);
+    const int ntile = (d.nx + TI - 1) / TI;
+    kernel<<<dim3(ntile * nz_loc), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, vy, dy, T(1) / dy, dt / dy,
+                                                          dt * T(0.5));
+  };
+  if (adv_arrays(ADV_CP) * (size_t)(d.ny + 2) * sizeof(T) <= 227 * 1024)
+    go(k_advcty<T, ADV_CP>, adv_arrays(ADV_CP));
+  else
+    go(k_advcty<T, ADV_C>, adv_arrays(ADV_C));
   count_launch();
 }
 
@@ -443,46 +454,50 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
     const T rks = rksz ? rksz[mb + (k - 1) * ms] : T(0.5) * (rk1 * Kk1 + rk * Kk);
     return rks * (qk1 - qk) * l_dz[k];
   };
-  // Window of originals: c(k-1), c(k), c(k+1); rho, K at k-1, k, k+1.
-  T cm = C(kb - 1), c0 = C(kb), cp = C(kb + 1);
+  // Window of originals: c(k), c(k+1); rho, K, c/rho at k-1, k, k+1.
+  const T cm = C(kb - 1);
+  T c0 = C(kb), cp = C(kb + 1);
   T rm = (kb > 1) ? R(kb - 1) : T(0), r0 = R(kb), rp = (kb < nz) ? R(kb + 1) : T(0);
   T Km = (kb > 1) ? K(kb - 1) : T(0), K0 = K(kb), Kp = (kb < nz) ? K(kb + 1) : T(0);
   auto Q = [&](T cv, T rv, int kk) { return c_over_rho(cv, rv, lrz, mb + (long long)(kk - 1) * ms); };
   T qm = (kb > 1) ? Q(cm, rm, kb - 1) : T(0), q0 = Q(c0, r0, kb), qp = (kb < nz) ? Q(cp, rp, kb + 1) : T(0);
   // gradb of the first interior cell needs the face (kb-1, kb).
-  T fprev = (kb >= 3) ? face(kb - 1, qm, q0, rm, r0, Km, K0) : T(0);
-  for (int k = kb; k <= ke; ++k) {
-    T work;
-    if (k == 1) {  // bottom (diffz.f90:32-39); kb == 1 here
-      const T rkst = K(2) * R(2);
-      const T rksb = K(1) * R(1);
-      const T gradt = rkst * ((cp / rp) - (c0 / r0)) * l_dz[1];
-      T gradb = rksb * ((c0 / r0) - (cm / r0)) * l_dz[0];
-      gradb = fmax2(T(0), gradb);
-      work = dt * (gradt - gradb) * l_dzdz[1];
-      fprev = face(1, q0, qp, r0, rp, K0, Kp);  // interior face (1,2) for k = 2
-    } else if (k == nz) {  // top (diffz.f90:51-58)
-      const T rkst = K0 * r0;
-      const T rksb = Km * rm;
-      T gradt = rkst * ((cp / r0) - (c0 / r0)) * l_dz[nz];
-      const T gradb = rksb * ((c0 / r0) - (cm / rm)) * l_dz[nz - 1];
-      gradt = fmin2(T(0), gradt);
-      work = dt * (gradt - gradb) * l_dz[nz];
-    } else {  // interior (diffz.f90:41-47)
-      if (k == 2 && kb == 2) fprev = face(1, qm, q0, rm, r0, Km, K0);
-      const T gradt = face(k, q0, qp, r0, rp, K0, Kp);
-      const T gradb = fprev;
-      work = dt * (gradt - gradb) * l_dzdz[k];
-      fprev = gradt;
-    }
+  T fprev = (kb >= 2) ? face(kb - 1, qm, q0, rm, r0, Km, K0) : T(0);
+  // stores cell k and advances the window (originals)
+  auto put = [&](int k, T work) {
     cc[cb + k * cs] = c0 + work;
-    // advance the window (originals)
     if (k < ke) {
-      cm = c0; c0 = cp; cp = C(k + 2);
+      c0 = cp; cp = C(k + 2);
       rm = r0; r0 = rp; rp = (k + 2 <= nz) ? R(k + 2) : T(0);
       Km = K0; K0 = Kp; Kp = (k + 2 <= nz) ? K(k + 2) : T(0);
       qm = q0; q0 = qp; qp = (k + 2 <= nz) ? Q(cp, rp, k + 2) : T(0);
     }
+  };
+  // The end levels stand outside the loop: inside, their operations are
+  // issued for every level with their predicates off (12.7 binary64
+  // instructions per cell instead of 8.7).
+  int k = kb;
+  if (k == 1) {  // bottom (diffz.f90:32-39)
+    const T rkst = K(2) * R(2);
+    const T rksb = K(1) * R(1);
+    const T gradt = rkst * (qp - q0) * l_dz[1];
+    const T gradb = max0(rksb * (q0 - Q(cm, r0, 1)) * l_dz[0]);
+    fprev = face(1, q0, qp, r0, rp, K0, Kp);  // interior face (1,2) for k = 2
+    put(1, dt * (gradt - gradb) * l_dzdz[1]);
+    ++k;
+  }
+  for (const int kl = min(ke, nz - 1); k <= kl; ++k) {  // interior (diffz.f90:41-47)
+    const T gradt = face(k, q0, qp, r0, rp, K0, Kp);
+    const T gradb = fprev;
+    fprev = gradt;
+    put(k, dt * (gradt - gradb) * l_dzdz[k]);
+  }
+  if (k == nz && k <= ke) {  // top (diffz.f90:51-58)
+    const T rkst = K0 * r0;
+    const T rksb = Km * rm;
+    const T gradt = min0(rkst * (Q(cp, r0, nz) - q0) * l_dz[nz]);
+    const T gradb = rksb * (q0 - qm) * l_dz[nz - 1];
+    put(nz, dt * (gradt - gradb) * l_dz[nz]);
   }
 }
 
@@ -528,34 +543,35 @@ struct DiffSrc {  // the line's factors in global memory: position q at m1 + (q-
   __device__ void at(int q, T& l, T& p) const { diff_factors(lrp, pkp, rho, rkh, m1 + (q - 1) * ms, l, p); }
 };
 
-// ff(q) = fk(q)*(cl(q+1) - cl(q)): the interior face flux, gradr of cell q
-// and gradl of cell q+1 (diffx.f90:34-40), formed once per face.
+// The face fluxes of a class's line from the staged cv = c and cl = c/rho, at
+// q = 1..n-1 the interior ff(q) = fk(q)*(cl(q+1)-cl(q)), gradr of cell q and
+// gradl of cell q+1 (diffx.f90:34-40), formed once per face.  The end cells'
+// four (diffx.f90:22-33, 44-55), which are not averaged, follow: ff(n) is
+// cell n's gradr, ff(0) (from q = n+1) cell 1's gradl, ff(n+1) cell 1's gradr
+// and ff(n+2) cell n's gradl.  Neighbouring threads form them by the same
+// operations, so that a warp issues them once.
 template <class T>
-__device__ __forceinline__ T diff_line_cell(int q, int n, const T* cv, const T* cl, const T* ff,
-                                            const DiffSrc<T>& src, int st, T dtdx2) {
-  // st: stride between consecutive line positions in the staged arrays
-  auto Cq = [&](int a) { return cv[a * st]; };
-  auto Q = [&](int a) { return cl[a * st]; };
-  T gradr, gradl;
-  if (q == 1) {
-    T l1, p1, l2, p2;
-    src.at(1, l1, p1);
-    src.at(2, l2, p2);
-    gradr = p2 * (Q(2) - Q(1));
-    gradl = p1 * (Q(1) - Cq(0) * l1);
-    gradl = fmax2(T(0), gradl);
-  } else if (q == n) {
-    T ln, pn, lm, pm;
-    src.at(n, ln, pn);
-    src.at(n - 1, lm, pm);
-    gradr = pn * (Cq(n + 1) * ln - Q(n));
-    gradl = pm * (Q(n) - Q(n - 1));
-    gradr = fmin2(T(0), gradr);
-  } else {
-    gradr = ff[q * st];
-    gradl = ff[(q - 1) * st];
+__device__ __forceinline__ void diff_line_face(int q, int n, const T* cv, const T* cl, const T* fk, T* ff,
+                                               const DiffSrc<T>& src, int st) {
+  if (q < n) {
+    ff[q * st] = fk[q * st] * (cl[(q + 1) * st] - cl[q * st]);
+    return;
   }
-  return Cq(q) + dtdx2 * (gradr - gradl);
+  const int e = q - n;  // 0: gradr(n), 1: gradl(1), 2: gradr(1), 3: gradl(n)
+  T l, p, unused;
+  src.at(e == 0 ? n : 1, l, unused);
+  src.at(e == 0 ? n : e == 1 ? 1 : e == 2 ? 2 : max(n - 1, 1), unused, p);
+  const T ghost = cv[(e == 0 ? n + 1 : 0) * st] * l;
+  const T hi = e == 0 ? ghost : cl[(e == 1 ? 1 : e == 2 ? 2 : n) * st];
+  const T lo = e == 1 ? ghost : cl[(e == 0 ? n : e == 2 ? 1 : n - 1) * st];
+  const T f = p * (hi - lo);
+  ff[(e == 0 ? n : e == 1 ? 0 : e == 2 ? n + 1 : n + 2) * st] = e == 0 ? min0(f) : e == 1 ? max0(f) : f;
+}
+
+template <class T>
+__device__ __forceinline__ T diff_line_cell(int q, int n, T cq, const T* ff, int st, T dtdx2) {
+  // st: stride between consecutive line positions in the staged arrays
+  return cq + dtdx2 * (ff[(q == 1 ? n + 1 : q) * st] - ff[(q == n && q > 1 ? n + 2 : q - 1) * st]);
 }
 
 // Stages the class-independent factors of position q (1..n) of a line:
@@ -574,7 +590,7 @@ __device__ __forceinline__ void diff_stage(int q, int n, const DiffSrc<T>& src, 
 
 // One block per x line (j,k) through classes 0..ncls-1.
 template <class T>
-__global__ void k_diffx(T* c, long long cstride, int ncls, Dims d, int iz_loc, T dx, T dt, const T* rkh,
+__global__ void k_diffx(T* c, long long cstride, int ncls, Dims d, int iz_loc, T dtdx2, const T* rkh,
                         const T* rho, const T* lrp, const T* pkp) {
   extern __shared__ unsigned char smem_raw[];
   const int nx = d.nx, ny = d.ny;
@@ -586,7 +602,6 @@ __global__ void k_diffx(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
   const int j = blockIdx.x % ny + 1, k = blockIdx.x / ny + iz_loc;
   const DiffSrc<T> src{lrp, pkp, rho, rkh, d.M(1, j, k), 1};
   for (int q = threadIdx.x + 1; q <= nx; q += blockDim.x) diff_stage(q, nx, src, lr + q, fk + q);
-  const T dtdx2 = dt / (dx * dx);
   for (int ic = 0; ic < ncls; ++ic) {
     T* cc = c + (long long)ic * cstride + d.C(0, j, k);
     __syncthreads();  // factors staged; the previous class is done with cv, cl
@@ -596,16 +611,16 @@ __global__ void k_diffx(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
       if (q >= 1 && q <= nx) cl[q] = v * lr[q];
     }
     __syncthreads();
-    for (int q = threadIdx.x + 1; q < nx; q += blockDim.x) ff[q] = fk[q] * (cl[q + 1] - cl[q]);
+    for (int q = threadIdx.x + 1; q < nx + 4; q += blockDim.x) diff_line_face(q, nx, cv, cl, fk, ff, src, 1);
     __syncthreads();
     for (int q = threadIdx.x + 1; q <= nx; q += blockDim.x)
-      cc[q] = diff_line_cell(q, nx, cv, cl, ff, src, 1, dtdx2);
+      cc[q] = diff_line_cell(q, nx, cv[q], ff, 1, dtdx2);
   }
 }
 
 // One block per tile of TI adjacent y lines at one k, through classes 0..ncls-1.
 template <class T>
-__global__ void k_diffy(T* c, long long cstride, int ncls, Dims d, int iz_loc, T dy, T dt, const T* rkh,
+__global__ void k_diffy(T* c, long long cstride, int ncls, Dims d, int iz_loc, T dtdy2, const T* rkh,
                         const T* rho, const T* lrp, const T* pkp) {
   extern __shared__ unsigned char smem_raw[];
   const int nx = d.nx, ny = d.ny, TI = blockDim.x;
@@ -625,7 +640,6 @@ __global__ void k_diffy(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
   const DiffSrc<T> src{lrp, pkp, rho, rkh, d.M(act ? i : nx, 1, k), nx};
   if (act)
     for (int q = ty + 1; q <= ny; q += TJ) diff_stage(q, ny, src, lr + q * TI, fk + q * TI);
-  const T dtdy2 = dt / (dy * dy);
   for (int ic = 0; ic < ncls; ++ic) {
     T* cc = c + (long long)ic * cstride;
     __syncthreads();
@@ -637,21 +651,21 @@ __global__ void k_diffy(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
       }
     __syncthreads();
     if (act)
-      for (int q = ty + 1; q < ny; q += TJ) ff[q * TI] = fk[q * TI] * (cl[(q + 1) * TI] - cl[q * TI]);
+      for (int q = ty + 1; q < ny + 4; q += TJ) diff_line_face(q, ny, cv, cl, fk, ff, src, TI);
     __syncthreads();
     if (act)
       for (int q = ty + 1; q <= ny; q += TJ)
-        cc[base + q * rowstride] = diff_line_cell(q, ny, cv, cl, ff, src, TI, dtdy2);
+        cc[base + q * rowstride] = diff_line_cell(q, ny, cv[q * TI], ff, TI, dtdy2);
   }
 }
 
 template <class T>
 void launch_diffx(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, T dx, T dt,
                   const T* rkh, const T* rho, const T* lr, const T* pk, int ncls, cudaStream_t s) {
-  const size_t sm = 5 * (size_t)(d.nx + 2) * sizeof(T);
+  const size_t sm = (5 * (size_t)(d.nx + 2) + 1) * sizeof(T);  // ff has one more
   set_smem((const void*)k_diffx<T>, sm);
   const int bs = d.nx >= 256 ? 256 : 128;
-  k_diffx<T><<<dim3(d.ny * nz_loc), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, dx, dt, rkh, rho, lr, pk);
+  k_diffx<T><<<dim3(d.ny * nz_loc), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, dt / (dx * dx), rkh, rho, lr, pk);
   count_launch();
 }
 
@@ -662,10 +676,10 @@ void launch_diffy(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, T dy,
   int TI = pick_ti(d.ny, sizeof(T), 5);
   while (TI > 4 && 5 * (size_t)(d.ny + 2) * TI * sizeof(T) > 48 * 1024) TI >>= 1;
   const int TJ = 256 / TI;
-  const size_t sm = 5 * (size_t)(d.ny + 2) * TI * sizeof(T);
+  const size_t sm = (5 * (size_t)(d.ny + 2) + 1) * TI * sizeof(T);  // ff has one more row
   set_smem((const void*)k_diffy<T>, sm);
   const int ntile = (d.nx + TI - 1) / TI;
-  k_diffy<T><<<dim3(ntile * nz_loc), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, dy, dt,
+  k_diffy<T><<<dim3(ntile * nz_loc), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, dt / (dy * dy),
                                                              rkh, rho, lr, pk);
   count_launch();
 }
