@@ -21,6 +21,17 @@ int reduce_blocks(long long n) {
   return (int)std::max<long long>(1, std::min<long long>((n + RB - 1) / RB, RMAXB));
 }
 
+// s = s + b rounded; returns the exact error.  The operand of the larger
+// magnitude is found by integer comparison, which leaves Dekker's three
+// operations for the error-free sum instead of TwoSum's six.
+__device__ __forceinline__ double add_exact(double& s, double b) {
+  const long long bs = dbits(s), bb = dbits(b);
+  const bool sw = (bs & 0x7fffffffffffffffLL) < (bb & 0x7fffffffffffffffLL);
+  const double hi = bitsd(sw ? bb : bs), lo = bitsd(sw ? bs : bb);
+  s = hi + lo;
+  return lo - (s - hi);
+}
+
 // Sum of n DDs p[0], p[stride], ... by one warp (all lanes call it; lane 0 has
 // the sum): each lane adds its share in order, then the lanes' sums are added
 // pairwise.  The high parts by TwoSum, its exact errors and the low parts in
@@ -430,7 +441,7 @@ __global__ void k_finddt(Dims d, int nc, double dX1, double dX2, const double* d
       den = dz[k] + dz[k - 1];
     }
     const double vzm = vz[m];
-    double low = (1.0 - 1e-12) * __longlong_as_double((long long)*(volatile unsigned long long*)&block_best);
+    double low = (1.0 - 1e-12) * bitsd((long long)*(volatile unsigned long long*)&block_best);
     for (int ic = 0; ic < nc; ++ic) {
       const double* vs = vset + (long long)ic * s3;
       const double v = absd(vzm + vs[m]), dv = vs[mhi] - vs[mlo];
@@ -438,11 +449,11 @@ __global__ void k_finddt(Dims d, int nc, double dX1, double dX2, const double* d
       // reference's; only what may exceed the block's maximum is formed as the
       // reference does (non-negative values and NaN patterns order as integers)
       const double est = fma(v, rz, fma(absd(dv), rden, pre));
-      if (__double_as_longlong(est) < __double_as_longlong(low)) continue;
+      if (dbits(est) < dbits(low)) continue;
       const double dtcni = pre + div_rn_recip(v, ddz, rz) + absd(div_rn_recip(dv, den, rden));
       // MAX(best, dtcni) (a NaN dtcni is skipped)
-      const long long db = __double_as_longlong(dtcni);
-      if (db <= 0x7ff0000000000000LL && db > __double_as_longlong(best)) {
+      const long long db = dbits(dtcni);
+      if (db <= 0x7ff0000000000000LL && db > dbits(best)) {
         best = dtcni;
         atomicMax(&block_best, (unsigned long long)db);
         low = fmax(low, (1.0 - 1e-12) * best);
@@ -451,7 +462,7 @@ __global__ void k_finddt(Dims d, int nc, double dX1, double dX2, const double* d
   }
   for (int off = 16; off > 0; off >>= 1) best = fmax2(best, __shfl_down_sync(0xffffffffu, best, off));
   if ((threadIdx.x & 31) == 0 && best > 0.0)
-    atomicMax(dtcn_bits, (unsigned long long)__double_as_longlong(best));
+    atomicMax(dtcn_bits, (unsigned long long)dbits(best));
 }
 
 void launch_finddt(Dims d, int nc, double dX1, double dX2, const double* dz, const double* vx,
@@ -488,7 +499,7 @@ __device__ __forceinline__ bool nonfinite_bits(float v) {
   return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u;
 }
 __device__ __forceinline__ bool nonfinite_bits(double v) {
-  return ((unsigned long long)__double_as_longlong(v) & 0x7ff0000000000000ull) == 0x7ff0000000000000ull;
+  return ((unsigned long long)dbits(v) & 0x7ff0000000000000ull) == 0x7ff0000000000000ull;
 }
 template <class T>
 __global__ void k_count_nonfinite(const T* __restrict__ a, long long n, unsigned long long* count) {

@@ -449,7 +449,7 @@ __device__ __forceinline__ void ganser_step(const ClassConst& k, const GanserCel
 // |v - vold| <= 1e-3 on the magnitude bits (the same order for non-negative
 // values; a NaN difference is above it as in binary64)
 __device__ __forceinline__ bool ganser_done(double v, double vold) {
-  return (__double_as_longlong(v - vold) & 0x7fffffffffffffffLL) <= __double_as_longlong(1e-3);
+  return (dbits(v - vold) & 0x7fffffffffffffffLL) <= dbits(1e-3);
 }
 
 // Sources/setvset.f90:65-181 for one call of the other drag models; returns
@@ -694,7 +694,7 @@ __global__ void k_chain_check(ChainGeom g, const double* entry, const double* ex
                               int* nbad, int cap) {
   const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (s < 1 || s >= g.nseg) return;
-  if (__double_as_longlong(entry[s]) != __double_as_longlong(exitv[s - 1])) {
+  if (dbits(entry[s]) != dbits(exitv[s - 1])) {
     const int slot = atomicAdd(nbad, 1);
     if (slot < cap) bad[slot] = (int)s;
   }
@@ -727,7 +727,7 @@ __global__ void k_chain_fix(ChainGeom g, int modv, ChainIO io, double* entry, do
     int next = 1;  // index into bad[] of the next listed segment after s
     while (s < g.nseg) {
       const double expect = exitv[s - 1];
-      if (__double_as_longlong(entry[s]) != __double_as_longlong(expect)) {
+      if (dbits(entry[s]) != dbits(expect)) {
         double cd = expect;
         int nc_flag = 0;
         entry[s] = cd;

@@ -20,6 +20,8 @@
 // a non-normal or huge value, exp beyond +-700) fall back to CUDA's log/exp.
 #pragma once
 
+#include "f3d_common.cuh"
+
 namespace f3d {
 
 struct DMathTab {
@@ -39,12 +41,12 @@ __device__ __forceinline__ void dmath_tab_init(DMathTab& t) {
 }
 
 __device__ __forceinline__ double dm_log(const DMathTab& t, double x) {
-  const long long ix = __double_as_longlong(x);
+  const long long ix = dbits(x);
   // 2^-1000 <= x <= 2^1000 (positive, normal, finite), as one unsigned compare
   if ((unsigned long long)(ix - 0x0170000000000000LL) > 0x7d00000000000000ULL) return log(x);
   const int k = (int)(ix >> 52) - 1023;
   const int j = (int)((ix >> 45) & 127);
-  const double z = __longlong_as_double((ix & 0x000FFFFFFFFFFFFFLL) | 0x3FF0000000000000LL);
+  const double z = bitsd((ix & 0x000FFFFFFFFFFFFFLL) | 0x3FF0000000000000LL);
   const double r = fma(z, t.invc[j], -1.0);
   double q = fma(r, 1.0 / 7.0, -1.0 / 6.0);
   q = fma(q, r, 1.0 / 5.0);
@@ -60,10 +62,10 @@ __device__ __forceinline__ double dm_log(const DMathTab& t, double x) {
 
 __device__ __forceinline__ double dm_exp(const DMathTab& t, double a) {
   // |a| <= 700 (NaN excluded), as one integer compare on the magnitude bits
-  if ((__double_as_longlong(a) & 0x7fffffffffffffffLL) > 0x4085e00000000000LL) return exp(a);
+  if ((dbits(a) & 0x7fffffffffffffffLL) > 0x4085e00000000000LL) return exp(a);
   const double shift = 0x1.8p52;                        // rounds a*64/ln2 to an integer
   const double kd = fma(a, 0x1.71547652b82fep+6, shift);
-  const long long n = __double_as_longlong(kd) - __double_as_longlong(shift);
+  const long long n = dbits(kd) - dbits(shift);
   const double kn = kd - shift;
   double r = fma(kn, -0x1.62e42fefa0000p-7, a);        // kn * (ln2/64)_hi is exact
   r = fma(kn, -0x1.cf79abc9e3b3ap-46, r);
@@ -73,7 +75,7 @@ __device__ __forceinline__ double dm_exp(const DMathTab& t, double a) {
   q = fma(q, r, 0.5);
   const double em1 = fma(q, r * r, r);  // e^r - 1
   const long long m52 = (long long)((unsigned long long)(n >> 6) << 52);  // 2^m in the exponent field
-  const double s = __longlong_as_double(__double_as_longlong(t.e2[n & 63]) + m52);
+  const double s = bitsd(dbits(t.e2[n & 63]) + m52);
   return fma(s, em1, s);
 }
 
