@@ -34,22 +34,27 @@ __device__ __forceinline__ double add_exact(double& s, double b) {
 
 // Sum of n DDs p[0], p[stride], ... by one warp (all lanes call it; lane 0 has
 // the sum): each lane adds its share in order, then the lanes' sums are added
-// pairwise.  The high parts by TwoSum, its exact errors and the low parts in
-// binary64 beside it (the cascaded sum of Ogita, Rump and Oishi, below): the
+// pairwise.  The high parts by error-free sums, their errors and the low parts
+// in binary64 beside them (the cascaded sum of Ogita, Rump and Oishi, below): the
 // dependent chain is one addition per term, where a double-double addition's
 // is nine.  An SM issues two lanes of binary64 per clock, so a block's
 // reduction is left to one warp per sum instead of a tree in every warp.
 __device__ __forceinline__ DD warp_sum_dd(const DD* p, int n, int stride) {
   const int lane = threadIdx.x & 31;
   double s = 0.0, e = 0.0;
-  auto add = [&](double hi, double lo) {
-    const double t = s + hi, bb = t - s;
-    e = e + (((s - (t - bb)) + (hi - bb)) + lo);
-    s = t;
-  };
-  for (int q = lane; q < n; q += 32) {
-    const DD v = p[(long long)q * stride];
-    add(v.hi, v.lo);
+  auto add = [&](double hi, double lo) { e = e + (add_exact(s, hi) + lo); };
+  // eight loads in flight: one at a time, the last block's sum of 743 partials
+  // waited 24 times for the L2
+  for (int q0 = lane; q0 < n; q0 += 8 * 32) {
+    DD v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int q = q0 + 32 * u;
+      v[u] = q < n ? p[(long long)q * stride] : DD{0.0, 0.0};
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (q0 + 32 * u < n) add(v[u].hi, v[u].lo);
   }
   for (int off = 16; off > 0; off >>= 1) {
     const double hi = __shfl_down_sync(0xffffffffu, s, off), lo = __shfl_down_sync(0xffffffffu, e, off);
@@ -115,6 +120,18 @@ __host__ __device__ inline Cm2Items cm2_items(const Dims& d, int iz_loc, int nz_
   return r;
 }
 
+// Threads per block: a class's term is seven binary64 operations, 112 cycles
+// per warp and SM, so that few items are spread over the SMs in small blocks
+// (80x80x25 cells, 6 classes: 225 blocks of 64 instead of 57 of 256).
+int cm2_threads(const Cm2Items& it) {
+  const int n = it.nT + it.nX + it.nY;
+  return n <= 304 * 64 ? 64 : n <= 304 * 128 ? 128 : RB;
+}
+int cm2_blocks(const Cm2Items& it) {
+  const int n = it.nT + it.nX + it.nY, t = cm2_threads(it);
+  return std::max(1, std::min((n + t - 1) / t, RMAXB));
+}
+
 // Cascaded TwoSum (Ogita, Rump and Oishi, "Accurate sum and dot product",
 // SIAM J. Sci. Comput. 26 (2005), Algorithm 4.4): s carries the running
 // binary64 sum, e the exact rounding errors of its additions summed in
@@ -122,12 +139,7 @@ __host__ __device__ inline Cm2Items cm2_items(const Dims& d, int iz_loc, int nz_
 struct DS {
   double s, e;
 };
-__device__ __forceinline__ void ds_add(DS& a, double b) {
-  const double s = a.s + b;
-  const double bb = s - a.s;
-  a.e = a.e + ((a.s - (s - bb)) + (b - bb));
-  a.s = s;
-}
+__device__ __forceinline__ void ds_add(DS& a, double b) { a.e = a.e + add_exact(a.s, b); }
 __device__ __forceinline__ DD ds_dd(DS a) {
   const double hi = a.s + a.e;
   return DD{hi, a.e - (hi - a.s)};
@@ -146,7 +158,7 @@ __device__ __forceinline__ void face_terms(const T* cc, long long hb, int nc_loc
 #pragma unroll
     for (int u = 0; u < CB; ++u) {
       if (cv[u] == T(0)) continue;
-      const double t = w * (double)cv[u];
+      const double t = w * widen(cv[u]);
       ds_add(acc, side ? t : -t);
     }
   }
@@ -159,7 +171,7 @@ __device__ DD block_sum_ds(DS a) {
   __shared__ DD sh[RB];
   sh[threadIdx.x] = ds_dd(a);
   DD v = dd_zero();
-  if (__syncthreads_or(a.s != 0.0 || a.e != 0.0) && threadIdx.x < 32) v = warp_sum_dd(sh, RB, 1);
+  if (__syncthreads_or(a.s != 0.0 || a.e != 0.0) && threadIdx.x < 32) v = warp_sum_dd(sh, blockDim.x, 1);
   return v;
 }
 
@@ -202,13 +214,16 @@ __device__ __forceinline__ void cmass2d_item(int u, const Cm2Items& it, const T*
     const T* cc = c0 + d.C(i, j, nz + 1);
     for (int q0 = 0; q0 < nc_loc; q0 += CB) {
       T cv[CB];
+      double sv[CB];  // likewise all in flight at a time
 #pragma unroll
       for (int u = 0; u < CB; ++u) cv[u] = q0 + u < nc_loc ? cc[(q0 + u) * hb] : T(0);
 #pragma unroll
+      for (int u = 0; u < CB; ++u) sv[u] = cv[u] != T(0) ? vs[(q0 + u) * s3] : 0.0;
+#pragma unroll
       for (int u = 0; u < CB; ++u) {
         if (cv[u] == T(0)) continue;  // an exact zero term (finite velocities)
-        const double velo = w + vs[(q0 + u) * s3];
-        ds_add(acc, da * velo * (double)cv[u]);
+        const double velo = w + sv[u];
+        ds_add(acc, da * velo * widen(cv[u]));
       }
     }
     return;
@@ -246,7 +261,7 @@ __global__ void k_cmass2d(const T* c, const double* vx, const double* vy, const 
   const Cm2Items it = cm2_items(d, iz_loc, nz_loc);
   const int ntot = it.nT + it.nX + it.nY;
   DS acc{0.0, 0.0};
-  for (int u = blockIdx.x * RB + threadIdx.x; u < ntot; u += gridDim.x * RB)
+  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < ntot; u += gridDim.x * blockDim.x)
     cmass2d_item<T>(u, it, c, vx, vy, vz, vset, d, ic_loc, nc_loc, iz_loc, nz_loc, dx, dy, dz, dt,
                     acc);
   const DD v = block_sum_ds(acc);
@@ -275,7 +290,7 @@ __global__ void k_cmass2d_batch(const BatchAux* tab, const int* bstep, DD* parti
 
 size_t cmass2d_scratch_bytes(Dims d, int iz_loc, int nz_loc) {
   const Cm2Items it = cm2_items(d, iz_loc, nz_loc);
-  return reduce_scratch_bytes((long long)it.nT + it.nX + it.nY, 1);
+  return sizeof(DD) * (size_t)cm2_blocks(it) + 256;
 }
 
 template <class T>
@@ -284,9 +299,9 @@ void launch_cmass2d(const T* c, const double* vx, const double* vy, const double
                     double dx, double dy, const double* dz, double dt, void* scratch,
                     double* out, cudaStream_t s, unsigned* done) {
   const Cm2Items it = cm2_items(d, iz_loc, nz_loc);
-  const int nb = reduce_blocks((long long)it.nT + it.nX + it.nY);
+  const int nb = cm2_blocks(it);
   DD* partial = reinterpret_cast<DD*>(scratch);
-  k_cmass2d<T><<<nb, RB, 0, s>>>(c, vx, vy, vz, vset, d, ic_loc, nc_loc, iz_loc, nz_loc, dx, dy, dz,
+  k_cmass2d<T><<<nb, cm2_threads(it), 0, s>>>(c, vx, vy, vz, vset, d, ic_loc, nc_loc, iz_loc, nz_loc, dx, dy, dz,
                                  dt, partial, done, out);
   count_launch();
   if (!done) {

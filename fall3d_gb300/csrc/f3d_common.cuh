@@ -42,6 +42,16 @@ __device__ __forceinline__ double bitsd(long long b) {
   return r;
 }
 
+// A binary32 value widened with integer operations (the conversion
+// instruction goes through the binary64 pipe, which the kernels of
+// binary64 sums are bound by); exponent 0 and 255 take the conversion.
+__device__ __forceinline__ double widen(float v) {
+  const unsigned u = __float_as_uint(v), e = (u >> 23) & 255u;
+  if (e - 1u >= 254u) return (double)v;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
 // |x| and x > 0 of binary64 values on the bit patterns (integer operations;
 // the binary64 pipe is the plain form's bottleneck): clearing the sign bit
 // is fabs, NaN included; x > 0 holds exactly for the patterns of positive

@@ -32,16 +32,6 @@ struct OutClasses {
   __device__ int at(int i) const { return cls_more ? cls_more[i] : (int)cls[i]; }
 };
 
-// A binary32 value widened with integer operations (the conversion
-// instruction goes through the binary64 pipe, which these kernels are bound
-// by); exponent 0 and 255 take the conversion.
-__device__ __forceinline__ double widen(float v) {
-  const unsigned u = __float_as_uint(v), e = (u >> 23) & 255u;
-  if (e - 1u >= 254u) return (double)v;
-  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
-}
-__device__ __forceinline__ double widen(double v) { return v; }
-
 // sum over the listed classes of c(i,j,k,ic) (0 + c1 + c2 + ...).  A zero
 // leaves the sum as it is and is skipped; eight loads are in flight.
 template <class T>
