@@ -161,21 +161,45 @@ __device__ __forceinline__ void adv_z_work(T c0, T cp, T vk, T vk_1, T pm, T sm,
   w2 = z.hdzm1 * (T(1) - Crk) * sigma * av * z.dzz;
 }
 
+// The column kernels take a thread per column, or where that leaves the chip
+// idle a thread per piece of it: blocks of 32 columns by blockDim.y pieces of
+// the levels iz_loc .. iz_loc+nz_loc-1.  A column's pieces are in one block,
+// which reads what they need of each other before any of them writes.
+struct ColPiece {
+  int kb, ke;  // its levels (kb > ke: none)
+};
+__device__ __forceinline__ ColPiece col_piece(int iz_loc, int nz_loc) {
+  const int len = (nz_loc + blockDim.y - 1) / blockDim.y, kb = iz_loc + threadIdx.y * len;
+  return ColPiece{kb, min(kb + len, iz_loc + nz_loc) - 1};
+}
+// Pieces while the columns' warps are fewer than 8 per SM, of at least four
+// levels each: a piece forms two levels' terms of its own before its first.
+// With and without: 32x28x14 cells and 4 classes advctzc 15 and 22 us, diffz 14
+// and 18; 80x80x25 and 6 classes 48 and 45, 28 and 33; 201x149x41 and one class
+// 64 and 71, 41 and 66; with twice as many warps advctzc 54 and 70 us at the
+// latter two.
+static dim3 col_block(long long cols, int ncls, int nz_loc) {
+  const long long warps = (cols + 31) / 32 * ncls;
+  int p = 1;
+  while (p < 8 && warps * p < 152 * 8 && nz_loc >= 4 * (2 * p)) p *= 2;
+  return p == 1 ? dim3(128) : dim3(32, p);
+}
+
 template <class T>
 __global__ void k_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* vz,
                           const T* vset, long long vstride, const T* dz, T dt) {
   extern __shared__ unsigned char smem_raw[];
   ZTab<T>* tab = reinterpret_cast<ZTab<T>*>(smem_raw);
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  for (int k = threadIdx.x + 1; k <= nz; k += blockDim.x) {
+  for (int k = threadIdx.y * blockDim.x + threadIdx.x + 1; k <= nz; k += blockDim.x * blockDim.y) {
     tab[k].dzz = T(2) / (dz[k] + dz[k - 1]);
     tab[k].dzk = T(1) / dz[k];
     tab[k].dzk_1 = T(1) / dz[k - 1];
     tab[k].hdzm1 = dt * T(0.5) * dz[k - 1];
   }
   __syncthreads();
-  const long long col = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (col >= (long long)nx * ny) return;
+  const long long col = min(blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)nx * ny - 1);
+  const bool act = col == blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int i = (int)(col % nx) + 1, j = (int)(col / nx) + 1;
   T* cc = c + (long long)blockIdx.y * cstride;
   const T* vs = vset + (long long)blockIdx.y * vstride;
@@ -184,23 +208,32 @@ __global__ void k_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_lo
   auto VK = [&](int k) { return vz[mb + (k - 1) * ms] + vs[mb + (k - 1) * ms]; };
   auto CO = [&](int k) { return cc[cb + k * cs]; };
   const T dznz = T(1) / dz[nz];
-  const int kb = iz_loc, ke = iz_loc + nz_loc - 1;
-  T c_m1 = CO(kb - 1), c_0 = CO(kb), c_p1 = CO(kb + 1);
-  T vk_0 = VK(kb), vk_m1 = VK(kb > 1 ? kb - 1 : 1);
-  T w1_k, w2_k, w2_km, pk, dk;
-  adv_z_work(c_0, c_p1, vk_0, vk_m1, vk_m1 * c_m1, (c_0 - c_m1) * tab[kb].dzk_1, tab[kb], dt, w1_k, w2_k, pk, dk);
-  if (kb == 1) {
-    w2_km = w2_k;
-  } else {
-    T w1_dummy, p_dummy, d_dummy;
-    const T c_m2 = CO(kb - 2), vk_m2 = VK(kb - 1 > 1 ? kb - 2 : 1);
-    adv_z_work(c_m1, c_0, vk_m1, vk_m2, vk_m2 * c_m2, (c_m1 - c_m2) * tab[kb - 1].dzk_1, tab[kb - 1], dt, w1_dummy, w2_km,
-               p_dummy, d_dummy);
+  const ColPiece pc = col_piece(iz_loc, nz_loc);
+  const int kb = pc.kb, ke = pc.ke;
+  T c_0 = T(0), c_p1 = T(0), vk_0 = T(0), w1_k, w2_k, w2_km, pk, dk, c_e1 = T(0), c_e2 = T(0);
+  if (kb <= ke) {
+    const T c_m1 = CO(kb - 1), vk_m1 = VK(kb > 1 ? kb - 1 : 1);
+    c_0 = CO(kb);
+    c_p1 = CO(kb + 1);
+    vk_0 = VK(kb);
+    c_e1 = CO(ke + 1);  // the next piece's first two, before it overwrites them
+    c_e2 = CO(min(ke + 2, nz + 1));
+    adv_z_work(c_0, c_p1, vk_0, vk_m1, vk_m1 * c_m1, (c_0 - c_m1) * tab[kb].dzk_1, tab[kb], dt, w1_k, w2_k, pk, dk);
+    if (kb == 1) {
+      w2_km = w2_k;
+    } else {
+      T w1_dummy, p_dummy, d_dummy;
+      const T c_m2 = CO(kb - 2), vk_m2 = VK(kb - 1 > 1 ? kb - 2 : 1);
+      adv_z_work(c_m1, c_0, vk_m1, vk_m2, vk_m2 * c_m2, (c_m1 - c_m2) * tab[kb - 1].dzk_1, tab[kb - 1], dt, w1_dummy,
+                 w2_km, p_dummy, d_dummy);
+    }
   }
+  if (blockDim.y > 1) __syncthreads();  // every piece has read its neighbours' originals
+  if (!act) return;
   for (int k = kb; k <= ke; ++k) {
     T w1_n, w2_n, c_p2 = T(0), vk_p1 = T(0);
     if (k + 1 <= nz) {
-      c_p2 = CO(k + 2);
+      c_p2 = k + 2 <= ke ? CO(k + 2) : k + 1 == ke ? c_e1 : c_e2;
       vk_p1 = VK(k + 1);
       adv_z_work(c_p1, c_p2, vk_p1, vk_0, pk, dk, tab[k + 1], dt, w1_n, w2_n, pk, dk);
     } else {
@@ -214,24 +247,20 @@ __global__ void k_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_lo
     w2_km = w2_k;
     w2_k = w2_n;
     w1_k = w1_n;
-    c_m1 = c_0;
     c_0 = c_p1;
     c_p1 = c_p2;
-    vk_m1 = vk_0;
     vk_0 = vk_p1;
   }
-  (void)c_m1;
-  (void)vk_m1;
 }
 
 template <class T>
 void launch_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* vz,
                     const T* vset, long long vstride, const T* dz, T dt, int ncls,
                     cudaStream_t s) {
-  const int bs = 128;
   const long long cols = (long long)d.nx * d.ny;
+  const dim3 bs = col_block(cols, ncls, nz_loc);
   const size_t sm = sizeof(ZTab<T>) * (d.nz + 1);
-  k_advctzc<T><<<dim3((unsigned)((cols + bs - 1) / bs), ncls), bs, sm, s>>>(
+  k_advctzc<T><<<dim3((unsigned)((cols + bs.x - 1) / bs.x), ncls), bs, sm, s>>>(
       c, cstride, d, nz_loc, iz_loc, vz, vset, vstride, dz, dt);
   count_launch();
 }
@@ -317,7 +346,7 @@ __global__ void k_advctx(T* c, long long cstride, int ncls, Dims d, int iz_loc, 
     L.v[q] = vq;
     adv_line_coef(vq, vl[q > 1 ? q - 1 : 1], auxv, dth, L.a[q], L.b[q]);
   }
-  for (int ic = 0; ic < ncls; ++ic) {
+  for (int ic = blockIdx.y; ic < ncls; ic += gridDim.y) {
     T* cc = c + (long long)ic * cstride + d.C(0, j, k);
     __syncthreads();  // the coefficients are staged; the previous class is done with p, dc, w1, w2
     for (int q = threadIdx.x; q <= nx; q += blockDim.x) adv_line_stage<ADV_DP>(L, q, nx, 1, cc, 1);
@@ -350,7 +379,7 @@ __global__ void k_advcty(T* c, long long cstride, int ncls, Dims d, int iz_loc, 
       L.v[q * TI] = vq;
       adv_line_coef(vq, vy[vb + (long long)(q > 1 ? q - 1 : 1) * nx], auxv, dth, L.a[q * TI], L.b[q * TI]);
     }
-  for (int ic = 0; ic < ncls; ++ic) {
+  for (int ic = blockIdx.y; ic < ncls; ic += gridDim.y) {
     T* cc = c + (long long)ic * cstride + cbase;
     __syncthreads();
     if (act)
@@ -375,6 +404,21 @@ static int pick_ti(int nline, size_t elem, int arrays) {
   return 1;
 }
 
+// Narrower tiles (of at least 8 lines, two sectors of a row) while they are
+// fewer than two blocks per SM over all classes.
+static int fill_ti(int ti, int nx, int nz_loc, int ncls) {
+  while (ti > 8 && (long long)((nx + ti - 1) / ti) * nz_loc * ncls < 304) ti >>= 1;
+  return ti;
+}
+
+// The line kernels' blocks take a line (or tile of lines) through every class,
+// or where the lines are fewer than two blocks per SM, through every ny-th one.
+// 32x28x14 cells and 4 classes, with the narrower tiles: advcty 8 us instead of
+// 24, diffy 8 instead of 18; 80x80x25 and 6 classes 37 instead of 43, 24 of 29.
+static int class_splits(long long lines, int ncls) {
+  return (int)std::min<long long>(ncls, std::max<long long>(1, (304 + lines - 1) / lines));
+}
+
 static void set_smem(const void* fn, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
@@ -385,7 +429,7 @@ void launch_advctx(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, cons
   const size_t sm = adv_arrays(ADV_DP) * (size_t)(d.nx + 2) * sizeof(T);
   set_smem((const void*)k_advctx<T>, sm);
   const int bs = d.nx >= 256 ? 256 : 128;
-  k_advctx<T><<<dim3(d.ny * nz_loc), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, vx, dx, T(1) / dx, dt / dx, dt * T(0.5));
+  k_advctx<T><<<dim3(d.ny * nz_loc, class_splits((long long)d.ny * nz_loc, ncls)), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, vx, dx, T(1) / dx, dt / dx, dt * T(0.5));
   count_launch();
 }
 
@@ -393,12 +437,13 @@ template <class T>
 void launch_advcty(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* vy, T dy,
                    T dt, int ncls, cudaStream_t s) {
   auto go = [&](auto kernel, int arrays) {
-    const int TI = pick_ti(d.ny, sizeof(T), arrays);
+    const int TI = fill_ti(pick_ti(d.ny, sizeof(T), arrays), d.nx, nz_loc, ncls);
     const int TJ = 256 / TI;
     const size_t sm = arrays * (size_t)(d.ny + 2) * TI * sizeof(T);
     set_smem((const void*)kernel, sm);
     const int ntile = (d.nx + TI - 1) / TI;
-    kernel<<<dim3(ntile * nz_loc), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, vy, dy, T(1) / dy, dt / dy,
+    kernel<<<dim3(ntile * nz_loc, class_splits((long long)ntile * nz_loc, ncls)), dim3(TI, TJ), sm, s>>>(
+        c, cstride, ncls, d, iz_loc, vy, dy, T(1) / dy, dt / dy,
                                                           dt * T(0.5));
   };
   if (adv_arrays(ADV_CP) * (size_t)(d.ny + 2) * sizeof(T) <= 227 * 1024)
@@ -432,13 +477,13 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
   T* l_dz = reinterpret_cast<T*>(smem_raw);  // 0..nz
   T* l_dzdz = l_dz + (d.nz + 1);             // 1..nz
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  for (int k = threadIdx.x; k <= nz; k += blockDim.x) {
+  for (int k = threadIdx.y * blockDim.x + threadIdx.x; k <= nz; k += blockDim.x * blockDim.y) {
     l_dz[k] = T(1) / dz[k];
     if (k >= 1) l_dzdz[k] = T(2) / (dz[k] + dz[k - 1]);
   }
   __syncthreads();
-  const long long col = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (col >= (long long)nx * ny) return;
+  const long long col = min(blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)nx * ny - 1);
+  const bool act = col == blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int i = (int)(col % nx) + 1, j = (int)(col / nx) + 1;
   T* cc = c + (long long)blockIdx.y * cstride;
   const long long cb = d.C(i, j, 0), cs = (long long)d.px * (ny + 2);
@@ -446,7 +491,8 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
   auto C = [&](int k) { return cc[cb + k * cs]; };
   auto R = [&](int k) { return rho[mb + (k - 1) * ms]; };
   auto K = [&](int k) { return rkver[mb + (k - 1) * ms]; };
-  const int kb = iz_loc, ke = iz_loc + nz_loc - 1;
+  const ColPiece pc = col_piece(iz_loc, nz_loc);
+  const int ke = pc.ke, kb = min(pc.kb, ke);  // an empty piece reads a level inside and does not march
   // Interior face flux between k and k+1 (diffz.f90:42-45):
   //   0.5*(rho(k+1)K(k+1) + rho(k)K(k)) * (c(k+1)/rho(k+1) - c(k)/rho(k)) * l_dz(k)
   // rksz, when given, holds that face's 0.5*(...) for the meteo update
@@ -455,8 +501,10 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
     return rks * (qk1 - qk) * l_dz[k];
   };
   // Window of originals: c(k), c(k+1); rho, K, c/rho at k-1, k, k+1.
-  const T cm = C(kb - 1);
+  const T cm = C(kb - 1), c_e1 = C(ke + 1);  // the next piece's first, before it overwrites it
   T c0 = C(kb), cp = C(kb + 1);
+  if (blockDim.y > 1) __syncthreads();  // every piece has read its neighbours' originals
+  if (!act || pc.kb > ke) return;
   T rm = (kb > 1) ? R(kb - 1) : T(0), r0 = R(kb), rp = (kb < nz) ? R(kb + 1) : T(0);
   T Km = (kb > 1) ? K(kb - 1) : T(0), K0 = K(kb), Kp = (kb < nz) ? K(kb + 1) : T(0);
   auto Q = [&](T cv, T rv, int kk) { return c_over_rho(cv, rv, lrz, mb + (long long)(kk - 1) * ms); };
@@ -467,7 +515,7 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
   auto put = [&](int k, T work) {
     cc[cb + k * cs] = c0 + work;
     if (k < ke) {
-      c0 = cp; cp = C(k + 2);
+      c0 = cp; cp = k + 2 <= ke ? C(k + 2) : c_e1;
       rm = r0; r0 = rp; rp = (k + 2 <= nz) ? R(k + 2) : T(0);
       Km = K0; K0 = Kp; Kp = (k + 2 <= nz) ? K(k + 2) : T(0);
       qm = q0; q0 = qp; qp = (k + 2 <= nz) ? Q(cp, rp, k + 2) : T(0);
@@ -504,12 +552,11 @@ __global__ void k_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc,
 template <class T>
 void launch_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* dz, T dt,
                   const T* rkver, const T* rho, const T* rksz, const T* lrz, int ncls, cudaStream_t s) {
-  const int bs = 128;
   const long long cols = (long long)d.nx * d.ny;
+  const dim3 bs = col_block(cols, ncls, nz_loc);
   const size_t sm = 2 * sizeof(T) * (d.nz + 1);
-  k_diffz<T><<<dim3((unsigned)((cols + bs - 1) / bs), ncls), bs, sm, s>>>(c, cstride, d, nz_loc,
-                                                                         iz_loc, dz, dt, rkver, rho,
-                                                                         rksz, lrz);
+  k_diffz<T><<<dim3((unsigned)((cols + bs.x - 1) / bs.x), ncls), bs, sm, s>>>(c, cstride, d, nz_loc, iz_loc, dz, dt,
+                                                                              rkver, rho, rksz, lrz);
   count_launch();
 }
 
@@ -602,7 +649,7 @@ __global__ void k_diffx(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
   const int j = blockIdx.x % ny + 1, k = blockIdx.x / ny + iz_loc;
   const DiffSrc<T> src{lrp, pkp, rho, rkh, d.M(1, j, k), 1};
   for (int q = threadIdx.x + 1; q <= nx; q += blockDim.x) diff_stage(q, nx, src, lr + q, fk + q);
-  for (int ic = 0; ic < ncls; ++ic) {
+  for (int ic = blockIdx.y; ic < ncls; ic += gridDim.y) {
     T* cc = c + (long long)ic * cstride + d.C(0, j, k);
     __syncthreads();  // factors staged; the previous class is done with cv, cl
     for (int q = threadIdx.x; q <= nx + 1; q += blockDim.x) {
@@ -640,7 +687,7 @@ __global__ void k_diffy(T* c, long long cstride, int ncls, Dims d, int iz_loc, T
   const DiffSrc<T> src{lrp, pkp, rho, rkh, d.M(act ? i : nx, 1, k), nx};
   if (act)
     for (int q = ty + 1; q <= ny; q += TJ) diff_stage(q, ny, src, lr + q * TI, fk + q * TI);
-  for (int ic = 0; ic < ncls; ++ic) {
+  for (int ic = blockIdx.y; ic < ncls; ic += gridDim.y) {
     T* cc = c + (long long)ic * cstride;
     __syncthreads();
     if (act)
@@ -665,7 +712,7 @@ void launch_diffx(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, T dx,
   const size_t sm = (5 * (size_t)(d.nx + 2) + 1) * sizeof(T);  // ff has one more
   set_smem((const void*)k_diffx<T>, sm);
   const int bs = d.nx >= 256 ? 256 : 128;
-  k_diffx<T><<<dim3(d.ny * nz_loc), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, dt / (dx * dx), rkh, rho, lr, pk);
+  k_diffx<T><<<dim3(d.ny * nz_loc, class_splits((long long)d.ny * nz_loc, ncls)), bs, sm, s>>>(c, cstride, ncls, d, iz_loc, dt / (dx * dx), rkh, rho, lr, pk);
   count_launch();
 }
 
@@ -675,11 +722,12 @@ void launch_diffy(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, T dy,
   // at most ~48 KB per block, so that several blocks share an SM
   int TI = pick_ti(d.ny, sizeof(T), 5);
   while (TI > 4 && 5 * (size_t)(d.ny + 2) * TI * sizeof(T) > 48 * 1024) TI >>= 1;
+  TI = fill_ti(TI, d.nx, nz_loc, ncls);
   const int TJ = 256 / TI;
   const size_t sm = (5 * (size_t)(d.ny + 2) + 1) * TI * sizeof(T);  // ff has one more row
   set_smem((const void*)k_diffy<T>, sm);
   const int ntile = (d.nx + TI - 1) / TI;
-  k_diffy<T><<<dim3(ntile * nz_loc), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, dt / (dy * dy),
+  k_diffy<T><<<dim3(ntile * nz_loc, class_splits((long long)ntile * nz_loc, ncls)), dim3(TI, TJ), sm, s>>>(c, cstride, ncls, d, iz_loc, dt / (dy * dy),
                                                              rkh, rho, lr, pk);
   count_launch();
 }

@@ -1,5 +1,5 @@
 """The plain form's sweeps where their kernels can go wrong: the smallest
-lines, sides around a warp and a block, lines too long for the staged products
+lines, sides around a warp and a block, columns cut into pieces, lines too long for the staged products
 (advcty), tails that fall off through the subnormals to zero, signed zeros and
 non-finite values in the diffusion's end faces.  Against the oracle, bit for
 bit (NaN payloads aside)."""
@@ -8,12 +8,12 @@ import pytest
 
 import fall3d_gb300 as F
 import oracle_lib as O
-from helpers import assert_same_bits
+from helpers import assert_close, assert_same_bits, oracle_state
 
 pytestmark = pytest.mark.gpu
 
 SIZES = [(3, 3, 3), (4, 5, 3), (31, 4, 4), (32, 65, 5), (127, 3, 9), (129, 7, 4), (257, 33, 3), (5, 290, 4),
-         (3, 1451, 3), (3, 4200, 3)]
+         (3, 1451, 3), (3, 4200, 3), (9, 8, 33), (33, 5, 41), (6, 5, 63)]
 
 
 def _state(nx, ny, nz, special):
@@ -49,3 +49,21 @@ def test_sweeps(nx, ny, nz, special):
             getattr(lib, "orc_" + name)(O.p(a), *[O.p(v) if isinstance(v, np.ndarray) else v for v in args])
             getattr(F, name)(b, *args)
             assert_same_bits(b, a, f"{name} {args[:5]}")
+
+
+@pytest.mark.parametrize("nx,ny,nz,nc", [(20, 18, 9, 3), (70, 9, 19, 5), (9, 75, 33, 2)])
+def test_steps_of_split_classes_and_pieces(nx, ny, nz, nc):
+    """The plain form's steps where lines and columns do not fill the chip
+    (classes spread over blocks, narrow tiles, pieces of columns): the oracle's
+    state to the tolerance of whole runs (its settling velocities differ by a
+    few ulp, the sweeps by nothing)."""
+    s, o = oracle_state("small", seed=11, steps=6, nx=nx, ny=ny, nz=nz, nc=nc, run_h=1.0)
+    g = F.Context(s, F.PREC_FP64)
+    g.meteo(0)
+    g.source(0)
+    g.step(6)
+    g.sync()
+    fo, fg = o.fields(), g.fields()
+    for k in ("c", "cdry", "cwet"):
+        assert_close(fg[k], fo[k], 1e-12, 1e-9, k)
+    assert np.max(fg["c"]) > 0.0
