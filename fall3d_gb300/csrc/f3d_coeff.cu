@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(64, 8)
 // the same SM return at once, so that an SM idle at launch time does not fill
 // up with chain blocks and shut the steps out.  The working blocks take
 // segments from a counter until none is left.
-__global__ void __launch_bounds__(128, 4)
+__global__ void __launch_bounds__(128, 8)
     k_chain_beside(ChainGeom g, int modv, ChainIO io, const double* cd_state, double* entry, double* exitv,
                    int* nonconv, int* claim, unsigned long long* next) {
   __shared__ PowTab tab;

@@ -384,7 +384,7 @@ void sizloop_fused(f3d_ctx* x) {
   const FusedArgs a = f3d::ctx_fused_args(x, shape);
   {
     ProfScope ps(x, "step_fused");
-    launch_step_fused(a, x->maps2, x->cmap, shape, s);
+    launch_step_fused(a, x->maps2, x->cmap, shape, s, x->pref_ready && cudaEventQuery(x->ev_pref) == cudaErrorNotReady);
   }
   std::swap(x->c32, x->c32b);
   std::swap(x->cmap, x->cmapb);

@@ -99,7 +99,9 @@ void step_chunks(FusedArgs& a, int shape, int nwet);
 // warp); two columns per lane.  Results do not depend on the shape.
 // step_shape: the faster one for a launch of its own, where none was set.
 int step_shape(Dims d, int ncls);
-void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s);
+// beside: a look-ahead meteo update may run at the same time.
+void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s,
+                       bool beside = false);
 // The step kernel's fields from the scaled binary64 fields of a meteo update
 // whose finddt maximum is at *dtcn (dt = safety/max(dtcn,1e-13)).
 void launch_step_fields(Dims d, int nc, double safety, double dX1, double dX2, const double* dz,

@@ -71,7 +71,7 @@ constexpr int GUARD = 512;  // bytes before the staging area (reads one row abov
 
 template <int HY_, int NW_>
 struct Shape {
-  static constexpr int HYR = HY_, NWARP = NW_, NT = 32 * NW_, RPW = HY_ / NW_, TY = HY_ - 6, FS = RS * HY_,
+  static constexpr int HYR = HY_, NT = 32 * NW_, RPW = HY_ / NW_, TY = HY_ - 6, FS = RS * HY_,
                        NP = HX * HY_, MAP = HY_ == 32 ? 0 : 1, UNROLL = HY_ == 32 ? 1 : 2;
   static_assert(HY_ % NW_ == 0 && NW_ >= NF, "rows must divide among warps; a warp issues one field's copies");
 };
@@ -82,7 +82,6 @@ using Flat = Shape<16, 16>;
 // value of the column to the left / right of each of the lane's two columns
 __device__ __forceinline__ float2 left2(float2 v) { return make_float2(shup(v.y), v.x); }
 __device__ __forceinline__ float2 right2(float2 v) { return make_float2(v.y, shdn(v.x)); }
-__device__ __forceinline__ float cmp(const float2& v, int c) { return c ? v.y : v.x; }
 __device__ __forceinline__ float& cmp(float2& v, int c) { return c ? v.y : v.x; }
 
 __device__ __forceinline__ float2 lds2(const float* p) { return *reinterpret_cast<const float2*>(p); }
@@ -690,6 +689,20 @@ __global__ void __launch_bounds__(S::NT, min_blocks<S>())
                        item % a.nchunk);
 }
 
+// The 64x32 step while a look-ahead meteo update runs beside it: with at most
+// 112 registers a block leaves the settling chain's four 64-register warps
+// room on its SM (the 128 of the other build take the whole register file).
+// A forecast of 400x300x50 cells and 16 classes over eight meteo updates runs at
+// 9.70e10 cell-class-steps/s with it, 8.95e10 with the other build throughout
+// (whose blocks and the chain's exclude each other) and 8.5e10 with every
+// update made when due.
+template <bool XFIRST>
+__global__ void __maxnreg__(112) k_step_fused2_beside(const FusedArgs a, const __grid_constant__ StepMaps maps) {
+  const int item = blockIdx.x / a.ncls;
+  step_tile<Tall, XFIRST>(a, &maps.met, &maps.c, a.c_in, a.c_out, 1, (int)(blockIdx.x % a.ncls), item / a.nchunk,
+                          item % a.nchunk);
+}
+
 // ------------------------------------------------------------ batched form
 // The step of every scenario of a batch in one persistent launch: the work
 // items are (scenario, tile, piece, class), numbered scenario by scenario
@@ -906,7 +919,7 @@ void step_chunks(FusedArgs& a, int shape, int nwet) {
   }
 }
 
-void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s) {
+void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, int shape, cudaStream_t s, bool beside) {
   with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
     const size_t sm = step_smem<S>(a.d.nz);
@@ -917,7 +930,10 @@ void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, i
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       kernel<<<fused_tiles(a.d.nx, a.d.ny, shape) * a.ncls * a.nchunk, S::NT, sm, s>>>(a, m);
     };
-    a.xfirst ? go(k_step_fused2<S, true>) : go(k_step_fused2<S, false>);
+    if (beside && S::HYR == HY)
+      a.xfirst ? go(k_step_fused2_beside<true>) : go(k_step_fused2_beside<false>);
+    else
+      a.xfirst ? go(k_step_fused2<S, true>) : go(k_step_fused2<S, false>);
     return 0;
   });
   count_launch();
