@@ -93,10 +93,15 @@ int table_rebuild(f3d_batch* b) {
   b->max_nc = 0;
   const int nsou_blocks = (b->max_nsou + 127) / 128;
   b->max_nsou = 0;
+  long long items = 0;
+  for (int q = 0; q < n; ++q) {
+    const f3d_ctx* x = b->slot[b->active[q]].x;
+    items += (long long)fused_tiles(x->g.nx, x->g.ny, b->shape) * x->g.nc;
+  }
   for (int q = 0; q < n; ++q) {
     Scen& s = b->slot[b->active[q]];
     f3d_ctx* x = s.x;
-    FusedArgs a = ctx_fused_args(x, b->shape);
+    FusedArgs a = ctx_fused_args(x, b->shape, items);
     a.c_in = s.c_a;
     a.c_out = s.c_b;
     b->h_args[q] = a;

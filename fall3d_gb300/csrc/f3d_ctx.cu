@@ -398,7 +398,7 @@ void sizloop_fused(f3d_ctx* x) {
 }  // namespace
 
 namespace f3d {
-FusedArgs ctx_fused_args(f3d_ctx* x, int shape) {
+FusedArgs ctx_fused_args(f3d_ctx* x, int shape, long long batch_items) {
   const Dims d = x->d;
   FusedArgs a{};
   a.c_in = x->c32;
@@ -422,7 +422,7 @@ FusedArgs ctx_fused_args(f3d_ctx* x, int shape) {
   a.vset64 = x->vset;
   a.vdep64 = x->vdep;
   a.status = small_step_status(x);
-  step_chunks(a, shape, x->g.wetdep ? x->nwet : 0);
+  step_chunks(a, shape, x->g.wetdep ? x->nwet : 0, batch_items);
   return a;
 }
 }  // namespace f3d

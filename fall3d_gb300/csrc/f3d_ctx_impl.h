@@ -144,8 +144,9 @@ void ctx_advance(f3d_ctx* x);
 // the mass-budget log of endstep.f90:51 when due
 int ctx_log(f3d_ctx* x, f3d_log_record* log, int log_cap, int* nlog);
 // arguments of the fused precision-form step for the context's state, with
-// the column pieces of a launch of its own for tile shape `shape`
-FusedArgs ctx_fused_args(f3d_ctx* x, int shape);
+// the column pieces of a launch of its own for tile shape `shape`, or of one
+// of batch_items uncut tiles
+FusedArgs ctx_fused_args(f3d_ctx* x, int shape, long long batch_items = 0);
 int ctx_check_step_status(f3d_ctx* x);
 inline double* ctx_outmass(f3d_ctx* x) { return x->small; }
 // gravity current (f3d_gravity.cu): addradialwind on the scaled winds of

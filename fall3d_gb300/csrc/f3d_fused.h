@@ -91,8 +91,12 @@ inline int halo_pitch(int nx) { return (nx + 2 + 3) & ~3; }
 
 // How a context's column is cut (nchunk, kfirst, klen) so that the tiles of
 // all classes fill the device: nwet = highest level any wet deposition
-// reaches (0: none), which the first piece must hold.
-void step_chunks(FusedArgs& a, int shape, int nwet);
+// reaches (0: none), which the first piece must hold.  batch_items: the uncut
+// tiles of all classes of all scenarios of the launch (0: its own); a batch
+// that fills the device gains nothing from pieces, which cost four iterations
+// each (64 members of 64..320 by 64..320 cells: 10.2 ms per step, cut as for
+// launches of their own 10.7 ms).
+void step_chunks(FusedArgs& a, int shape, int nwet, long long batch_items);
 
 // Tile shapes (F3D_OPT_TILE), region x by y / threads: 0, 1 and 2 = 64x16 /
 // 512 (a row per warp, two blocks per SM), 3 = 64x32 / 512 (two rows per

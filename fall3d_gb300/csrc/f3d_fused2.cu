@@ -895,12 +895,12 @@ int fused_tiles(int nx, int ny, int shape) {
 // 299 against 285 at 243x191x37 and 11, 976 against 889 at 400x300x50 and 16.
 int step_shape(Dims d, int ncls) { return (long long)fused_tiles(d.nx, d.ny, 0) * ncls <= device_sms() ? 0 : 3; }
 
-void step_chunks(FusedArgs& a, int shape, int nwet) {
+void step_chunks(FusedArgs& a, int shape, int nwet, long long batch_items) {
   const int nz = a.d.nz;
   a.nchunk = 1;
   a.kfirst = nz;
   a.klen = nz;
-  const long long blocks = (long long)fused_tiles(a.d.nx, a.d.ny, shape) * a.ncls;
+  const long long blocks = std::max(batch_items, (long long)fused_tiles(a.d.nx, a.d.ny, shape) * a.ncls);
   const long long slots = (long long)device_sms() * with_shape(shape, [](auto s) { return min_blocks<decltype(s)>(); });
   // waves of blocks times iterations of the longest piece (plus ~3 for the start)
   long long best = ((blocks + slots - 1) / slots) * (nz + 4);
