@@ -158,7 +158,7 @@ int table_rebuild(f3d_batch* b) {
 // the kernels of one batch step, in stream order
 int enqueue_step(f3d_batch* b, int commit_only_fused) {
   const int n = (int)b->active.size();
-  BK(cudaMemsetAsync(b->d_counter, 0, sizeof(int), b->stream));
+  BK(cudaMemsetAsync(b->d_counter, 0, 2 * sizeof(int), b->stream));
   if (!commit_only_fused) launch_setsrc_batch(b->d_aux, b->d_bstep, n, b->max_nc, b->max_nsou, b->stream);
   launch_step_fused_batch(b->shape, b->grid, b->d_item_off, n, b->d_counter, b->d_bstep, b->d_iiter0,
                           commit_only_fused ? 0 : 1, b->max_nz, b->d_maps, b->stream);
@@ -223,7 +223,7 @@ int f3d_batch_create(int max_scenarios, f3d_batch** out) {
   ok = ok && cudaMalloc(&b->d_item_off, sizeof(int) * (n + 1)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_bstep, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_iiter0, sizeof(int) * n) == cudaSuccess;
-  ok = ok && cudaMalloc(&b->d_counter, sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&b->d_counter, 2 * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_red, cmass2d_batch_scratch_bytes(n)) == cudaSuccess;
   ok = ok && cudaMemsetAsync(b->d_red, 0, cmass2d_batch_scratch_bytes(n), b->stream) == cudaSuccess;  // block counters
   ok = ok && cudaMallocHost(&b->h_aux, sizeof(BatchAux) * n) == cudaSuccess;

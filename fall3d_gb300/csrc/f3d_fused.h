@@ -118,8 +118,8 @@ void launch_step_vk(Dims d, int nc, const double* vz, const double* vset, float*
 int fused_tiles(int nx, int ny, int shape);
 
 // Batched form: the arguments of up to F3D_BATCH_MAX scenarios in constant
-// memory (c_in / c_out are the scenario's two buffers), then one persistent
-// launch over the work items of all of them.
+// memory (c_in / c_out are the scenario's two buffers), then a persistent
+// launch per sweep order over the work items of all that take it; counter: two.
 #define F3D_BATCH_MAX 128
 struct BatchMaps {  // a scenario's tensor maps (device array in batch order)
   F2Maps met;

@@ -704,7 +704,7 @@ __global__ void __maxnreg__(112) k_step_fused2_beside(const FusedArgs a, const _
 }
 
 // ------------------------------------------------------------ batched form
-// The step of every scenario of a batch in one persistent launch: the work
+// The step of every scenario of a batch in persistent launches: the work
 // items are (scenario, tile, piece, class), numbered scenario by scenario
 // (item_off[s] .. item_off[s+1]-1, class fastest); each block takes the next
 // item from a counter until none is left.  A scenario's arguments live in
@@ -714,48 +714,60 @@ __global__ void __maxnreg__(112) k_step_fused2_beside(const FusedArgs a, const _
 __constant__ FusedArgs c_batch[F3D_BATCH_MAX];
 static_assert(sizeof(FusedArgs) * F3D_BATCH_MAX <= 48 * 1024, "batch argument table exceeds constant memory");
 
-// a call of its own, so that the two sweep orders do not share registers
+// Two launches per batch step, one per sweep order, each over the scenarios
+// whose step has that order (usually all or none): with both orders in one
+// kernel the march spills, 324 bytes when both are inlined, 104 and 228 as calls
+// of their own, 20 to 48 in this form (four scenarios of
+// 400x300x50 cells and 16 classes 9.48e10 -> 1.00e11 cell-class-steps/s, 64
+// members of 64..320 by 64..320 cells 7.18e10 -> 7.36e10).
 template <class S, bool XFIRST>
-__device__ __noinline__ void step_tile_call(const FusedArgs& a, const F2Maps* maps, const CMaps* cmap,
-                                            const float* c_in, float* c_out, const int commit, const int cls,
-                                            const int tile, const int chunk) {
-  step_tile<S, XFIRST>(a, maps, cmap, c_in, c_out, commit, cls, tile, chunk);
-}
-
-template <class S>
 __global__ void __launch_bounds__(S::NT, min_blocks<S>())
     k_step_fused2_batch(const int* __restrict__ item_off, int nscen, int* counter, const int* __restrict__ bstep,
                         const int* __restrict__ iiter0, int commit, const BatchMaps* __restrict__ maps) {
   __shared__ int s_item;
+  __shared__ int s_off[F3D_BATCH_MAX + 1], s_scn[F3D_BATCH_MAX + 1];  // this order's items and scenarios
   __shared__ FusedArgs s_args;
-  const int total = item_off[nscen];
+  for (int q = threadIdx.x; q < nscen; q += S::NT) {
+    s_off[q] = item_off[q + 1] - item_off[q];
+    s_scn[q] = ((iiter0[q] + bstep[q] + 1) % 2 == 0) == XFIRST;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {  // compacted in place: entry n is written at or before it is read
+    int n = 0, off = 0;
+    for (int q = 0; q < nscen; ++q) {
+      const int items = s_off[q];
+      if (!s_scn[q]) continue;
+      s_off[n] = off;
+      s_scn[n++] = q;
+      off += items;
+    }
+    s_off[n] = off;
+    s_item = n;
+  }
+  __syncthreads();
+  const int nsel = s_item, total = s_off[nsel];
   for (;;) {
     __syncthreads();  // the previous item is done with shared memory
     if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
     __syncthreads();
     const int item = s_item;
     if (item >= total) break;
-    int lo = 0, hi = nscen;  // item_off[lo] <= item < item_off[hi]
+    int lo = 0, hi = nsel;  // s_off[lo] <= item < s_off[hi]
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (item_off[mid] <= item) lo = mid;
+      if (s_off[mid] <= item) lo = mid;
       else hi = mid;
     }
+    const int scn = s_scn[lo], local = item - s_off[lo];
     for (int w = threadIdx.x; w < (int)(sizeof(FusedArgs) / 4); w += S::NT)
-      reinterpret_cast<int*>(&s_args)[w] = reinterpret_cast<const int*>(&c_batch[lo])[w];
+      reinterpret_cast<int*>(&s_args)[w] = reinterpret_cast<const int*>(&c_batch[scn])[w];
     __syncthreads();
     const FusedArgs& a = s_args;
-    const int local = item - item_off[lo], rest = local / a.ncls;
-    const int bs = bstep[lo];
+    const int rest = local / a.ncls, bs = bstep[scn];
     const float* cin = (bs & 1) ? a.c_out : a.c_in;
     float* cout = (bs & 1) ? const_cast<float*>(a.c_in) : a.c_out;
-    const int iiter = iiter0[lo] + bs + 1;
-    const CMaps* cm = (bs & 1) ? &maps[lo].b : &maps[lo].a;
-    const int cls = local % a.ncls, tile = rest / a.nchunk, chunk = rest % a.nchunk;
-    if (iiter % 2 == 0)
-      step_tile_call<S, true>(a, &maps[lo].met, cm, cin, cout, commit, cls, tile, chunk);
-    else
-      step_tile_call<S, false>(a, &maps[lo].met, cm, cin, cout, commit, cls, tile, chunk);
+    step_tile<S, XFIRST>(a, &maps[scn].met, (bs & 1) ? &maps[scn].b : &maps[scn].a, cin, cout, commit, local % a.ncls,
+                         rest / a.nchunk, rest % a.nchunk);
   }
 }
 
@@ -1001,11 +1013,14 @@ int fused_batch_grid(int shape, int max_nz) {
   return with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
     const size_t sm = step_smem<S>(max_nz);
-    int per_sm = 0;
-    if (cudaFuncSetAttribute(k_step_fused2_batch<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_fused2_batch<S>, S::NT, sm) != cudaSuccess)
-      return -1;
+    auto fit = [&](auto kernel) {
+      int per_sm = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::NT, sm) != cudaSuccess)
+        return 0;
+      return per_sm;
+    };
+    const int per_sm = std::min(fit(k_step_fused2_batch<S, true>), fit(k_step_fused2_batch<S, false>));
     return per_sm < 1 ? -1 : per_sm * device_sms();
   });
 }
@@ -1014,11 +1029,12 @@ void launch_step_fused_batch(int shape, int grid, const int* item_off, int nscen
                              const int* iiter0, int commit, int max_nz, const BatchMaps* maps, cudaStream_t s) {
   with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
-    k_step_fused2_batch<S><<<grid, S::NT, step_smem<S>(max_nz), s>>>(item_off, nscen, counter, bstep, iiter0, commit,
-                                                                    maps);
+    const size_t sm = step_smem<S>(max_nz);
+    k_step_fused2_batch<S, true><<<grid, S::NT, sm, s>>>(item_off, nscen, counter, bstep, iiter0, commit, maps);
+    k_step_fused2_batch<S, false><<<grid, S::NT, sm, s>>>(item_off, nscen, counter + 1, bstep, iiter0, commit, maps);
     return 0;
   });
-  count_launch();
+  count_launch(2);
 }
 
 }  // namespace f3d
