@@ -154,18 +154,22 @@ __global__ void k_out_plane(const double* f, long long n, const double* Hm1, voi
 }
 
 // deposit thickness, cm (printres_nc.f90:191-214): 1e2*(sum over particle
-// classes of cload(ic)/rhop(ic))/Hm1; the reciprocals of rhop once per block.
+// classes of cload(ic)/rhop(ic))/Hm1; the reciprocals of rhop once per block,
+// for OB classes at a time.
 __global__ void k_out_thick(const double* cload, long long pl, int np, const double* rhop,
                             const double* Hm1, void* out, int f32) {
-  extern __shared__ double rr[];
-  for (int ic = threadIdx.x; ic < np; ic += OB) rr[ic] = 1.0 / rhop[ic];
-  __syncthreads();
+  __shared__ double rr[OB];
   const long long p = blockIdx.x * (long long)OB + threadIdx.x;
-  if (p >= pl) return;
   double s = 0.0;
-  for (int ic = 1; ic <= np; ++ic)
-    s = s + div_rn_recip(cload[(long long)ic * pl + p], rhop[ic - 1], rr[ic - 1]);
-  put(out, p, 1e2 * s / Hm1[p], f32);
+  for (int i0 = 0; i0 < np; i0 += OB) {
+    const int n = min(OB, np - i0);
+    __syncthreads();  // the previous group's are read
+    if (threadIdx.x < n) rr[threadIdx.x] = 1.0 / rhop[i0 + threadIdx.x];
+    __syncthreads();
+    for (int u = 0; u < n && p < pl; ++u)
+      s = s + div_rn_recip(cload[(i0 + u + 1LL) * pl + p], rhop[i0 + u], rr[u]);
+  }
+  if (p < pl) put(out, p, 1e2 * s / Hm1[p], f32);
 }
 
 // concentration at a flight level, g/m3 (printres_nc.f90:542-573 and
@@ -593,8 +597,7 @@ int f3d_output(f3d_ctx* x, int var, int index, int asl, void* dst, int dst_type)
     case F3D_OUT_THICK:
       launch_getc0(x->cdry, x->cwet, x->cload, d, nc, np, s);
       if (var == F3D_OUT_THICK)
-        k_out_thick<<<blocks(pl), OB, sizeof(double) * (np > 0 ? np : 1), s>>>(x->cload, pl, np, x->rhop, x->Hm1,
-                                                                              res.p, o32);
+        k_out_thick<<<blocks(pl), OB, 0, s>>>(x->cload, pl, np, x->rhop, x->Hm1, res.p, o32);
       else
         k_out_plane<<<blocks(pl), OB, 0, s>>>((var == F3D_OUT_LOAD ? x->cload : x->cwet) + index * pl, pl,
                                               x->Hm1, res.p, o32);
