@@ -32,6 +32,10 @@ struct OutClasses {
   __device__ int at(int i) const { return cls_more ? cls_more[i] : (int)cls[i]; }
 };
 
+// x != 0 with no binary64 comparison
+__device__ __forceinline__ bool nonzero(float x) { return x != 0.0f; }
+__device__ __forceinline__ bool nonzero(double x) { return (dbits(x) << 1) != 0; }
+
 // sum over the listed classes of c(i,j,k,ic) (0 + c1 + c2 + ...).  A zero
 // leaves the sum as it is and is skipped; eight loads are in flight.
 template <class T>
@@ -43,7 +47,7 @@ __device__ __forceinline__ double class_sum(const T* c, long long hb, long long 
     for (int u = 0; u < 8; ++u) v[u] = n0 + u < cl.n ? c[(long long)cl.at(n0 + u) * hb + q] : T(0);
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      if (v[u] != T(0)) s = s + widen(v[u]);
+      if (nonzero(v[u])) s = s + widen(v[u]);
   }
   return s;
 }
@@ -229,7 +233,11 @@ __global__ void k_out_con_asl(const T* c, Dims d, const OutClasses cl, const dou
   const int i = (int)(p % d.nx) + 1, j = (int)(p / d.nx) + 1;
   const long long hb = d.halo();
   const double h = Hm1[p];
-  auto val = [&](int k) { return 1e3 * (class_sum<T>(c, hb, d.C(i, j, k), cl) / h); };
+  // the levels of the last pair: the next one mostly shares one of them (400x300x50
+  // cells, the plain form, sums of 8 classes: 2.05 ms; 2.67 ms with each pair formed
+  // anew and zeros found by binary64 comparisons)
+  int ka = 0;
+  double w[2] = {0.0, 0.0};
   const double zo = fmax2(0.0, topg[p]);
   for (int k = 1; k <= d.nz; ++k) {
     const double zasl = zlayer[k - 1];
@@ -238,7 +246,17 @@ __global__ void k_out_con_asl(const T* c, Dims d, const OutClasses cl, const dou
       for (int kk = 1; kk <= d.nz - 1; ++kk) {
         if (zasl >= zo + zlayer[kk - 1] && zasl <= zo + zlayer[kk]) {
           const double s = (zo + zlayer[kk] - zasl) / (zlayer[kk] - zlayer[kk - 1]);
-          v = s * val(kk) + (1.0 - s) * val(kk + 1);
+          if (kk != ka) {
+            const bool next = ka > 0 && kk == ka + 1;
+            if (next) w[0] = w[1];
+            for (int u = next ? 1 : 0; u < 2; ++u) {
+              const double x = 1e3 * (class_sum<T>(c, hb, d.C(i, j, kk + u), cl) / h);
+              if (u == 0) w[0] = x;
+              else w[1] = x;
+            }
+            ka = kk;
+          }
+          v = s * w[0] + (1.0 - s) * w[1];
           break;
         }
       }
