@@ -28,8 +28,18 @@
 
 namespace f3d {
 
+static int sms() {
+  static int nsm = 0;
+  if (!nsm) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return std::max(1, nsm);
+}
+
 // ------------------------------------------------------------- kappa3
-// Sources/kappa3.f90:50-236.  A thread takes K3_LEV levels of a column: what
+// Sources/kappa3.f90:50-236.  A thread takes up to K3_LEV levels of a column: what
 // depends on the column alone (the power of RAMS, the divisors) is formed once
 // and divisions by a column's or a level's divisor use its reciprocal
 // (div_rn_recip: the same quotient), since binary64 operations bound it
@@ -46,13 +56,14 @@ __global__ void k_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv
                          const double* dz, const double* zlayer, const double* Hm1,
                          const double* vx, const double* vy, const double* vptemp,
                          const double* ustar, const double* zi, const double* rl,
-                         double* rkver, double* rkhor) {
+                         double* rkver, double* rkhor, int levels) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const double vkarm = 0.4, beta1 = 9.2, beta2 = 13.0, rlamb = 30.0, rkhmin = 1e2, rkvmin = 1.0;
   const double hinf = 5.0, hsup = 5e3, alfa = 0.28, Khf = 8000.0, gi = 9.81;
-  const int k0 = blockIdx.y * K3_LEV + 1, k1 = min(nz, k0 + K3_LEV - 1);
+  const bool vert = modkv != 0, horiz = modkh != 0;
+  const int k0 = blockIdx.y * levels + 1, k1 = min(nz, k0 + levels - 1);
   __shared__ K3Level lev[K3_LEV + 1];  // levels k0-1 .. (k0-1: only for k = nz, below)
-  if (threadIdx.x <= K3_LEV) {
+  if (vert && threadIdx.x <= levels) {
     const int k = k0 - 1 + threadIdx.x;
     if (k >= 1 && k <= nz) {
       K3Level z;
@@ -77,17 +88,17 @@ __global__ void k_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv
     dvdz2 = fmax2(dvdz2, 1e-10);
     rich = gi * div_rn_recip(vptemp[m + pl] - vptemp[m - pl], z.dzs, z.rdzs) / (vptemp[m] * dvdz2);
   };
-  const double us = ustar[p], rlp = rl[p];
-  const double h = fmin2(fmax2(zi[p], hinf), hsup), rh = 1.0 / h;
-  const double dXX = Hm1[p] * dX1;
-  const double ddx = i == 1 || i == nx ? dXX : 2.0 * dXX, rddx = 1.0 / ddx;
-  const double ddy = j == 1 || j == ny ? dX2 : 2.0 * dX2, rddy = 1.0 / ddy;
+  const double us = vert ? ustar[p] : 0.0, rlp = vert ? rl[p] : 0.0;
+  const double h = vert ? fmin2(fmax2(zi[p], hinf), hsup) : 1.0, rh = vert ? 1.0 / h : 1.0;
+  const double dXX = horiz ? Hm1[p] * dX1 : 1.0;
+  const double ddx = i == 1 || i == nx ? dXX : 2.0 * dXX, rddx = horiz ? 1.0 / ddx : 1.0;
+  const double ddy = j == 1 || j == ny ? dX2 : 2.0 * dX2, rddy = horiz ? 1.0 / ddy : 1.0;
   const double Kmh = modkh == 1 ? 0.075 * pow(dXX * dX2, 2.0 / 3.0) : 0.0;
   const long long e = i == nx ? p : p + 1, w = i == 1 ? p : p - 1;
   const long long n = j == ny ? p : p + nx, s = j == 1 ? p : p - nx;
   for (int k = k0; k <= k1; ++k) {
     const long long o = (k - 1) * pl, m = p + o;
-    const double zl = lev[k - k0 + 1].zl;
+    const double zl = vert ? lev[k - k0 + 1].zl : 0.0;
     // vertical
     if (modkv == 0) {
       rkver[m] = rkv0;
@@ -158,14 +169,36 @@ __global__ void k_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv
   }
 }
 
+// both diffusivities constant
+__global__ void k_kappa3_const(long long n, double rkv0, double rkh0, double* rkver, double* rkhor) {
+  for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < n; m += (long long)gridDim.x * blockDim.x) {
+    rkver[m] = rkv0;
+    rkhor[m] = rkh0;
+  }
+}
+
 void launch_kappa3(Dims d, int modkv, int modkh, int coord_sys, double rkv0, double rkh0,
                    double Csh, double dX1, double dX2, double dx, double dy, const double* dz,
                    const double* zlayer, const double* Hm1, const double* vx, const double* vy,
                    const double* vptemp, const double* ustar, const double* zi, const double* rl,
                    double* rkver, double* rkhor, cudaStream_t s) {
-  k_kappa3<<<dim3((unsigned)((d.plane() + K3_B - 1) / K3_B), (d.nz + K3_LEV - 1) / K3_LEV), K3_B, 0, s>>>(
+  const long long cb = (d.plane() + K3_B - 1) / K3_B;
+  if (modkv == 0 && modkh == 0) {
+    const long long n = d.cells();
+    k_kappa3_const<<<(unsigned)std::min<long long>((n + 255) / 256, 8LL * sms()), 256, 0, s>>>(n, rkv0, rkh0, rkver,
+                                                                                            rkhor);
+    count_launch();
+    return;
+  }
+  // as many levels per thread as leave three blocks on two SMs, in groups of
+  // about the same size: 33x29x14 cells 40 us with one level, 83 with ten;
+  // 80x80x25 75 with five, 85 with ten and 99 with one; 121x101x30 114 with ten,
+  // 135 with three; 400x300x50 1.25 ms with ten, 2.49 with one (the call's wall clock)
+  const long long most = std::max<long long>(1, std::min<long long>(K3_LEV, 2 * cb * d.nz / (3LL * sms())));
+  const int groups = (int)((d.nz + most - 1) / most), levels = (d.nz + groups - 1) / groups;
+  k_kappa3<<<dim3((unsigned)cb, groups), K3_B, 0, s>>>(
       d, modkv, modkh, coord_sys, rkv0, rkh0, Csh, dX1, dX2, dx, dy, dz, zlayer, Hm1, vx, vy, vptemp, ustar, zi, rl,
-      rkver, rkhor);
+      rkver, rkhor, levels);
   count_launch();
 }
 
@@ -789,16 +822,6 @@ __global__ void k_vset_finish(long long s3, int nc, int np, int aggregate, doubl
   }
 }
 
-static int chain_sms() {
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return std::max(1, nsm);
-}
-
 static ChainGeom chain_geom(Dims d, int np) {
   ChainGeom g;
   g.d = d;
@@ -810,7 +833,7 @@ static ChainGeom chain_geom(Dims d, int np) {
   // costs the W cells of its warm-up: segments of about 1024 cells, but no
   // fewer than 3 warps per SM hold, and at most 12 warps' worth, whose
   // different lengths (2 to 6 iterations per cell by class) even out.
-  const long long warp_row = 32LL * chain_sms();
+  const long long warp_row = 32LL * sms();
   const long long n = std::min(12 * warp_row, std::max(3 * warp_row, g.L / 1024));
   g.S = std::max<long long>(64, (g.L + n - 1) / n);
   g.nseg = (g.L + g.S - 1) / g.S;
@@ -869,7 +892,7 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
       (void)carveout;
       cudaMemsetAsync(claim, 0, sizeof(int) * 256, s);
       cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
-      k_chain_beside<<<(unsigned)(4 * chain_sms()), 128, 0, s>>>(g, modv, io, cd_state, entry, exitv, nonconv, claim,
+      k_chain_beside<<<(unsigned)(4 * sms()), 128, 0, s>>>(g, modv, io, cd_state, entry, exitv, nonconv, claim,
                                                                  next);
     } else {
       k_chain_segments<<<(unsigned)nb, bs, 0, s>>>(g, modv, io, cd_state, entry, exitv, nonconv);
