@@ -934,18 +934,38 @@ __global__ void k_d2f(float* dst, const double* src, long long n) {
        q += (long long)gridDim.x * blockDim.x)
     dst[q] = (float)src[q];
 }
-// the same between arrays of rows of different pitch
+// The same between arrays of rows of different pitch.  A block takes groups of
+// whole rows, its threads the values one after the other across the row ends, so
+// that every load and store of a warp but those at a row's end is one line.
+constexpr int CONV_VALUES = 2048;  // of a group, about
 template <class D, class S>
-__global__ void k_convert_rows(D* dst, int dpitch, const S* src, int spitch, int w, long long rows) {
-  const int lane = threadIdx.x & 31;
-  for (long long r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8LL)
-    for (int i = lane; i < w; i += 32) dst[r * dpitch + i] = (D)src[r * spitch + i];
+__global__ void __launch_bounds__(256) k_convert_rows(D* dst, int dpitch, const S* src, int spitch, int w,
+                                                      int group, long long rows) {
+  const int dr = 256 / w, di = 256 % w, row = threadIdx.x / w, col = threadIdx.x % w;
+  for (long long r0 = blockIdx.x * (long long)group; r0 < rows; r0 += gridDim.x * (long long)group) {
+    const int n = (int)min((long long)group, rows - r0);
+    D* const o = dst + r0 * dpitch;
+    const S* const a = src + r0 * spitch;
+    int r = row, i = col;
+#pragma unroll 8
+    while (r < n) {
+      o[r * dpitch + i] = (D)a[r * spitch + i];
+      r += dr;
+      i += di;
+      if (i >= w) {
+        i -= w;
+        ++r;
+      }
+    }
+  }
 }
 template <class D, class S>
 static void convert_rows(D* dst, int dpitch, const S* src, int spitch, int w, long long rows, cudaStream_t s) {
   if (rows <= 0) return;
-  k_convert_rows<D, S><<<(int)std::min<long long>((rows + 7) / 8, 152LL * 16), 256, 0, s>>>(dst, dpitch, src, spitch,
-                                                                                         w, rows);
+  const int group = std::max(1, CONV_VALUES / w);
+  const long long nb = (rows + group - 1) / group;
+  k_convert_rows<D, S><<<(unsigned)std::min<long long>(nb, 152LL * 64), 256, 0, s>>>(dst, dpitch, src, spitch, w,
+                                                                                    group, rows);
   count_launch();
 }
 void launch_d2f_rows(float* dst, int dpitch, const double* src, int spitch, int w, long long rows, cudaStream_t s) {
