@@ -198,5 +198,6 @@ void launch_d2f(float* dst, const double* src, long long n, cudaStream_t s);
 // rows of w values between arrays of different row pitch
 void launch_d2f_rows(float* dst, int dpitch, const double* src, int spitch, int w, long long rows, cudaStream_t s);
 void launch_f2d_rows(double* dst, int dpitch, const float* src, int spitch, int w, long long rows, cudaStream_t s);
+void launch_copy_rows(float* dst, int dpitch, const float* src, int spitch, int w, long long rows, cudaStream_t s);
 
 }  // namespace f3d

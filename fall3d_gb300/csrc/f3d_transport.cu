@@ -974,6 +974,9 @@ void launch_d2f_rows(float* dst, int dpitch, const double* src, int spitch, int 
 void launch_f2d_rows(double* dst, int dpitch, const float* src, int spitch, int w, long long rows, cudaStream_t s) {
   convert_rows(dst, dpitch, src, spitch, w, rows, s);
 }
+void launch_copy_rows(float* dst, int dpitch, const float* src, int spitch, int w, long long rows, cudaStream_t s) {
+  convert_rows(dst, dpitch, src, spitch, w, rows, s);
+}
 void launch_d2f(float* dst, const double* src, long long n, cudaStream_t s) {
   if (n <= 0) return;
   const int nb = (int)std::min<long long>((n + 255) / 256, 152LL * 16);

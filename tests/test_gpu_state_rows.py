@@ -44,3 +44,31 @@ def test_state_round_trips(prec, nx, ny, nz, nc, tmp_path):
         assert np.array_equal(f["cdry"], dry) and np.array_equal(f["cwet"], wet)
     for x in (g, h, e):
         x.close()
+
+
+@pytest.mark.parametrize("nx", [12, 13, 14, 31])
+def test_steps_after_a_restore(nx, tmp_path):
+    """A restore uses the step's second buffer: the steps that follow in the
+    same context give the bits of those that followed the save, whatever the
+    padding and whichever buffer the state was in."""
+    s = synth.make_scenario("small", seed=6, nx=nx, ny=11, nz=9, nc=3, run_h=0.5)
+    g = F.Context(s, F.PREC_FP32)
+    g.meteo(0)
+    g.source(0)
+    for before in (2, 3):
+        g.step(before)
+        t = g.state()
+        path = tmp_path / f"{before}.ckpt"
+        g.save(path)
+        g.step(5)
+        want, out = g.fields(), g.state()["outmass"]
+        g.restore(path)
+        g.meteo(0)
+        g.source(0)
+        g.set_time(t["time"], t["iiter"])
+        g.step(5)
+        got = g.fields()
+        for k in ("c", "cdry", "cwet"):
+            assert np.array_equal(got[k], want[k]), (before, k)
+        assert g.state()["outmass"] == out
+    g.close()
