@@ -879,7 +879,10 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
   cudaMemsetAsync(nbad, 0, sizeof(int), s);
   cudaMemsetAsync(status, 0, sizeof(int), s);
   if (np > 0 && g.L > 0) {
-    if (!have_classes) launch_class_consts(np, modv, diam, rhop, psi, sphe, scratch, s);
+    if (!have_classes) {
+      k_class_consts<<<(np + 31) / 32, 32, 0, s>>>(np, modv, diam, rhop, psi, sphe, cc);
+      count_launch();
+    }
     k_visc<<<(int)std::min<long long>((d.cells() + 255) / 256, 152LL * 16), 256, 0, s>>>(d.cells(), modv, tempe,
                                                                                          rho, visc, cf);
     const ChainIO io{cc, visc, cf, rho, vset, iters};
@@ -908,14 +911,6 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
         d.cells(), nc, np, aggregate, vset_factor, vset);
     count_launch();
   }
-}
-
-void launch_class_consts(int np, int modv, const double* diam, const double* rhop, const double* psi,
-                         const double* sphe, void* scratch, cudaStream_t s) {
-  if (np <= 0) return;
-  k_class_consts<<<(np + 31) / 32, 32, 0, s>>>(np, modv, diam, rhop, psi, sphe,
-                                               reinterpret_cast<ClassConst*>(scratch));
-  count_launch();
 }
 
 }  // namespace f3d

@@ -468,10 +468,12 @@ int meteo_enqueue(f3d_ctx* x, cudaStream_t s, const double* u, const double* v, 
   launch_kappa3(d, g.modkv, g.modkh, g.coord_sys, g.rkv0, g.rkh0, g.Csh, g.dX1, g.dX2, g.dx, g.dy,
                 x->dz, x->zlayer, x->Hm1, x->vx, x->vy, x->vptemp, x->ustar, x->zi, x->rl, x->rkver,
                 x->rkhor, s);
-  // meteo.f90:81 setvset (unscaled rho), continuing the cd chain
+  // meteo.f90:81 setvset (unscaled rho), continuing the cd chain; the class
+  // constants (0.2 ms) are made with the first update, their inputs never change
   launch_setvset(d, g.nc, g.np, g.modv, x->diam, x->rhop, x->psi, x->sphe, x->tempe, x->rho,
                  g.aggregate, g.vset_factor, x->vset, x->iters, cd_state, x->vset_scratch, status, s,
-                 beside_step, 1);
+                 beside_step, x->have_classes);
+  x->have_classes = 1;
   // meteo.f90:100 setvdrydep (tempe(:,:,1), unscaled rho(:,:,1))
   launch_setvdrydep(d, g.nc, x->diam, x->zlayer, x->ldu, x->rl, x->znt, x->ustar, x->tempe, x->rho,
                     x->vdep, s);
@@ -753,7 +755,6 @@ int f3d_ctx_create(const f3d_grid* g, f3d_ctx** out) {
   if (!rc) rc = upload(x, x->rhop, g->rhop, nc);
   if (!rc) rc = upload(x, x->psi, g->psi, nc);
   if (!rc) rc = upload(x, x->sphe, g->sphe, nc);
-  if (!rc) launch_class_consts(g->np, g->modv, x->diam, x->rhop, x->psi, x->sphe, x->vset_scratch, x->stream);
   const double cd0 = 1.0;  // setvset.f90:89
   if (!rc && cudaMemcpyAsync(small_cd(x), &cd0, sizeof cd0, cudaMemcpyHostToDevice, x->stream) != cudaSuccess)
     rc = f3d::ctx_error(F3D_ERR_CUDA, "upload failed");

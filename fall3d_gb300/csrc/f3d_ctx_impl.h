@@ -99,6 +99,7 @@ struct f3d_ctx {
   // scratch
   void* red_scratch = nullptr;
   void* vset_scratch = nullptr;
+  int have_classes = 0;  // it holds the class constants
   void* out_plane = nullptr;  // result of a 2-D output variable, made on first use
   double* small = nullptr;  // [0] outmass, [1..4] budget, [8] cd, [16] dtcn bits, [24] status, [40..41] non-finite counts
   // host scalars of the time loop

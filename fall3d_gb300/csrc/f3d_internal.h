@@ -181,15 +181,13 @@ size_t setvset_scratch_bytes(Dims d, int np);
 // beside_step != 0: the chain runs as one block of four 64-register warps per
 // SM, which fits next to a resident step-kernel block (a look-ahead update on
 // a second stream); the results do not depend on it.
+// have_classes != 0: the scratch holds the class constants of an earlier call
+// with the same classes.
 void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const double* rhop,
                     const double* psi, const double* sphe, const double* tempe,
                     const double* rho, int aggregate, double vset_factor, double* vset,
                     int* iters, double* cd_state, void* scratch, int* status, cudaStream_t s,
                     int beside_step = 0, int have_classes = 0);
-// The class constants of launch_setvset, kept at the start of its scratch: a
-// caller whose classes stay the same makes them once (have_classes).
-void launch_class_consts(int np, int modv, const double* diam, const double* rhop, const double* psi,
-                         const double* sphe, void* scratch, cudaStream_t s);
 // The drag iteration's table-driven log (op 0) and exp (op 1) on n values.
 void launch_dmath_eval(int op, long long n, const double* x, double* y, cudaStream_t s);
 
