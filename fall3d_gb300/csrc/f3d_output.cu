@@ -27,9 +27,9 @@ struct OutClasses {
   int n;
   const int* cls_more;
   const double *q_more, *r_more;
-  unsigned short cls[CMAX];
+  int cls[CMAX];
   double q[CMAX], r[CMAX];
-  __device__ int at(int i) const { return cls_more ? cls_more[i] : (int)cls[i]; }
+  __device__ int at(int i) const { return cls_more ? cls_more[i] : cls[i]; }
 };
 
 // x != 0 with no binary64 comparison
@@ -489,7 +489,7 @@ int class_list(f3d_ctx* x, const std::vector<int>& cls, const std::vector<double
   o = OutClasses{};
   o.n = (int)cls.size();
   if (cls.size() <= (size_t)CMAX) {
-    for (size_t i = 0; i < cls.size(); ++i) o.cls[i] = (unsigned short)cls[i];
+    for (size_t i = 0; i < cls.size(); ++i) o.cls[i] = cls[i];
     for (size_t i = 0; i < q.size(); ++i) {
       o.q[i] = q[i];
       o.r[i] = r[i];

@@ -1,5 +1,6 @@
 """Output variables of contexts with very many classes: more than the doubles of
-a block's default shared memory.  Bit for bit the oracle's restatement."""
+a block's default shared memory, and class numbers beyond 16 bits.  Bit for bit
+the oracle's restatement."""
 import numpy as np
 import pytest
 
@@ -24,4 +25,16 @@ def test_thickness(nc):
     f = dict(c=np.zeros((nc, 5, 5, 5)), cdry=dry, cwet=wet)
     for v in (F.OUT_LOAD, F.OUT_THICK):
         assert np.array_equal(g.output(v), O.output(s.grid, f, v))
+    g.close()
+
+
+def test_class_numbers_beyond_16_bits():
+    nc = 65600
+    s, g = _context(nc)
+    c = np.zeros((nc, 5, 5, 5))
+    c[:, 1:-1, 1:-1, 1:-1] = np.arange(1, nc + 1)[:, None, None, None]
+    g.upload_state(c)
+    hm = np.asarray(s.grid["Hm1"])
+    for index in (1, 65535, 65536, 65537, nc):  # class `index`
+        assert np.array_equal(g.output(F.OUT_CON, index), 1e3 * (np.full((3, 3, 3), float(index)) / hm)), index
     g.close()
