@@ -382,9 +382,11 @@ void sizloop_fused(f3d_ctx* x) {
   cudaStream_t s = x->stream;
   const int shape = x->tile_set ? x->opt_tile : step_shape(d, nc);
   const FusedArgs a = f3d::ctx_fused_args(x, shape);
+  // a look-ahead update in flight: the 64x32 step that leaves it room on the SMs
+  const bool beside = shape == 3 && x->pref_ready && cudaEventQuery(x->ev_pref) == cudaErrorNotReady;
   {
-    ProfScope ps(x, "step_fused");
-    launch_step_fused(a, x->maps2, x->cmap, shape, s, x->pref_ready && cudaEventQuery(x->ev_pref) == cudaErrorNotReady);
+    ProfScope ps(x, beside ? "step_beside" : "step_fused");
+    launch_step_fused(a, x->maps2, x->cmap, shape, s, beside);
   }
   std::swap(x->c32, x->c32b);
   std::swap(x->cmap, x->cmapb);
