@@ -316,11 +316,12 @@ def setvset(nx, ny, nz, nc, np_, modv, diam, rhop, psi, sphe, tempe, rho, aggreg
 
 
 def dmath_eval(op, x):
-    """Diagnostic: the drag iteration's table-driven binary64 log (op 0) or
-    exp (op 1) of every value of the float64 array x, or (op 2) the
+    """Diagnostic: the library's own binary64 functions of the float64 array
+    x: a table-driven log (op 0) or exp (op 1) of every value, (op 2) the
     quotients a/b of the pairs x = (a0, b0, a1, b1, ...) formed from the
-    reciprocal of b as the plain form's sweeps divide.  Returns a new
-    array (one value per pair for op 2)."""
+    reciprocal of b as the plain form's sweeps divide, or the Ganser drag
+    iteration's x**(0.6567-1) (op 4), 1/sqrt(x) (op 5) and 1/x (op 6).
+    Returns a new array (one value per pair for op 2)."""
     x = np.ascontiguousarray(x, dtype=np.float64).ravel()
     if op == 2:
         if x.size % 2:

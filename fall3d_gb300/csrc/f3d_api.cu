@@ -619,7 +619,8 @@ int f3d_setvset(const int* nx, const int* ny, const int* nz, const int* nc, cons
 }
 
 int f3d_dmath_eval(int op, long long n, const double* x, double* y) {
-  if (op < 0 || op > 2 || n < 0) return set_error(F3D_ERR_ARG, "op must be 0 (log), 1 (exp) or 2 (quotient), n >= 0");
+  if (op < 0 || op > 6 || op == 3 || n < 0)
+    return set_error(F3D_ERR_ARG, "op must be 0 (log), 1 (exp), 2 (quotient), 4 (power), 5 (1/sqrt) or 6 (1/x), n >= 0");
   if (n > 0 && (!x || !y)) return set_error(F3D_ERR_ARG, "NULL argument");
   Marshal m;
   const double* dx = m.arr(x, (size_t)n * (op == 2 ? 2 : 1), false);

@@ -792,13 +792,23 @@ __global__ void k_chain_status(ChainGeom g, const int* nonconv, int* status) {
   if (s < g.nseg && nonconv[s]) atomicOr(status, 1);
 }
 
+// f3d_dmath_eval; ops 4 to 6: the Ganser iteration's power, 1/sqrt and 1/x
 __global__ void k_dmath_eval(int op, long long n, const double* x, double* y) {
   __shared__ DMathTab tab;
+  __shared__ PowTab pow_tab;
   dmath_tab_init(tab);
+  pow_tab_init(pow_tab);
   __syncthreads();
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x)
-    y[q] = op == 0 ? dm_log(tab, x[q]) : op == 1 ? dm_exp(tab, x[q]) : div_rn_recip(x[2 * q], x[2 * q + 1], 1.0 / x[2 * q + 1]);
+       q += (long long)gridDim.x * blockDim.x) {
+    const double v = x[op == 2 ? 2 * q : q];
+    y[q] = op == 0   ? dm_log(tab, v)
+           : op == 1 ? dm_exp(tab, v)
+           : op == 2 ? div_rn_recip(v, x[2 * q + 1], 1.0 / x[2 * q + 1])
+           : op == 4 ? (pow_in_range(v) ? pow_a(pow_tab, v) : pow(v, kPowA))
+           : op == 5 ? ganser_rsqrt(v)
+                     : (mid_range(v) ? rcp_fast(v) : 1.0 / v);
+  }
 }
 
 void launch_dmath_eval(int op, long long n, const double* x, double* y, cudaStream_t s) {

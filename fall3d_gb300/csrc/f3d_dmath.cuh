@@ -1,8 +1,9 @@
-// f3d_dmath.cuh -- table-driven binary64 logarithm and exponential for the
+// f3d_dmath.cuh -- binary64 functions in few operations: those of the
 // settling-velocity iteration (vsettl), whose cost on GB300 is the number of
-// binary64 operations per drag iteration.
+// binary64 operations per drag iteration (further down), and a table-driven
+// logarithm and exponential, which only the diagnostic f3d_dmath_eval reaches.
 //
-// Methods (published):
+// Methods of the latter (published):
 //  * exp: P. T. P. Tang, "Table-driven implementation of the exponential
 //    function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989.
 //    a = (64 m + j) ln2/64 + r with |r| <= ln2/128, exp(a) = 2^m 2^(j/64) e^r,
@@ -14,8 +15,8 @@
 //    with the tabulated reciprocal), |r| <= 2^-8, and
 //    log x = k ln2 - log(1/c) + log1p(r), log1p by its Taylor series to r^7.
 //
-// Accuracy: the truncated series are below 2^-64; the results are within
-// a few units in the last place (the tests bound both against a
+// Accuracy of these: the truncated series are below 2^-64; the results are
+// within a few units in the last place (the tests bound both against a
 // high-precision evaluation).  Arguments outside the reduced ranges (log of
 // a non-normal or huge value, exp beyond +-700) fall back to CUDA's log/exp.
 #pragma once
@@ -93,8 +94,8 @@ constexpr double kPowA = 0.6567 - 1.0;
 constexpr int kPowEmin = -64, kPowN = 128;  // exponents k of the table
 struct PowTab {
   double invc[256];   // RN(1 / (1 + (j + 1/2)/256))
-  double powc[256];   // RN(invc[j]^-a)
-  double pow2[kPowN]; // RN(2^(a (kPowEmin + j)))
+  double powc[256];   // invc[j]^-a
+  double pow2[kPowN]; // 2^(a (kPowEmin + j))
 };
 __device__ __forceinline__ void pow_tab_init(PowTab& t) {
   for (int j = threadIdx.x; j < 256; j += blockDim.x) {
@@ -123,9 +124,15 @@ __device__ __forceinline__ double pow_a(const PowTab& t, double x) {
   return fma(s * r, q, s);
 }
 
-// 1/sqrt(x) and 1/x from the hardware's approximations (relative error at
-// most 2^-20) by one step of third order each, whose own error is below
-// 2^-60; x in [2^-1000, 2^1000].
+// 1/sqrt(x) and 1/x, x in [2^-1000, 2^1000], from the hardware's approximations
+// y by one step of Chebyshev's method (J. F. Traub, Iterative Methods for the
+// Solution of Equations, 1964), y - f/f' (1 + f f''/(2 f'^2)), of third order:
+//   f(y) = 1/y - x,   e = 1 - x y:    y (1 + e + e^2);
+//   f(y) = 1/y^2 - x, h = 1 - x y^2:  y (1 + h/2 + 3/8 h^2).
+// With a relative error d of y, the first leaves d^3 and the second, the next term
+// of the series of (1 - h)^(-1/2) being 5/16 h^3 at h = 2 d, 5/2 d^3.  d measured over
+// 1.3e9 arguments in [1, 4): 2^-19.94 and 2^-20.04; so 2^-59.8 and 2^-58.8, beside
+// the roundings of the last operations (1.02 and 1.6 times 2^-53 in all).
 __device__ __forceinline__ double rsqrt_fast(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -188,7 +188,7 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
                     const double* rho, int aggregate, double vset_factor, double* vset,
                     int* iters, double* cd_state, void* scratch, int* status, cudaStream_t s,
                     int beside_step = 0, int have_classes = 0);
-// The drag iteration's table-driven log (op 0) and exp (op 1) on n values.
+// f3d_dmath_eval's functions on n values (or pairs, op 2).
 void launch_dmath_eval(int op, long long n, const double* x, double* y, cudaStream_t s);
 
 // Conversions for the FP32 form.

@@ -250,12 +250,13 @@ int f3d_setvset(const int* nx, const int* ny, const int* nz, const int* nc,
                 const double* tempe, const double* rho, const int* aggregate,
                 const double* vset_factor, double* vset, double* cd);
 
-/* Diagnostic: the binary64 log (op 0) or exp (op 1) that setvset's Ganser
- * drag iteration uses in place of pow (a table-driven restatement, within a
- * few ulp), on n host or device values; op 2: the quotients a/b of n pairs
- * x = (a0, b0, a1, b1, ...) formed from the reciprocal of b the way the
- * plain form's sweeps divide (equal to the IEEE quotient).  No reference
- * counterpart. */
+/* Diagnostic: the library's own binary64 functions on n host or device
+ * values.  Op 0 and 1: a table-driven log and exp (within a few ulp; not used
+ * elsewhere); op 2: the quotients a/b of n pairs x = (a0, b0, a1, b1, ...)
+ * formed from the reciprocal of b the way the plain form's sweeps divide
+ * (equal to the IEEE quotient); op 4, 5 and 6: x**(0.6567-1), 1/sqrt(x) and
+ * 1/x as setvset's Ganser drag iteration forms them (within 8.2, 1.6 and 1.02
+ * times 2^-53).  No reference counterpart. */
 int f3d_dmath_eval(int op, long long n, const double* x, double* y);
 
 /* Sources/setvdrydep.f90:1 setvdrydep (module state made explicit). */
