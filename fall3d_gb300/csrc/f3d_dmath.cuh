@@ -89,7 +89,10 @@ __device__ __forceinline__ double dm_exp(const DMathTab& t, double a) {
 // the top eight fraction bits of z, x^a = 2^(ka) c^a (1 + r)^a, r = z/c - 1,
 // |r| <= 2^-9: two table values and the binomial series to r^5 (the next term
 // is below 2^-57), 8 operations in place of the 23 of a logarithm and an
-// exponential.
+// exponential.  Within 8.2 * 2^-53 of the value: the tables' 2 and 1 ulp, their
+// product and the last rounding.  (The power of two's exponent a*k is rounded,
+// by up to 2^-49 at the ends of the range, which the table corrects: without
+// that the error was 12.9 * 2^-53.)
 constexpr double kPowA = 0.6567 - 1.0;
 constexpr int kPowEmin = -64, kPowN = 128;  // exponents k of the table
 struct PowTab {
@@ -103,7 +106,11 @@ __device__ __forceinline__ void pow_tab_init(PowTab& t) {
     t.invc[j] = ic;
     t.powc[j] = pow(ic, -kPowA);
   }
-  for (int j = threadIdx.x; j < kPowN; j += blockDim.x) t.pow2[j] = exp2(kPowA * (kPowEmin + j));
+  for (int j = threadIdx.x; j < kPowN; j += blockDim.x) {
+    const double k = kPowEmin + j, p = kPowA * k, l = fma(kPowA, k, -p);  // a*k = p + l
+    const double e = exp2(p);
+    t.pow2[j] = fma(e, l * 0.6931471805599453, e);  // 2^l = 1 + l ln 2, l below 2^-49
+  }
 }
 // the biased exponent lies in the table's range
 __device__ __forceinline__ bool pow_in_range(double x) {

@@ -1,5 +1,5 @@
-"""Functions of the settling chain's Ganser iteration
-(f3d_dmath_eval, ops 5 and 6), as the iteration calls them, against extended
+"""The three functions of the settling chain's Ganser iteration
+(f3d_dmath_eval, ops 4 to 6), as the iteration calls them, against extended
 precision (numpy longdouble: 64-bit significand on x86, IEEE quad on Arm).
 
 Bounds, from the operations (u = 2^-53):
@@ -7,9 +7,13 @@ Bounds, from the operations (u = 2^-53):
    2^-20), and the last multiply-add rounds once: 1.02 u.
  * 1/sqrt(x): 2.5 times that cube; the product x*y rounded before the
    residual (its error enters halved, u/2 * 1) and the last rounding: 1.6 u.
+ * x^(0.6567-1): the two table values (CUDA's pow and exp2, 2 and 1 ulp, an ulp
+   being at most 2 u), their product (u), the last rounding (u) and the series
+   (its next term: 0.1 u) with its own roundings, below 2^-8 u:
+   8.2 u.
 Arguments: the iteration's range, binade edges, the edges of the table's
 intervals, and both sides of the ranges beyond which CUDA's own functions are
-called (1 ulp for 1/x and sqrt by IEEE, 1 ulp for rsqrt)."""
+called (1 ulp for 1/x and sqrt by IEEE, 1 ulp for rsqrt, 2 for pow)."""
 import numpy as np
 import pytest
 
@@ -17,6 +21,7 @@ import fall3d_gb300 as F
 
 pytestmark = pytest.mark.gpu
 U = 2.0 ** -53
+A = np.longdouble(0.6567 - 1.0)  # the binary64 value the iteration uses
 
 
 def _around(v):
@@ -53,10 +58,16 @@ def test_reciprocal_square_root():
     _check(y[~inside], exact[~inside], 2.0)
 
 
+def test_power():
+    x = _args(-64, 64)
+    y = F.dmath_eval(4, x)
+    _check(y, x.astype(np.longdouble) ** A, 8.2)
+
+
 def test_special_values():
     x = np.array([0.0, np.inf, np.nan, -1.0, 5e-324, 1e308])
     with np.errstate(all="ignore"):
-        for op, f in ((6, lambda v: 1.0 / v), (5, lambda v: v ** -0.5)):
+        for op, f in ((6, lambda v: 1.0 / v), (5, lambda v: v ** -0.5), (4, lambda v: v ** float(A))):
             y, t = F.dmath_eval(op, x), f(x)
             assert np.array_equal(np.isnan(y), np.isnan(t)) and np.array_equal(np.isinf(y), np.isinf(t)), op
             ok = np.isfinite(t)
