@@ -271,6 +271,7 @@ int f3d_batch_add(f3d_batch* b, f3d_ctx* x, const f3d_met_series* met, const f3d
   if (!b || !x || !met || !src || !slot) return ctx_error(F3D_ERR_ARG, "NULL argument");
   if (x->prec != F3D_PREC_FP32 || !x->fused_ok)
     return ctx_error(F3D_ERR_ARG, "batched contexts must be precision-form (FP32) contexts of the fused step");
+  if (x->g.nz > fused2_max_nz(true)) return ctx_error(F3D_ERR_ARG, "too many levels for a batch");
   if (x->gc_on) return ctx_error(F3D_ERR_ARG, "the gravity current is not supported in a batch");
   if (x->agr_on) return ctx_error(F3D_ERR_ARG, "aggregation is not supported in a batch");
   ctx_prefetch_drop(x);  // the batch makes each update when it is due

@@ -690,7 +690,7 @@ int f3d_ctx_create(const f3d_grid* g, f3d_ctx** out) {
   for (int k = 1; k < g->nz; ++k)
     if (!(g->zlayer[k] >= g->zlayer[k - 1])) x->fused_ok = 0;
   if (x->d.halo() >= (1LL << 31) || x->d.cells() >= (1LL << 31)) x->fused_ok = 0;
-  if (g->nz > f3d::fused2_max_nz()) x->fused_ok = 0;  // the step kernel's per-level table
+  if (g->nz > f3d::fused2_max_nz(false)) x->fused_ok = 0;  // the step kernel's per-level table
   // the highest priority: a look-ahead meteo update on the context's second
   // stream (lowest priority) runs in what the steps leave free
   int prio_least = 0, prio_greatest = 0;

@@ -85,8 +85,9 @@ struct CMaps {
 // 0 on success
 int make_step_maps(const FusedArgs& a, F2Maps* out);
 int make_c_maps(Dims d, int ncls, const float* c, CMaps* out);
-// the largest nz whose per-level table the step kernel's shared memory holds
-int fused2_max_nz();
+// the largest nz whose per-level table fits into the step kernel's shared memory,
+// for a context's own step or in a batch (whose kernel keeps tables of its own)
+int fused2_max_nz(bool batch);
 inline int halo_pitch(int nx) { return (nx + 2 + 3) & ~3; }
 
 // How a context's column is cut (nchunk, kfirst, klen) so that the tiles of

@@ -951,9 +951,22 @@ void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, i
   count_launch();
 }
 
-int fused2_max_nz() {
-  const size_t cap = (size_t)227 * 1024, base = step_smem<Tall>(0);
-  return cap > base ? (int)((cap - base) / sizeof(ZTab)) - 1 : 0;
+int fused2_max_nz(bool batch) {
+  static const auto limit = [](std::initializer_list<const void*> kernels) {
+    size_t fixed = 0;  // the kernels' own shared memory beside the dynamic one
+    for (const void* k : kernels) {
+      cudaFuncAttributes at{};
+      if (cudaFuncGetAttributes(&at, k) != cudaSuccess) return 0;
+      fixed = std::max(fixed, at.sharedSizeBytes);
+    }
+    const size_t cap = (size_t)227 * 1024, base = step_smem<Tall>(0) + fixed;
+    return cap > base ? (int)((cap - base) / sizeof(ZTab)) : 0;
+  };
+  static const int alone = limit({(const void*)k_step_fused2<Tall, true>, (const void*)k_step_fused2<Tall, false>,
+                                  (const void*)k_step_fused2_beside<true>, (const void*)k_step_fused2_beside<false>});
+  static const int in_batch = limit({(const void*)k_step_fused2_batch<Tall, true>,
+                                     (const void*)k_step_fused2_batch<Tall, false>});
+  return batch ? in_batch : alone;
 }
 
 // cuTensorMapEncodeTiled, reached through the runtime's driver entry point
