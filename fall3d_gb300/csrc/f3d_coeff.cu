@@ -832,20 +832,25 @@ __global__ void k_vset_finish(long long s3, int nc, int np, int aggregate, doubl
   }
 }
 
-static ChainGeom chain_geom(Dims d, int np) {
+static ChainGeom chain_geom(Dims d, int np, int modv) {
   ChainGeom g;
   g.d = d;
   g.L = d.cells() * np;
   g.W = 64;
-  // The segments are the threads of one launch.  Three warps per SM already
-  // keep the binary64 pipe busy (an iteration's 26 operations take 416 clocks
-  // of it per warp, about half of the iteration's latency), and every segment
-  // costs the W cells of its warm-up: segments of about 1024 cells, but no
-  // fewer than 3 warps per SM hold, and at most 12 warps' worth, whose
-  // different lengths (2 to 6 iterations per cell by class) even out.
+  // The segments are the threads of one launch.  Every one costs the W cells of
+  // its warm-up and the longest ends the launch (2 to 6 iterations per cell by
+  // class): segments of about 256 cells, but no fewer than 8 warps per SM hold, and
+  // at most 12 warps' worth.  Whole columns of an iterating model, so that the
+  // lanes of a warp go through the levels together; the closed form reads in order
+  // with segments of any length.  Update, ms, with segments of 1024 cells and 3 warps
+  // at least, with 256 and 8, and with whole columns:
+  //   300x220x30, 8 classes: Ganser 7.5, 6.2, 5.3; Wilson 29.1, 20.4, 16.0; Dellino 10.0, 7.5, 8.1
+  //   243x191x37, 11:        Ganser 9.5, 7.3, 5.5; Wilson 43.0, 27.1, 16.9; Dellino  9.9, 8.5, 8.7
+  //   400x300x50, 16:        Ganser 24.2, 24.2, 21.3; Wilson 88.1, 88.1, 69.6 (12 warps in all cases)
   const long long warp_row = 32LL * sms();
-  const long long n = std::min(12 * warp_row, std::max(3 * warp_row, g.L / 1024));
+  const long long n = std::min(12 * warp_row, std::max(8 * warp_row, g.L / 256));
   g.S = std::max<long long>(64, (g.L + n - 1) / n);
+  if (modv != 4) g.S = (g.S + d.nz - 1) / d.nz * d.nz;
   g.nseg = (g.L + g.S - 1) / g.S;
   return g;
 }
@@ -857,7 +862,7 @@ static constexpr int kBadCap = 8192;
 static constexpr size_t region(size_t bytes) { return (bytes + 255) & ~size_t(255); }
 
 size_t setvset_scratch_bytes(Dims d, int np) {
-  const ChainGeom g = chain_geom(d, np);
+  const ChainGeom g = chain_geom(d, np, 4);  // the model with the most segments
   return region(sizeof(ClassConst) * (size_t)(np + 1)) + 2 * region(sizeof(double) * (size_t)g.nseg) +
          region(sizeof(int) * (size_t)g.nseg) + region(sizeof(int) * 8) + region(sizeof(int) * kBadCap) +
          region(sizeof(double) * (size_t)d.cells()) + region(2 * sizeof(double) * (size_t)d.cells()) +
@@ -869,7 +874,7 @@ void launch_setvset(Dims d, int nc, int np, int modv, const double* diam, const 
                     const double* rho, int aggregate, double vset_factor, double* vset,
                     int* iters, double* cd_state, void* scratch, int* status, cudaStream_t s,
                     int beside_step, int have_classes) {
-  const ChainGeom g = chain_geom(d, np);
+  const ChainGeom g = chain_geom(d, np, modv);
   unsigned char* p = reinterpret_cast<unsigned char*>(scratch);
   auto take = [&](size_t bytes) {
     unsigned char* r = p;
