@@ -22,8 +22,6 @@ template <class T>
 F3D_HD T fmin2(T a, T b) { return (b < a || isnan(a)) ? b : a; }
 template <class T>
 F3D_HD T sign1(T b) { return isnan(b) ? T(1) : (signbit(b) ? T(-1) : T(1)); }
-template <class T>
-F3D_HD T fabs_t(T x) { return x < T(0) ? -x : (x == T(0) ? T(0) : x); }
 
 // A binary64 value's bit pattern and back, by moves that the compiler does
 // not look through: it turns integer operations on the pattern that it
@@ -218,16 +216,4 @@ F3D_HD DD dd_add_d(DD a, double b) {
   double hi = s + lo;
   lo = lo - (hi - s);
   return DD{hi, lo};
-}
-F3D_HD DD dd_add(DD a, DD b) {
-  double s = a.hi + b.hi;
-  double bb = s - a.hi;
-  double err = (a.hi - (s - bb)) + (b.hi - bb);
-  double lo = a.lo + b.lo + err;
-  double hi = s + lo;
-  lo = lo - (hi - s);
-  return DD{hi, lo};
-}
-__device__ __forceinline__ DD dd_shfl_down(DD v, int off) {
-  return DD{__shfl_down_sync(0xffffffffu, v.hi, off), __shfl_down_sync(0xffffffffu, v.lo, off)};
 }
