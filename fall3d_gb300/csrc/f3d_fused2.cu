@@ -716,10 +716,14 @@ static_assert(sizeof(FusedArgs) * F3D_BATCH_MAX <= 48 * 1024, "batch argument ta
 
 // Two launches per batch step, one per sweep order, each over the scenarios
 // whose step has that order (usually all or none): with both orders in one
-// kernel the march spills, 324 bytes when both are inlined, 104 and 228 as calls
-// of their own, 20 to 48 in this form (four scenarios of
-// 400x300x50 cells and 16 classes 9.48e10 -> 1.00e11 cell-class-steps/s, 64
-// members of 64..320 by 64..320 cells 7.18e10 -> 7.36e10).
+// kernel the 64x32 march spills, 324 bytes when both are inlined, 104 and 228 as
+// calls of their own, 20 to 48 in this form (four scenarios of 400x300x50 cells and
+// 16 classes 9.48e10 -> 1.00e11 cell-class-steps/s, 64 members of 64..320 by
+// 64..320 cells 7.18e10 -> 7.36e10; the 64x16 march, at 64 registers, spills 232 and
+// 244).  Where both orders have scenarios the launches follow one another, each
+// with a tail of its own: 12 members of 64..200 by 64..200 cells take 0.79 ms a step
+// when they agree and 0.88 ms when half of them are a step behind, 12 of
+// 200x180x40 cells and 12 classes 2.63 and 2.71 (0.99 and 1.00, 3.32 and 3.32 before the flux form).
 template <class S, bool XFIRST>
 __global__ void __launch_bounds__(S::NT, min_blocks<S>())
     k_step_fused2_batch(const int* __restrict__ item_off, int nscen, int* counter, const int* __restrict__ bstep,

@@ -3,7 +3,7 @@ per-kernel DRAM table is measured on:
 
 * the 400x300x50 grid with 16 classes (precipitation band, wet deposition on)
   in both forms: one meteo update (the coefficient chain, finddt, the
-  binary32 copies and halo-layout fields), two steps of every step path
+  binary32 copies and the step kernel's fields), two steps of every step path
   (per-routine binary64 sweeps, per-routine binary32 sweeps, the fused step
   of every tile shape), the budgets, every output variable and a flight
   level cut;
@@ -34,7 +34,7 @@ def _context_kernels(s, prec, steps=2):
     g.source(0)
     g.meteo(0)
     if prec == F.PREC_FP32:
-        for fused, tile in ((0, 0), (1, 0), (1, 1), (1, 2), (1, 3)):
+        for fused, tile in ((0, 0), (1, 0), (1, 3)):
             g.set_option(F.OPT_FUSED, fused)
             g.set_option(F.OPT_TILE, tile)
             g.step(steps)

@@ -555,11 +555,12 @@ int f3d_ctx_restore(f3d_ctx* ctx, const char* path);
                             with a decreasing zlayer or >= 2^31 cells per
                             class always use the per-routine kernels.     */
 #define F3D_OPT_TILE  2  /* fused kernel tile region x by y / threads:
-                            0, 1, 2 = 64x16/512, 3 = 64x32/512 (default;
-                            where it was not set, a context's own step
-                            takes 64x16 on grids whose 64x16 tiles are no
-                            more than the SMs), with two columns per lane;
-                            results do not depend on it                    */
+                            0, 1, 2 = 64x16/512 (0: a batch's default until
+                            one is set or tuned), 3 = 64x32/512 (a context's
+                            default; where it was not set, a context's own
+                            step takes 64x16 on grids whose 64x16 tiles are
+                            no more than the SMs), with two columns per
+                            lane; results do not depend on it              */
 #define F3D_OPT_GRAPH 3  /* batches: 1 = replay one CUDA graph per batch step
                             (default), 0 = launch the kernels one by one   */
 #define F3D_OPT_PREFETCH 4 /* f3d_run: 1 = compute the next DBS snapshot's
