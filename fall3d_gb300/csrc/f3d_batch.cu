@@ -68,7 +68,7 @@ struct f3d_batch {
   void* d_red = nullptr;
   // pinned staging of the tables
   BatchAux* h_aux = nullptr;
-  FusedArgs* h_args = nullptr;
+  FusedArgs *h_args = nullptr, *d_args = nullptr;
   BatchMaps* h_maps = nullptr;  // the scenarios' tensor maps, batch order
   BatchMaps* d_maps = nullptr;
   int *h_item_off = nullptr, *h_bstep = nullptr, *h_iiter0 = nullptr;
@@ -143,7 +143,7 @@ int table_rebuild(f3d_batch* b) {
   if ((b->max_nsou + 127) / 128 != nsou_blocks) b->graph_dirty = true;  // setsrc's grid changed
   b->h_item_off[n] = off;
   if (n > 0) {
-    if (upload_batch_args(b->h_args, n, b->stream)) return ctx_error(F3D_ERR_CUDA, "constant table upload failed");
+    BK(cudaMemcpyAsync(b->d_args, b->h_args, sizeof(FusedArgs) * n, cudaMemcpyHostToDevice, b->stream));
     BK(cudaMemcpyAsync(b->d_aux, b->h_aux, sizeof(BatchAux) * n, cudaMemcpyHostToDevice, b->stream));
     BK(cudaMemcpyAsync(b->d_maps, b->h_maps, sizeof(BatchMaps) * n, cudaMemcpyHostToDevice, b->stream));
     BK(cudaMemcpyAsync(b->d_bstep, b->h_bstep, sizeof(int) * n, cudaMemcpyHostToDevice, b->stream));
@@ -160,7 +160,7 @@ int enqueue_step(f3d_batch* b, int commit_only_fused) {
   const int n = (int)b->active.size();
   BK(cudaMemsetAsync(b->d_counter, 0, 2 * sizeof(int), b->stream));
   if (!commit_only_fused) launch_setsrc_batch(b->d_aux, b->d_bstep, n, b->max_nc, b->max_nsou, b->stream);
-  launch_step_fused_batch(b->shape, b->grid, b->d_item_off, n, b->d_counter, b->d_bstep, b->d_iiter0,
+  launch_step_fused_batch(b->shape, b->grid, b->d_args, b->d_item_off, n, b->d_counter, b->d_bstep, b->d_iiter0,
                           commit_only_fused ? 0 : 1, b->max_nz, b->d_maps, b->stream);
   if (!commit_only_fused) {
     launch_cmass2d_batch(b->d_aux, b->d_bstep, n, b->cap, b->d_red, b->stream);
@@ -228,6 +228,7 @@ int f3d_batch_create(int max_scenarios, f3d_batch** out) {
   ok = ok && cudaMemsetAsync(b->d_red, 0, cmass2d_batch_scratch_bytes(n), b->stream) == cudaSuccess;  // block counters
   ok = ok && cudaMallocHost(&b->h_aux, sizeof(BatchAux) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_args, sizeof(FusedArgs) * n) == cudaSuccess;
+  ok = ok && cudaMalloc(&b->d_args, sizeof(FusedArgs) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_maps, sizeof(BatchMaps) * n) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_maps, sizeof(BatchMaps) * n) == cudaSuccess;
   ok = ok && cudaMallocHost(&b->h_item_off, sizeof(int) * (n + 1)) == cudaSuccess;
@@ -254,6 +255,7 @@ int f3d_batch_destroy(f3d_batch* b) {
   cudaFree(b->d_red);
   cudaFreeHost(b->h_aux);
   cudaFreeHost(b->h_args);
+  cudaFree(b->d_args);
   cudaFreeHost(b->h_maps);
   cudaFree(b->d_maps);
   cudaFreeHost(b->h_item_off);

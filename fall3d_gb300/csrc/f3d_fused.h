@@ -118,19 +118,19 @@ void launch_step_vk(Dims d, int nc, const double* vz, const double* vset, float*
 // tiles of one class of an nx x ny grid for a tile shape
 int fused_tiles(int nx, int ny, int shape);
 
-// Batched form: the arguments of up to F3D_BATCH_MAX scenarios in constant
-// memory (c_in / c_out are the scenario's two buffers), then a persistent
-// launch per sweep order over the work items of all that take it; counter: two.
+// Batched form: a persistent launch per sweep order over the work items of all
+// scenarios (at most F3D_BATCH_MAX) that take it.  args: device array of the
+// scenarios' arguments, whose c_in / c_out are the scenario's two buffers; counter: two.
 #define F3D_BATCH_MAX 128
 struct BatchMaps {  // a scenario's tensor maps (device array in batch order)
   F2Maps met;
   CMaps a, b;
 };
-int upload_batch_args(const FusedArgs* h, int n, cudaStream_t s);
 // sets the kernel's shared-memory limit and returns its persistent grid (-1 on error)
 int fused_batch_grid(int shape, int max_nz);
-void launch_step_fused_batch(int shape, int grid, const int* item_off, int nscen, int* counter, const int* bstep,
-                             const int* iiter0, int commit, int max_nz, const BatchMaps* maps, cudaStream_t s);
+void launch_step_fused_batch(int shape, int grid, const FusedArgs* args, const int* item_off, int nscen, int* counter,
+                             const int* bstep, const int* iiter0, int commit, int max_nz, const BatchMaps* maps,
+                             cudaStream_t s);
 void launch_wet_lambda(long long n, double dt, const double* prate, double* lam, cudaStream_t s);
 
 }  // namespace f3d

@@ -707,12 +707,11 @@ __global__ void __maxnreg__(112) k_step_fused2_beside(const FusedArgs a, const _
 // The step of every scenario of a batch in persistent launches: the work
 // items are (scenario, tile, piece, class), numbered scenario by scenario
 // (item_off[s] .. item_off[s+1]-1, class fastest); each block takes the next
-// item from a counter until none is left.  A scenario's arguments live in
-// constant memory; its buffers alternate with the number of batch steps it
+// item from a counter until none is left.  A scenario's arguments are copied
+// to shared memory with each item; its buffers alternate with the number of batch steps it
 // has taken (bstep[s] even: c_in -> c_out, odd: c_out -> c_in), and the x/y
 // order follows iiter = iiter0[s] + bstep[s] + 1 (sizloop.f90:42-48).
-__constant__ FusedArgs c_batch[F3D_BATCH_MAX];
-static_assert(sizeof(FusedArgs) * F3D_BATCH_MAX <= 48 * 1024, "batch argument table exceeds constant memory");
+static_assert(sizeof(FusedArgs) % 4 == 0, "copied by words");
 
 // Two launches per batch step, one per sweep order, each over the scenarios
 // whose step has that order (usually all or none): with both orders in one
@@ -726,8 +725,9 @@ static_assert(sizeof(FusedArgs) * F3D_BATCH_MAX <= 48 * 1024, "batch argument ta
 // 200x180x40 cells and 12 classes 2.63 and 2.71 (0.99 and 1.00, 3.32 and 3.32 before the flux form).
 template <class S, bool XFIRST>
 __global__ void __launch_bounds__(S::NT, min_blocks<S>())
-    k_step_fused2_batch(const int* __restrict__ item_off, int nscen, int* counter, const int* __restrict__ bstep,
-                        const int* __restrict__ iiter0, int commit, const BatchMaps* __restrict__ maps) {
+    k_step_fused2_batch(const FusedArgs* __restrict__ args, const int* __restrict__ item_off, int nscen, int* counter,
+                        const int* __restrict__ bstep, const int* __restrict__ iiter0, int commit,
+                        const BatchMaps* __restrict__ maps) {
   __shared__ int s_item;
   __shared__ int s_off[F3D_BATCH_MAX + 1], s_scn[F3D_BATCH_MAX + 1];  // this order's items and scenarios
   __shared__ FusedArgs s_args;
@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(S::NT, min_blocks<S>())
     }
     const int scn = s_scn[lo], local = item - s_off[lo];
     for (int w = threadIdx.x; w < (int)(sizeof(FusedArgs) / 4); w += S::NT)
-      reinterpret_cast<int*>(&s_args)[w] = reinterpret_cast<const int*>(&c_batch[scn])[w];
+      reinterpret_cast<int*>(&s_args)[w] = __ldg(reinterpret_cast<const int*>(args + scn) + w);
     __syncthreads();
     const FusedArgs& a = s_args;
     const int rest = local / a.ncls, bs = bstep[scn];
@@ -1018,14 +1018,6 @@ int make_c_maps(Dims d, int ncls, const float* c, CMaps* out) {
   return step_map(d, c, (long long)(d.nz + 2) * ncls, &out->m[0], &out->m[1]);
 }
 
-int upload_batch_args(const FusedArgs* h, int n, cudaStream_t s) {
-  if (n > F3D_BATCH_MAX) return 1;
-  return cudaMemcpyToSymbolAsync(c_batch, h, sizeof(FusedArgs) * (size_t)n, 0, cudaMemcpyHostToDevice, s) ==
-                 cudaSuccess
-             ? 0
-             : 1;
-}
-
 int fused_batch_grid(int shape, int max_nz) {
   return with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
@@ -1042,13 +1034,15 @@ int fused_batch_grid(int shape, int max_nz) {
   });
 }
 
-void launch_step_fused_batch(int shape, int grid, const int* item_off, int nscen, int* counter, const int* bstep,
-                             const int* iiter0, int commit, int max_nz, const BatchMaps* maps, cudaStream_t s) {
+void launch_step_fused_batch(int shape, int grid, const FusedArgs* args, const int* item_off, int nscen, int* counter,
+                             const int* bstep, const int* iiter0, int commit, int max_nz, const BatchMaps* maps,
+                             cudaStream_t s) {
   with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
     const size_t sm = step_smem<S>(max_nz);
-    k_step_fused2_batch<S, true><<<grid, S::NT, sm, s>>>(item_off, nscen, counter, bstep, iiter0, commit, maps);
-    k_step_fused2_batch<S, false><<<grid, S::NT, sm, s>>>(item_off, nscen, counter + 1, bstep, iiter0, commit, maps);
+    k_step_fused2_batch<S, true><<<grid, S::NT, sm, s>>>(args, item_off, nscen, counter, bstep, iiter0, commit, maps);
+    k_step_fused2_batch<S, false><<<grid, S::NT, sm, s>>>(args, item_off, nscen, counter + 1, bstep, iiter0, commit,
+                                                         maps);
     return 0;
   });
   count_launch(2);
