@@ -126,7 +126,7 @@ struct BatchMaps {  // a scenario's tensor maps (device array in batch order)
   F2Maps met;
   CMaps a, b;
 };
-// sets the kernel's shared-memory limit and returns its persistent grid (-1 on error)
+// sets the kernels' shared-memory limit (that of the longest column) and returns their persistent grid (-1 on error)
 int fused_batch_grid(int shape, int max_nz);
 void launch_step_fused_batch(int shape, int grid, const FusedArgs* args, const int* item_off, int nscen, int* counter,
                              const int* bstep, const int* iiter0, int commit, int max_nz, const BatchMaps* maps,

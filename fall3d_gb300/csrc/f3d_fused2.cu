@@ -943,7 +943,10 @@ void launch_step_fused(const FusedArgs& a, const F2Maps& maps, const CMaps& c, i
     m.met = maps;
     m.c = c;
     auto go = [&](auto kernel) {
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      // the limit of the longest column, not of this one: another thread may be
+      // launching the kernel for a longer one
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)step_smem<S>(std::max(a.d.nz, fused2_max_nz(false))));
       kernel<<<fused_tiles(a.d.nx, a.d.ny, shape) * a.ncls * a.nchunk, S::NT, sm, s>>>(a, m);
     };
     if (beside && S::HYR == HY)
@@ -1024,7 +1027,8 @@ int fused_batch_grid(int shape, int max_nz) {
     const size_t sm = step_smem<S>(max_nz);
     auto fit = [&](auto kernel) {
       int per_sm = 0;
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess ||
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)step_smem<S>(std::max(max_nz, fused2_max_nz(true)))) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::NT, sm) != cudaSuccess)
         return 0;
       return per_sm;

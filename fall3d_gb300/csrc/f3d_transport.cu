@@ -419,8 +419,10 @@ static int class_splits(long long lines, int ncls) {
   return (int)std::min<long long>(ncls, std::max<long long>(1, (304 + lines - 1) / lines));
 }
 
+// Always the most a block can have: a limit by the launch's own size would be
+// lowered by another thread's launch of the same kernel on a shorter line.
 static void set_smem(const void* fn, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
 template <class T>
