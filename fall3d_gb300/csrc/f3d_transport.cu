@@ -172,16 +172,19 @@ __device__ __forceinline__ ColPiece col_piece(int iz_loc, int nz_loc) {
   const int len = (nz_loc + blockDim.y - 1) / blockDim.y, kb = iz_loc + threadIdx.y * len;
   return ColPiece{kb, min(kb + len, iz_loc + nz_loc) - 1};
 }
-// Pieces while the columns' warps are fewer than 8 per SM, of at least four
-// levels each: a piece forms two levels' terms of its own before its first.
-// With and without: 32x28x14 cells and 4 classes advctzc 15 and 22 us, diffz 14
-// and 18; 80x80x25 and 6 classes 48 and 45, 28 and 33; 201x149x41 and one class
-// 64 and 71, 41 and 66; with twice as many warps advctzc 54 and 70 us at the
-// latter two.
-static dim3 col_block(long long cols, int ncls, int nz_loc) {
+// Pieces while the columns' warps are fewer than warps_per_sm, of at least four
+// levels each: a piece forms two levels' terms of its own before its first, which
+// costs advctzc more than diffz.  us, cut and uncut:
+//   32x28x14 cells, 4 classes (112 warps)  advctzc 15, 22; diffz 14, 18
+//   201x149x41, one class (936)            advctzc 64, 70; diffz 64, 98
+//   70x70x25, 7 classes (1078)             advctzc 47, 45; diffz 27, 32
+//   80x80x25, 6 classes (1200)             advctzc 47, 45; diffz 27, 32
+//   160x121x40, 2 classes (1210)           advctzc 70, 67; diffz 57, 77
+// With twice as many warps advctzc loses more: 54 and 70 us at 80x80x25 and 201x149x41.
+static dim3 col_block(long long cols, int ncls, int nz_loc, int warps_per_sm) {
   const long long warps = (cols + 31) / 32 * ncls;
   int p = 1;
-  while (p < 8 && warps * p < 152 * 8 && nz_loc >= 4 * (2 * p)) p *= 2;
+  while (p < 8 && warps * p < 152LL * warps_per_sm && nz_loc >= 4 * (2 * p)) p *= 2;
   return p == 1 ? dim3(128) : dim3(32, p);
 }
 
@@ -258,7 +261,7 @@ void launch_advctzc(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, con
                     const T* vset, long long vstride, const T* dz, T dt, int ncls,
                     cudaStream_t s) {
   const long long cols = (long long)d.nx * d.ny;
-  const dim3 bs = col_block(cols, ncls, nz_loc);
+  const dim3 bs = col_block(cols, ncls, nz_loc, 7);
   const size_t sm = sizeof(ZTab<T>) * (d.nz + 1);
   k_advctzc<T><<<dim3((unsigned)((cols + bs.x - 1) / bs.x), ncls), bs, sm, s>>>(
       c, cstride, d, nz_loc, iz_loc, vz, vset, vstride, dz, dt);
@@ -555,7 +558,7 @@ template <class T>
 void launch_diffz(T* c, long long cstride, Dims d, int nz_loc, int iz_loc, const T* dz, T dt,
                   const T* rkver, const T* rho, const T* rksz, const T* lrz, int ncls, cudaStream_t s) {
   const long long cols = (long long)d.nx * d.ny;
-  const dim3 bs = col_block(cols, ncls, nz_loc);
+  const dim3 bs = col_block(cols, ncls, nz_loc, 8);
   const size_t sm = 2 * sizeof(T) * (d.nz + 1);
   k_diffz<T><<<dim3((unsigned)((cols + bs.x - 1) / bs.x), ncls), bs, sm, s>>>(c, cstride, d, nz_loc, iz_loc, dz, dt,
                                                                               rkver, rho, rksz, lrz);
