@@ -583,7 +583,8 @@ int f3d_get_option(const f3d_ctx* ctx, int key, int* value);
 int f3d_ctx_stream(f3d_ctx* ctx, void** stream);
 
 /* Per-kernel timing with CUDA events recorded on the context's stream
- * around every launch of f3d_step while enabled.  f3d_profile_read returns,
+ * around every launch of f3d_step while enabled (a step_fused launch beside a
+ * look-ahead meteo update is listed as step_beside).  f3d_profile_read returns,
  * for up to cap kernel kinds, the name, launch count and total milliseconds
  * since the last reset (it synchronises the stream). */
 int f3d_profile_enable(f3d_ctx* ctx, int enable);
