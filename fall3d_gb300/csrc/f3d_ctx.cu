@@ -514,6 +514,7 @@ int meteo_enqueue(f3d_ctx* x, cudaStream_t s, const double* u, const double* v, 
 // aggregation flags (Fall3d.f90:94-96).
 int meteo_finish(f3d_ctx* x, unsigned long long dtcn_bits, int status, int nwet) {
   x->nwet = nwet;
+  x->met_by_run = 0;
   if (status) return f3d::ctx_error(F3D_ERR_NOCONV, "No convergence in vsettl routine");
   double dtcn;
   memcpy(&dtcn, &dtcn_bits, sizeof dtcn);
@@ -886,10 +887,11 @@ int f3d_step(f3d_ctx* x) {
   if (!x) return f3d::ctx_error(F3D_ERR_ARG, "NULL context");
   if (!x->have_met) return f3d::ctx_error(F3D_ERR_STATE, "f3d_step before f3d_meteo");
   if (x->agr_on && x->agr_due) {  // Fall3d.f90:101-110: agrpar after this step's updates
-    const int rc = x->agr_replay > 0 ? f3d::agg_restore_vset(x, x->agr_replay) : f3d::agg_agrpar(x);
+    int rc = x->agr_replay > 0 ? f3d::agg_restore_vset(x, x->agr_replay) : f3d::agg_agrpar(x);
+    if (!rc && x->agr_replay > 0 && x->agr_again) rc = f3d::agg_agrpar(x);
     if (rc) return rc;
     x->agr_due = 0;
-    x->agr_replay = 0;
+    x->agr_replay = x->agr_again = 0;
   }
   f3d::ctx_advance(x);
   const Dims d = x->d;
@@ -1071,6 +1073,7 @@ struct CkptHeader {
 };
 const char kCkptMagic[8] = {'F', '3', 'D', 'C', 'K', 'P', 'T', '1'};
 const long long kCkptAggr = 0x5247474146334446LL;  // the optional aggregation section
+const long long kCkptAgain = 1LL << 32;  // with its agrpar count: a source update is due, and another agrpar with it
 
 // c between the device and a checkpoint's host block, whose rows hold nx+2
 // values: one copy of the whole where the device's are as long.  The precision
@@ -1130,7 +1133,11 @@ int f3d_ctx_save(f3d_ctx* x, const char* path) {
       CK(cudaMemcpyAsync(agf.data() + q * s3, src[q], s3 * sizeof(double), cudaMemcpyDeviceToHost, s));
   }
   CK(cudaMemcpyAsync(&h.outmass, small_outmass(x), sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&h.cd_prev, small_cd_prev(x), sizeof(double), cudaMemcpyDeviceToHost, s));
+  // the updates that a restored run replays at this time: the current
+  // intervals' own, or where the next one is due already, that one, which the
+  // uninterrupted run enters from the chain's present value
+  const bool met_due = x->met_by_run && x->meteo_time <= x->time, src_due = x->met_by_run && x->source_time <= x->time;
+  CK(cudaMemcpyAsync(&h.cd_prev, met_due ? small_cd(x) : small_cd_prev(x), sizeof(double), cudaMemcpyDeviceToHost, s));
   if (int rc = ckpt_state(x, c.data(), true)) return rc;
   CK(cudaMemcpyAsync(cdry.data(), x->cdry, pl2 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(cwet.data(), x->cwet, pl2 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1141,7 +1148,9 @@ int f3d_ctx_save(f3d_ctx* x, const char* path) {
             fwrite(cdry.data(), sizeof(double), pl2, f) == pl2 && fwrite(cwet.data(), sizeof(double), pl2, f) == pl2;
   if (ok && x->agr_on) {  // aggregation: the agrsrc step counter, agrpar calls since the meteo update,
                           // Maggr and Alagr, Abagr, Asagr, Adagr
-    const long long agg[3] = {kCkptAggr, x->agr_ipass, x->agr_npar};
+    // (a due meteo update starts that count again, a due source update adds a call)
+    const long long calls = met_due ? 0 : x->agr_npar + (src_due && x->agr_npar > 0 ? kCkptAgain : 0);
+    const long long agg[3] = {kCkptAggr, x->agr_ipass, calls};
     ok = fwrite(agg, sizeof agg, 1, f) == 1 && fwrite(agf.data(), sizeof(double), agf.size(), f) == agf.size();
   }
   ok = (fclose(f) == 0) && ok;
@@ -1193,7 +1202,8 @@ int f3d_ctx_restore(f3d_ctx* x, const char* path) {
     for (int q = 0; q < 5; ++q)
       CK(cudaMemcpyAsync(dst[q], agf.data() + q * s3, s3 * sizeof(double), cudaMemcpyHostToDevice, s));
     x->agr_ipass = (int)agg[1];
-    x->agr_replay = (int)agg[2];  // vset scalings owed after the replayed updates (0: none made yet)
+    x->agr_replay = (int)(agg[2] & (kCkptAgain - 1));  // vset scalings owed after the replayed updates (0: none made yet)
+    x->agr_again = (agg[2] & kCkptAgain) != 0;
   }
   CK(cudaStreamSynchronize(s));
   x->time = h.time;
@@ -1202,6 +1212,7 @@ int f3d_ctx_restore(f3d_ctx* x, const char* path) {
   // the next f3d_run replays the updates of the current meteo and source
   // intervals (Fall3d.f90:83-101 select them from the time)
   x->run_started = 1;
+  x->met_by_run = 0;
   x->meteo_time = h.time;
   x->source_time = h.time;
   x->meteotime = 1;
@@ -1395,6 +1406,7 @@ int ctx_run_prepare(f3d_ctx* x, const f3d_met_series* met, const f3d_src_series*
                        met->prate ? met->prate + o2 : nullptr, met->ldu);
       }
       if (rc) return rc;
+      x->met_by_run = 1;
       x->meteo_time = (double)endsec - met->time_lag;
       // the next snapshot's update while this interval steps: the update due
       // at meteo_time reads snapshot itime + 1 (the steps are shorter than

@@ -53,7 +53,9 @@ struct f3d_ctx {
   // aggregation in transport (f3d_set_aggregation)
   int agr_on = 0, agr_iaggr = 0, agr_ndtagr = 1, agr_ipass = 0, agr_due = 0;
   int agr_npar = 0;    // agrpar calls since the last meteo update
+  int met_by_run = 0;  // the last meteo update was made by the run loop, which knows when the next is due
   int agr_replay = 0;  // agrpar calls owed by a restored run
+  int agr_again = 0;   // and one more, of the source update that was due
   double agr_Df = 3.0, agr_sumNi = 0.0;
   std::vector<double> agr_fc;  // fc(1:np)
   double *agr_fc_dev = nullptr, *agr_cls = nullptr;
