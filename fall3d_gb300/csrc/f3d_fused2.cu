@@ -693,9 +693,9 @@ __global__ void __launch_bounds__(S::NT, min_blocks<S>())
 // 112 registers a block leaves the settling chain's four 64-register warps
 // room on its SM (the 128 of the other build take the whole register file).
 // A forecast of 400x300x50 cells and 16 classes over eight meteo updates runs at
-// 9.70e10 cell-class-steps/s with it, 8.95e10 with the other build throughout
-// (whose blocks and the chain's exclude each other) and 8.5e10 with every
-// update made when due.
+// 9.84e10 cell-class-steps/s with it, 6.7e10 to 7.6e10 with the other build
+// throughout (whose blocks and the chain's exclude each other) and 8.5e10 to
+// 9.0e10 with every update made when due.
 template <bool XFIRST>
 __global__ void __maxnreg__(112) k_step_fused2_beside(const FusedArgs a, const __grid_constant__ StepMaps maps) {
   const int item = blockIdx.x / a.ncls;
