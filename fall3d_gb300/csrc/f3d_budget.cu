@@ -406,7 +406,7 @@ void launch_getc0(double* cdry, double* cwet, double* cload, Dims d, int nc, int
 // formed from that divisor's reciprocal (div_rn_recip: the same quotient).
 // Bound by the binary64 pipe: a class's two terms are formed exactly only
 // where an estimate of four operations reaches the largest value the block
-// has seen (400x300x50 cells, 16 classes: 3.69 ms -> 1.47 ms).
+// has seen (400x300x50 cells, 16 classes: 3.69 ms -> 1.24 ms).
 __global__ void k_finddt(Dims d, int nc, double dX1, double dX2, const double* dz,
                          const double* vx, const double* vy, const double* vz,
                          const double* vset, const double* rkh1, const double* rkhor,

@@ -43,7 +43,7 @@ static int sms() {
 // depends on the column alone (the power of RAMS, the divisors) is formed once
 // and divisions by a column's or a level's divisor use its reciprocal
 // (div_rn_recip: the same quotient), since binary64 operations bound it
-// (400x300x50 cells: 2.61 ms one cell per thread, 1.51 ms so).
+// (400x300x50 cells: 2.72 ms one cell per thread, 0.98 ms so).
 constexpr int K3_LEV = 10, K3_B = 128;
 
 struct K3Level {  // of level k (kappa3.f90:64-96)
